@@ -149,9 +149,15 @@ struct Binning {
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // ---- launchers (k_analysis.cu) ----
-// First and last column of every row of B (bmin = INT32_MAX, bmax = -1 for
-// empty rows; any column order).
-void launch_row_minmax(const CsrDev &B, int32_t *bmin, int32_t *bmax, int *unsorted, cudaStream_t s, int num_sms);
+// Checks an operand (row pointers, column range; badPtr and badIdx may be
+// null) and gives the first and last column of every row (INT32_MAX and -1
+// for empty rows) and in *unsorted (zeroed by the caller) how many entries do
+// not ascend.
+void launch_check_operand(const CsrDev &M, int32_t *bmin, int32_t *bmax, int *badPtr, int *badIdx, int *unsorted,
+                          cudaStream_t s, int num_sms);
+// Replaces them by the smallest and largest column when *unsorted is not 0.
+void launch_row_minmax(const CsrDev &B, int32_t *bmin, int32_t *bmax, const int *unsorted, cudaStream_t s,
+                       int num_sms);
 void launch_row_products(const CsrDev &A, const int32_t *Bp, const int32_t *bmin, const int32_t *bmax,
                          const RowInfo &ri, uint8_t *symBin, int *err, const Tuning &t, cudaStream_t s,
                          int num_sms);
@@ -197,8 +203,6 @@ void launch_symbolic_bin(const SymArgs &a, int bin, int32_t begin, int32_t n, cu
 // bin sizes, so a stream capture holds it).
 void launch_symbolic_bin_dd(const SymArgs &a, int bin, cudaStream_t s, int *launches);
 void launch_f32_to_f64(const float *src, double *dst, int64_t n, cudaStream_t s);
-void launch_validate_ptr(const int32_t *ptr, int64_t m, int64_t nnz, int *flag, cudaStream_t s);
-void launch_validate_idx(const int32_t *idx, int64_t nnz, int64_t ncols, int *flag, cudaStream_t s);
 
 // One work item of the dense bin: row, or the piece of it over the column
 // slabs [s0, s1) whose entries start `off` entries into C's row (s0 < 0:

@@ -335,7 +335,7 @@ int validate_host(dbd_ctx *c, const dbd_csr_view *v, const char *name) {
     return DBD_OK;
 }
 
-int finish_operand(dbd_ctx *c, Operand &op, const CsrDev &d);
+int finish_operand(dbd_ctx *c, Operand &op, const CsrDev &d, const char *name);
 
 int load_operand(dbd_ctx *c, Operand &op, const dbd_csr_view *v, const char *name) {
     int rc = validate_host(c, v, name);
@@ -350,19 +350,6 @@ int load_operand(dbd_ctx *c, Operand &op, const dbd_csr_view *v, const char *nam
     d.nnz = v->nnz;
     const size_t ne = (size_t)v->nnz;
     if (v->on_device) {
-        // Validate on the device: row_ptr first, then indices (only once the
-        // row_ptr is known to span [0, nnz]).
-        CK(c, c->flags.ensure(4 * sizeof(int)));
-        CK(c, cudaMemsetAsync(c->flags.p, 0, 4 * sizeof(int), c->stream));
-        launch_validate_ptr(v->row_ptr, v->n_rows, v->nnz, c->flags.as<int>(), c->stream);
-        int hf[4];
-        CK(c, cudaMemcpyAsync(hf, c->flags.p, sizeof(hf), cudaMemcpyDeviceToHost, c->stream));
-        CK(c, cudaStreamSynchronize(c->stream));
-        if (hf[0]) return set_err(c, DBD_ERR_INVALID, std::string(name) + ": malformed row_ptr");
-        launch_validate_idx(v->col_idx, v->nnz, v->n_cols, c->flags.as<int>() + 1, c->stream);
-        CK(c, cudaMemcpyAsync(hf, c->flags.p, sizeof(hf), cudaMemcpyDeviceToHost, c->stream));
-        CK(c, cudaStreamSynchronize(c->stream));
-        if (hf[1]) return set_err(c, DBD_ERR_INVALID, std::string(name) + ": column index out of range");
         d.ptr = v->row_ptr;
         d.idx = v->col_idx;
         if (v->val_fp32) {
@@ -390,24 +377,30 @@ int load_operand(dbd_ctx *c, Operand &op, const dbd_csr_view *v, const char *nam
         d.idx = op.idx.as<int32_t>();
         d.val = op.val.as<double>();
     }
-    return finish_operand(c, op, d);
+    return finish_operand(c, op, d, name);
 }
 
-// Sortedness and row column ranges of an operand now on the device.
-int finish_operand(dbd_ctx *c, Operand &op, const CsrDev &d) {
+// Checks of an operand now on the device (row_ptr spanning [0, nnz] and
+// every column in range before anything reads through them), the first and
+// last column of every row (the column windows of the products' rows) and
+// whether every row ascends strictly (cursors, plain accumulation, runs).
+int finish_operand(dbd_ctx *c, Operand &op, const CsrDev &d, const char *name) {
     op.dev = d;
-    // Row column ranges (the column windows of the products' rows) and
-    // whether every row ascends strictly (cursors, plain accumulation, runs).
     CK(c, c->flags.ensure(4 * sizeof(int)));
-    CK(c, cudaMemsetAsync(c->flags.as<int>() + 2, 0, sizeof(int), c->stream));
+    int *flags = c->flags.as<int>();
+    CK(c, cudaMemsetAsync(flags, 0, 3 * sizeof(int), c->stream));
     CK(c, op.bmin.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(d.m, 1)));
     CK(c, op.bmax.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(d.m, 1)));
-    launch_row_minmax(d, op.bmin.as<int32_t>(), op.bmax.as<int32_t>(), c->flags.as<int>() + 2, c->stream,
-                      c->num_sms);
-    int unsorted = 0;
-    CK(c, cudaMemcpyAsync(&unsorted, c->flags.as<int>() + 2, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    launch_check_operand(d, op.bmin.as<int32_t>(), op.bmax.as<int32_t>(), flags, flags + 1, flags + 2, c->stream,
+                         c->num_sms);
+    int hf[3] = {0, 0, 0};
+    CK(c, cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    op.sorted = unsorted ? 0 : 1;
+    if (hf[0]) return set_err(c, DBD_ERR_INVALID, std::string(name) + ": malformed row_ptr");
+    if (hf[1]) return set_err(c, DBD_ERR_INVALID, std::string(name) + ": column index out of range");
+    op.sorted = hf[2] ? 0 : 1;
+    if (!op.sorted)
+        launch_row_minmax(d, op.bmin.as<int32_t>(), op.bmax.as<int32_t>(), flags + 2, c->stream, c->num_sms);
     op.loaded = true;
     c->divided = false;
     return DBD_OK;
@@ -1772,7 +1765,7 @@ int dbd_spgemm_batched(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const d
     da.ptr = c->A.ptr.as<int32_t>();
     da.idx = c->A.idx.as<int32_t>();
     da.val = c->A.val.as<double>();
-    rc = finish_operand(c, c->A, da);
+    rc = finish_operand(c, c->A, da, "A");
     if (rc) return rc;
     c->b_is_a = square;
     if (!square) {
@@ -1783,7 +1776,7 @@ int dbd_spgemm_batched(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const d
         db.ptr = c->B.ptr.as<int32_t>();
         db.idx = c->B.idx.as<int32_t>();
         db.val = c->B.val.as<double>();
-        rc = finish_operand(c, c->B, db);
+        rc = finish_operand(c, c->B, db, "B");
         if (rc) return rc;
     }
     c->batchCount = count;
@@ -1971,6 +1964,7 @@ int dbd_batch_enqueue(dbd_ctx *c, void *stream) {
     const CsrDev &A = c->A.dev, &B = opB(c);
     const Operand &opb = c->bpSquare ? c->A : c->B;
     int launches = 0;
+    launch_check_operand(B, opb.bmin.as<int32_t>(), opb.bmax.as<int32_t>(), nullptr, nullptr, flags + 2, s, c->num_sms);
     launch_row_minmax(B, opb.bmin.as<int32_t>(), opb.bmax.as<int32_t>(), flags + 2, s, c->num_sms);
     launch_row_products(A, B.ptr, opb.bmin.as<int32_t>(), opb.bmax.as<int32_t>(), row_info(c), c->symBin.as<uint8_t>(),
                         c->err.as<int>(), c->tune, s, c->num_sms);

