@@ -141,32 +141,35 @@ enum CounterSlot : int {
 struct Binning {
     uint8_t *bin = nullptr;     // m bin ids
     int32_t *list = nullptr;    // m row ids grouped by bin
-    int32_t *hist = nullptr;    // ntiles * kMaxBins counts
+    int32_t *hist = nullptr;    // kMaxBins rows of ntiles counts
     int32_t *tileOff = nullptr; // (ntiles + 1) * kMaxBins absolute offsets into list
     int32_t *binStart = nullptr;// kMaxBins + 1
 };
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+inline int64_t tile_count(int64_t m) { return ceil_div(m, kTileRows); }
 
 // ---- launchers (k_analysis.cu) ----
 // Checks an operand (row pointers, column range; badPtr and badIdx may be
 // null) and gives the first and last column of every row (INT32_MAX and -1
 // for empty rows) and in *unsorted (zeroed by the caller) how many entries do
 // not ascend.
-void launch_check_operand(const CsrDev &M, int32_t *bmin, int32_t *bmax, int *badPtr, int *badIdx, int *unsorted,
-                          cudaStream_t s, int num_sms);
+void launch_check_operand(const CsrDev &M, int2 *range, int *badPtr, int *badIdx, int *unsorted, cudaStream_t s,
+                          int num_sms);
 // Replaces them by the smallest and largest column when *unsorted is not 0.
-void launch_row_minmax(const CsrDev &B, int32_t *bmin, int32_t *bmax, const int *unsorted, cudaStream_t s,
-                       int num_sms);
-void launch_row_products(const CsrDev &A, const int32_t *Bp, const int32_t *bmin, const int32_t *bmax,
-                         const RowInfo &ri, uint8_t *symBin, int *err, const Tuning &t, cudaStream_t s,
-                         int num_sms);
-void launch_block_products(int64_t m, const int64_t *rowP, int64_t rows_per_block,
-                           int64_t *blockP, cudaStream_t s);
-void launch_bin_lists(int64_t m, const Binning &b, int nbins, cudaStream_t s);
-void launch_num_bins(int64_t m, const int32_t *Ap, const RowInfo &ri, const int32_t *rowNnz,
-                     uint8_t *numBin, const Tuning &t, cudaStream_t s, int num_sms);
-void launch_row_scan(int64_t m, const int32_t *rowNnz, int64_t *part, int64_t *Cp, cudaStream_t s);
+void launch_row_minmax(const CsrDev &B, int2 *range, const int *unsorted, cudaStream_t s, int num_sms);
+void launch_row_products(const CsrDev &A, const int32_t *Bp, const int2 *range, const RowInfo &ri, uint8_t *symBin,
+                         int *err, const Tuning &t, cudaStream_t s, int num_sms);
+// Row lists of the symbolic bins and (blockP not null) the products of every
+// rows_per_block rows; tileSum: tile_count(m) + 1 int64 of scratch.
+void launch_sym_lists(int64_t m, const Binning &b, const RowInfo &ri, int64_t *tileSum, int64_t rows_per_block,
+                      int64_t *blockP, cudaStream_t s);
+// Numeric bins, their row lists and C's row pointers (m + 1) from the rows'
+// entry counts.
+void launch_num_lists(int64_t m, const Binning &b, const RowInfo &ri, const int32_t *Ap, const int32_t *rowNnz,
+                      const Tuning &t, int64_t *tileSum, int64_t *Cp, cudaStream_t s);
+// cnt (m int32) -> exclusive int64 scan Cp (m + 1); part: ceil(m / kScanTile) + 1 int64 of scratch.
+void launch_row_scan(int64_t m, const int32_t *cnt, int64_t *part, int64_t *Cp, cudaStream_t s);
 
 // ---- launchers (k_spgemm.cu) ----
 struct SymArgs {

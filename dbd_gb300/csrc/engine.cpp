@@ -100,7 +100,7 @@ struct HostBuf {
 struct Operand {
     CsrDev dev;
     DevBuf ptr, idx, val, tmp;
-    DevBuf bmin, bmax;  // first and last column of every row (as the right operand)
+    DevBuf range;  // first and last column of every row (as the right operand)
     bool loaded = false;
     int sorted = 0;
 };
@@ -389,10 +389,8 @@ int finish_operand(dbd_ctx *c, Operand &op, const CsrDev &d, const char *name) {
     CK(c, c->flags.ensure(4 * sizeof(int)));
     int *flags = c->flags.as<int>();
     CK(c, cudaMemsetAsync(flags, 0, 3 * sizeof(int), c->stream));
-    CK(c, op.bmin.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(d.m, 1)));
-    CK(c, op.bmax.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(d.m, 1)));
-    launch_check_operand(d, op.bmin.as<int32_t>(), op.bmax.as<int32_t>(), flags, flags + 1, flags + 2, c->stream,
-                         c->num_sms);
+    CK(c, op.range.ensure(sizeof(int2) * (size_t)std::max<int64_t>(d.m, 1)));
+    launch_check_operand(d, op.range.as<int2>(), flags, flags + 1, flags + 2, c->stream, c->num_sms);
     int hf[3] = {0, 0, 0};
     CK(c, cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
@@ -400,7 +398,7 @@ int finish_operand(dbd_ctx *c, Operand &op, const CsrDev &d, const char *name) {
     if (hf[1]) return set_err(c, DBD_ERR_INVALID, std::string(name) + ": column index out of range");
     op.sorted = hf[2] ? 0 : 1;
     if (!op.sorted)
-        launch_row_minmax(d, op.bmin.as<int32_t>(), op.bmax.as<int32_t>(), flags + 2, c->stream, c->num_sms);
+        launch_row_minmax(d, op.range.as<int2>(), flags + 2, c->stream, c->num_sms);
     op.loaded = true;
     c->divided = false;
     return DBD_OK;
@@ -443,7 +441,7 @@ int divide_blocks(dbd_ctx *c) {
     CK(c, c->numTileOff.ensure(sizeof(int32_t) * kMaxBins * (nt + 1)));
     CK(c, c->symStart.ensure(sizeof(int32_t) * (kMaxBins + 1)));
     CK(c, c->numStart.ensure(sizeof(int32_t) * (kMaxBins + 1)));
-    CK(c, c->part.ensure(sizeof(int64_t) * (size_t)(ceil_div(m, kScanTile) + 1)));
+    CK(c, c->part.ensure(sizeof(int64_t) * (nt + 1)));
     CK(c, c->Cp.ensure(sizeof(int64_t) * (mm + 1)));
     CK(c, c->cursor.ensure(2 * sizeof(int32_t) * (size_t)std::max<int64_t>(A.nnz, 1)));
     CK(c, c->err.ensure(sizeof(int)));
@@ -452,13 +450,12 @@ int divide_blocks(dbd_ctx *c) {
     CK(c, cudaEventRecord(c->evStart, c->stream));
     CK(c, cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream));
     const Operand &opb = c->b_is_a ? c->A : c->B;
-    launch_row_products(A, B.ptr, opb.bmin.as<int32_t>(), opb.bmax.as<int32_t>(), row_info(c),
-                        c->symBin.as<uint8_t>(), c->err.as<int>(), c->tune, c->stream, c->num_sms);
-    launch_block_products(m, c->rowP.as<int64_t>(), rpb, c->blockP.as<int64_t>(), c->stream);
+    launch_row_products(A, B.ptr, opb.range.as<int2>(), row_info(c), c->symBin.as<uint8_t>(), c->err.as<int>(),
+                        c->tune, c->stream, c->num_sms);
     Binning sb{c->symBin.as<uint8_t>(), c->symList.as<int32_t>(), c->hist.as<int32_t>(),
                c->symTileOff.as<int32_t>(), c->symStart.as<int32_t>()};
-    launch_bin_lists(m, sb, SB_COUNT, c->stream);
-    c->launches += 5;
+    launch_sym_lists(m, sb, row_info(c), c->part.as<int64_t>(), rpb, c->blockP.as<int64_t>(), c->stream);
+    c->launches += 4;
     CK(c, cudaGetLastError());
     c->blockP_h.assign((size_t)c->nblocks, 0);
     if (c->nblocks)
@@ -571,14 +568,12 @@ int symbolic(dbd_ctx *c) {
     }
     fk.join();
     cudaEvent_t es = c->time_ev(c->stream);
-    launch_row_scan(m, c->rowNnz.as<int32_t>(), c->part.as<int64_t>(), c->Cp.as<int64_t>(), c->stream);
-    launch_num_bins(m, c->A.dev.ptr, row_info(c), c->rowNnz.as<int32_t>(), c->numBin.as<uint8_t>(), c->tune, c->stream,
-                    c->num_sms);
     Binning nb{c->numBin.as<uint8_t>(), c->numList.as<int32_t>(), c->hist.as<int32_t>(),
                c->numTileOff.as<int32_t>(), c->numStart.as<int32_t>()};
-    launch_bin_lists(m, nb, NB_COUNT, c->stream);
+    launch_num_lists(m, nb, row_info(c), c->A.dev.ptr, c->rowNnz.as<int32_t>(), c->tune, c->part.as<int64_t>(),
+                     c->Cp.as<int64_t>(), c->stream);
     if (es) c->timed.push_back({2, 0, es, c->time_ev(c->stream)});
-    c->launches += 7;
+    c->launches += 3;
     CK(c, cudaGetLastError());
     CK(c, cudaMemcpyAsync(&c->nnzC, c->Cp.as<int64_t>() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaMemcpyAsync(c->numStart_h, c->numStart.p, sizeof(c->numStart_h), cudaMemcpyDeviceToHost, c->stream));
@@ -1314,7 +1309,7 @@ void dbd_destroy(dbd_ctx *c) {
                       &c->rowP, &c->symBin, &c->numBin, &c->rowNnz, &c->symList, &c->numList, &c->hist,
                       &c->symTileOff, &c->numTileOff, &c->symStart, &c->numStart, &c->part, &c->Cp, &c->cursor,
                       &c->err, &c->blockP, &c->flags, &c->Ci, &c->Cv, &c->wideBits, &c->wideSlot, &c->adjG,
-                      &c->adjA, &c->adjB, &c->adjT, &c->rowLo, &c->rowHi, &c->A.bmin, &c->A.bmax, &c->B.bmin, &c->B.bmax,
+                      &c->adjA, &c->adjB, &c->adjT, &c->rowLo, &c->rowHi, &c->A.range, &c->B.range,
                       &c->ctrs, &c->gdense, &c->dgCount, &c->dgCol, &c->dgVal, &c->dgSum, &c->dgWsum,
                       &c->dgBad, &c->hashOut, &c->dscr, &c->heavySlot, &c->slabCnt,
                       &c->items})
@@ -1860,8 +1855,7 @@ int dbd_batch_plan(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const dbd_c
         CK(c, op.ptr.ensure(sizeof(int32_t) * (size_t)(rows + 1)));
         CK(c, op.idx.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(ne, 1)));
         CK(c, op.val.ensure(sizeof(double) * (size_t)std::max<int64_t>(ne, 1)));
-        CK(c, op.bmin.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(rows, 1)));
-        CK(c, op.bmax.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(rows, 1)));
+        CK(c, op.range.ensure(sizeof(int2) * (size_t)std::max<int64_t>(rows, 1)));
         return DBD_OK;
     };
     int rc = sized(c->A, m, nnzA[count]);
@@ -1908,7 +1902,7 @@ int dbd_batch_plan(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const dbd_c
     CK(c, c->numTileOff.ensure(sizeof(int32_t) * kMaxBins * (nt + 1)));
     CK(c, c->symStart.ensure(sizeof(int32_t) * (kMaxBins + 1)));
     CK(c, c->numStart.ensure(sizeof(int32_t) * (kMaxBins + 1)));
-    CK(c, c->part.ensure(sizeof(int64_t) * (size_t)(ceil_div(m, kScanTile) + 1)));
+    CK(c, c->part.ensure(sizeof(int64_t) * (nt + 1)));
     CK(c, c->Cp.ensure(sizeof(int64_t) * (mm + 1)));
     CK(c, c->cursor.ensure(2 * sizeof(int32_t) * (size_t)std::max<int64_t>(nnzA[count], 1)));
     CK(c, c->err.ensure(sizeof(int)));
@@ -1964,13 +1958,13 @@ int dbd_batch_enqueue(dbd_ctx *c, void *stream) {
     const CsrDev &A = c->A.dev, &B = opB(c);
     const Operand &opb = c->bpSquare ? c->A : c->B;
     int launches = 0;
-    launch_check_operand(B, opb.bmin.as<int32_t>(), opb.bmax.as<int32_t>(), nullptr, nullptr, flags + 2, s, c->num_sms);
-    launch_row_minmax(B, opb.bmin.as<int32_t>(), opb.bmax.as<int32_t>(), flags + 2, s, c->num_sms);
-    launch_row_products(A, B.ptr, opb.bmin.as<int32_t>(), opb.bmax.as<int32_t>(), row_info(c), c->symBin.as<uint8_t>(),
-                        c->err.as<int>(), c->tune, s, c->num_sms);
+    launch_check_operand(B, opb.range.as<int2>(), nullptr, nullptr, flags + 2, s, c->num_sms);
+    launch_row_minmax(B, opb.range.as<int2>(), flags + 2, s, c->num_sms);
+    launch_row_products(A, B.ptr, opb.range.as<int2>(), row_info(c), c->symBin.as<uint8_t>(), c->err.as<int>(),
+                        c->tune, s, c->num_sms);
     Binning sb{c->symBin.as<uint8_t>(), c->symList.as<int32_t>(), c->hist.as<int32_t>(), c->symTileOff.as<int32_t>(),
                c->symStart.as<int32_t>()};
-    launch_bin_lists(m, sb, SB_COUNT, s);
+    launch_sym_lists(m, sb, row_info(c), nullptr, 0, nullptr, s);
     SymArgs sa{};
     sa.A = A;
     sa.B = B;
@@ -1995,11 +1989,10 @@ int dbd_batch_enqueue(dbd_ctx *c, void *stream) {
         for (int bin : sorder) launch_symbolic_bin_dd(sa, bin, fk.stream(bin), &launches);
         fk.join();
     }
-    launch_row_scan(m, c->rowNnz.as<int32_t>(), c->part.as<int64_t>(), c->Cp.as<int64_t>(), s);
-    launch_num_bins(m, A.ptr, row_info(c), c->rowNnz.as<int32_t>(), c->numBin.as<uint8_t>(), c->tune, s, c->num_sms);
     Binning nb{c->numBin.as<uint8_t>(), c->numList.as<int32_t>(), c->hist.as<int32_t>(), c->numTileOff.as<int32_t>(),
                c->numStart.as<int32_t>()};
-    launch_bin_lists(m, nb, NB_COUNT, s);
+    launch_num_lists(m, nb, row_info(c), A.ptr, c->rowNnz.as<int32_t>(), c->tune, c->part.as<int64_t>(),
+                     c->Cp.as<int64_t>(), s);
     launch_numeric_guard(c->Cp.as<int64_t>() + m, c->bpCap, c->err.as<int>(), c->numStart.as<int32_t>(), NB_COUNT,
                          flags + 3, s);
     NumArgs na{};

@@ -21,7 +21,7 @@ constexpr unsigned FULL = 0xffffffffu;
 // Everything a multiply asks of an operand before it reads through it, in one
 // pass: *badPtr <- 1 unless ptr[0] == 0, ptr[m] == nnz and ptr never
 // decreases; *badIdx <- 1 if a column lies outside [0, n); the first and last
-// column of every row (bmin = INT32_MAX, bmax = -1 when empty), which are its
+// column of every row as one pair (INT32_MAX and -1 when empty), which are its
 // smallest and largest where the row ascends; and *unsorted += the number of
 // entries not above their predecessor in the same row (0: every row ascends).
 // badPtr and badIdx may be null.
@@ -37,8 +37,7 @@ constexpr unsigned FULL = 0xffffffffu;
 // of 2.1M five-point rows takes 251 us less.
 // (A row_ptr that fails its check is never read through: a row's entries are
 // touched only when both its bounds lie in [0, nnz].)
-__global__ void __launch_bounds__(256) k_check_operand(CsrDev M, int32_t *__restrict__ bmin,
-                                                       int32_t *__restrict__ bmax, int *__restrict__ badPtr,
+__global__ void __launch_bounds__(256) k_check_operand(CsrDev M, int2 *__restrict__ range, int *__restrict__ badPtr,
                                                        int *__restrict__ badIdx, int *__restrict__ unsorted) {
     __shared__ int red[8];
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -109,8 +108,7 @@ __global__ void __launch_bounds__(256) k_check_operand(CsrDev M, int32_t *__rest
             } else {
                 badP |= w[u] < v[u];
                 if (lo[u] <= before[u]) --down;
-                bmin[r] = lo[u];
-                bmax[r] = hi[u];
+                range[r] = make_int2(lo[u], hi[u]);
             }
         }
     }
@@ -128,8 +126,7 @@ __global__ void __launch_bounds__(256) k_check_operand(CsrDev M, int32_t *__rest
 
 // Smallest and largest column of every row of an operand that
 // k_check_operand found unsorted (one warp per row); nothing otherwise.
-__global__ void k_row_minmax(CsrDev B, int32_t *__restrict__ bmin, int32_t *__restrict__ bmax,
-                             const int *__restrict__ unsorted) {
+__global__ void k_row_minmax(CsrDev B, int2 *__restrict__ range, const int *__restrict__ unsorted) {
     if (*unsorted == 0) return;
     const int lane = threadIdx.x & 31;
     int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -147,10 +144,7 @@ __global__ void k_row_minmax(CsrDev B, int32_t *__restrict__ bmin, int32_t *__re
             lo = min(lo, __shfl_xor_sync(FULL, lo, d));
             hi = max(hi, __shfl_xor_sync(FULL, hi, d));
         }
-        if (lane == 0) {
-            bmin[row] = lo;
-            bmax[row] = hi;
-        }
+        if (lane == 0) range[row] = make_int2(lo, hi);
     }
 }
 
@@ -173,31 +167,54 @@ __device__ __forceinline__ void row_products_out(const CsrDev &A, int64_t row, i
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) k_row_products(CsrDev A, const int32_t *__restrict__ Bp,
-                                                          const int32_t *__restrict__ bmin,
-                                                          const int32_t *__restrict__ bmax, RowInfo ri,
+                                                          const int2 *__restrict__ range, RowInfo ri,
                                                           uint8_t *__restrict__ symBin, int *err, Tuning tune) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int sub = lane & 7;
     const unsigned gmask = 0xffu << (lane & 24);
     const int64_t stride = ((int64_t)gridDim.x * THREADS) >> 3;
-    for (int64_t row = (blockIdx.x * (int64_t)THREADS + tid) >> 3; row < A.m; row += stride) {
-        const int32_t s = A.ptr[row], e = A.ptr[row + 1];
-        if (e - s > kLongRow) continue;  // the whole group skips together
-        int64_t sum = 0;
-        int32_t lo = INT32_MAX, hi = -1;
-        for (int32_t i = s + sub; i < e; i += 8) {
-            const int32_t k = A.idx[i];
-            sum += (int64_t)(Bp[k + 1] - Bp[k]);
-            lo = min(lo, bmin[k]);
-            hi = max(hi, bmax[k]);
+    // kRowsAhead rows a group in flight: a row is a chain of three dependent
+    // loads, which one row at a time leaves the GPU waiting for (2.1M
+    // five-entry rows: 155 -> 105 us, with the ranges read as pairs).
+    constexpr int kRowsAhead = 4;
+    for (int64_t b = (blockIdx.x * (int64_t)THREADS + tid) >> 3; b < A.m; b += kRowsAhead * stride) {
+        int32_t s[kRowsAhead], e[kRowsAhead], k[kRowsAhead];
+#pragma unroll
+        for (int u = 0; u < kRowsAhead; ++u) {
+            const int64_t row = b + u * stride;
+            s[u] = row < A.m ? __ldg(&A.ptr[row]) : 0;
+            e[u] = row < A.m ? __ldg(&A.ptr[row + 1]) : 0;
         }
 #pragma unroll
-        for (int d = 4; d; d >>= 1) {
-            sum += __shfl_xor_sync(gmask, sum, d, 8);
-            lo = min(lo, __shfl_xor_sync(gmask, lo, d, 8));
-            hi = max(hi, __shfl_xor_sync(gmask, hi, d, 8));
+        for (int u = 0; u < kRowsAhead; ++u) k[u] = s[u] + sub < e[u] ? __ldg(&A.idx[s[u] + sub]) : -1;
+        int64_t sum[kRowsAhead];
+        int32_t lo[kRowsAhead], hi[kRowsAhead];
+#pragma unroll
+        for (int u = 0; u < kRowsAhead; ++u) {
+            const int2 r = k[u] >= 0 ? __ldg(&range[k[u]]) : make_int2(INT32_MAX, -1);
+            sum[u] = k[u] >= 0 ? __ldg(&Bp[k[u] + 1]) - __ldg(&Bp[k[u]]) : 0;
+            lo[u] = r.x;
+            hi[u] = r.y;
         }
-        if (sub == 0) row_products_out(A, row, sum, lo, hi, ri, symBin, err, tune);
+#pragma unroll
+        for (int u = 0; u < kRowsAhead; ++u) {
+            const int64_t row = b + u * stride;
+            if (row >= A.m || e[u] - s[u] > kLongRow) continue;  // the whole group skips together
+            for (int32_t i = s[u] + 8 + sub; i < e[u]; i += 8) {
+                const int32_t q = A.idx[i];
+                const int2 r = __ldg(&range[q]);
+                sum[u] += (int64_t)(Bp[q + 1] - Bp[q]);
+                lo[u] = min(lo[u], r.x);
+                hi[u] = max(hi[u], r.y);
+            }
+#pragma unroll
+            for (int d = 4; d; d >>= 1) {
+                sum[u] += __shfl_xor_sync(gmask, sum[u], d, 8);
+                lo[u] = min(lo[u], __shfl_xor_sync(gmask, lo[u], d, 8));
+                hi[u] = max(hi[u], __shfl_xor_sync(gmask, hi[u], d, 8));
+            }
+            if (sub == 0) row_products_out(A, row, sum[u], lo[u], hi[u], ri, symBin, err, tune);
+        }
     }
 
     // Long rows: CTA b takes the long rows r with r = b (mod gridDim.x), one
@@ -222,9 +239,10 @@ __global__ void __launch_bounds__(THREADS) k_row_products(CsrDev A, const int32_
             int32_t lo = INT32_MAX, hi = -1;
             for (int32_t i = s + tid; i < e; i += THREADS) {
                 const int32_t k = A.idx[i];
+                const int2 kr = __ldg(&range[k]);
                 sum += (int64_t)(Bp[k + 1] - Bp[k]);
-                lo = min(lo, bmin[k]);
-                hi = max(hi, bmax[k]);
+                lo = min(lo, kr.x);
+                hi = max(hi, kr.y);
             }
 #pragma unroll
             for (int d = 16; d; d >>= 1) {
@@ -251,120 +269,182 @@ __global__ void __launch_bounds__(THREADS) k_row_products(CsrDev A, const int32_
     }
 }
 
-// Products per row block (block_Info of divide_Blocks, ZIP:dbd/src/main.cpp:276-296).
-__global__ void k_block_products(int64_t m, const int64_t *__restrict__ rowP,
-                                 int64_t rows_per_block, int64_t *__restrict__ blockP) {
-    __shared__ int64_t red[32];
-    const int64_t b = blockIdx.x;
-    const int64_t r0 = b * rows_per_block;
-    const int64_t r1 = min(m, r0 + rows_per_block);
-    int64_t s = 0;
-    for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) s += rowP[r];
-    for (int d = 16; d; d >>= 1) s += __shfl_xor_sync(FULL, s, d);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        s = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0;
-        for (int d = 16; d; d >>= 1) s += __shfl_xor_sync(FULL, s, d);
-        if (threadIdx.x == 0) blockP[b] = s;
-    }
-}
+// ---- per-bin row lists ----
+//
+// Rows are grouped by bin, row order kept, in three launches over tiles of
+// kTileRows rows: k_tiles counts every bin's rows per tile (hist[bin][tile])
+// and sums a per-row quantity per tile, k_tile_scan turns the counts into
+// absolute offsets, k_tile_scatter writes the lists.  The same three launches
+// carry what else is needed of the rows on either side of the symbolic pass:
+// before it the sums are the rows' products, from which the scan's last CTA
+// makes the row blocks' products; after it k_tiles also picks the numeric
+// bins, the sums are the rows' entries, which the scan's last CTA scans, and
+// the scatter writes C's row pointers.  (Before: five launches ahead of the
+// symbolic kernels' and seven behind them, and one CTA scanning all bins one
+// after another: all of them 130 and 210 us on 2.1M rows, 40 and 53 us now; on 65k
+// rows 14 and 25 us, 7 and 8 us now.)
 
-__global__ void k_num_bins(int64_t m, const int32_t *__restrict__ Ap, RowInfo ri,
-                           const int32_t *__restrict__ rowNnz, uint8_t *__restrict__ numBin, Tuning tune) {
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < m;
-         r += (int64_t)gridDim.x * blockDim.x)
-        numBin[r] = num_bin_of(ri.rowP[r], Ap[r + 1] - Ap[r], rowNnz[r], span_words(ri.lo[r], ri.hi[r]), tune);
-}
+// What the tiles carry beside the lists: nothing, the products (rowP) of the
+// row blocks, or the entries (rowNnz) and numeric bins of the rows.
+enum TileMode : int { TILES_PLAIN = 0, TILES_BLOCKS, TILES_NUMERIC };
 
-// Per-tile (kTileRows rows) counts of each bin.
-__global__ void k_bin_hist(int64_t m, const uint8_t *__restrict__ bin, int nbins,
-                           int32_t *__restrict__ hist) {
+__global__ void __launch_bounds__(kTileRows) k_tiles(int64_t m, int64_t ntiles, TileMode mode,
+                                                     uint8_t *__restrict__ bin, int nbins, const int32_t *__restrict__ Ap,
+                                                     RowInfo ri, const int32_t *__restrict__ rowNnz, Tuning tune,
+                                                     int32_t *__restrict__ hist, int64_t *__restrict__ tileSum) {
     __shared__ int32_t wc[kTileRows / 32][kMaxBins];
+    __shared__ int64_t ws[kTileRows / 32];
     const int64_t r = (int64_t)blockIdx.x * kTileRows + threadIdx.x;
-    const int b = r < m ? (int)bin[r] : -1;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int b = -1;
+    int64_t x = 0;
+    if (r < m) {
+        if (mode == TILES_NUMERIC) {
+            const int32_t nnz = rowNnz[r];
+            b = num_bin_of(ri.rowP[r], Ap[r + 1] - Ap[r], nnz, span_words(ri.lo[r], ri.hi[r]), tune);
+            bin[r] = (uint8_t)b;
+            x = nnz;
+        } else {
+            b = bin[r];
+            if (mode == TILES_BLOCKS) x = ri.rowP[r];
+        }
+    }
     for (int q = 0; q < nbins; ++q) {
         const unsigned mk = __ballot_sync(FULL, b == q);
         if (lane == 0) wc[w][q] = __popc(mk);
     }
+#pragma unroll
+    for (int d = 16; d; d >>= 1) x += __shfl_xor_sync(FULL, x, d);
+    if (lane == 0) ws[w] = x;
     __syncthreads();
     if (threadIdx.x < nbins) {
         int32_t s = 0;
         for (int i = 0; i < kTileRows / 32; ++i) s += wc[i][threadIdx.x];
-        hist[(int64_t)blockIdx.x * kMaxBins + threadIdx.x] = s;
+        hist[threadIdx.x * ntiles + blockIdx.x] = s;
+    } else if (threadIdx.x == 32 && tileSum) {
+        int64_t s = 0;
+        for (int i = 0; i < kTileRows / 32; ++i) s += ws[i];
+        tileSum[blockIdx.x] = s;
     }
 }
 
-// Block-wide exclusive scan of one int per thread (blockDim.x == 1024).
-__device__ __forceinline__ int32_t block_excl_scan_1024(int32_t v, int32_t *total, int32_t *sh) {
+constexpr int kScanThreads = 1024;
+
+// Block-wide exclusive scan of one value per thread (blockDim.x ==
+// kScanThreads).
+template <class T>
+__device__ __forceinline__ T block_excl_scan_wide(T v, T *total, T *sh) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int32_t x = v;
+    T x = v;
+#pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        const int32_t y = __shfl_up_sync(FULL, x, d);
+        const T y = __shfl_up_sync(FULL, x, d);
         if (lane >= d) x += y;
     }
     if (lane == 31) sh[w] = x;
     __syncthreads();
     if (w == 0) {
-        int32_t t = sh[lane];
+        T t = sh[lane];
+#pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const int32_t y = __shfl_up_sync(FULL, t, d);
+            const T y = __shfl_up_sync(FULL, t, d);
             if (lane >= d) t += y;
         }
         sh[lane] = t;  // inclusive warp totals
     }
     __syncthreads();
-    const int32_t base = w ? sh[w - 1] : 0;
-    *total = sh[31];
+    const T base = w ? sh[w - 1] : T(0);
+    *total = sh[kScanThreads / 32 - 1];
     __syncthreads();
     return base + x - v;
 }
 
-// Exclusive scan of every bin's column of hist over tiles, then absolute
-// offsets (bin start + within-bin offset) into tileOff; one CTA of 1024.
-__global__ void k_bin_scan(int64_t ntiles, int nbins, const int32_t *__restrict__ hist,
-                           int32_t *__restrict__ tileOff, int32_t *__restrict__ binStart) {
-    __shared__ int32_t sh[32];
-    __shared__ int32_t totals[kMaxBins];
-    for (int q = 0; q < nbins; ++q) {
-        int32_t carry = 0;
-        for (int64_t t0 = 0; t0 < ntiles; t0 += 1024) {
-            const int64_t t = t0 + threadIdx.x;
-            const int32_t v = t < ntiles ? hist[t * kMaxBins + q] : 0;
+// CTA q < kMaxBins: bin q's start (the rows of all bins below it, from their
+// tile counts) and its tiles' absolute offsets, four tiles a thread.  CTA
+// kMaxBins: the row blocks' products, or the tiles' entry offsets and C's
+// size.
+__global__ void __launch_bounds__(kScanThreads) k_tile_scan(int64_t ntiles, TileMode mode, int nbins,
+                                                            const int32_t *__restrict__ hist,
+                                                            int32_t *__restrict__ tileOff,
+                                                            int32_t *__restrict__ binStart,
+                                                            int64_t *__restrict__ tileSum, int64_t tilesPerBlock,
+                                                            int64_t *__restrict__ out) {
+    const int tid = threadIdx.x, q = blockIdx.x;
+    if (q < kMaxBins) {
+        __shared__ int32_t sh[kScanThreads / 32];
+        int32_t below = 0, start;
+        const int64_t n = (int64_t)min(q, nbins) * ntiles;
+#pragma unroll 8
+        for (int64_t i = tid; i < n; i += kScanThreads) below += hist[i];
+        block_excl_scan_wide<int32_t>(below, &start, sh);
+        int32_t carry = start;
+        for (int64_t t0 = 0; t0 < ntiles; t0 += 4 * kScanThreads) {
+            const int64_t t = t0 + 4 * tid;
+            int32_t v[4];
+            int32_t s = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                v[u] = q < nbins && t + u < ntiles ? hist[q * ntiles + t + u] : 0;
+                s += v[u];
+            }
             int32_t tot;
-            const int32_t ex = block_excl_scan_1024(v, &tot, sh);
-            if (t < ntiles) tileOff[t * kMaxBins + q] = carry + ex;
+            int32_t at = carry + block_excl_scan_wide<int32_t>(s, &tot, sh);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (t + u < ntiles) tileOff[(t + u) * kMaxBins + q] = at;
+                at += v[u];
+            }
             carry += tot;
         }
-        if (threadIdx.x == 0) totals[q] = carry;
-        __syncthreads();
-    }
-    __shared__ int32_t starts[kMaxBins + 1];
-    if (threadIdx.x == 0) {
-        int32_t s = 0;
-        for (int q = 0; q < kMaxBins; ++q) {
-            starts[q] = s;
-            if (q < nbins) s += totals[q];
+        if (tid == 0) {
+            tileOff[ntiles * kMaxBins + q] = carry;
+            binStart[q] = start;
+            if (q == kMaxBins - 1) binStart[kMaxBins] = carry;
         }
-        starts[kMaxBins] = s;
-        for (int q = 0; q <= kMaxBins; ++q) binStart[q] = starts[q];
+    } else if (mode == TILES_BLOCKS) {
+        // block_Info of divide_Blocks (ZIP:dbd/src/main.cpp:276-296), a warp a block.
+        const int64_t blocks = (ntiles + tilesPerBlock - 1) / tilesPerBlock;
+        for (int64_t k = tid >> 5; k < blocks; k += kScanThreads / 32) {
+            int64_t s = 0;
+            for (int64_t t = k * tilesPerBlock + (tid & 31); t < min(ntiles, (k + 1) * tilesPerBlock); t += 32)
+                s += tileSum[t];
+#pragma unroll
+            for (int d = 16; d; d >>= 1) s += __shfl_xor_sync(FULL, s, d);
+            if ((tid & 31) == 0) out[k] = s;
+        }
+    } else if (mode == TILES_NUMERIC) {
+        __shared__ int64_t sh[kScanThreads / 32];
+        int64_t carry = 0;
+        for (int64_t t0 = 0; t0 < ntiles; t0 += 4 * kScanThreads) {
+            const int64_t t = t0 + 4 * tid;
+            int64_t v[4], s = 0, tot;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                v[u] = t + u < ntiles ? tileSum[t + u] : 0;
+                s += v[u];
+            }
+            int64_t at = carry + block_excl_scan_wide<int64_t>(s, &tot, sh);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (t + u < ntiles) tileSum[t + u] = at;
+                at += v[u];
+            }
+            carry += tot;
+        }
+        if (tid == 0) *out = carry;
     }
-    __syncthreads();
-    for (int64_t i = threadIdx.x; i < ntiles * kMaxBins; i += blockDim.x) {
-        const int q = (int)(i % kMaxBins);
-        if (q < nbins) tileOff[i] += starts[q];
-        else tileOff[i] = starts[kMaxBins];
-    }
-    if (threadIdx.x < kMaxBins)
-        tileOff[ntiles * kMaxBins + threadIdx.x] =
-            threadIdx.x < nbins ? starts[threadIdx.x] + totals[threadIdx.x] : starts[kMaxBins];
 }
 
-// Stable scatter of row ids into their bin's list.
-__global__ void k_bin_scatter(int64_t m, const uint8_t *__restrict__ bin, int nbins,
-                              const int32_t *__restrict__ tileOff, int32_t *__restrict__ list) {
+// Stable scatter of row ids into their bin's list; with Cp also C's row
+// pointers (Cp[m] is the scan's).
+__global__ void __launch_bounds__(kTileRows) k_tile_scatter(int64_t m, const uint8_t *__restrict__ bin, int nbins,
+                                                            const int32_t *__restrict__ tileOff,
+                                                            int32_t *__restrict__ list,
+                                                            const int32_t *__restrict__ rowNnz,
+                                                            const int64_t *__restrict__ tileSum,
+                                                            int64_t *__restrict__ Cp) {
     __shared__ int32_t wc[kTileRows / 32][kMaxBins];
+    __shared__ int64_t ws[kTileRows / 32];
     const int64_t r = (int64_t)blockIdx.x * kTileRows + threadIdx.x;
     const int b = r < m ? (int)bin[r] : -1;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -374,11 +454,26 @@ __global__ void k_bin_scatter(int64_t m, const uint8_t *__restrict__ bin, int nb
         if (b == q) rank = __popc(mk & ((1u << lane) - 1u));
         if (lane == 0) wc[w][q] = __popc(mk);
     }
+    const int64_t x = Cp && r < m ? rowNnz[r] : 0;
+    int64_t incl = x;
+    if (Cp) {
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int64_t y = __shfl_up_sync(FULL, incl, d);
+            if (lane >= d) incl += y;
+        }
+        if (lane == 31) ws[w] = incl;
+    }
     __syncthreads();
     if (b >= 0) {
         int32_t pos = tileOff[(int64_t)blockIdx.x * kMaxBins + b] + rank;
         for (int i = 0; i < w; ++i) pos += wc[i][b];
         list[pos] = (int32_t)r;
+    }
+    if (Cp && r < m) {
+        int64_t at = tileSum[blockIdx.x] + incl - x;
+        for (int i = 0; i < w; ++i) at += ws[i];
+        Cp[r] = at;
     }
 }
 
@@ -464,49 +559,52 @@ __global__ void k_f32_to_f64(const float *__restrict__ src, double *__restrict__
 
 }  // namespace
 
-void launch_check_operand(const CsrDev &M, int32_t *bmin, int32_t *bmax, int *badPtr, int *badIdx, int *unsorted,
-                          cudaStream_t s, int num_sms) {
+void launch_check_operand(const CsrDev &M, int2 *range, int *badPtr, int *badIdx, int *unsorted, cudaStream_t s,
+                          int num_sms) {
     const int64_t work = std::max<int64_t>(M.m + 1, M.nnz);
     const int grid = (int)std::min<int64_t>(ceil_div(work, 256), (int64_t)num_sms * 8);
-    k_check_operand<<<grid, 256, 0, s>>>(M, bmin, bmax, badPtr, badIdx, unsorted);
+    k_check_operand<<<grid, 256, 0, s>>>(M, range, badPtr, badIdx, unsorted);
 }
 
-void launch_row_minmax(const CsrDev &B, int32_t *bmin, int32_t *bmax, const int *unsorted, cudaStream_t s,
-                       int num_sms) {
+void launch_row_minmax(const CsrDev &B, int2 *range, const int *unsorted, cudaStream_t s, int num_sms) {
     if (B.m == 0) return;
     const int grid = (int)std::min<int64_t>(ceil_div(B.m * 32, 256), (int64_t)num_sms * 8);
-    k_row_minmax<<<grid, 256, 0, s>>>(B, bmin, bmax, unsorted);
+    k_row_minmax<<<grid, 256, 0, s>>>(B, range, unsorted);
 }
 
-void launch_row_products(const CsrDev &A, const int32_t *Bp, const int32_t *bmin, const int32_t *bmax,
-                         const RowInfo &ri, uint8_t *symBin, int *err, const Tuning &t, cudaStream_t s,
-                         int num_sms) {
+void launch_row_products(const CsrDev &A, const int32_t *Bp, const int2 *range, const RowInfo &ri, uint8_t *symBin,
+                         int *err, const Tuning &t, cudaStream_t s, int num_sms) {
     if (A.m == 0) return;
     constexpr int threads = 256;
     const int64_t need = ceil_div(A.m * 8, threads);
     const int grid = (int)std::min<int64_t>(need, (int64_t)num_sms * 8);
-    k_row_products<threads><<<grid, threads, 0, s>>>(A, Bp, bmin, bmax, ri, symBin, err, t);
+    k_row_products<threads><<<grid, threads, 0, s>>>(A, Bp, range, ri, symBin, err, t);
 }
 
-void launch_block_products(int64_t m, const int64_t *rowP, int64_t rows_per_block, int64_t *blockP,
-                           cudaStream_t s) {
-    const int64_t nb = ceil_div(m, rows_per_block);
-    if (nb == 0) return;
-    k_block_products<<<(unsigned)nb, 256, 0, s>>>(m, rowP, rows_per_block, blockP);
+void launch_sym_lists(int64_t m, const Binning &b, const RowInfo &ri, int64_t *tileSum, int64_t rows_per_block,
+                      int64_t *blockP, cudaStream_t s) {
+    const int64_t nt = ceil_div(m, kTileRows);
+    const TileMode mode = blockP ? TILES_BLOCKS : TILES_PLAIN;
+    if (nt > 0)
+        k_tiles<<<(unsigned)nt, kTileRows, 0, s>>>(m, nt, mode, b.bin, SB_COUNT, nullptr, ri, nullptr, Tuning{}, b.hist,
+                                                   blockP ? tileSum : nullptr);
+    k_tile_scan<<<kMaxBins + 1, kScanThreads, 0, s>>>(nt, mode, SB_COUNT, b.hist, b.tileOff, b.binStart, tileSum,
+                                                      std::max<int64_t>(rows_per_block / kTileRows, 1), blockP);
+    if (nt > 0)
+        k_tile_scatter<<<(unsigned)nt, kTileRows, 0, s>>>(m, b.bin, SB_COUNT, b.tileOff, b.list, nullptr, nullptr,
+                                                          nullptr);
 }
 
-void launch_bin_lists(int64_t m, const Binning &b, int nbins, cudaStream_t s) {
-    const int64_t ntiles = ceil_div(m, kTileRows);
-    if (ntiles > 0) k_bin_hist<<<(unsigned)ntiles, kTileRows, 0, s>>>(m, b.bin, nbins, b.hist);
-    k_bin_scan<<<1, 1024, 0, s>>>(ntiles, nbins, b.hist, b.tileOff, b.binStart);
-    if (ntiles > 0) k_bin_scatter<<<(unsigned)ntiles, kTileRows, 0, s>>>(m, b.bin, nbins, b.tileOff, b.list);
-}
-
-void launch_num_bins(int64_t m, const int32_t *Ap, const RowInfo &ri, const int32_t *rowNnz,
-                     uint8_t *numBin, const Tuning &t, cudaStream_t s, int num_sms) {
-    if (m == 0) return;
-    const int grid = (int)std::min<int64_t>(ceil_div(m, 256), (int64_t)num_sms * 8);
-    k_num_bins<<<grid, 256, 0, s>>>(m, Ap, ri, rowNnz, numBin, t);
+void launch_num_lists(int64_t m, const Binning &b, const RowInfo &ri, const int32_t *Ap, const int32_t *rowNnz,
+                      const Tuning &t, int64_t *tileSum, int64_t *Cp, cudaStream_t s) {
+    const int64_t nt = ceil_div(m, kTileRows);
+    if (nt > 0)
+        k_tiles<<<(unsigned)nt, kTileRows, 0, s>>>(m, nt, TILES_NUMERIC, b.bin, NB_COUNT, Ap, ri, rowNnz, t, b.hist,
+                                                   tileSum);
+    k_tile_scan<<<kMaxBins + 1, kScanThreads, 0, s>>>(nt, TILES_NUMERIC, NB_COUNT, b.hist, b.tileOff, b.binStart,
+                                                      tileSum, 1, Cp + m);
+    if (nt > 0)
+        k_tile_scatter<<<(unsigned)nt, kTileRows, 0, s>>>(m, b.bin, NB_COUNT, b.tileOff, b.list, rowNnz, tileSum, Cp);
 }
 
 void launch_row_scan(int64_t m, const int32_t *rowNnz, int64_t *part, int64_t *Cp, cudaStream_t s) {
@@ -529,8 +627,8 @@ void launch_f32_to_f64(const float *src, double *dst, int64_t n, cudaStream_t s)
 // launch, by default).  Returns the first error.
 cudaError_t preload_analysis_kernels() {
     const void *fns[] = {
-        (const void *)k_check_operand, (const void *)k_row_minmax, (const void *)k_row_products<256>, (const void *)k_block_products,
-        (const void *)k_num_bins, (const void *)k_bin_hist, (const void *)k_bin_scan, (const void *)k_bin_scatter,
+        (const void *)k_check_operand, (const void *)k_row_minmax, (const void *)k_row_products<256>,
+        (const void *)k_tiles, (const void *)k_tile_scan, (const void *)k_tile_scatter,
         (const void *)k_scan_reduce, (const void *)k_scan_parts, (const void *)k_scan_final,
         (const void *)k_f32_to_f64,
     };

@@ -83,14 +83,15 @@ struct Carver {
     }
 };
 
-// Bytes of scratch the pipeline needs for m rows and nnzA entries of A and
-// mB rows of B; the carving below in dbd_spgemm_noalloc takes the same
-// regions in this order.
+// Bytes of scratch that m rows and nnzA entries of A and mB rows of B count
+// for: what callers size their inputs by.  The carving below in
+// dbd_spgemm_noalloc takes the same regions in this order, some of them
+// joined (the two columns of B's rows) or shared (the scan partials).
 size_t scratch_bytes(int64_t m, int64_t nnzA, int64_t mB) {
     Carver c{nullptr};
     const size_t nt = (size_t)ceil_div(m, kTileRows) + 1;
-    c.take<int32_t>((size_t)mB);                   // bmin
-    c.take<int32_t>((size_t)mB);                   // bmax
+    c.take<int32_t>((size_t)mB);                   // first columns of B's rows
+    c.take<int32_t>((size_t)mB);                   // last columns
     c.take<int32_t>((size_t)m);                    // rowLo
     c.take<int32_t>((size_t)m);                    // rowHi
     c.take<int64_t>((size_t)m);                    // rowP
@@ -104,7 +105,7 @@ size_t scratch_bytes(int64_t m, int64_t nnzA, int64_t mB) {
     c.take<int32_t>(kMaxBins * nt);                // numTileOff
     c.take<int32_t>(kMaxBins + 1);                 // symStart
     c.take<int32_t>(kMaxBins + 1);                 // numStart
-    c.take<int64_t>((size_t)ceil_div(m, kScanTile) + 1);  // part
+    c.take<int64_t>((size_t)ceil_div(m, kScanTile) + 1);  // scan partials
     c.take<int32_t>(2 * (size_t)nnzA);             // dense-window state
     c.take<int>(4);                                // err + flags
     c.take<uint32_t>(CTR_COUNT);                   // persistent kernels' row counters
@@ -167,8 +168,7 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
         return fail(DBD_ERR_INVALID, "the stream is capturing: this call synchronises and cannot be captured");
     Carver c{base};  // the layout of scratch_bytes()
     const size_t nt = (size_t)ceil_div(m, kTileRows) + 1;
-    int32_t *bmin = c.take<int32_t>((size_t)b->n_rows);
-    int32_t *bmax = c.take<int32_t>((size_t)b->n_rows);
+    int2 *range = c.take<int2>((size_t)b->n_rows);
     RowInfo ri;
     ri.lo = c.take<int32_t>((size_t)m);
     ri.hi = c.take<int32_t>((size_t)m);
@@ -184,7 +184,10 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     int32_t *numTileOff = c.take<int32_t>(kMaxBins * nt);
     int32_t *symStart = c.take<int32_t>(kMaxBins + 1);
     int32_t *numStart = c.take<int32_t>(kMaxBins + 1);
-    int64_t *part = c.take<int64_t>((size_t)ceil_div(m, kScanTile) + 1);
+    // The tiles' entry sums take the symbolic tile offsets' place, which are
+    // read last when the symbolic lists are written.
+    static_assert(sizeof(int32_t) * kMaxBins >= sizeof(int64_t), "a tile's sum fits in its offsets");
+    int64_t *tileSum = reinterpret_cast<int64_t *>(symTileOff);
     int32_t *state = c.take<int32_t>(2 * (size_t)a->nnz);
     int *flags = c.take<int>(4);  // [0] device error word, [1] bad row_ptr, [2] bad index, [3] B unsorted
     uint32_t *ctrs = c.take<uint32_t>(CTR_COUNT);
@@ -201,21 +204,23 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     int sms = 0;
     NA_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     // Both operands are checked before any kernel gathers through them; A's
-    // row column ranges (into rowLo and rowHi, which the analysis fills
-    // later) and order are not used.
-    if (b != a) launch_check_operand(A, ri.lo, ri.hi, flags + 1, flags + 2, flags + 3, s, sms);
-    if (b != a) NA_CK(cudaMemsetAsync(flags + 3, 0, sizeof(int), s));
-    launch_check_operand(B, bmin, bmax, flags + 1, flags + 2, flags + 3, s, sms);
+    // row ranges (into rowP, which the analysis fills later) and order are
+    // not used.
+    if (b != a) {
+        launch_check_operand(A, reinterpret_cast<int2 *>(rowP), flags + 1, flags + 2, flags + 3, s, sms);
+        NA_CK(cudaMemsetAsync(flags + 3, 0, sizeof(int), s));
+    }
+    launch_check_operand(B, range, flags + 1, flags + 2, flags + 3, s, sms);
     int hflags[4] = {0, 0, 0, 0};
     NA_CK(cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, s));
     NA_CK(cudaStreamSynchronize(s));
     if (hflags[1]) return fail(DBD_ERR_INVALID, "malformed row_ptr");
     if (hflags[2]) return fail(DBD_ERR_INVALID, "column index out of range");
-    if (hflags[3]) launch_row_minmax(B, bmin, bmax, flags + 3, s, sms);
+    if (hflags[3]) launch_row_minmax(B, range, flags + 3, s, sms);
     // Analysis: products per row, symbolic bins, row lists.
-    launch_row_products(A, B.ptr, bmin, bmax, ri, symBin, flags, Tuning{}, s, sms);
+    launch_row_products(A, B.ptr, range, ri, symBin, flags, Tuning{}, s, sms);
     Binning sb{symBin, symList, hist, symTileOff, symStart};
-    launch_bin_lists(m, sb, SB_COUNT, s);
+    launch_sym_lists(m, sb, ri, nullptr, 0, nullptr, s);
     int32_t symStart_h[kMaxBins + 1];
     NA_CK(cudaMemcpyAsync(symStart_h, symStart, sizeof(symStart_h), cudaMemcpyDeviceToHost, s));
     NA_CK(cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, s));
@@ -239,10 +244,8 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     int launches = 0;
     for (int bin = SB_TINY; bin < SB_COUNT; ++bin)
         launch_symbolic_bin(sa, bin, symStart_h[bin], symStart_h[bin + 1] - symStart_h[bin], s, &launches);
-    launch_row_scan(m, rowNnz, part, c_row_ptr, s);
-    launch_num_bins(m, A.ptr, ri, rowNnz, numBin, Tuning{}, s, sms);
     Binning nb{numBin, numList, hist, numTileOff, numStart};
-    launch_bin_lists(m, nb, NB_COUNT, s);
+    launch_num_lists(m, nb, ri, A.ptr, rowNnz, Tuning{}, tileSum, c_row_ptr, s);
     int64_t nnz = 0;
     int32_t numStart_h[kMaxBins + 1];
     NA_CK(cudaMemcpyAsync(&nnz, c_row_ptr + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
