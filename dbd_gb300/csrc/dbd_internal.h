@@ -135,7 +135,7 @@ enum DevErr : int { DEV_OK = 0, DEV_TABLE_FULL = 1, DEV_COUNT_MISMATCH = 2, DEV_
 // Counter slots for dynamically scheduled kernels (zeroed per multiply).
 enum CounterSlot : int {
     CTR_SYM_TINY = 0, CTR_SYM_HWARP, CTR_SYM_HCTA, CTR_SYM_WIDE, CTR_NUM_GDENSE, CTR_NUM_RANKWIN, CTR_NUM_DSCR,
-    CTR_HEAVY, CTR_ITEMS, CTR_COUNT = 16
+    CTR_HEAVY, CTR_ITEMS, CTR_ADJOINT, CTR_COUNT = 16
 };
 
 struct Binning {
@@ -278,7 +278,8 @@ void launch_numeric_bin(const NumArgs &a, int bin, int32_t lo, int32_t hi, cudaS
 
 // Adjoint of C = A*B over fixed patterns: given G = dL/dC on C's pattern
 // (Cp, Ci), dA[e] = sum_k G(i,k) B(j,k) for e = (i,j) in A and
-// dB[f] += A(i,j) G(i,k) for f = (j,k) in B.  dA and dB start at zero.
+// dB[f] += A(i,j) G(i,k) for f = (j,k) in B (dB null: dA only).  dA and dB
+// start at zero: entries without products are not written.
 struct AdjArgs {
     CsrDev A, B;
     const int64_t *Cp;
@@ -286,11 +287,20 @@ struct AdjArgs {
     const double *G;
     double *dA;
     double *dB;
-    const int32_t *order;  // rows of A in the forward's numeric bin order (null: 0..m-1)
-    int64_t nrows;
+    const int32_t *order;  // rows of A in the forward's numeric bin order
+    uint32_t *ctr;         // row counter of the CTA kernel
+    // With dB null: where to keep every product A(i,j) * G(i,k) for the
+    // deterministic dB pass (null: nowhere), entry e's from off[e] on in B's
+    // row order.
+    double *prod = nullptr;
+    const int64_t *off = nullptr;
+    int64_t prodCap = 0;
     int *err;
 };
-void launch_adjoint(const AdjArgs &a, cudaStream_t s, int *launches);
+// Rows order[lo, hi) whose rows of C hold at most 512 entries (one warp each).
+void launch_adjoint_warp(const AdjArgs &a, int32_t lo, int32_t hi, cudaStream_t s, int *launches);
+// Rows order[lo, hi) of any size, the last ones first.
+void launch_adjoint_cta(const AdjArgs &a, int32_t lo, int32_t hi, int num_sms, cudaStream_t s, int *launches);
 // dB = mask_B(A^T G) on its own: one warp per row k of B, each lane one
 // entry (k, j), summing A(i,k) * G(i,j) over column k of A in row order
 // (colPtr / perm / rowOf: A's entries grouped by column, stably).
@@ -303,6 +313,9 @@ struct AdjDbArgs {
     const int64_t *Cp;
     const int32_t *Ci;
     const double *G;
+    const double *prod = nullptr;  // the dA pass's products (AdjArgs), or null: G by search
+    const int64_t *off = nullptr;
+    int64_t prodCap = 0;
     double *dB;
     int *err;
     int32_t *extra;         // nnz(B): segments after the first, per entry
@@ -314,6 +327,10 @@ struct AdjDbArgs {
 // vals: two pairs of nnz(A) uint32 buffers; scratch: stable_sort_scratch_bytes).
 void launch_adjoint_transpose(const CsrDev &A, int32_t *rowOf, uint32_t *keys0, uint32_t *vals0, uint32_t *keys1,
                               uint32_t *vals1, void *scratch, int32_t *colPtr, const uint32_t **perm, cudaStream_t s);
+// len[e]: products of A entry e; off: their exclusive scan (nnz(A) + 1).
+// scanPart: ceil(nnz(A) / kScanTile) + 1 int64.
+void launch_entry_products(const CsrDev &A, const CsrDev &B, int32_t *len, int64_t *scanPart, int64_t *off,
+                           cudaStream_t s);
 // partCap for a.part: the further segments number at most the forward's
 // products over the segment length.  scanPart: ceil(nnz(B) / kScanTile) + 1
 // int64 for the scan of the segment counts.
@@ -381,6 +398,7 @@ void launch_hash_words(const uint32_t *w, int64_t n, uint64_t salt, uint64_t *ac
 
 // One-time kernel attribute setup (dynamic shared memory limits).
 void init_kernel_attributes();
+void init_adjoint_attributes();
 // Load the kernels of k_analysis.cu / k_spgemm.cu now instead of at their
 // first launch (cudaFuncGetAttributes on each); the first error is returned.
 cudaError_t preload_analysis_kernels();

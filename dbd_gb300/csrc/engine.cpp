@@ -155,6 +155,7 @@ struct dbd_ctx {
     int64_t patA = -1, patB = -1;
     DevBuf adjG, adjA, adjB;    // device copies for host-side adjoint arguments
     DevBuf adjT;                // A grouped by column for the deterministic dB pass
+    DevBuf adjProd, adjOff;     // its products as the dA pass computed them, and where each A entry's start
     // Batched products: the pairs' placement (device copy of the pair
     // descriptors and offsets, staged through pinned memory), the per-row
     // column shift of the concatenated A, and the pair count of the last
@@ -417,6 +418,7 @@ int divide_blocks(dbd_ctx *c) {
     if (A.n != B.m) return set_err(c, DBD_ERR_INVALID, "inner dimensions differ (A.n_cols != B.n_rows)");
     const auto t0 = Clock::now();
     drop_graph(c);  // the plan it replays is replaced
+    c->patternOk = false;  // so are the arrays an adjoint would read the last product's rows from
     c->launches = 0;
     c->tused = c->sused = 0;
     c->timed.clear();
@@ -1292,6 +1294,7 @@ int dbd_create(const dbd_config *cfg_in, dbd_ctx **out) {
     cudaEventCreate(&c->evNumA);
     cudaEventCreate(&c->evNumB);
     init_kernel_attributes();
+    init_adjoint_attributes();
     if (cudaGetLastError() != cudaSuccess) {
         dbd_destroy(c);
         return DBD_ERR_CUDA;
@@ -1309,7 +1312,7 @@ void dbd_destroy(dbd_ctx *c) {
                       &c->rowP, &c->symBin, &c->numBin, &c->rowNnz, &c->symList, &c->numList, &c->hist,
                       &c->symTileOff, &c->numTileOff, &c->symStart, &c->numStart, &c->part, &c->Cp, &c->cursor,
                       &c->err, &c->blockP, &c->flags, &c->Ci, &c->Cv, &c->wideBits, &c->wideSlot, &c->adjG,
-                      &c->adjA, &c->adjB, &c->adjT, &c->rowLo, &c->rowHi, &c->A.range, &c->B.range,
+                      &c->adjA, &c->adjB, &c->adjT, &c->adjProd, &c->adjOff, &c->rowLo, &c->rowHi, &c->A.range, &c->B.range,
                       &c->ctrs, &c->gdense, &c->dgCount, &c->dgCol, &c->dgVal, &c->dgSum, &c->dgWsum,
                       &c->dgBad, &c->hashOut, &c->dscr, &c->heavySlot, &c->slabCnt,
                       &c->items})
@@ -1584,10 +1587,38 @@ int dbd_spgemm_adjoint(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b,
     aa.dA = dA;
     aa.dB = det ? nullptr : dB;  // deterministic: dB by its own pass below
     aa.order = c->numList.as<int32_t>();
-    aa.nrows = c->m;
+    aa.ctr = c->ctrs.as<uint32_t>() + CTR_ADJOINT;
     aa.err = c->err.as<int>();
     int launches = 0;
-    launch_adjoint(aa, c->stream, &launches);
+    if (det && B.nnz > 0 && A.nnz > 0 && 8.0 * (double)c->products <= c->cfg.gpu_gib * kGiB / 8) {
+        // The products of the dA pass are kept for the dB pass within an
+        // eighth of the GPU budget (as the wide rows' bitmaps are) and where
+        // the device has the room; otherwise the dB pass looks G up again.
+        const size_t oLen = (8 * (size_t)(A.nnz + 1) + 15) / 16 * 16;
+        const size_t oScan = oLen + (4 * (size_t)A.nnz + 15) / 16 * 16;
+        if (c->adjProd.ensure(8 * (size_t)std::max<int64_t>(c->products, 1)) == cudaSuccess &&
+            c->adjOff.ensure(oScan + 8 * (size_t)(ceil_div(A.nnz, kScanTile) + 1)) == cudaSuccess) {
+            char *p = c->adjOff.as<char>();
+            launch_entry_products(A, B, reinterpret_cast<int32_t *>(p + oLen), reinterpret_cast<int64_t *>(p + oScan),
+                                  reinterpret_cast<int64_t *>(p), c->stream);
+            aa.prod = c->adjProd.as<double>();
+            aa.off = reinterpret_cast<const int64_t *>(p);
+            aa.prodCap = c->products;
+        } else {
+            cudaGetLastError();
+        }
+    }
+    // The numeric bins between the CTA rank rows and the dense ones hold the
+    // rows of C that need a CTA (numWarpMax entries or more); a warp takes the
+    // others, at most kDenseWarpWords * 32 entries long.
+    c->sused = 0;
+    {
+        Fork fk(c);
+        launch_adjoint_cta(aa, c->numStart_h[NB_RANKS], c->numStart_h[NB_DENSEW], c->num_sms, fk.stream(0), &launches);
+        launch_adjoint_warp(aa, c->numStart_h[NB_TINY], c->numStart_h[NB_RANKS], fk.stream(1), &launches);
+        launch_adjoint_warp(aa, c->numStart_h[NB_DENSEW], c->numStart_h[NB_COUNT], fk.stream(2), &launches);
+        fk.join();
+    }
     if (det && B.nnz > 0) {
         // A grouped by column (stably, so rows ascend in every column), then
         // dB by segments of every column (launch_adjoint_db).
@@ -1621,6 +1652,9 @@ int dbd_spgemm_adjoint(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b,
         ab.Cp = c->Cp.as<int64_t>();
         ab.Ci = c->Ci.as<int32_t>();
         ab.G = dG;
+        ab.prod = aa.prod;
+        ab.off = aa.off;
+        ab.prodCap = aa.prodCap;
         ab.dB = dB;
         ab.err = c->err.as<int>();
         ab.extra = reinterpret_cast<int32_t *>(p + oExtra);

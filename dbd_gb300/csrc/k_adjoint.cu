@@ -4,10 +4,11 @@
 // device (CSR, columns ascending in every row):
 //   dA = mask_A(G * B^T)   dA(i,k) = sum_j G(i,j) * B(k,j)
 //   dB = mask_B(A^T * G)   dB(k,j) = sum_i A(i,k) * G(i,j)
-// k_adjoint takes both from A's rows (dB by FP64 reductions); with the
+// k_adjoint_warp and k_adjoint_cta take both from A's rows (dB by FP64 reductions); with the
 // deterministic option dB comes from its own pass over B's pattern
 // (k_entry_rows, the stable radix sort of k_mtx.cu, k_col_ptr, then the
 // k_adjoint_db kernels).
+#include "cta_stage.cuh"
 #include "dbd_internal.h"
 #include "warp_chunk.cuh"
 
@@ -28,51 +29,265 @@ __device__ __forceinline__ int64_t find_col(const int32_t *__restrict__ ci, int6
     return (lo < end && ci[lo] == k) ? lo : end;
 }
 
-// One warp per row of A, rows in the forward's numeric order heaviest bins
-// first.  Every product (e = (i,k), f = (k,j)) looks up g = G(i,j) in C's
-// row i, adds A[e] * g to dB[f] (FP64 reduction at L2) and g * B[f] to dA[e]
-// (summed over the adjacent lanes that share e first).
-__global__ void __launch_bounds__(256) k_adjoint(AdjArgs a) {
-    const int lane = threadIdx.x & 31;
-    const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (item >= a.nrows) return;
-    const int32_t row = a.order ? a.order[a.nrows - 1 - item] : (int32_t)item;
+// Rows of C of at most kAdjWarpNnz entries: one warp per row of A.  The row's
+// columns and G sit in shared memory, so a product's G(i,j) is a binary
+// search there instead of one through L2 (each step of which the product
+// would wait for); eight lanes take one entry of A at a time, four entries a
+// step, so that short B rows fill the warp without an owner search and an
+// entry's dA is one sum over eight lanes.  Two FP64 instructions a product:
+// the fused multiply-add into dA and the multiply whose sum into dB the L2
+// does.  100k rows of 256 products: 380 -> 242 us.
+constexpr int kAdjWarpNnz = 512;
+constexpr int kAdjWarpRows = 4;  // 24 KB a CTA
+
+__global__ void __launch_bounds__(32 * kAdjWarpRows) k_adjoint_warp(AdjArgs a, int32_t lo, int32_t n) {
+    __shared__ double gs[kAdjWarpRows][kAdjWarpNnz];
+    __shared__ int32_t cs[kAdjWarpRows][kAdjWarpNnz];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t item = (int64_t)blockIdx.x * kAdjWarpRows + w;
+    if (item >= n) return;
+    const int32_t row = a.order[lo + item];
     const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
-    const int64_t c0 = a.Cp[row], c1 = a.Cp[row + 1];
-    for (int32_t e = e0; e < e1; e += 32) {
-        const Chunk c = load_chunk(a.A, a.B, e, e1, lane);
-        for (int32_t t0 = 0; t0 < c.total; t0 += 32) {
-            const int32_t t = t0 + lane;
-            const int o = chunk_owner(c, t);
-            const int32_t incl_o = __shfl_sync(FULL, c.incl, o);
-            const int32_t len_o = __shfl_sync(FULL, c.len, o);
-            const int32_t bs_o = __shfl_sync(FULL, c.bs, o);
-            const double av = __shfl_sync(FULL, c.a, o);
-            const bool valid = t < c.total;
-            double ga = 0.0;
-            if (valid) {
-                const int32_t pos = bs_o + (t - (incl_o - len_o));
-                const int32_t k = a.B.idx[pos];
-                const int64_t q = find_col(a.Ci, c0, c1, k);
-                if (q < c1) {
-                    const double g = a.G[q];
-                    ga = __dmul_rn(g, a.B.val[pos]);
-                    if (a.dB) atomicAdd(&a.dB[pos], __dmul_rn(av, g));
-                } else {
-                    raise(a.err, DEV_COUNT_MISMATCH);
+    const int64_t c0 = a.Cp[row], nc64 = a.Cp[row + 1] - c0;
+    if (nc64 > kAdjWarpNnz) {  // not the bins' row
+        if (lane == 0) raise(a.err, DEV_COUNT_MISMATCH);
+        return;
+    }
+    const int nc = (int)nc64;
+    const double *g = gs[w];
+    const int32_t *c = cs[w];
+    for (int i = lane; i < nc; i += 32) {
+        cs[w][i] = __ldg(&a.Ci[c0 + i]);
+        gs[w][i] = __ldg(&a.G[c0 + i]);
+    }
+    __syncwarp();
+    int top = 1;
+    while (2 * top < nc) top <<= 1;
+    const int sub = lane & 7, grp = lane >> 3;
+    const unsigned gmask = 0xffu << (lane & 24);
+    for (int32_t eb = e0; eb < e1; eb += 32) {
+        int32_t bs = 0, len = 0;
+        double av = 0.0;
+        int64_t off = 0;
+        if (eb + lane < e1) {
+            if (a.prod) off = __ldg(&a.off[eb + lane]);
+            const int32_t k = __ldg(&a.A.idx[eb + lane]);
+            bs = __ldg(&a.B.ptr[k]);
+            len = __ldg(&a.B.ptr[k + 1]) - bs;
+            av = __ldg(&a.A.val[eb + lane]);
+        }
+        const int ne = min(32, e1 - eb);
+        for (int q = 0; q < ne; q += 4) {
+            const int32_t s = __shfl_sync(FULL, bs, q + grp), l = __shfl_sync(FULL, len, q + grp);
+            const double x = __shfl_sync(FULL, av, q + grp);
+            double *keep = nullptr;
+            if (a.prod) {
+                const int64_t o = __shfl_sync(FULL, off, q + grp);
+                if (o + l <= a.prodCap) keep = a.prod + o;
+                else raise(a.err, DEV_COUNT_MISMATCH);  // the patterns are not the forward's
+            }
+            double acc = 0.0;
+            for (int32_t i0 = sub; i0 < l; i0 += 16) {
+                // Two products a lane in flight.
+                int32_t k[2];
+                double b[2];
+                int at[2] = {0, 0};
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int32_t i = i0 + 8 * u;
+                    k[u] = i < l ? __ldg(&a.B.idx[s + i]) : -1;
+                    b[u] = i < l ? __ldg(&a.B.val[s + i]) : 0.0;
+                }
+                for (int step = top; step >= 1; step >>= 1) {
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+                        if (at[u] + step < nc && c[at[u] + step] <= k[u]) at[u] += step;
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (k[u] < 0) continue;
+                    if (nc == 0 || c[at[u]] != k[u]) {
+                        raise(a.err, DEV_COUNT_MISMATCH);
+                        continue;
+                    }
+                    const double gv = g[at[u]];
+                    acc = __fma_rn(gv, b[u], acc);
+                    if (a.dB) atomicAdd(&a.dB[s + i0 + 8 * u], __dmul_rn(x, gv));
+                    else if (keep) keep[i0 + 8 * u] = __dmul_rn(x, gv);
                 }
             }
-            // Lanes of one entry are adjacent: sum ga over each run of equal o.
-            const int key = valid ? o : -1 - lane;
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int ok = __shfl_down_sync(FULL, key, d);
-                const double og = __shfl_down_sync(FULL, ga, d);
-                if (lane + d < 32 && ok == key) ga += og;
-            }
-            const int pk = __shfl_up_sync(FULL, key, 1);
-            if (valid && (lane == 0 || pk != key)) atomicAdd(&a.dA[e + o], ga);
+            for (int d = 4; d; d >>= 1) acc += __shfl_xor_sync(gmask, acc, d, 8);
+            if (sub == 0 && q + grp < ne) a.dA[eb + q + grp] = acc;
         }
+    }
+}
+
+// Rows of more entries: persistent CTAs take rows from a counter, from the
+// heaviest bin on.  The row's entries are staged with their B rows' lengths
+// and the warps take equal contiguous shares of its products (a warp a row,
+// the form before, walked a power-law hub's half a million products alone:
+// 3.65 ms on R-MAT 2^14, 0.26 ms now, 0.30 keeping the products).  A row of C within kRankWordsMax
+// 32-column words is ranked through a bitmap and the words' first positions
+// in shared memory, two shared loads and a bit count a lookup; a wider one by
+// binary search.  Four steps of B loads, then their four loads of G, are in
+// flight together.
+// dA of an entry is summed by the lanes it falls on, in registers while the
+// warp stays on it, and stored by the warp it starts in; the parts of an
+// entry that warps further on hold are added by one thread, in warp order
+// (a fixed order either way).
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_adjoint_cta(AdjArgs a, int32_t lo, int32_t n, int maxWords) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    using L = StageLayout<THREADS>;
+    constexpr int NW = THREADS / 32;
+    __shared__ int32_t sh[NW];
+    __shared__ int32_t partEnt[NW];
+    __shared__ double partSum[NW];
+    __shared__ int32_t next;
+    int32_t *pre = reinterpret_cast<int32_t *>(smem + L::pre);
+    int32_t *bst = reinterpret_cast<int32_t *>(smem + L::bst);
+    double *av = reinterpret_cast<double *>(smem + L::av);
+    int32_t *src = reinterpret_cast<int32_t *>(smem + L::bytes);
+    uint32_t *bits = reinterpret_cast<uint32_t *>(src + THREADS);
+    int32_t *wpre = reinterpret_cast<int32_t *>(bits + maxWords);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (;;) {
+        if (tid == 0) next = (int32_t)atomicAdd(a.ctr, 1u);
+        __syncthreads();
+        const int32_t item = next;
+        if (item >= n) break;
+        const int32_t row = a.order[lo + n - 1 - item];
+        const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
+        const int64_t c0 = a.Cp[row], c1 = a.Cp[row + 1];
+        const int32_t w0 = c1 > c0 ? a.Ci[c0] >> 5 : 0;
+        const int words = c1 > c0 ? (a.Ci[c1 - 1] >> 5) - w0 + 1 : 0;
+        const bool ranked = words <= maxWords;
+        if (ranked) {
+            for (int i = tid; i < words; i += THREADS) bits[i] = 0u;
+            __syncthreads();
+            for (int64_t i = c0 + tid; i < c1; i += THREADS) {
+                const int32_t c = __ldg(&a.Ci[i]);
+                const int32_t before = i > c0 ? __ldg(&a.Ci[i - 1]) : -1;
+                const int w = (c >> 5) - w0;
+                atomicOr(&bits[w], 1u << (c & 31));
+                if (before < 0 || (before >> 5) != (c >> 5)) wpre[w] = (int32_t)(i - c0);
+            }
+        }
+        // Position of column c in C's row, or -1.
+        auto find = [&](int32_t c) -> int64_t {
+            if (ranked) {
+                const uint32_t w = (uint32_t)((c >> 5) - w0);
+                if (w >= (uint32_t)words) return -1;
+                const uint32_t word = bits[w], bit = 1u << (c & 31);
+                return word & bit ? c0 + wpre[w] + __popc(word & (bit - 1u)) : -1;
+            }
+            const int64_t q = find_col(a.Ci, c0, c1, c);
+            return q < c1 ? q : -1;
+        };
+        for (int32_t eb = e0; eb < e1; eb += THREADS) {
+            int nb;
+            const int32_t total = stage_entries<THREADS, true>(a.A, a.B, eb, min(THREADS, e1 - eb), pre, bst, av, &nb,
+                                                               sh, false, 0, 0, nullptr, false, src);
+            int32_t tb, te;
+            warp_share<THREADS>(total, &tb, &te);
+            if (lane == 0) partEnt[warp] = -1;
+            // The batch's products follow each other in the kept array.
+            double *keep = nullptr;
+            if (a.prod) {
+                const int64_t o = a.off[eb];
+                if (o + total <= a.prodCap) keep = a.prod + o;
+                else raise(a.err, DEV_COUNT_MISMATCH);  // the patterns are not the forward's
+            }
+            if (tb < te) {
+                RangeWalk walk(pre, bst, nb, tb);
+                int cur = walk.e0;              // the entry being summed, in acc over the lanes
+                bool later = pre[cur] < tb;     // it starts in an earlier warp
+                double acc = 0.0;
+                auto flush = [&]() {
+                    double s = acc;
+#pragma unroll
+                    for (int d = 16; d; d >>= 1) s += __shfl_xor_sync(FULL, s, d);
+                    if (lane == 0) {
+                        if (later) {
+                            partEnt[warp] = src[cur];
+                            partSum[warp] = s;
+                        } else {
+                            a.dA[src[cur]] = s;
+                        }
+                    }
+                    later = false;
+                };
+                constexpr int U = 4;
+                for (int32_t g0 = tb; g0 < te; g0 += 32 * U) {
+                    int32_t pos[U], col[U];
+                    int ent[U];
+                    bool val[U];
+                    double bv[U], gv[U];
+                    walk.template place<U>(pre, bst, nb, g0, te, pos, ent, val);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        col[u] = val[u] ? __ldg(&a.B.idx[pos[u]]) : 0;
+                        bv[u] = val[u] ? __ldg(&a.B.val[pos[u]]) : 0.0;
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int64_t q = val[u] ? find(col[u]) : -1;
+                        if (val[u] && q < 0) raise(a.err, DEV_COUNT_MISMATCH);
+                        gv[u] = q >= 0 ? __ldg(&a.G[q]) : 0.0;
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        if (val[u] && (a.dB || keep)) {
+                            const double x = __dmul_rn(av[ent[u]], gv[u]);
+                            if (a.dB) atomicAdd(&a.dB[pos[u]], x);
+                            else keep[g0 + 32 * u + lane] = x;
+                        }
+                        const int e = ent[u];
+                        if (val[u] && e == cur) acc = __fma_rn(gv[u], bv[u], acc);
+                        const unsigned other = __ballot_sync(FULL, val[u] && e != cur);
+                        if (other == 0u) continue;
+                        flush();
+                        // The valid lanes lead the step and their entries do not
+                        // decrease: the last one's entry is summed next, entries
+                        // between it and cur lie within this step.
+                        const int last = __shfl_sync(FULL, e, 31 - __clz(other));
+                        const bool mid = val[u] && e != cur && e != last;
+                        if (__any_sync(FULL, mid)) {
+                            const int key = mid ? e : -1 - lane;
+                            double p = mid ? __dmul_rn(gv[u], bv[u]) : 0.0;
+#pragma unroll
+                            for (int d = 1; d < 32; d <<= 1) {
+                                const int ok = __shfl_down_sync(FULL, key, d);
+                                const double op = __shfl_down_sync(FULL, p, d);
+                                if (lane + d < 32 && ok == key) p += op;
+                            }
+                            const int pk = __shfl_up_sync(FULL, key, 1);
+                            if (mid && (lane == 0 || pk != key)) a.dA[src[e]] = p;
+                        }
+                        acc = val[u] && e == last ? __dmul_rn(gv[u], bv[u]) : 0.0;
+                        cur = last;
+                    }
+                }
+                flush();
+            }
+            __syncthreads();
+            if (tid == 0) {
+                for (int w = 1; w < NW; ++w)
+                    if (partEnt[w] >= 0) a.dA[partEnt[w]] += partSum[w];
+            }
+            __syncthreads();
+        }
+        __syncthreads();  // every thread has read `next` before it changes
+    }
+}
+
+// Products of every A entry (the length of its B row).
+__global__ void __launch_bounds__(256) k_entry_products(CsrDev A, const int32_t *__restrict__ Bp,
+                                                        int32_t *__restrict__ len) {
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < A.nnz; e += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t k = A.idx[e];
+        len[e] = Bp[k + 1] - Bp[k];
     }
 }
 
@@ -122,9 +337,32 @@ __device__ __forceinline__ int64_t b_row_of(const CsrDev &B, int64_t f) {
     return lo;
 }
 
-// Sum of A(i,k) * G(i,j) over the entries [p, pe) of A's column grouping.
-__device__ __forceinline__ double column_sum(const AdjDbArgs &a, int32_t p, int32_t pe, int32_t j) {
+// Sum of A(i,k) * G(i,j) over the entries [p, pe) of A's column grouping, in
+// order, for entry f = (k,j) of B, the at-th of its row.  With the dA pass's
+// products kept (a.prod, entry e's from off[e] on in B's row order) a term is
+// one load, next to its neighbours' for the threads of the same row; without,
+// a binary search of C's row i, a chain of about 16 dependent loads.  R-MAT
+// 2^14 (16.8M products): 126 + 365 us in the two passes that call it with
+// the search, 16 + 74 us with the products.
+__device__ __forceinline__ double column_sum(const AdjDbArgs &a, int32_t p, int32_t pe, int32_t j, int64_t at) {
     double acc = 0.0;
+    if (a.prod) {
+        constexpr int U = 8;
+        for (; p < pe; p += U) {
+            int64_t q[U];
+            double x[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) q[u] = p + u < pe ? (int64_t)__ldg(&a.perm[p + u]) : -1;
+#pragma unroll
+            for (int u = 0; u < U; ++u) q[u] = q[u] >= 0 ? __ldg(&a.off[q[u]]) : -1;
+#pragma unroll
+            for (int u = 0; u < U; ++u) x[u] = q[u] >= 0 && q[u] + at < a.prodCap ? __ldg(&a.prod[q[u] + at]) : 0.0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (p + u < pe) acc += x[u];
+        }
+        return acc;
+    }
     for (; p < pe; ++p) {
         const uint32_t e = a.perm[p];
         const int32_t i = a.rowOf[e];
@@ -142,7 +380,7 @@ __global__ void __launch_bounds__(256) k_adjoint_db(AdjDbArgs a) {
     const int64_t k = b_row_of(a.B, f);
     const int32_t p0 = a.colPtr[k], p1 = a.colPtr[k + 1];
     const int32_t len = p1 - p0;
-    a.dB[f] = column_sum(a, p0, len > kAdjSeg ? p0 + kAdjSeg : p1, a.B.idx[f]);
+    a.dB[f] = column_sum(a, p0, len > kAdjSeg ? p0 + kAdjSeg : p1, a.B.idx[f], f - a.B.ptr[k]);
     a.extra[f] = len > kAdjSeg ? (len - 1) / kAdjSeg : 0;
 }
 
@@ -167,7 +405,7 @@ __global__ void __launch_bounds__(256) k_adjoint_db_tail(AdjDbArgs a) {
         const int64_t k = b_row_of(a.B, f);
         const int32_t p1 = a.colPtr[k + 1];
         const int64_t pb = (int64_t)a.colPtr[k] + (1 + (g - a.xStart[f])) * kAdjSeg;
-        a.part[g] = column_sum(a, (int32_t)pb, (int32_t)min((int64_t)p1, pb + kAdjSeg), a.B.idx[f]);
+        a.part[g] = column_sum(a, (int32_t)pb, (int32_t)min((int64_t)p1, pb + kAdjSeg), a.B.idx[f], f - a.B.ptr[k]);
     }
 }
 
@@ -180,6 +418,8 @@ __global__ void __launch_bounds__(256) k_adjoint_db_sum(AdjDbArgs a) {
     for (int64_t g = x0; g < x1; ++g) acc += a.part[g];
     a.dB[f] = acc;
 }
+
+constexpr int kAdjCtaThreads = 512;
 
 }  // namespace
 
@@ -195,6 +435,13 @@ void launch_adjoint_transpose(const CsrDev &A, int32_t *rowOf, uint32_t *keys0, 
     *perm = vs;
 }
 
+void launch_entry_products(const CsrDev &A, const CsrDev &B, int32_t *len, int64_t *scanPart, int64_t *off,
+                           cudaStream_t s) {
+    if (A.nnz > 0)
+        k_entry_products<<<(unsigned)std::min<int64_t>(ceil_div(A.nnz, 256), 65535), 256, 0, s>>>(A, B.ptr, len);
+    launch_row_scan(A.nnz, len, scanPart, off, s);
+}
+
 int64_t adjoint_db_part_cap(int64_t products) { return products / kAdjSeg + 1; }
 
 void launch_adjoint_db(const AdjDbArgs &a, int64_t *scanPart, int num_sms, cudaStream_t s) {
@@ -206,10 +453,32 @@ void launch_adjoint_db(const AdjDbArgs &a, int64_t *scanPart, int num_sms, cudaS
     k_adjoint_db_sum<<<grid, 256, 0, s>>>(a);
 }
 
-void launch_adjoint(const AdjArgs &a, cudaStream_t s, int *launches) {
-    if (a.nrows <= 0) return;
-    k_adjoint<<<(unsigned)ceil_div(a.nrows, 8), 256, 0, s>>>(a);
+// Dynamic shared memory of the CTA kernel for bitmaps of `words` words.
+static size_t smem_adjoint_cta(int words) {
+    return StageLayout<kAdjCtaThreads>::bytes + 4 * (size_t)kAdjCtaThreads + 8 * (size_t)words;
+}
+
+void launch_adjoint_warp(const AdjArgs &a, int32_t lo, int32_t hi, cudaStream_t s, int *launches) {
+    if (hi <= lo) return;
+    k_adjoint_warp<<<(unsigned)ceil_div(hi - lo, kAdjWarpRows), 32 * kAdjWarpRows, 0, s>>>(a, lo, hi - lo);
     ++*launches;
+}
+
+void launch_adjoint_cta(const AdjArgs &a, int32_t lo, int32_t hi, int num_sms, cudaStream_t s, int *launches) {
+    if (hi <= lo) return;
+    // A matrix of few columns needs no more bitmap than they take.
+    const int words = (int)std::min<int64_t>(kRankWordsMax, a.B.n / 32 + 2);
+    const size_t smem = smem_adjoint_cta(words);
+    const int per_sm = std::max(1, std::min(2048 / kAdjCtaThreads, (int)((227 * 1024) / (smem + 1024))));
+    const int grid = (int)std::min<int64_t>(hi - lo, (int64_t)std::max(num_sms, 1) * per_sm);
+    cudaMemsetAsync(a.ctr, 0, sizeof(uint32_t), s);
+    k_adjoint_cta<kAdjCtaThreads><<<(unsigned)grid, kAdjCtaThreads, smem, s>>>(a, lo, hi - lo, words);
+    ++*launches;
+}
+
+void init_adjoint_attributes() {
+    cudaFuncSetAttribute(k_adjoint_cta<kAdjCtaThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem_adjoint_cta(kRankWordsMax));
 }
 
 }  // namespace dbd
