@@ -79,7 +79,7 @@ struct Tuning {
     int32_t symHashSpanWords = kWideHashSpanWords;  // symbolic CTA rows hash above this span
     int32_t denseWarpWords = kDenseWarpWords; // numeric rows on one warp's dense window
     int32_t midSpanWords = 0;                 // numeric rows on one warp's rank window (off: the
-                                              // bucket-sorted warp hash measures faster)
+                                              // register-sorted warp hash measures faster)
     int32_t denseMethod = 0;                  // dense bin: 0 rank windows, 1 global slots, 2 FP64 windows,
                                               // 3 one pass into FP64 scratch rows
 };

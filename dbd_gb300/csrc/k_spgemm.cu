@@ -16,9 +16,9 @@
 //                               the union of the B rows' column runs when
 //                               each is one run); warp bitmap ranks
 //   short rows  (<= 256 nnz)    one warp per row: symbolic by a shared hash
-//                               table; numeric by expand-sort-compress for
-//                               rows of at most 256 products, else by the
-//                               table, compaction and a bucket sort
+//                               table; numeric by expand-sort-compress in
+//                               registers for rows of at most 512 products, else by the
+//                               table, compaction and a bitonic sort
 //   CTA rows                    the row's A entries staged in shared memory,
 //                               warps over consecutive products with several
 //                               B loads in flight (warp_range_ld): hash
@@ -94,6 +94,8 @@ __device__ __forceinline__ bool in_window(uint32_t rel, uint32_t limit, int *err
 constexpr int kWideLoads = 4;
 // Steps of B loads a warp-hash row keeps in flight.
 constexpr int kHashWarpLoads = 2;
+// Warp-hash rows of at most this many products are sorted instead of hashed.
+constexpr int kEscMax = 512;
 
 // Position in B of product t (all lanes call; result valid when t < total).
 __device__ __forceinline__ int32_t chunk_pos(const Chunk &c, int32_t t, double *a_out) {
@@ -309,12 +311,12 @@ constexpr int kSymTinyWarps = 4;  // 16.5 KB a CTA
 constexpr int kNumTinyWarps = 2;  // 24.8 KB a CTA
 
 // Batcher's merge exchange: the comparators of stage (P, K), then the next.
-template <int N, int P, int K>
-__device__ __forceinline__ void merge_exchange(uint32_t (&key)[N]) {
+template <int N, int P, int K, class T>
+__device__ __forceinline__ void merge_exchange(T (&key)[N]) {
 #pragma unroll
     for (int x = K % P; x < N - K; ++x) {
         if ((x - K % P) % (2 * K) < K && x / (2 * P) == (x + K) / (2 * P)) {
-            const uint32_t lo = min(key[x], key[x + K]), hi = max(key[x], key[x + K]);
+            const T lo = min(key[x], key[x + K]), hi = max(key[x], key[x + K]);
             key[x] = lo;
             key[x + K] = hi;
         }
@@ -1025,90 +1027,12 @@ __device__ __forceinline__ void group_bitonic(uint64_t *buf, int N, int gt) {
     }
 }
 
-// One warp orders n <= kBucketN packed (column << 32 | slot) entries of a
-// row whose columns lie in [lo, lo + span): a counting sort by bucket
-// (256 buckets of equal column width, each lane owning 8), then insertion
-// sort inside each bucket.  Rows of uniform columns put a few entries in
-// each bucket, so this costs a few operations per entry instead of a
-// bitonic network.  Returns false (nothing written) when a bucket holds
-// more than 32 entries (clustered columns); the caller sorts otherwise.
-constexpr int kBuckets = 256;
-__device__ __forceinline__ bool warp_bucket_order(const uint64_t *in, int n, int32_t lo, int64_t span, int *cnts,
-                                                  uint64_t *out) {
-    const int lane = threadIdx.x & 31;
-    for (int b = lane; b < kBuckets; b += 32) cnts[b] = 0;
-    __syncwarp();
-    constexpr int PER = kNumWarpMax / 32;  // entries per lane
-    uint64_t key[PER];
-    int bk[PER], rk[PER];
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-        const int i = lane + 32 * u;
-        bk[u] = -1;
-        if (i < n) {
-            key[u] = in[i];
-            const int64_t rel = (int64_t)(int32_t)(key[u] >> 32) - lo;
-            bk[u] = (int)min((int64_t)kBuckets - 1, max((int64_t)0, rel * kBuckets / span));
-            rk[u] = atomicAdd(&cnts[bk[u]], 1);
-        }
-    }
-    __syncwarp();
-    // Lane l owns buckets [8 l, 8 l + 8): counts -> starts.
-    int c8[8], mine = 0, mx = 0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        c8[q] = cnts[8 * lane + q];
-        mine += c8[q];
-        mx = max(mx, c8[q]);
-    }
-#pragma unroll
-    for (int d = 16; d; d >>= 1) mx = max(mx, __shfl_xor_sync(FULL, mx, d));
-    if (mx > 32) return false;
-    int incl = mine;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int y = __shfl_up_sync(FULL, incl, d);
-        if (lane >= d) incl += y;
-    }
-    int st = incl - mine;
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        cnts[8 * lane + q] = st;
-        st += c8[q];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < PER; ++u)
-        if (bk[u] >= 0) out[cnts[bk[u]] + rk[u]] = key[u];
-    __syncwarp();
-    // Insertion sort inside each of this lane's buckets (by column).
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int s0 = cnts[8 * lane + q], c = c8[q];
-        for (int i = 1; i < c; ++i) {
-            const uint64_t v = out[s0 + i];
-            int j = i - 1;
-            while (j >= 0 && (out[s0 + j] >> 32) > (v >> 32)) {
-                out[s0 + j + 1] = out[s0 + j];
-                --j;
-            }
-            out[s0 + j + 1] = v;
-        }
-    }
-    __syncwarp();
-    return true;
-}
-
 // Compacts the occupied slots of a (keys, vals) table into sbuf (which
 // aliases keys) as packed (column, slot) pairs, sorts them and writes the
-// row.  GROUP threads per row; all of them call.  One-warp rows pass
-// bucket buffers (cnts, bbuf) and are ordered by warp_bucket_order when
-// their columns spread evenly.
+// row.  GROUP threads per row; all of them call.
 template <int GROUP, int ROWS, int TABLE>
 __device__ __forceinline__ void table_write_sorted(const NumArgs &a, int32_t row, int32_t *keys, const double *vals,
-                                                   int *gcnt, int gt, int *cnts = nullptr,
-                                                   uint64_t *bbuf = nullptr) {
+                                                   int *gcnt, int gt) {
     constexpr int KPT = TABLE / GROUP;
     constexpr int NMAX = TABLE / 2;
     const int lane = threadIdx.x & 31;
@@ -1134,58 +1058,102 @@ __device__ __forceinline__ void table_write_sorted(const NumArgs &a, int32_t row
     const int64_t expect = a.Cp[row + 1] - a.Cp[row];
     if (gt == 0 && (n != expect || n > NMAX)) raise(a.err, DEV_COUNT_MISMATCH);
     const int nn = min(n, NMAX);
-    const uint64_t *sorted = sbuf;
-    bool done = false;
-    if constexpr (GROUP == 32 && ROWS > 1 && NMAX <= kNumWarpMax) {
-        if (cnts) {
-            const int32_t lo = a.rowLo[row];
-            const int64_t span = max((int64_t)1, (int64_t)a.rowHi[row] - lo + 1);
-            done = warp_bucket_order(sbuf, nn, lo, span, cnts, bbuf);
-            if (done) sorted = bbuf;
-        }
-    }
-    if (!done) {
-        int N = 1;
-        while (N < nn) N <<= 1;
-        for (int i = nn + gt; i < N; i += GROUP) sbuf[i] = ~0ull;
-        group_sync<GROUP, ROWS>();
-        group_bitonic<GROUP, ROWS>(sbuf, N, gt);
-    }
+    int N = 1;
+    while (N < nn) N <<= 1;
+    for (int i = nn + gt; i < N; i += GROUP) sbuf[i] = ~0ull;
+    group_sync<GROUP, ROWS>();
+    group_bitonic<GROUP, ROWS>(sbuf, N, gt);
     const int64_t obase = a.Cp[row] - a.outBase;
     const int32_t shift = col_shift(a, row);
     const int wn = (int)min((int64_t)nn, expect);
     for (int i = gt; i < wn; i += GROUP) {
-        const uint64_t v = sorted[i];
+        const uint64_t v = sbuf[i];
         a.Ci[obase + i] = (int32_t)(v >> 32) - shift;
         a.Cv[obase + i] = vals[(uint32_t)v];
     }
 }
 
-// Shared bytes per warp of the warp hash kernel: keys, values and the bucket
-// counters.  Rows of at most kNumWarpMax products (expand-sort-compress) sort
-// into the upper half of the values, which they do not use; the table path
-// sorts its compacted keys in place (bitonic).  7 KB per warp.
-constexpr size_t warp_hash_bytes(int table) { return 12 * (size_t)table + 4 * (size_t)kBuckets; }
+// Shared bytes per warp of the warp hash kernel: keys and values (which rows
+// sorted in registers use for their products).  6 KB per warp.
+constexpr size_t warp_hash_bytes(int table) { return 12 * (size_t)table; }
 
-// Warp hash rows: keys int32[TABLE] then values double[TABLE] per row.
-// A row of at most kNumWarpMax products, by one warp without a hash table
-// (expand, sort, compress): every product's column and value go to shared
-// memory, a bucket counting sort (or a bitonic sort when columns cluster)
-// orders them by column, and each run of equal columns is summed by the lane
-// holding its first entry and written at the run's rank.  pk holds
-// kNumWarpMax packed (column << 32 | product) keys, pv the products' values.
-template <int ROWS>
-__device__ __forceinline__ void esc_row(const NumArgs &a, int32_t row, int32_t e0, int32_t e1, int n, uint64_t *pk,
-                                        double *pv, int *cnts, uint64_t *bbuf) {
+// Sorts 32 R keys ascending over a warp's registers: key[r] of lane l is the
+// (R l + r)-th afterwards.  Each lane sorts its own R (merge_exchange); then
+// runs of neighbouring lanes are merged: the first step of a merge compares
+// mirrored positions, the others positions one stride apart (Batcher's
+// bitonic merge, all comparators the same way round), strides of R and more
+// by shuffles, shorter ones inside the lane.
+template <int R, class K>
+__device__ __forceinline__ void warp_sort(K (&key)[R]) {
+    const int lane = threadIdx.x & 31;
+    merge_exchange<R, 1, 1>(key);
+#pragma unroll
+    for (int m = 2; m <= 32; m <<= 1) {  // runs of m lanes
+        K other[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) other[r] = __shfl_xor_sync(FULL, key[R - 1 - r], m - 1);
+        const bool low = (lane & (m >> 1)) == 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) key[r] = low ? min(key[r], other[r]) : max(key[r], other[r]);
+#pragma unroll
+        for (int d = m >> 2; d >= 1; d >>= 1) {
+            const bool lo = (lane & d) == 0;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const K x = __shfl_xor_sync(FULL, key[r], d);
+                key[r] = lo ? min(key[r], x) : max(key[r], x);
+            }
+        }
+#pragma unroll
+        for (int d = R >> 1; d >= 1; d >>= 1) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                if ((r & d) == 0) {
+                    const K lo = min(key[r], key[r + d]), hi = max(key[r], key[r + d]);
+                    key[r] = lo;
+                    key[r + d] = hi;
+                }
+            }
+        }
+    }
+}
+
+// Where a warp keeps entry p of up to 1024 it writes R consecutive ones a lane
+// and reads 32 consecutive ones a step: rotated by p / 32 in its group of 32,
+// so that neither hits a bank more than twice.
+__device__ __forceinline__ int rotated(int p) { return (p & ~31) | ((p + (p >> 5)) & 31); }
+
+// A row of at most 32 R products by one warp without a hash table (expand,
+// sort, compress): every product's value goes to shared memory and its
+// (column, product) key is sorted in registers (warp_sort), which puts equal
+// columns next to each other in Gustavson order.  A lane sums the runs inside
+// its R keys; a run over several lanes is finished by the lane that holds its
+// first key, from the others' leading sums.  The row's entries are gathered in
+// shared memory and written 32 consecutive ones a step.
+//
+// A bucket counting sort in shared memory with each lane writing R
+// consecutive entries, the form before, was bound by the L1: 60M bank
+// conflicts and 20M store requests for 100k rows of 256 products (91% of L1
+// throughput busy): 455 -> 227 us, 550k rows of about 144 products 1611 ->
+// 1106 us.  What bounds it now is latency, at 32 warps an SM (64 registers, 6 KB
+// a warp; at 92 registers and 20 warps 272 us).  kbuf and pv
+// hold 32 R entries each; columns lie in [rlo, rlo + 2^(bits of K - log2(32 R))).
+template <int R, class K>
+__device__ __forceinline__ void esc_row(const NumArgs &a, int32_t row, int32_t e0, int32_t e1, int n, int32_t rlo,
+                                        K *kbuf, double *pv) {
+    constexpr int N = 32 * R;
+    constexpr int SHIFT = ilog2(N);
+    constexpr K NONE = ~K(0);
+    constexpr int U = R < 4 ? R : 4;  // steps of B loads in flight
     const int lane = threadIdx.x & 31;
     int32_t tb = 0;  // products of the earlier chunks
     for (int32_t e = e0; e < e1; e += 32) {
         const Chunk c = load_chunk(a.A, a.B, e, e1, lane);
-        for (int32_t t0 = 0; t0 < c.total; t0 += 32 * kHashWarpLoads) {
-            int32_t j[kHashWarpLoads];
-            double av[kHashWarpLoads];
+        for (int32_t t0 = 0; t0 < c.total; t0 += 32 * U) {
+            int32_t j[U];
+            double av[U];
 #pragma unroll
-            for (int u = 0; u < kHashWarpLoads; ++u) {
+            for (int u = 0; u < U; ++u) {
                 j[u] = -1;
                 av[u] = 0.0;
                 const int32_t t = t0 + 32 * u + lane;
@@ -1194,18 +1162,18 @@ __device__ __forceinline__ void esc_row(const NumArgs &a, int32_t row, int32_t e
                     if (t < c.total && tb + t < n) j[u] = jj;
                 }
             }
-            int32_t col[kHashWarpLoads];
-            double bv[kHashWarpLoads];
+            int32_t col[U];
+            double bv[U];
 #pragma unroll
-            for (int u = 0; u < kHashWarpLoads; ++u) {
+            for (int u = 0; u < U; ++u) {
                 col[u] = j[u] >= 0 ? __ldg(&a.B.idx[j[u]]) : 0;
                 bv[u] = j[u] >= 0 ? __ldg(&a.B.val[j[u]]) : 0.0;
             }
 #pragma unroll
-            for (int u = 0; u < kHashWarpLoads; ++u) {
+            for (int u = 0; u < U; ++u) {
                 if (j[u] >= 0) {
                     const int t = tb + t0 + 32 * u + lane;
-                    pk[t] = ((uint64_t)(uint32_t)col[u] << 32) | (uint32_t)t;
+                    kbuf[t] = (K)(uint32_t)(col[u] - rlo) << SHIFT | (K)t;
                     pv[t] = __dmul_rn(av[u], bv[u]);
                 }
             }
@@ -1213,27 +1181,48 @@ __device__ __forceinline__ void esc_row(const NumArgs &a, int32_t row, int32_t e
         tb += c.total;
     }
     __syncwarp();
-    const int32_t rlo = a.rowLo[row];
-    const int64_t span = max((int64_t)1, (int64_t)a.rowHi[row] - rlo + 1);
-    const uint64_t *sorted = bbuf;
-    if (!warp_bucket_order(pk, n, rlo, span, cnts, bbuf)) {
-        int N = 1;
-        while (N < n) N <<= 1;
-        for (int i = n + lane; i < N; i += 32) pk[i] = ~0ull;
-        __syncwarp();
-        group_bitonic<32, ROWS>(pk, N, lane);
-        sorted = pk;
-    }
-    // Lane l takes sorted entries [8 l, 8 l + 8): the first entry of each
-    // run of equal columns is a head; heads before it give its rank.
-    constexpr int PER = kNumWarpMax / 32;
-    uint32_t headMask = 0;
+    K key[R];
 #pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int i = PER * lane + q;
-        if (i < n && (i == 0 || (sorted[i] >> 32) != (sorted[i - 1] >> 32))) headMask |= 1u << q;
+    for (int r = 0; r < R; ++r) key[r] = 32 * r + lane < n ? kbuf[32 * r + lane] : NONE;
+    warp_sort<R>(key);
+    // Values, and which keys start a column's run.
+    double v[R];
+    uint32_t heads = 0;
+    const K before = __shfl_up_sync(FULL, key[R - 1], 1);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const bool valid = R * lane + r < n;
+        v[r] = valid ? pv[(int)(key[r] & (K)(N - 1))] : 0.0;
+        const K prev = r > 0 ? key[r > 0 ? r - 1 : 0] : before;
+        if (valid && ((r == 0 && lane == 0) || (key[r] >> SHIFT) != (prev >> SHIFT))) heads |= 1u << r;
     }
-    const int mine = __popc(headMask);
+    __syncwarp();
+    // Sums of the runs in this lane, each left in its last key's v: lead is
+    // the part of an earlier lane's run, the run of the last head may go on.
+    double lead = 0.0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (R * lane + r < n && !((heads >> r) & 1u)) {
+            if ((heads & ((1u << r) - 1u)) == 0u) lead += v[r];
+            else v[r] += v[r > 0 ? r - 1 : 0];
+        }
+    }
+    // Lanes whose last key's run goes on take the following lanes' leads.
+    const bool leads = R * lane < n && !(heads & 1u);  // this lane starts inside a run
+    const unsigned goOn = __ballot_sync(FULL, leads);
+    const unsigned bare = __ballot_sync(FULL, heads == 0u);
+    double more = 0.0;
+    bool open = heads != 0u && lane < 31 && ((goOn >> (lane + 1)) & 1u);
+    const bool goesOn = open;
+    for (int d = 1; __any_sync(FULL, open); ++d) {
+        const double x = __shfl_down_sync(FULL, lead, d);
+        if (open) {
+            more += x;
+            open = lane + d < 31 && ((bare >> (lane + d)) & 1u) && ((goOn >> (lane + d + 1)) & 1u);
+        }
+    }
+    // Ranks, then the row gathered in order.
+    const int mine = __popc(heads);
     int incl = mine;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -1241,21 +1230,27 @@ __device__ __forceinline__ void esc_row(const NumArgs &a, int32_t row, int32_t e
         if (lane >= d) incl += y;
     }
     const int total = __shfl_sync(FULL, incl, 31);
+    const int64_t obase = a.Cp[row] - a.outBase;
     const int64_t expect = a.Cp[row + 1] - a.Cp[row];
     if (lane == 0 && total != expect) raise(a.err, DEV_COUNT_MISMATCH);
-    const int64_t obase = a.Cp[row] - a.outBase;
-    const int32_t shift = col_shift(a, row);
-    int64_t pos = incl - mine;
-    for (uint32_t m = headMask; m; m &= m - 1u) {
-        const int i = PER * lane + __ffs(m) - 1;
-        const uint64_t k0 = sorted[i];
-        double sum = pv[(uint32_t)k0];
-        for (int jx = i + 1; jx < n && (sorted[jx] >> 32) == (k0 >> 32); ++jx) sum = __dadd_rn(sum, pv[(uint32_t)sorted[jx]]);
-        if (pos < expect) {
-            a.Ci[obase + pos] = (int32_t)(k0 >> 32) - shift;
-            a.Cv[obase + pos] = sum;
+    int32_t *cbuf = reinterpret_cast<int32_t *>(kbuf);
+    int p = incl - mine;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if ((heads >> r) & 1u) cbuf[rotated(p++)] = (int32_t)(key[r] >> SHIFT);
+        // The run's last key in this lane: the next one is a head or there is none.
+        const bool ends = R * lane + r < n && (r == R - 1 || R * lane + r + 1 >= n || ((heads >> (r + 1)) & 1u));
+        if (ends && (heads & ((2u << r) - 1u))) {
+            if (goesOn && p == incl) v[r] += more;
+            pv[rotated(p - 1)] = v[r];
         }
-        ++pos;
+    }
+    __syncwarp();
+    const int32_t shift = col_shift(a, row) - rlo;
+    const int wn = (int)min((int64_t)total, expect);
+    for (int i = lane; i < wn; i += 32) {
+        a.Ci[obase + i] = cbuf[rotated(i)] - shift;
+        a.Cv[obase + i] = pv[rotated(i)];
     }
 }
 
@@ -1269,13 +1264,33 @@ __device__ __forceinline__ void num_hash_warp_rows(const NumArgs &a, int32_t lo,
     unsigned char *base_ptr = smem + (size_t)g * warp_hash_bytes(TABLE);
     int32_t *keys = reinterpret_cast<int32_t *>(base_ptr);
     double *vals = reinterpret_cast<double *>(base_ptr + 4 * (size_t)TABLE);
-    int *cnts = reinterpret_cast<int *>(base_ptr + 12 * (size_t)TABLE);
     const int32_t row = a.list[lo + item];
     const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
-    if (a.rowP[row] <= kNumWarpMax && TABLE >= 2 * kNumWarpMax) {
-        esc_row<ROWS>(a, row, e0, e1, (int)a.rowP[row], reinterpret_cast<uint64_t *>(keys), vals, cnts,
-                      reinterpret_cast<uint64_t *>(vals + kNumWarpMax));
-        return;
+    // Expand-sort-compress where the products fit the registers and the
+    // columns the keys; the table takes the others.
+    static_assert(TABLE >= kEscMax, "the table's arrays hold the products");
+    const int64_t P = a.rowP[row];
+    if (P <= kEscMax) {
+        const int32_t rlo = a.rowLo[row];
+        const int64_t span = (int64_t)a.rowHi[row] - rlo + 1;
+        uint32_t *kb = reinterpret_cast<uint32_t *>(keys);
+        if (P <= 128 && span < (1 << 25)) {
+            esc_row<4, uint32_t>(a, row, e0, e1, (int)P, rlo, kb, vals);
+            return;
+        }
+        if (P <= 256 && span < (1 << 24)) {
+            esc_row<8, uint32_t>(a, row, e0, e1, (int)P, rlo, kb, vals);
+            return;
+        }
+        if (P <= 256) {
+            esc_row<8, unsigned long long>(a, row, e0, e1, (int)P, rlo, reinterpret_cast<unsigned long long *>(keys),
+                                           vals);
+            return;
+        }
+        if (span < (1 << 23)) {
+            esc_row<16, uint32_t>(a, row, e0, e1, (int)P, rlo, kb, vals);
+            return;
+        }
     }
     for (int i = lane; i < TABLE; i += 32) {
         keys[i] = EMPTY;
@@ -1319,14 +1334,14 @@ __device__ __forceinline__ void num_hash_warp_rows(const NumArgs &a, int32_t lo,
 }
 
 template <int ROWS, int TABLE>
-__global__ void __launch_bounds__(32 * ROWS) k_num_hash_warp(NumArgs a, int32_t lo, int32_t count) {
+__global__ void __launch_bounds__(32 * ROWS, 8) k_num_hash_warp(NumArgs a, int32_t lo, int32_t count) {
     num_hash_warp_rows<ROWS, TABLE>(a, lo, count, blockIdx.x);
 }
 
 // The same rows launched device-driven: the bin's rows from the bin table
 // on the device, covered by a grid-stride loop.
 template <int ROWS, int TABLE>
-__global__ void __launch_bounds__(32 * ROWS) k_num_hash_warp_dd(NumArgs a, int bin) {
+__global__ void __launch_bounds__(32 * ROWS, 8) k_num_hash_warp_dd(NumArgs a, int bin) {
     const int32_t lo = a.binStart[bin], count = a.binStart[bin + 1] - lo;
     for (int64_t vb = blockIdx.x; vb * ROWS < count; vb += gridDim.x) {
         num_hash_warp_rows<ROWS, TABLE>(a, lo, count, vb);
