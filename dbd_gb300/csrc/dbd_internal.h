@@ -146,6 +146,31 @@ struct Binning {
     int32_t *binStart = nullptr;// kMaxBins + 1
 };
 
+// Control words of a multiply on the device, one block so that one memset
+// clears them: flags of A (0-3) and of B (4-7) -- row_ptr malformed, a column
+// out of range, entries not ascending; 3: a batch's output over its capacity,
+// 7: a batch's malformed pair -- then the error word and the counters.
+enum CtlWord : int {
+    CTL_A = 0, CTL_OVER = 3, CTL_B = 4, CTL_PAIR = 7, CTL_ERR = 8, CTL_CTR = 16, CTL_COUNT = CTL_CTR + CTR_COUNT
+};
+
+// What a pass's last kernel leaves for the host in pinned memory (no copies:
+// the host reads it once the stream has been waited for).
+struct Mailbox {
+    int32_t flags[8];
+    int32_t err, heavy;
+    int64_t nnz;
+    int32_t binStart[kMaxBins + 1];
+    int64_t blockP[1];  // as many as the multiply has row blocks
+};
+// Where it comes from (to null: nothing is left).
+struct Mail {
+    Mailbox *to = nullptr;
+    const int32_t *ctl = nullptr;       // control words
+    const int32_t *binStart = nullptr;
+    const int64_t *nnz = nullptr;       // C's size (null: before the symbolic pass)
+};
+
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline int64_t tile_count(int64_t m) { return ceil_div(m, kTileRows); }
 
@@ -158,16 +183,19 @@ void launch_check_operand(const CsrDev &M, int2 *range, int *badPtr, int *badIdx
                           int num_sms);
 // Replaces them by the smallest and largest column when *unsorted is not 0.
 void launch_row_minmax(const CsrDev &B, int2 *range, const int *unsorted, cudaStream_t s, int num_sms);
+// ctl (may be null): control words; with an operand's check failed every row is
+// left empty and neither operand is read.
 void launch_row_products(const CsrDev &A, const int32_t *Bp, const int2 *range, const RowInfo &ri, uint8_t *symBin,
-                         int *err, const Tuning &t, cudaStream_t s, int num_sms);
+                         int *err, const int32_t *ctl, const Tuning &t, cudaStream_t s, int num_sms);
 // Row lists of the symbolic bins and (blockP not null) the products of every
-// rows_per_block rows; tileSum: tile_count(m) + 1 int64 of scratch.
-void launch_sym_lists(int64_t m, const Binning &b, const RowInfo &ri, int64_t *tileSum, int64_t rows_per_block,
-                      int64_t *blockP, cudaStream_t s);
+// rows_per_block rows; empty rows' entry counts are cleared.  tileSum:
+// tile_count(m) + 1 int64 of scratch.
+void launch_sym_lists(int64_t m, const Binning &b, const RowInfo &ri, int32_t *rowNnz, int64_t *tileSum,
+                      int64_t rows_per_block, int64_t *blockP, const Mail &mail, cudaStream_t s);
 // Numeric bins, their row lists and C's row pointers (m + 1) from the rows'
 // entry counts.
 void launch_num_lists(int64_t m, const Binning &b, const RowInfo &ri, const int32_t *Ap, const int32_t *rowNnz,
-                      const Tuning &t, int64_t *tileSum, int64_t *Cp, cudaStream_t s);
+                      const Tuning &t, int64_t *tileSum, int64_t *Cp, const Mail &mail, cudaStream_t s);
 // cnt (m int32) -> exclusive int64 scan Cp (m + 1); part: ceil(m / kScanTile) + 1 int64 of scratch.
 void launch_row_scan(int64_t m, const int32_t *cnt, int64_t *part, int64_t *Cp, cudaStream_t s);
 

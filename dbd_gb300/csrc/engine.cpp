@@ -102,6 +102,7 @@ struct Operand {
     DevBuf ptr, idx, val, tmp;
     DevBuf range;  // first and last column of every row (as the right operand)
     bool loaded = false;
+    bool pending = false;  // checked on the device, the result not read yet (judge_operands)
     int sorted = 0;
 };
 
@@ -133,10 +134,11 @@ struct dbd_ctx {
 
     // work arrays
     DevBuf rowP, symBin, numBin, rowNnz, symList, numList, hist, symTileOff, numTileOff, symStart,
-        numStart, part, Cp, cursor, err, blockP, flags;
+        numStart, part, Cp, cursor;
+    DevBuf ctl;              // control words (CtlWord), allocated once
+    HostBuf mailBuf;         // Mailbox: what the host reads back of a pass
     DevBuf Ci, Cv;           // resident product or device output ring
     DevBuf Cf;               // float32 values of each device slot (out_val_fp32 in the copying scopes)
-    DevBuf ctrs;             // row counters of the persistent kernels
     DevBuf gdense;           // global dense slots of the dense bin
     int gSlots = 0;
     int64_t gStride = 0;
@@ -233,6 +235,20 @@ struct dbd_ctx {
         cudaEventRecord(e, s);
         return e;
     }
+    int *flags() const { return ctl.as<int>(); }
+    int *err() const { return ctl.as<int>() + CTL_ERR; }
+    uint32_t *ctrs() const { return ctl.as<uint32_t>() + CTL_CTR; }
+    Mailbox *mail() const { return mailBuf.as<Mailbox>(); }
+    // Timing events of a multiply's chunks, kept between multiplies.
+    std::vector<cudaEvent_t> cpool;
+    cudaEvent_t chunk_ev(size_t i) {
+        while (cpool.size() <= i) {
+            cudaEvent_t e = nullptr;
+            cudaEventCreate(&e);
+            cpool.push_back(e);
+        }
+        return cpool[i];
+    }
     cudaEvent_t sync_ev() {
         if (sused == spool.size()) {
             cudaEvent_t e;
@@ -302,19 +318,22 @@ int cuda_fail(dbd_ctx *c, cudaError_t e, const char *what) {
         if (_e != cudaSuccess) return cuda_fail((ctx), _e, #call);  \
     } while (0)
 
+// The error word as a status.
+int device_err(dbd_ctx *c, int h, const char *stage) {
+    if (h == DEV_OK) return DBD_OK;
+    const char *what = h == DEV_TABLE_FULL       ? "hash table full"
+                       : h == DEV_COUNT_MISMATCH ? "numeric/symbolic count mismatch"
+                       : h == DEV_ROW_TOO_LONG   ? "a row has more than 2^31 products"
+                       : h == DEV_OUT_OF_WINDOW  ? "a column lies outside its row's window (B changed after loading?)"
+                                                 : "unknown";
+    return set_err(c, DBD_ERR_DEVICE_CHECK, std::string(stage) + ": device check failed: " + what);
+}
+
+// Waits for the stream and reads the error word.
 int check_device_err(dbd_ctx *c, const char *stage) {
-    int h = 0;
-    CK(c, cudaMemcpyAsync(&h, c->err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(c, cudaMemcpyAsync(&c->mail()->err, c->err(), sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    if (h != DEV_OK) {
-        const char *what = h == DEV_TABLE_FULL       ? "hash table full"
-                           : h == DEV_COUNT_MISMATCH ? "numeric/symbolic count mismatch"
-                           : h == DEV_ROW_TOO_LONG   ? "a row has more than 2^31 products"
-                           : h == DEV_OUT_OF_WINDOW  ? "a column lies outside its row's window (B changed after loading?)"
-                                                     : "unknown";
-        return set_err(c, DBD_ERR_DEVICE_CHECK, std::string(stage) + ": device check failed: " + what);
-    }
-    return DBD_OK;
+    return device_err(c, c->mail()->err, stage);
 }
 
 // Host-side validation of a host CSR operand (O(n + nnz)).
@@ -336,12 +355,12 @@ int validate_host(dbd_ctx *c, const dbd_csr_view *v, const char *name) {
     return DBD_OK;
 }
 
-int finish_operand(dbd_ctx *c, Operand &op, const CsrDev &d, const char *name);
+int check_operand(dbd_ctx *c, Operand &op, const CsrDev &d);
 
 int load_operand(dbd_ctx *c, Operand &op, const dbd_csr_view *v, const char *name) {
     int rc = validate_host(c, v, name);
     if (rc) return rc;
-    op.loaded = false;
+    op.loaded = op.pending = false;
     c->batchCount = 0;
     c->replayOk = false;  // operand buffers may move: the captured numeric graph is stale
     drop_graph(c);
@@ -378,30 +397,84 @@ int load_operand(dbd_ctx *c, Operand &op, const dbd_csr_view *v, const char *nam
         d.idx = op.idx.as<int32_t>();
         d.val = op.val.as<double>();
     }
-    return finish_operand(c, op, d, name);
+    return check_operand(c, op, d);
 }
 
-// Checks of an operand now on the device (row_ptr spanning [0, nnz] and
-// every column in range before anything reads through them), the first and
-// last column of every row (the column windows of the products' rows) and
-// whether every row ascends strictly (cursors, plain accumulation, runs).
-int finish_operand(dbd_ctx *c, Operand &op, const CsrDev &d, const char *name) {
+// Enqueues the checks of an operand now on the device (row_ptr spanning
+// [0, nnz], every column in range), the first and last column of every row
+// (the column windows of the products' rows) and whether every row ascends
+// strictly (cursors, plain accumulation, runs).  The operand's flags are
+// zero.  Nothing reads through the operand before judge_operands but kernels
+// that look at the flags themselves, so a multiply waits for its operands'
+// checks and its work estimate once.
+int check_operand(dbd_ctx *c, Operand &op, const CsrDev &d) {
     op.dev = d;
-    CK(c, c->flags.ensure(4 * sizeof(int)));
-    int *flags = c->flags.as<int>();
-    CK(c, cudaMemsetAsync(flags, 0, 3 * sizeof(int), c->stream));
+    int *flags = c->flags() + (&op == &c->B ? CTL_B : CTL_A);
     CK(c, op.range.ensure(sizeof(int2) * (size_t)std::max<int64_t>(d.m, 1)));
     launch_check_operand(d, op.range.as<int2>(), flags, flags + 1, flags + 2, c->stream, c->num_sms);
-    int hf[3] = {0, 0, 0};
-    CK(c, cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
-    if (hf[0]) return set_err(c, DBD_ERR_INVALID, std::string(name) + ": malformed row_ptr");
-    if (hf[1]) return set_err(c, DBD_ERR_INVALID, std::string(name) + ": column index out of range");
-    op.sorted = hf[2] ? 0 : 1;
-    if (!op.sorted)
+    if (&op == &c->B || c->b_is_a)  // the right operand
         launch_row_minmax(d, op.range.as<int2>(), flags + 2, c->stream, c->num_sms);
-    op.loaded = true;
+    CK(c, cudaGetLastError());
+    op.loaded = op.pending = true;
     c->divided = false;
+    return DBD_OK;
+}
+
+int settle_operands(dbd_ctx *c);
+
+// Clears the control words (flags of both operands, error word, counters).
+int clear_ctl(dbd_ctx *c) {
+    CK(c, cudaMemsetAsync(c->ctl.p, 0, sizeof(int32_t) * CTL_COUNT, c->stream));
+    return DBD_OK;
+}
+
+// The pending checks' results, from flags the host has read.
+int judge_operands(dbd_ctx *c, const int32_t *flags) {
+    int rc = DBD_OK;
+    if (const int32_t bad = flags[CTL_PAIR])
+        rc = set_err(c, DBD_ERR_INVALID, (bad & 1) ? "a pair's row_ptr does not span [0, nnz] monotonically"
+                                                   : "a pair's column index is out of range");
+    for (Operand *op : {&c->A, &c->B}) {
+        if (!op->pending) continue;
+        op->pending = false;
+        const bool isB = op == &c->B;
+        const int32_t *f = flags + (isB ? CTL_B : CTL_A);
+        op->sorted = f[2] ? 0 : 1;
+        if (flags[CTL_PAIR]) op->loaded = false;
+        if (f[0] || f[1]) {
+            op->loaded = false;
+            if (!rc)
+                rc = set_err(c, DBD_ERR_INVALID, std::string(isB ? "B: " : "A: ") +
+                                                     (f[0] ? "malformed row_ptr" : "column index out of range"));
+        }
+    }
+    return rc;
+}
+
+// Waits for the pending checks.
+int settle_operands(dbd_ctx *c) {
+    if (!c->A.pending && !c->B.pending) return DBD_OK;
+    CK(c, cudaMemcpyAsync(c->mail()->flags, c->flags(), sizeof(c->mail()->flags), cudaMemcpyDeviceToHost, c->stream));
+    CK(c, cudaStreamSynchronize(c->stream));
+    return judge_operands(c, c->mail()->flags);
+}
+
+// Loads A and B (null: A again), their checks pending.  A fault of A's is
+// reported ahead of one of B's.
+int load_pair(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b) {
+    c->A.pending = c->B.pending = false;
+    c->b_is_a = b == nullptr;
+    int rc = clear_ctl(c);
+    if (!rc) rc = load_operand(c, c->A, a, "A");
+    if (rc) return rc;
+    if (b) {
+        rc = load_operand(c, c->B, b, "B");
+        if (rc) {
+            const std::string msg = c->last_error;
+            const int ra = settle_operands(c);
+            return ra ? ra : set_err(c, rc, msg);
+        }
+    }
     return DBD_OK;
 }
 
@@ -415,7 +488,10 @@ int divide_blocks(dbd_ctx *c) {
         return set_err(c, DBD_ERR_INVALID, "load A and B before dividing blocks");
     const CsrDev &A = c->A.dev;
     const CsrDev &B = opB(c);
-    if (A.n != B.m) return set_err(c, DBD_ERR_INVALID, "inner dimensions differ (A.n_cols != B.n_rows)");
+    if (A.n != B.m) {
+        const int rc = settle_operands(c);
+        return rc ? rc : set_err(c, DBD_ERR_INVALID, "inner dimensions differ (A.n_cols != B.n_rows)");
+    }
     const auto t0 = Clock::now();
     drop_graph(c);  // the plan it replays is replaced
     c->patternOk = false;  // so are the arrays an adjoint would read the last product's rows from
@@ -446,28 +522,32 @@ int divide_blocks(dbd_ctx *c) {
     CK(c, c->part.ensure(sizeof(int64_t) * (nt + 1)));
     CK(c, c->Cp.ensure(sizeof(int64_t) * (mm + 1)));
     CK(c, c->cursor.ensure(2 * sizeof(int32_t) * (size_t)std::max<int64_t>(A.nnz, 1)));
-    CK(c, c->err.ensure(sizeof(int)));
-    CK(c, c->blockP.ensure(sizeof(int64_t) * (size_t)std::max<int64_t>(c->nblocks, 1)));
+    CK(c, c->mailBuf.ensure(sizeof(Mailbox) + sizeof(int64_t) * (size_t)c->nblocks));
 
     CK(c, cudaEventRecord(c->evStart, c->stream));
-    CK(c, cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream));
+    // The error word and the counters; the flags may hold pending checks.
+    CK(c, cudaMemsetAsync(c->err(), 0, sizeof(int32_t) * (CTL_COUNT - CTL_ERR), c->stream));
     const Operand &opb = c->b_is_a ? c->A : c->B;
-    launch_row_products(A, B.ptr, opb.range.as<int2>(), row_info(c), c->symBin.as<uint8_t>(), c->err.as<int>(),
-                        c->tune, c->stream, c->num_sms);
+    launch_row_products(A, B.ptr, opb.range.as<int2>(), row_info(c), c->symBin.as<uint8_t>(), c->err(),
+                        c->flags(), c->tune, c->stream, c->num_sms);
     Binning sb{c->symBin.as<uint8_t>(), c->symList.as<int32_t>(), c->hist.as<int32_t>(),
                c->symTileOff.as<int32_t>(), c->symStart.as<int32_t>()};
-    launch_sym_lists(m, sb, row_info(c), c->part.as<int64_t>(), rpb, c->blockP.as<int64_t>(), c->stream);
+    Mail mail;
+    mail.to = c->mail();
+    mail.ctl = c->flags();
+    mail.binStart = c->symStart.as<int32_t>();
+    launch_sym_lists(m, sb, row_info(c), c->rowNnz.as<int32_t>(), c->part.as<int64_t>(), rpb, c->mail()->blockP, mail,
+                     c->stream);
     c->launches += 4;
     CK(c, cudaGetLastError());
-    c->blockP_h.assign((size_t)c->nblocks, 0);
-    if (c->nblocks)
-        CK(c, cudaMemcpyAsync(c->blockP_h.data(), c->blockP.p, sizeof(int64_t) * (size_t)c->nblocks,
-                              cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaMemcpyAsync(c->symStart_h, c->symStart.p, sizeof(c->symStart_h), cudaMemcpyDeviceToHost,
-                          c->stream));
     CK(c, cudaEventRecord(c->evPre, c->stream));
-    int rc = check_device_err(c, "work estimate");
+    CK(c, cudaStreamSynchronize(c->stream));
+    int rc = judge_operands(c, c->mail()->flags);
     if (rc) return rc;
+    rc = device_err(c, c->mail()->err, "work estimate");
+    if (rc) return rc;
+    memcpy(c->symStart_h, c->mail()->binStart, sizeof(c->symStart_h));
+    c->blockP_h.assign(c->mail()->blockP, c->mail()->blockP + c->nblocks);
 
     // Segmenter + categoriser on the per-block products (host, O(blocks)).
     int64_t total = 0, mx = 0;
@@ -511,19 +591,16 @@ int divide_blocks(dbd_ctx *c) {
 
 int symbolic(dbd_ctx *c) {
     const int64_t m = c->m;
-    CK(c, cudaMemsetAsync(c->rowNnz.p, 0, sizeof(int32_t) * (size_t)std::max<int64_t>(m, 1), c->stream));
     SymArgs sa;
     sa.A = c->A.dev;
     sa.B = opB(c);
     sa.list = c->symList.as<int32_t>();
     sa.binStart = c->symStart.as<int32_t>();
     sa.rowNnz = c->rowNnz.as<int32_t>();
-    CK(c, c->ctrs.ensure(sizeof(uint32_t) * CTR_COUNT));
-    CK(c, cudaMemsetAsync(c->ctrs.p, 0, sizeof(uint32_t) * CTR_COUNT, c->stream));
-    sa.ctr = c->ctrs.as<uint32_t>();
+    sa.ctr = c->ctrs();
     sa.numSms = c->num_sms;
     sa.bSorted = opB_sorted(c);
-    sa.err = c->err.as<int>();
+    sa.err = c->err();
     sa.rowLo = c->rowLo.as<int32_t>();
     sa.rowP = c->rowP.as<int64_t>();
     sa.rowHi = c->rowHi.as<int32_t>();
@@ -536,7 +613,6 @@ int symbolic(dbd_ctx *c) {
         const int64_t cap = std::min<int64_t>({m, c->products / kHeavyP, 262144});
         CK(c, c->heavySlot.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(m, 1)));
         CK(c, c->slabCnt.ensure(sizeof(int32_t) * (size_t)kMaxSlabs * (size_t)cap));
-        CK(c, cudaMemsetAsync(c->heavySlot.p, 0xff, sizeof(int32_t) * (size_t)std::max<int64_t>(m, 1), c->stream));
         sa.heavySlot = c->heavySlot.as<int32_t>();
         sa.slabCnt = c->slabCnt.as<int32_t>();
         sa.heavyCap = (int)cap;
@@ -572,23 +648,23 @@ int symbolic(dbd_ctx *c) {
     cudaEvent_t es = c->time_ev(c->stream);
     Binning nb{c->numBin.as<uint8_t>(), c->numList.as<int32_t>(), c->hist.as<int32_t>(),
                c->numTileOff.as<int32_t>(), c->numStart.as<int32_t>()};
+    Mail mail;
+    mail.to = c->mail();
+    mail.ctl = c->flags();
+    mail.binStart = c->numStart.as<int32_t>();
+    mail.nnz = c->Cp.as<int64_t>() + m;
     launch_num_lists(m, nb, row_info(c), c->A.dev.ptr, c->rowNnz.as<int32_t>(), c->tune, c->part.as<int64_t>(),
-                     c->Cp.as<int64_t>(), c->stream);
+                     c->Cp.as<int64_t>(), mail, c->stream);
     if (es) c->timed.push_back({2, 0, es, c->time_ev(c->stream)});
     c->launches += 3;
     CK(c, cudaGetLastError());
-    CK(c, cudaMemcpyAsync(&c->nnzC, c->Cp.as<int64_t>() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaMemcpyAsync(c->numStart_h, c->numStart.p, sizeof(c->numStart_h), cudaMemcpyDeviceToHost, c->stream));
-    uint32_t heavy = 0;
-    if (c->heavyCap > 0)
-        CK(c, cudaMemcpyAsync(&heavy, c->ctrs.as<uint32_t>() + CTR_HEAVY, sizeof(heavy), cudaMemcpyDeviceToHost,
-                              c->stream));
-    c->numTileOff_h.assign((size_t)kMaxBins * (size_t)(c->ntiles + 1), 0);
-    CK(c, cudaMemcpyAsync(c->numTileOff_h.data(), c->numTileOff.p, sizeof(int32_t) * c->numTileOff_h.size(),
-                          cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaEventRecord(c->evSym, c->stream));
-    int rc = check_device_err(c, "symbolic");
+    CK(c, cudaStreamSynchronize(c->stream));
+    int rc = device_err(c, c->mail()->err, "symbolic");
     if (rc) return rc;
+    c->nnzC = c->mail()->nnz;
+    memcpy(c->numStart_h, c->mail()->binStart, sizeof(c->numStart_h));
+    const uint32_t heavy = c->heavyCap > 0 ? (uint32_t)c->mail()->heavy : 0u;
     for (int q = 0; q < NB_COUNT; ++q) c->stats.rows_per_bin[q] = c->numStart_h[q + 1] - c->numStart_h[q];
     c->stats.nnz_c = c->nnzC;
     // Dense-bin work items: one per row plus the extra pieces of heavy rows
@@ -620,13 +696,13 @@ void numeric_rows(dbd_ctx *c, int64_t r0, int64_t r1, int64_t outBase, int32_t *
     na.Cv = Cv;
     na.state = c->cursor.as<int32_t>();
     na.bSorted = opB_sorted(c);
-    na.err = c->err.as<int>();
+    na.err = c->err();
     na.rowP = c->rowP.as<int64_t>();
     na.rowLo = c->rowLo.as<int32_t>();
     na.rowHi = c->rowHi.as<int32_t>();
     na.tune = c->tune;
     na.numSms = c->num_sms;
-    na.ctr = c->ctrs.as<uint32_t>();
+    na.ctr = c->ctrs();
     if (c->gSlots > 0) {
         const size_t slot = gdense_slot_bytes(c->gStride);
         char *base = c->gdense.as<char>();
@@ -654,14 +730,15 @@ void numeric_rows(dbd_ctx *c, int64_t r0, int64_t r1, int64_t outBase, int32_t *
     if (c->batchCount > 0) na.colShift = c->rowShift.as<int32_t>();
     const int64_t t0 = r0 / kTileRows;
     const int64_t t1 = (r1 >= c->m) ? c->ntiles : r1 / kTileRows;
+    const bool whole = r0 == 0 && r1 >= c->m;  // the tiles' offsets are on the host only for chunks
     // Bins run concurrently, one stream each; heaviest first so that their
     // long CTAs start early.
     static const int order[] = {NB_DENSE, NB_RANKL, NB_HCTA_L, NB_RANKS, NB_HCTA_S,
                                 NB_HWARP, NB_RANKM, NB_RANKW, NB_DENSEW, NB_TINY};
     Fork fk(c);
     for (int b : order) {
-        const int32_t lo = c->numTileOff_h[(size_t)t0 * kMaxBins + b];
-        const int32_t hi = c->numTileOff_h[(size_t)t1 * kMaxBins + b];
+        const int32_t lo = whole ? c->numStart_h[b] : c->numTileOff_h[(size_t)t0 * kMaxBins + b];
+        const int32_t hi = whole ? c->numStart_h[b + 1] : c->numTileOff_h[(size_t)t1 * kMaxBins + b];
         if (hi <= lo) continue;
         cudaStream_t s = fk.stream(b);
         cudaEvent_t e0 = c->time_ev(s);
@@ -839,8 +916,6 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
     const int64_t m = c->m, nnz = c->nnzC;
     const double gpu_budget = c->cfg.gpu_gib * kGiB;
     const double host_budget = c->cfg.host_gib * kGiB;
-    size_t free_b = 0, total_b = 0;
-    CK(c, cudaMemGetInfo(&free_b, &total_b));
     // Device memory already held by operands and work arrays.
     const double used = (double)(c->A.ptr.cap + c->A.idx.cap + c->A.val.cap + c->B.ptr.cap + c->B.idx.cap +
                                  c->B.val.cap + c->rowP.cap + c->symBin.cap + c->numBin.cap + c->rowNnz.cap +
@@ -848,7 +923,16 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
                                  c->numTileOff.cap + c->part.cap + c->Cp.cap + c->cursor.cap +
                                  (c->gSlots ? c->gdense.cap : 0) + (c->scrSlots ? c->dscr.cap : 0) +
                                  c->wideBits.cap + c->heavySlot.cap + c->slabCnt.cap + c->items.cap);
-    const double dev_avail = std::min(gpu_budget - used, (double)free_b - 512.0 * 1024 * 1024);
+    double dev_avail = gpu_budget - used;
+    // What the device has free matters where C's arrays have yet to be
+    // allocated (asking takes 25 us).
+    const size_t held = (size_t)std::max<int64_t>(nnz, 1);
+    if (scope != DBD_SCOPE_KERNEL || 12.0 * (double)nnz > std::max(0.0, dev_avail) ||
+        c->Ci.cap < sizeof(int32_t) * held || c->Cv.cap < sizeof(double) * held) {
+        size_t free_b = 0, total_b = 0;
+        CK(c, cudaMemGetInfo(&free_b, &total_b));
+        dev_avail = std::min(dev_avail, (double)free_b - 512.0 * 1024 * 1024);
+    }
     const bool copies = scope != DBD_SCOPE_KERNEL;
     // The reference's output layout (float32 values): the copying scopes
     // round each chunk's FP64 values once on the device, so 8 bytes per
@@ -947,6 +1031,10 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
         }
         rc = plan_chunks(c, cpBlk, cap_entries, b0, chunks);
         if (rc) return rc;
+        c->numTileOff_h.resize((size_t)kMaxBins * (size_t)(c->ntiles + 1));
+        CK(c, cudaMemcpyAsync(c->numTileOff_h.data(), c->numTileOff.p, sizeof(int32_t) * c->numTileOff_h.size(),
+                              cudaMemcpyDeviceToHost, c->stream));
+        CK(c, cudaStreamSynchronize(c->stream));
     }
     c->stats.n_chunks = (int32_t)chunks.size();
     const int nslots = resident ? 1 : nslots_dev;
@@ -1067,10 +1155,10 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
     std::vector<cudaEvent_t> evNum(chunks.size()), evCopy(chunks.size()), evNum0(chunks.size()),
         evCopy0(chunks.size());
     for (size_t i = 0; i < chunks.size(); ++i) {
-        cudaEventCreate(&evNum[i]);
-        cudaEventCreate(&evCopy[i]);
-        cudaEventCreate(&evNum0[i]);
-        cudaEventCreate(&evCopy0[i]);
+        evNum[i] = c->chunk_ev(4 * i);
+        evCopy[i] = c->chunk_ev(4 * i + 1);
+        evNum0[i] = c->chunk_ev(4 * i + 2);
+        evCopy0[i] = c->chunk_ev(4 * i + 3);
     }
     double t_d2h_issue = 0.0;
     CK(c, cudaEventRecord(c->evNumA, c->stream));
@@ -1148,8 +1236,9 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
         }
     }
     CK(c, cudaEventRecord(c->evNumB, c->stream));
+    cudaMemcpyAsync(&c->mail()->err, c->err(), sizeof(int), cudaMemcpyDeviceToHost, c->stream);
     cudaError_t se = cudaStreamSynchronize(c->stream);
-    cudaError_t ce = cudaStreamSynchronize(c->copy_stream);
+    cudaError_t ce = copies ? cudaStreamSynchronize(c->copy_stream) : cudaSuccess;
     if (consume) {
         {
             std::lock_guard<std::mutex> lk(mu);
@@ -1164,10 +1253,6 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
         if (!se && cudaEventElapsedTime(&x, evNum0[i], evNum[i]) == cudaSuccess) chunks_ms += x;
         if (!se && !ce && scope != DBD_SCOPE_KERNEL && cudaEventElapsedTime(&x, evCopy0[i], evCopy[i]) == cudaSuccess)
             copy_ms += x;
-        cudaEventDestroy(evNum[i]);
-        cudaEventDestroy(evCopy[i]);
-        cudaEventDestroy(evNum0[i]);
-        cudaEventDestroy(evCopy0[i]);
     }
     cudaGetLastError();  // events of chunks that a failed loop left unrecorded
     c->stats.t_chunks_ms = chunks_ms;
@@ -1181,7 +1266,7 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
     }
     c->dgDevOk = dev_dg;
     c->dgHostOk = host_dg && !werr;
-    rc = check_device_err(c, "numeric");
+    rc = device_err(c, c->mail()->err, "numeric");
     if (rc) return rc;
     if (scope == DBD_SCOPE_IO) {
         int rc2 = werr;
@@ -1295,6 +1380,11 @@ int dbd_create(const dbd_config *cfg_in, dbd_ctx **out) {
     cudaEventCreate(&c->evNumB);
     init_kernel_attributes();
     init_adjoint_attributes();
+    if (c->ctl.ensure(sizeof(int32_t) * CTL_COUNT) != cudaSuccess ||
+        c->mailBuf.ensure(sizeof(Mailbox) + sizeof(int64_t) * 4096) != cudaSuccess) {
+        dbd_destroy(c);
+        return DBD_ERR_CUDA;
+    }
     if (cudaGetLastError() != cudaSuccess) {
         dbd_destroy(c);
         return DBD_ERR_CUDA;
@@ -1311,12 +1401,13 @@ void dbd_destroy(dbd_ctx *c) {
     for (DevBuf *b : {&c->A.ptr, &c->A.idx, &c->A.val, &c->A.tmp, &c->B.ptr, &c->B.idx, &c->B.val, &c->B.tmp,
                       &c->rowP, &c->symBin, &c->numBin, &c->rowNnz, &c->symList, &c->numList, &c->hist,
                       &c->symTileOff, &c->numTileOff, &c->symStart, &c->numStart, &c->part, &c->Cp, &c->cursor,
-                      &c->err, &c->blockP, &c->flags, &c->Ci, &c->Cv, &c->wideBits, &c->wideSlot, &c->adjG,
+                      &c->ctl, &c->Ci, &c->Cv, &c->wideBits, &c->wideSlot, &c->adjG,
                       &c->adjA, &c->adjB, &c->adjT, &c->adjProd, &c->adjOff, &c->rowLo, &c->rowHi, &c->A.range, &c->B.range,
-                      &c->ctrs, &c->gdense, &c->dgCount, &c->dgCol, &c->dgVal, &c->dgSum, &c->dgWsum,
+                      &c->gdense, &c->dgCount, &c->dgCol, &c->dgVal, &c->dgSum, &c->dgWsum,
                       &c->dgBad, &c->hashOut, &c->dscr, &c->heavySlot, &c->slabCnt,
                       &c->items})
         b->release();
+    c->mailBuf.release();
     c->hCp.release();
     c->hCi.release();
     c->hCv.release();
@@ -1328,6 +1419,7 @@ void dbd_destroy(dbd_ctx *c) {
     c->batchHost.release();
     for (cudaEvent_t e : c->tpool) cudaEventDestroy(e);
     for (cudaEvent_t e : c->spool) cudaEventDestroy(e);
+    for (cudaEvent_t e : c->cpool) cudaEventDestroy(e);
     for (int b = 0; b < kMaxBins; ++b) {
         if (c->bin_streams[b]) {
             cudaStreamSynchronize(c->bin_streams[b]);
@@ -1373,14 +1465,18 @@ int dbd_load_a(dbd_ctx *c, const dbd_csr_view *a) {
     if (!c || !a) return DBD_ERR_INVALID;
     cudaSetDevice(c->cfg.device);
     c->b_is_a = false;
-    return load_operand(c, c->A, a, "A");
+    CK(c, cudaMemsetAsync(c->flags(), 0, sizeof(int32_t) * CTL_ERR, c->stream));
+    int rc = load_operand(c, c->A, a, "A");
+    return rc ? rc : settle_operands(c);
 }
 
 int dbd_load_b(dbd_ctx *c, const dbd_csr_view *b) {
     if (!c || !b) return DBD_ERR_INVALID;
     cudaSetDevice(c->cfg.device);
     c->b_is_a = false;
-    return load_operand(c, c->B, b, "B");
+    CK(c, cudaMemsetAsync(c->flags(), 0, sizeof(int32_t) * CTL_ERR, c->stream));
+    int rc = load_operand(c, c->B, b, "B");
+    return rc ? rc : settle_operands(c);
 }
 
 int dbd_divide_blocks(dbd_ctx *c, int64_t *num_blocks) {
@@ -1505,17 +1601,13 @@ int dbd_spgemm(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b, dbd_sco
                dbd_csr_out *out, dbd_stats *st) {
     if (!c || !a) return DBD_ERR_INVALID;
     cudaSetDevice(c->cfg.device);
-    int rc = load_operand(c, c->A, a, "A");
+    int rc = load_pair(c, a, b && b != a ? b : nullptr);
     if (rc) return rc;
-    if (!b || b == a) {
-        c->b_is_a = true;
-    } else {
-        c->b_is_a = false;
-        rc = load_operand(c, c->B, b, "B");
-        if (rc) return rc;
+    rc = divide_blocks(c);  // waits for the operands' checks with its own results
+    if (rc) {
+        cudaStreamSynchronize(c->stream);  // nothing may still read the caller's arrays
+        return rc;
     }
-    rc = divide_blocks(c);
-    if (rc) return rc;
     rc = distribute(c, scope, out_dir);
     if (rc) return rc;
     if (st) *st = c->stats;
@@ -1552,13 +1644,9 @@ int dbd_spgemm_adjoint(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b,
         if (!c->patternOk) return set_err(c, DBD_ERR_BUDGET, "C's pattern does not fit the device budget");
     } else {
         // Same patterns as the last multiply: only the values may have changed.
-        rc = load_operand(c, c->A, a, "A");
+        rc = load_pair(c, a, bb == a ? nullptr : bb);
+        if (!rc) rc = settle_operands(c);
         if (rc) return rc;
-        c->b_is_a = bb == a;
-        if (!c->b_is_a) {
-            rc = load_operand(c, c->B, bb, "B");
-            if (rc) return rc;
-        }
     }
     const CsrDev &A = c->A.dev;
     const CsrDev &B = opB(c);
@@ -1577,7 +1665,7 @@ int dbd_spgemm_adjoint(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b,
     }
     if (A.nnz > 0) CK(c, cudaMemsetAsync(dA, 0, sizeof(double) * (size_t)A.nnz, c->stream));
     if (B.nnz > 0) CK(c, cudaMemsetAsync(dB, 0, sizeof(double) * (size_t)B.nnz, c->stream));
-    CK(c, cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream));
+    CK(c, cudaMemsetAsync(c->err(), 0, sizeof(int), c->stream));
     AdjArgs aa;
     aa.A = A;
     aa.B = B;
@@ -1587,8 +1675,8 @@ int dbd_spgemm_adjoint(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b,
     aa.dA = dA;
     aa.dB = det ? nullptr : dB;  // deterministic: dB by its own pass below
     aa.order = c->numList.as<int32_t>();
-    aa.ctr = c->ctrs.as<uint32_t>() + CTR_ADJOINT;
-    aa.err = c->err.as<int>();
+    aa.ctr = c->ctrs() + CTR_ADJOINT;
+    aa.err = c->err();
     int launches = 0;
     if (det && B.nnz > 0 && A.nnz > 0 && 8.0 * (double)c->products <= c->cfg.gpu_gib * kGiB / 8) {
         // The products of the dA pass are kept for the dB pass within an
@@ -1656,7 +1744,7 @@ int dbd_spgemm_adjoint(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b,
         ab.off = aa.off;
         ab.prodCap = aa.prodCap;
         ab.dB = dB;
-        ab.err = c->err.as<int>();
+        ab.err = c->err();
         ab.extra = reinterpret_cast<int32_t *>(p + oExtra);
         ab.xStart = reinterpret_cast<int64_t *>(p + oStart);
         ab.part = reinterpret_cast<double *>(p + oPart);
@@ -1773,20 +1861,15 @@ int dbd_spgemm_batched(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const d
     const int64_t *dnnzA = drow + n1, *drowB = dnnzA + n1, *dnnzB = drowB + n1;
     int64_t *dCoff = const_cast<int64_t *>(dnnzB + 2 * n1);
     CK(c, c->rowShift.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(rowA[count], 1)));
-    CK(c, c->flags.ensure(4 * sizeof(int)));
-    CK(c, cudaMemsetAsync(c->flags.p, 0, sizeof(int), c->stream));
+    rc = clear_ctl(c);
+    if (rc) return rc;
     launch_batch_gather(dpa, drow, dnnzA, count, rowA[count], nnzA[count], c->A.ptr.as<int32_t>(),
-                        c->A.idx.as<int32_t>(), c->A.val.as<double>(), c->rowShift.as<int32_t>(), c->flags.as<int>(),
+                        c->A.idx.as<int32_t>(), c->A.val.as<double>(), c->rowShift.as<int32_t>(), c->flags() + CTL_PAIR,
                         c->stream);
     if (!square)
         launch_batch_gather(dpa + count, drowB, dnnzB, count, rowB[count], nnzB[count], c->B.ptr.as<int32_t>(),
-                            c->B.idx.as<int32_t>(), c->B.val.as<double>(), nullptr, c->flags.as<int>(), c->stream);
+                            c->B.idx.as<int32_t>(), c->B.val.as<double>(), nullptr, c->flags() + CTL_PAIR, c->stream);
     CK(c, cudaGetLastError());
-    int bad = 0;
-    CK(c, cudaMemcpyAsync(&bad, c->flags.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
-    if (bad) return set_err(c, DBD_ERR_INVALID, (bad & 1) ? "a pair's row_ptr does not span [0, nnz] monotonically"
-                                                          : "a pair's column index is out of range");
     CsrDev da;
     da.m = rowA[count];
     da.n = rowB[count];
@@ -1794,9 +1877,10 @@ int dbd_spgemm_batched(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const d
     da.ptr = c->A.ptr.as<int32_t>();
     da.idx = c->A.idx.as<int32_t>();
     da.val = c->A.val.as<double>();
-    rc = finish_operand(c, c->A, da, "A");
-    if (rc) return rc;
+    c->A.pending = c->B.pending = false;
     c->b_is_a = square;
+    rc = check_operand(c, c->A, da);
+    if (rc) return rc;
     if (!square) {
         CsrDev db;
         db.m = rowB[count];
@@ -1805,14 +1889,18 @@ int dbd_spgemm_batched(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const d
         db.ptr = c->B.ptr.as<int32_t>();
         db.idx = c->B.idx.as<int32_t>();
         db.val = c->B.val.as<double>();
-        rc = finish_operand(c, c->B, db, "B");
+        rc = check_operand(c, c->B, db);
         if (rc) return rc;
     }
     c->batchCount = count;
     c->batchNnzA.assign(nnzA, nnzA + n1);
     c->batchNnzB.assign(nnzB, nnzB + n1);
-    rc = divide_blocks(c);
-    if (rc) return rc;
+    rc = divide_blocks(c);  // waits for the pairs' checks with its own results
+    if (rc) {
+        c->batchCount = 0;
+        cudaStreamSynchronize(c->stream);  // nothing may still read the pairs' arrays
+        return rc;
+    }
     rc = distribute(c, scope, nullptr);
     c->patternOk = false;  // C's columns are pair-local: no adjoint on this pattern
     if (rc) return rc;
@@ -1896,7 +1984,6 @@ int dbd_batch_plan(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const dbd_c
     if (!rc && !square) rc = sized(c->B, rowB[count], nnzB[count]);
     if (rc) return rc;
     CK(c, c->rowShift.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(m, 1)));
-    CK(c, c->flags.ensure(4 * sizeof(int)));
     CsrDev da{}, db{};
     da.m = m;
     da.n = rowB[count];
@@ -1939,8 +2026,6 @@ int dbd_batch_plan(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const dbd_c
     CK(c, c->part.ensure(sizeof(int64_t) * (nt + 1)));
     CK(c, c->Cp.ensure(sizeof(int64_t) * (mm + 1)));
     CK(c, c->cursor.ensure(2 * sizeof(int32_t) * (size_t)std::max<int64_t>(nnzA[count], 1)));
-    CK(c, c->err.ensure(sizeof(int)));
-    CK(c, c->ctrs.ensure(sizeof(uint32_t) * CTR_COUNT));
     CK(c, c->Ci.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(c_capacity, 1)));
     CK(c, c->Cv.ensure(sizeof(double) * (size_t)std::max<int64_t>(c_capacity, 1)));
     // Every kernel of the run is loaded (and every grid looked up) now, so
@@ -1976,11 +2061,8 @@ int dbd_batch_enqueue(dbd_ctx *c, void *stream) {
     const int64_t *drow = reinterpret_cast<const int64_t *>(c->batchDev.as<char>() + descBytes);
     const int64_t *dnnzA = drow + n1, *drowB = dnnzA + n1, *dnnzB = drowB + n1;
     int64_t *dCoff = const_cast<int64_t *>(dnnzB + 2 * n1);
-    int *flags = c->flags.as<int>();
-    CK(c, cudaMemsetAsync(flags, 0, 4 * sizeof(int), s));
-    CK(c, cudaMemsetAsync(c->err.p, 0, sizeof(int), s));
-    CK(c, cudaMemsetAsync(c->ctrs.p, 0, sizeof(uint32_t) * CTR_COUNT, s));
-    CK(c, cudaMemsetAsync(c->rowNnz.p, 0, sizeof(int32_t) * (size_t)std::max<int64_t>(m, 1), s));
+    int *flags = c->flags();
+    CK(c, cudaMemsetAsync(c->ctl.p, 0, sizeof(int32_t) * CTL_COUNT, s));
     // The pairs' current contents, gathered into the concatenated operands.
     launch_batch_gather(dpa, drow, dnnzA, count, m, c->A.dev.nnz, c->A.ptr.as<int32_t>(), c->A.idx.as<int32_t>(),
                         c->A.val.as<double>(), c->rowShift.as<int32_t>(), flags, s);
@@ -1994,19 +2076,19 @@ int dbd_batch_enqueue(dbd_ctx *c, void *stream) {
     int launches = 0;
     launch_check_operand(B, opb.range.as<int2>(), nullptr, nullptr, flags + 2, s, c->num_sms);
     launch_row_minmax(B, opb.range.as<int2>(), flags + 2, s, c->num_sms);
-    launch_row_products(A, B.ptr, opb.range.as<int2>(), row_info(c), c->symBin.as<uint8_t>(), c->err.as<int>(),
+    launch_row_products(A, B.ptr, opb.range.as<int2>(), row_info(c), c->symBin.as<uint8_t>(), c->err(), nullptr,
                         c->tune, s, c->num_sms);
     Binning sb{c->symBin.as<uint8_t>(), c->symList.as<int32_t>(), c->hist.as<int32_t>(), c->symTileOff.as<int32_t>(),
                c->symStart.as<int32_t>()};
-    launch_sym_lists(m, sb, row_info(c), nullptr, 0, nullptr, s);
+    launch_sym_lists(m, sb, row_info(c), c->rowNnz.as<int32_t>(), nullptr, 0, nullptr, Mail{}, s);
     SymArgs sa{};
     sa.A = A;
     sa.B = B;
     sa.list = c->symList.as<int32_t>();
     sa.binStart = c->symStart.as<int32_t>();
     sa.rowNnz = c->rowNnz.as<int32_t>();
-    sa.ctr = c->ctrs.as<uint32_t>();
-    sa.err = c->err.as<int>();
+    sa.ctr = c->ctrs();
+    sa.err = c->err();
     sa.rowLo = c->rowLo.as<int32_t>();
     sa.rowHi = c->rowHi.as<int32_t>();
     sa.rowP = c->rowP.as<int64_t>();
@@ -2026,8 +2108,8 @@ int dbd_batch_enqueue(dbd_ctx *c, void *stream) {
     Binning nb{c->numBin.as<uint8_t>(), c->numList.as<int32_t>(), c->hist.as<int32_t>(), c->numTileOff.as<int32_t>(),
                c->numStart.as<int32_t>()};
     launch_num_lists(m, nb, row_info(c), A.ptr, c->rowNnz.as<int32_t>(), c->tune, c->part.as<int64_t>(),
-                     c->Cp.as<int64_t>(), s);
-    launch_numeric_guard(c->Cp.as<int64_t>() + m, c->bpCap, c->err.as<int>(), c->numStart.as<int32_t>(), NB_COUNT,
+                     c->Cp.as<int64_t>(), Mail{}, s);
+    launch_numeric_guard(c->Cp.as<int64_t>() + m, c->bpCap, c->err(), c->numStart.as<int32_t>(), NB_COUNT,
                          flags + 3, s);
     NumArgs na{};
     na.A = A;
@@ -2041,7 +2123,7 @@ int dbd_batch_enqueue(dbd_ctx *c, void *stream) {
     na.state = c->cursor.as<int32_t>();
     na.bSorted = 0;
     na.bUnsorted = flags + 2;
-    na.err = c->err.as<int>();
+    na.err = c->err();
     na.rowP = c->rowP.as<int64_t>();
     na.rowLo = c->rowLo.as<int32_t>();
     na.rowHi = c->rowHi.as<int32_t>();
@@ -2049,7 +2131,7 @@ int dbd_batch_enqueue(dbd_ctx *c, void *stream) {
     na.tune = c->tune;
     na.tune.denseMethod = 0;
     na.numSms = c->num_sms;
-    na.ctr = c->ctrs.as<uint32_t>();
+    na.ctr = c->ctrs();
     static const int norder[] = {NB_DENSE, NB_RANKL, NB_HCTA_L, NB_RANKS, NB_HCTA_S,
                                  NB_HWARP, NB_RANKM, NB_RANKW, NB_DENSEW, NB_TINY};
     {
@@ -2077,8 +2159,8 @@ int dbd_batch_result(dbd_ctx *c, int64_t *c_row_off, int64_t *c_nnz_off, dbd_csr
     const size_t n1 = (size_t)count + 1;
     int hf[4] = {0, 0, 0, 0}, derr = 0;
     int64_t nnz = 0;
-    CK(c, cudaMemcpy(hf, c->flags.p, sizeof(hf), cudaMemcpyDeviceToHost));
-    CK(c, cudaMemcpy(&derr, c->err.p, sizeof(int), cudaMemcpyDeviceToHost));
+    CK(c, cudaMemcpy(hf, c->flags(), sizeof(hf), cudaMemcpyDeviceToHost));
+    CK(c, cudaMemcpy(&derr, c->err(), sizeof(int), cudaMemcpyDeviceToHost));
     CK(c, cudaMemcpy(&nnz, c->Cp.as<int64_t>() + m, sizeof(int64_t), cudaMemcpyDeviceToHost));
     if (hf[0]) return set_err(c, DBD_ERR_INVALID, (hf[0] & 1) ? "a pair's row_ptr does not span [0, nnz] monotonically"
                                                                : "a pair's column index is out of range");
@@ -2247,7 +2329,7 @@ int dbd_update_values(dbd_ctx *c, int64_t count, const double *const *a_val, con
         c->tused = c->sused = 0;
         CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         c->capturing = true;
-        cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream);
+        cudaMemsetAsync(c->err(), 0, sizeof(int), c->stream);
         numeric_rows(c, 0, c->m, 0, c->Ci.as<int32_t>(), c->Cv.as<double>());
         c->capturing = false;
         cudaGraph_t g = nullptr;

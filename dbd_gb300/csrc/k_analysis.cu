@@ -168,7 +168,17 @@ __device__ __forceinline__ void row_products_out(const CsrDev &A, int64_t row, i
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) k_row_products(CsrDev A, const int32_t *__restrict__ Bp,
                                                           const int2 *__restrict__ range, RowInfo ri,
-                                                          uint8_t *__restrict__ symBin, int *err, Tuning tune) {
+                                                          uint8_t *__restrict__ symBin, int *err,
+                                                          const int32_t *__restrict__ ctl, Tuning tune) {
+    if (ctl && (ctl[CTL_A] | ctl[CTL_A + 1] | ctl[CTL_B] | ctl[CTL_B + 1] | ctl[CTL_PAIR])) {
+        for (int64_t r = blockIdx.x * (int64_t)THREADS + threadIdx.x; r < A.m; r += (int64_t)gridDim.x * THREADS) {
+            ri.rowP[r] = 0;
+            ri.lo[r] = INT32_MAX;
+            ri.hi[r] = -1;
+            symBin[r] = SB_EMPTY;
+        }
+        return;
+    }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int sub = lane & 7;
     const unsigned gmask = 0xffu << (lane & 24);
@@ -290,7 +300,7 @@ enum TileMode : int { TILES_PLAIN = 0, TILES_BLOCKS, TILES_NUMERIC };
 
 __global__ void __launch_bounds__(kTileRows) k_tiles(int64_t m, int64_t ntiles, TileMode mode,
                                                      uint8_t *__restrict__ bin, int nbins, const int32_t *__restrict__ Ap,
-                                                     RowInfo ri, const int32_t *__restrict__ rowNnz, Tuning tune,
+                                                     RowInfo ri, int32_t *__restrict__ rowNnz, Tuning tune,
                                                      int32_t *__restrict__ hist, int64_t *__restrict__ tileSum) {
     __shared__ int32_t wc[kTileRows / 32][kMaxBins];
     __shared__ int64_t ws[kTileRows / 32];
@@ -306,6 +316,7 @@ __global__ void __launch_bounds__(kTileRows) k_tiles(int64_t m, int64_t ntiles, 
             x = nnz;
         } else {
             b = bin[r];
+            if (b == SB_EMPTY) rowNnz[r] = 0;  // no symbolic kernel takes it
             if (mode == TILES_BLOCKS) x = ri.rowP[r];
         }
     }
@@ -436,16 +447,26 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_scan(int64_t ntiles, Tile
 }
 
 // Stable scatter of row ids into their bin's list; with Cp also C's row
-// pointers (Cp[m] is the scan's).
+// pointers (Cp[m] is the scan's).  The first CTA leaves what the host decides
+// the next launches by in its mailbox: pageable copies of the same words cost
+// a pass 12 us each.
 __global__ void __launch_bounds__(kTileRows) k_tile_scatter(int64_t m, const uint8_t *__restrict__ bin, int nbins,
                                                             const int32_t *__restrict__ tileOff,
                                                             int32_t *__restrict__ list,
                                                             const int32_t *__restrict__ rowNnz,
                                                             const int64_t *__restrict__ tileSum,
-                                                            int64_t *__restrict__ Cp) {
+                                                            int64_t *__restrict__ Cp, Mail mail) {
     __shared__ int32_t wc[kTileRows / 32][kMaxBins];
     __shared__ int64_t ws[kTileRows / 32];
     const int64_t r = (int64_t)blockIdx.x * kTileRows + threadIdx.x;
+    if (mail.to && blockIdx.x == 0) {
+        const int t = threadIdx.x;
+        if (t < 8) mail.to->flags[t] = mail.ctl[t];
+        else if (t < 8 + kMaxBins + 1) mail.to->binStart[t - 8] = mail.binStart[t - 8];
+        else if (t == 32) mail.to->err = mail.ctl[CTL_ERR];
+        else if (t == 33) mail.to->heavy = mail.ctl[CTL_CTR + CTR_HEAVY];
+        else if (t == 34 && mail.nnz) mail.to->nnz = *mail.nnz;
+    }
     const int b = r < m ? (int)bin[r] : -1;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int rank = 0;
@@ -573,38 +594,39 @@ void launch_row_minmax(const CsrDev &B, int2 *range, const int *unsorted, cudaSt
 }
 
 void launch_row_products(const CsrDev &A, const int32_t *Bp, const int2 *range, const RowInfo &ri, uint8_t *symBin,
-                         int *err, const Tuning &t, cudaStream_t s, int num_sms) {
+                         int *err, const int32_t *ctl, const Tuning &t, cudaStream_t s, int num_sms) {
     if (A.m == 0) return;
     constexpr int threads = 256;
     const int64_t need = ceil_div(A.m * 8, threads);
     const int grid = (int)std::min<int64_t>(need, (int64_t)num_sms * 8);
-    k_row_products<threads><<<grid, threads, 0, s>>>(A, Bp, range, ri, symBin, err, t);
+    k_row_products<threads><<<grid, threads, 0, s>>>(A, Bp, range, ri, symBin, err, ctl, t);
 }
 
-void launch_sym_lists(int64_t m, const Binning &b, const RowInfo &ri, int64_t *tileSum, int64_t rows_per_block,
-                      int64_t *blockP, cudaStream_t s) {
-    const int64_t nt = ceil_div(m, kTileRows);
+void launch_sym_lists(int64_t m, const Binning &b, const RowInfo &ri, int32_t *rowNnz, int64_t *tileSum,
+                      int64_t rows_per_block, int64_t *blockP, const Mail &mail, cudaStream_t s) {
+    const int64_t nt = tile_count(m);
     const TileMode mode = blockP ? TILES_BLOCKS : TILES_PLAIN;
     if (nt > 0)
-        k_tiles<<<(unsigned)nt, kTileRows, 0, s>>>(m, nt, mode, b.bin, SB_COUNT, nullptr, ri, nullptr, Tuning{}, b.hist,
+        k_tiles<<<(unsigned)nt, kTileRows, 0, s>>>(m, nt, mode, b.bin, SB_COUNT, nullptr, ri, rowNnz, Tuning{}, b.hist,
                                                    blockP ? tileSum : nullptr);
     k_tile_scan<<<kMaxBins + 1, kScanThreads, 0, s>>>(nt, mode, SB_COUNT, b.hist, b.tileOff, b.binStart, tileSum,
                                                       std::max<int64_t>(rows_per_block / kTileRows, 1), blockP);
-    if (nt > 0)
-        k_tile_scatter<<<(unsigned)nt, kTileRows, 0, s>>>(m, b.bin, SB_COUNT, b.tileOff, b.list, nullptr, nullptr,
-                                                          nullptr);
+    if (nt > 0 || mail.to)
+        k_tile_scatter<<<(unsigned)std::max<int64_t>(nt, 1), kTileRows, 0, s>>>(m, b.bin, SB_COUNT, b.tileOff, b.list,
+                                                                               nullptr, nullptr, nullptr, mail);
 }
 
 void launch_num_lists(int64_t m, const Binning &b, const RowInfo &ri, const int32_t *Ap, const int32_t *rowNnz,
-                      const Tuning &t, int64_t *tileSum, int64_t *Cp, cudaStream_t s) {
-    const int64_t nt = ceil_div(m, kTileRows);
+                      const Tuning &t, int64_t *tileSum, int64_t *Cp, const Mail &mail, cudaStream_t s) {
+    const int64_t nt = tile_count(m);
     if (nt > 0)
-        k_tiles<<<(unsigned)nt, kTileRows, 0, s>>>(m, nt, TILES_NUMERIC, b.bin, NB_COUNT, Ap, ri, rowNnz, t, b.hist,
-                                                   tileSum);
+        k_tiles<<<(unsigned)nt, kTileRows, 0, s>>>(m, nt, TILES_NUMERIC, b.bin, NB_COUNT, Ap, ri,
+                                                   const_cast<int32_t *>(rowNnz), t, b.hist, tileSum);
     k_tile_scan<<<kMaxBins + 1, kScanThreads, 0, s>>>(nt, TILES_NUMERIC, NB_COUNT, b.hist, b.tileOff, b.binStart,
                                                       tileSum, 1, Cp + m);
-    if (nt > 0)
-        k_tile_scatter<<<(unsigned)nt, kTileRows, 0, s>>>(m, b.bin, NB_COUNT, b.tileOff, b.list, rowNnz, tileSum, Cp);
+    if (nt > 0 || mail.to)
+        k_tile_scatter<<<(unsigned)std::max<int64_t>(nt, 1), kTileRows, 0, s>>>(m, b.bin, NB_COUNT, b.tileOff, b.list,
+                                                                               rowNnz, tileSum, Cp, mail);
 }
 
 void launch_row_scan(int64_t m, const int32_t *rowNnz, int64_t *part, int64_t *Cp, cudaStream_t s) {

@@ -9,7 +9,9 @@
 // pipeline (row products, bins, row lists, per-tile offsets, row counts, scan
 // partials, dense-window cursors and next columns, the error word) is carved out of the
 // file-scope array below instead of cudaMalloc'ed, and the pipeline runs on
-// the caller's stream without creating streams or events.
+// the caller's stream without creating streams or events.  What the host reads
+// back (bin sizes, nnz(C), the error word) the kernels leave in pinned words
+// allocated by the first call on a device.
 //
 // The array is kDbdNoallocScratchBytes (32 MiB) per GPU, held by every GPU
 // that loads this library until the process exits.
@@ -31,6 +33,7 @@ constexpr int kMaxDevices = 64;
 std::mutex g_setup_mu;
 bool g_setup_done[kMaxDevices] = {};
 unsigned char *g_scratch_addr[kMaxDevices] = {};
+Mailbox *g_mail[kMaxDevices] = {};  // pinned: what a call reads back
 thread_local char g_msg[256];
 
 // Failures are reported by the return code and one stderr line.
@@ -44,9 +47,10 @@ int fail(int code, const char *msg) {
     return report(code);
 }
 
-// Device address of the scratch array on the current device (set-up once
-// per device: kernel attributes and cudaGetSymbolAddress).
-int device_scratch(int dev, unsigned char **out) {
+// Device address of the scratch array on the current device and the pinned
+// words a call reads back (set-up once per device: kernel attributes and
+// loading, cudaGetSymbolAddress, the pinned words).
+int device_scratch(int dev, unsigned char **out, Mailbox **mail) {
     if (dev < 0 || dev >= kMaxDevices) return fail(DBD_ERR_INVALID, "device ordinal out of range");
     std::lock_guard<std::mutex> lk(g_setup_mu);
     if (!g_setup_done[dev]) {
@@ -65,10 +69,18 @@ int device_scratch(int dev, unsigned char **out) {
             snprintf(g_msg, sizeof(g_msg), "cudaGetSymbolAddress: %s", cudaGetErrorString(e));
             return report(DBD_ERR_CUDA);
         }
+        void *h = nullptr;
+        e = cudaMallocHost(&h, sizeof(Mailbox));
+        if (e != cudaSuccess) {
+            snprintf(g_msg, sizeof(g_msg), "cudaMallocHost: %s", cudaGetErrorString(e));
+            return report(DBD_ERR_OOM_HOST);
+        }
+        g_mail[dev] = static_cast<Mailbox *>(h);
         g_scratch_addr[dev] = static_cast<unsigned char *>(p);
         g_setup_done[dev] = true;
     }
     *out = g_scratch_addr[dev];
+    *mail = g_mail[dev];
     return DBD_OK;
 }
 
@@ -154,7 +166,8 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     int dev = 0;
     NA_CK(cudaGetDevice(&dev));
     unsigned char *base = nullptr;
-    int rc = device_scratch(dev, &base);
+    Mailbox *box = nullptr;
+    int rc = device_scratch(dev, &base, &box);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream_handle;
     // The call synchronises with the host twice (bin sizes, nnz(C)), which a
@@ -189,13 +202,12 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     static_assert(sizeof(int32_t) * kMaxBins >= sizeof(int64_t), "a tile's sum fits in its offsets");
     int64_t *tileSum = reinterpret_cast<int64_t *>(symTileOff);
     int32_t *state = c.take<int32_t>(2 * (size_t)a->nnz);
-    int *flags = c.take<int>(4);  // [0] device error word, [1] bad row_ptr, [2] bad index, [3] B unsorted
-    uint32_t *ctrs = c.take<uint32_t>(CTR_COUNT);
+    int32_t *ctl = c.take<int32_t>(CTL_COUNT);
+    int *err = ctl + CTL_ERR;
+    uint32_t *ctrs = reinterpret_cast<uint32_t *>(ctl + CTL_CTR);
 
     // The array keeps the previous call's contents: clear what starts at zero.
-    NA_CK(cudaMemsetAsync(flags, 0, 4 * sizeof(int), s));
-    NA_CK(cudaMemsetAsync(ctrs, 0, sizeof(uint32_t) * CTR_COUNT, s));
-    NA_CK(cudaMemsetAsync(rowNnz, 0, sizeof(int32_t) * (size_t)(m > 0 ? m : 1), s));
+    NA_CK(cudaMemsetAsync(ctl, 0, sizeof(int32_t) * CTL_COUNT, s));
     CsrDev A, B;
     A.m = a->n_rows; A.n = a->n_cols; A.nnz = a->nnz;
     A.ptr = a->row_ptr; A.idx = a->col_idx; A.val = (const double *)a->val;
@@ -203,30 +215,31 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     B.ptr = b->row_ptr; B.idx = b->col_idx; B.val = (const double *)b->val;
     int sms = 0;
     NA_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // Both operands are checked before any kernel gathers through them; A's
-    // row ranges (into rowP, which the analysis fills later) and order are
-    // not used.
-    if (b != a) {
-        launch_check_operand(A, reinterpret_cast<int2 *>(rowP), flags + 1, flags + 2, flags + 3, s, sms);
-        NA_CK(cudaMemsetAsync(flags + 3, 0, sizeof(int), s));
-    }
-    launch_check_operand(B, range, flags + 1, flags + 2, flags + 3, s, sms);
-    int hflags[4] = {0, 0, 0, 0};
-    NA_CK(cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, s));
-    NA_CK(cudaStreamSynchronize(s));
-    if (hflags[1]) return fail(DBD_ERR_INVALID, "malformed row_ptr");
-    if (hflags[2]) return fail(DBD_ERR_INVALID, "column index out of range");
-    if (hflags[3]) launch_row_minmax(B, range, flags + 3, s, sms);
+    // Both operands are checked before any kernel gathers through them (the
+    // work estimate looks at the flags; the host reads them with its results).
+    // A's row ranges (into rowP, which the analysis fills later) are not used.
+    if (b != a)
+        launch_check_operand(A, reinterpret_cast<int2 *>(rowP), ctl + CTL_A, ctl + CTL_A + 1, ctl + CTL_A + 2, s, sms);
+    launch_check_operand(B, range, ctl + CTL_B, ctl + CTL_B + 1, ctl + CTL_B + 2, s, sms);
+    launch_row_minmax(B, range, ctl + CTL_B + 2, s, sms);
     // Analysis: products per row, symbolic bins, row lists.
-    launch_row_products(A, B.ptr, range, ri, symBin, flags, Tuning{}, s, sms);
+    launch_row_products(A, B.ptr, range, ri, symBin, err, ctl, Tuning{}, s, sms);
     Binning sb{symBin, symList, hist, symTileOff, symStart};
-    launch_sym_lists(m, sb, ri, nullptr, 0, nullptr, s);
-    int32_t symStart_h[kMaxBins + 1];
-    NA_CK(cudaMemcpyAsync(symStart_h, symStart, sizeof(symStart_h), cudaMemcpyDeviceToHost, s));
-    NA_CK(cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, s));
+    Mail mail;
+    mail.to = box;
+    mail.ctl = ctl;
+    mail.binStart = symStart;
+    launch_sym_lists(m, sb, ri, rowNnz, nullptr, 0, nullptr, mail, s);
     NA_CK(cudaStreamSynchronize(s));
     NA_CK(cudaGetLastError());
-    if (hflags[0]) return fail(DBD_ERR_DEVICE_CHECK, "a row has more than 2^31 products");
+    for (const int32_t *f : {box->flags + CTL_A, box->flags + CTL_B}) {
+        if (f[0]) return fail(DBD_ERR_INVALID, "malformed row_ptr");
+        if (f[1]) return fail(DBD_ERR_INVALID, "column index out of range");
+    }
+    if (box->err) return fail(DBD_ERR_DEVICE_CHECK, "a row has more than 2^31 products");
+    int32_t symStart_h[kMaxBins + 1];
+    memcpy(symStart_h, box->binStart, sizeof(symStart_h));
+    const int sorted = box->flags[CTL_B + 2] ? 0 : 1;
     // Symbolic, row pointer, numeric bins.
     SymArgs sa;
     sa.A = A;
@@ -236,8 +249,8 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     sa.rowNnz = rowNnz;
     sa.ctr = ctrs;
     sa.numSms = sms;
-    sa.bSorted = hflags[3] ? 0 : 1;
-    sa.err = flags;
+    sa.bSorted = sorted;
+    sa.err = err;
     sa.rowLo = ri.lo;
     sa.rowP = ri.rowP;
     sa.rowHi = ri.hi;
@@ -245,15 +258,15 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     for (int bin = SB_TINY; bin < SB_COUNT; ++bin)
         launch_symbolic_bin(sa, bin, symStart_h[bin], symStart_h[bin + 1] - symStart_h[bin], s, &launches);
     Binning nb{numBin, numList, hist, numTileOff, numStart};
-    launch_num_lists(m, nb, ri, A.ptr, rowNnz, Tuning{}, tileSum, c_row_ptr, s);
-    int64_t nnz = 0;
-    int32_t numStart_h[kMaxBins + 1];
-    NA_CK(cudaMemcpyAsync(&nnz, c_row_ptr + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    NA_CK(cudaMemcpyAsync(numStart_h, numStart, sizeof(numStart_h), cudaMemcpyDeviceToHost, s));
-    NA_CK(cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, s));
+    mail.binStart = numStart;
+    mail.nnz = c_row_ptr + m;
+    launch_num_lists(m, nb, ri, A.ptr, rowNnz, Tuning{}, tileSum, c_row_ptr, mail, s);
     NA_CK(cudaStreamSynchronize(s));
     NA_CK(cudaGetLastError());
-    if (hflags[0]) return fail(DBD_ERR_DEVICE_CHECK, "symbolic phase: device check failed");
+    if (box->err) return fail(DBD_ERR_DEVICE_CHECK, "symbolic phase: device check failed");
+    const int64_t nnz = box->nnz;
+    int32_t numStart_h[kMaxBins + 1];
+    memcpy(numStart_h, box->binStart, sizeof(numStart_h));
     *c_nnz = nnz;
     if (nnz > c_capacity) {
         snprintf(g_msg, sizeof(g_msg), "output needs %lld entries, capacity is %lld", (long long)nnz,
@@ -270,8 +283,8 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     na.Ci = c_col_idx;
     na.Cv = c_val;
     na.state = state;
-    na.bSorted = hflags[3] ? 0 : 1;
-    na.err = flags;
+    na.bSorted = sorted;
+    na.err = err;
     na.rowP = rowP;
     na.rowLo = ri.lo;
     na.numSms = sms;
@@ -279,9 +292,9 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     na.ctr = ctrs;
     for (int bin = NB_TINY; bin < NB_COUNT; ++bin)
         launch_numeric_bin(na, bin, numStart_h[bin], numStart_h[bin + 1], s, &launches);
-    NA_CK(cudaMemcpyAsync(hflags, flags, sizeof(int), cudaMemcpyDeviceToHost, s));
+    NA_CK(cudaMemcpyAsync(&box->err, err, sizeof(int), cudaMemcpyDeviceToHost, s));
     NA_CK(cudaStreamSynchronize(s));
     NA_CK(cudaGetLastError());
-    if (hflags[0]) return fail(DBD_ERR_DEVICE_CHECK, "numeric phase: device check failed");
+    if (box->err) return fail(DBD_ERR_DEVICE_CHECK, "numeric phase: device check failed");
     return DBD_OK;
 }

@@ -512,7 +512,8 @@ void dbd_writer_close(dbd_writer *w);
  * square A with 2 entries per row fits up to about 610k rows (31 + 8 + 16 =
  * 55 bytes per row) -- are rejected with DBD_ERR_BUDGET.  The first call on a
  * device sets that device up (its kernel attributes, the loading of every
- * kernel the pipeline launches, and the array's device address), so make the
+ * kernel the pipeline launches, the array's device address, and some 300
+ * bytes of pinned host memory that results are read back through), so make the
  * first call on each device before reserving the device's memory.
  * The call reads bin sizes and nnz(C) back to the host, so it cannot be
  * captured into a CUDA graph: on a capturing stream it returns

@@ -93,3 +93,56 @@ def test_malformed_device_operands_are_refused(n, fault):
             assert ("column" if "column" in fault else "row_ptr") in str(e.value)
         assert ctx.spgemm(good).C.n_rows == n
     del keep, keep2
+
+
+def _bad(n):
+    A = gen.banded(n, 1, 0)
+    A.col_idx[-1] = n
+    return A
+
+
+def test_checks_are_read_with_the_first_results():
+    """The operands' checks are waited for with the work estimate: A's fault is
+    reported ahead of B's and of mismatched sizes, nothing is multiplied, and
+    the context goes on working; the stage functions report them at once."""
+    bad, keep = _device(_bad(300))
+    good, keep2 = _device(gen.banded(300, 1, 0))
+    other, keep3 = _device(gen.banded(200, 1, 0))
+    with dbd.Context(cpu_gib=1, gpu_gib=1) as ctx:
+        for a, b, text in ((bad, bad, "A: column"), (bad, other, "A: column"), (good, other, "inner dimensions"),
+                           (good, bad, "B: column")):
+            with pytest.raises(dbd.DBDError, match=text):
+                ctx.spgemm(a, b)
+        for load, name in ((ctx.initialize_A, "A"), (ctx.initialize_B, "B")):
+            with pytest.raises(dbd.DBDError, match=f"{name}: column"):
+                load(bad)
+        with pytest.raises(dbd.DBDError, match="load A and B"):
+            ctx.divide_Blocks()
+        with pytest.raises(dbd.DBDError, match="a pair's column"):
+            ctx.spgemm_batched([good, bad, good])
+        ctx.initialize_A(good)
+        ctx.initialize_B(good)
+        ctx.divide_Blocks()
+        ctx.distribute_Workload("kernel")
+        first = ctx.result()
+        np.testing.assert_array_equal(first.val, ctx.spgemm(good).C.val)
+        assert ctx.spgemm_batched([good, good]).C[1].nnz == first.nnz
+    del keep, keep2, keep3
+
+
+def test_noalloc_refuses_malformed_operands():
+    import ctypes
+    from dbd_gb300 import _ffi
+    bad, keep = _device(_bad(300))
+    good, keep2 = _device(gen.banded(300, 1, 0))
+    ptr = torch.empty(301, dtype=torch.int64, device="cuda")
+    idx = torch.empty(3000, dtype=torch.int32, device="cuda")
+    val = torch.empty(3000, dtype=torch.float64, device="cuda")
+    nnz = ctypes.c_int64()
+    for a, b, rc in ((bad, None, -1), (bad, good, -1), (good, bad, -1), (good, good, 0), (good, None, 0)):
+        va, vb = a.view()[0], None if b is None else b.view()[0]
+        got = _ffi.load().dbd_spgemm_noalloc(ctypes.byref(va), None if vb is None else ctypes.byref(vb), ptr.data_ptr(),
+                                             idx.data_ptr(), val.data_ptr(), 3000, ctypes.byref(nnz), None)
+        assert got == rc
+        assert rc or nnz.value == 300 * 5 - 6
+    del keep, keep2
