@@ -69,13 +69,13 @@ __host__ __device__ __forceinline__ int span_words(int32_t lo, int32_t hi) {
 // compile-time size it selects against, so every choice keeps every row
 // inside its kernel's tables: warpSpanWords <= kWarpSpanWords, numWarpMax <=
 // kNumWarpMax, symWarpMax <= kSymWarpMax, rankWordsMax <= kRankWordsMax,
-// rankSharedMax <= kNumCtaLMax (the shared value array of the rank kernel).
+// rankSharedMax <= kNumCtaLMax (the small CTAs' 16-bit ranks hold them).
 struct Tuning {
     int32_t warpSpanWords = kWarpSpanWords;   // narrow rows: warp bitmap / warp rank kernels
     int32_t numWarpMax = kNumWarpMax;         // numeric rows on one warp (rank or hash)
     int32_t symWarpMax = kSymWarpMax;         // symbolic rows on a warp hash table
     int32_t rankWordsMax = kRankWordsMax;     // CTA rank kernels for windows up to this many words
-    int32_t rankSharedMax = kNumCtaLMax;      // rank rows accumulating in shared memory
+    int32_t rankSharedMax = kNumCtaLMax;      // rank rows on the small CTAs (256 threads)
     int32_t symHashSpanWords = kWideHashSpanWords;  // symbolic CTA rows hash above this span
     int32_t denseWarpWords = kDenseWarpWords; // numeric rows on one warp's dense window
     int32_t midSpanWords = 0;                 // numeric rows on one warp's rank window (off: the

@@ -22,9 +22,9 @@
 //   CTA rows                    the row's A entries staged in shared memory,
 //                               warps over consecutive products with several
 //                               B loads in flight (warp_range_ld): hash
-//                               tables for narrow-span rows, bitmap + word
-//                               ranks for rows within 2^18 columns (values in
-//                               shared memory or reduced into C in place)
+//                               tables for narrow-span rows, bitmap ranks
+//                               for rows within 2^18 columns (products
+//                               reduced into C in place)
 //   wide rows   (symbolic)      persistent CTAs, a shared bitmap over windows
 //                               of up to 2^19 columns that stays zero between
 //                               rows, kept for the numeric rank kernels
@@ -198,10 +198,7 @@ __device__ __forceinline__ void write_columns_balanced(const uint32_t *bits, con
         word = bits[w];
     }
     for (; p < r0; ++p) word &= word - 1u;  // drop the bits before rank r0
-    // out + r is 16-byte aligned when (k0 + r) % 4 == 0.
-    const uint32_t k0 = (uint32_t)(reinterpret_cast<uintptr_t>(out) >> 2) & 3u;
-    int32_t q0 = 0, q1 = 0, q2 = 0, q3 = 0;
-    for (; p < r1; ++p) {
+    auto next = [&]() -> int32_t {
         while (!word) {
             m &= m - 1u;
             while (!m) m = tmask[++g];
@@ -210,24 +207,16 @@ __device__ __forceinline__ void write_columns_balanced(const uint32_t *bits, con
         }
         const int b = __ffs(word) - 1;
         word &= word - 1u;
-        const int32_t c = (int32_t)(colbase + (w << 5) + b);
-        const uint32_t k = (k0 + (uint32_t)p) & 3u;
-        if (k == 0) q0 = c;
-        else if (k == 1) q1 = c;
-        else if (k == 2) q2 = c;
-        else q3 = c;
-        if (k == 3 || p + 1 == r1) {
-            const int32_t first = p - (int32_t)k;  // the quad's first rank
-            if (k == 3 && first >= r0) {
-                __stcs(reinterpret_cast<int4 *>(out + first), make_int4(q0, q1, q2, q3));
-            } else {
-                for (int32_t t = max(first, r0); t <= p; ++t) {
-                    const uint32_t kt = (k0 + (uint32_t)t) & 3u;
-                    __stcs(out + t, kt == 0 ? q0 : (kt == 1 ? q1 : (kt == 2 ? q2 : q3)));
-                }
-            }
-        }
+        return (int32_t)(colbase + (w << 5) + b);
+    };
+    // out + r is 16-byte aligned when (k0 + r) % 4 == 0.
+    const uint32_t k0 = (uint32_t)(reinterpret_cast<uintptr_t>(out) >> 2) & 3u;
+    for (; p < r1 && ((k0 + (uint32_t)p) & 3u); ++p) __stcs(out + p, next());
+    for (; p + 4 <= r1; p += 4) {
+        const int32_t q0 = next(), q1 = next(), q2 = next(), q3 = next();
+        __stcs(reinterpret_cast<int4 *>(out + p), make_int4(q0, q1, q2, q3));
     }
+    for (; p < r1; ++p) __stcs(out + p, next());
 }
 
 template <int GROUP, int ROWS>
@@ -1405,35 +1394,53 @@ __global__ void __launch_bounds__(THREADS) k_num_hash_cta_dd(NumArgs a, int bin)
     }
 }
 
-// Rank rows (C has at most 2^18 columns): one CTA per row.  Pass 1 sets the
-// row's columns in a shared bitmap over all of C's columns; a scan of the
-// words' popcounts gives every column its rank among the row's columns, which
-// is its position in C's row.  Pass 2 accumulates every product into
-// vals[rank].  The output is in column order without hashing or sorting.
-// Rows with more than vcap entries accumulate vcap ranks per pass 2.  With
-// GLOBAL_ACC the row's slice of C's values is zeroed and accumulated in place
-// by FP64 reductions at L2 (no shared value array, no slices).
-template <int THREADS, bool GLOBAL_ACC>
-__device__ __forceinline__ void num_rank_rows(const NumArgs &a, int32_t lo, int maxWords, int vcap, int64_t vb) {
+// Rank rows (windows of at most 2^18 columns): one CTA per row.  The row's
+// columns are bits of a shared bitmap over its window (kept by the symbolic
+// pass, or set here by a pass over the products); each thread takes its own
+// consecutive words into registers, and a scan of their counts ranks every
+// pair of words, which gives a column's position in C's row by one 64-bit
+// load and a bit count.  Columns are written balanced by position, and a pass
+// over the products adds each one into C's row in place by an FP64 reduction
+// at L2.  No hashing, no sorting, no values in shared memory.
+//
+// P is the type of the pairs' ranks: 16 bits for the rows of the small CTAs
+// (at most kNumCtaLMax entries), which with 44 KB a CTA puts five of them on
+// an SM; a row is a chain of short phases with barriers between them, so what
+// bounds it is how many rows an SM has in flight.  Rows of up to 4096 entries used to
+// accumulate in shared memory (compare-and-swap loops around a multiply-add,
+// 102 KB and 256 threads a CTA, two CTAs per SM): R-MAT 2^18, 57k such rows
+// 3.13 -> 1.70 ms; 33k larger ones (512 threads, two CTAs an SM: three
+// spill and take 5.4) 5.01 -> 4.76 ms, where the reductions' 25 sectors a step
+// keep L1 at 62% and L2 at 54% of their throughput.
+// CTAs an SM is to hold: 64 registers a thread for the small ones.
+__host__ __device__ constexpr int rank_ctas(int threads) { return threads == 256 ? 4 : 2; }
+
+// Where the rank kernel's bitmap starts behind the staging area.
+__host__ __device__ constexpr size_t rank_bits_at(int threads) {
+    return (threads == 256 ? StageLayout<256>::bytes : StageLayout<512>::bytes) / 16 * 16 + 16;
+}
+
+template <int THREADS, class P>
+__device__ __forceinline__ void num_rank_rows(const NumArgs &a, int32_t lo, int maxWords, int64_t vb) {
     extern __shared__ __align__(16) unsigned char smem[];
     using L = StageLayout<THREADS>;
     constexpr int NW = THREADS / 32;
+    constexpr int kWpt = kRankWordsMax / THREADS;  // words a thread owns at most
     __shared__ int32_t sh[NW];
     int32_t *pre = reinterpret_cast<int32_t *>(smem + L::pre);
     int32_t *bst = reinterpret_cast<int32_t *>(smem + L::bst);
     double *av = reinterpret_cast<double *>(smem + L::av);
-    uint32_t *bits = reinterpret_cast<uint32_t *>(smem + L::bytes);
-    int32_t *wpre = reinterpret_cast<int32_t *>(bits + maxWords);
-    double *vals = reinterpret_cast<double *>(wpre + maxWords);
+    uint32_t *bits = reinterpret_cast<uint32_t *>(smem + rank_bits_at(THREADS));
+    P *pairRank = reinterpret_cast<P *>(bits + maxWords);
     // Per thread, the rank of its first column and its non-empty words, kept
     // in the staging area (idle between the passes).
     static_assert(8 * THREADS <= L::bytes && kRankWordsMax <= 32 * THREADS, "rank groups");
     int32_t *tbase = pre;
     uint32_t *tmask = reinterpret_cast<uint32_t *>(pre + THREADS);
-    const int tid = threadIdx.x, lane = tid & 31;
+    const int tid = threadIdx.x;
     const int32_t row = a.list[lo + vb];
     const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
-    const int64_t expect = a.Cp[row + 1] - a.Cp[row];
+    const int32_t expect = (int32_t)(a.Cp[row + 1] - a.Cp[row]);  // at most the window's 2^18 columns
     const int64_t obase = a.Cp[row] - a.outBase;
     // The row's window: words [rw0, rw0 + nwords) of C's columns.
     const int32_t rlo = a.rowLo[row];
@@ -1441,13 +1448,10 @@ __device__ __forceinline__ void num_rank_rows(const NumArgs &a, int32_t lo, int 
     const int nwords = min(span_words(rlo, a.rowHi[row]), maxWords);
     const int32_t cbase = rw0 << 5;
     const int32_t obc = cbase - col_shift(a, row);  // column written for bit 0
+    double *cv = a.Cv + obase;
 
-    if (a.wideBits && sym_bin_of(a.rowP[row], e1 - e0, nwords, a.tune) == SB_WIDE) {
-        // The symbolic pass kept this row's bitmap.
-        const uint32_t *src = a.wideBits + (size_t)a.wideSlot[row] * kRankWordsMax;
-        for (int i = tid; i < nwords; i += THREADS) bits[i] = __ldcs(&src[i]);
-        __syncthreads();
-    } else {
+    const bool kept = a.wideBits && sym_bin_of(a.rowP[row], e1 - e0, nwords, a.tune) == SB_WIDE;
+    if (!kept) {
         for (int i = tid; i < nwords; i += THREADS) bits[i] = 0u;
         for (int32_t eb = e0; eb < e1; eb += THREADS) {
             int nb;
@@ -1464,36 +1468,53 @@ __device__ __forceinline__ void num_rank_rows(const NumArgs &a, int32_t lo, int 
             __syncthreads();
         }
     }
+    // C's values start at zero; the stores run while the row is ranked.
+    for (int i = tid; i < expect; i += THREADS) cv[i] = 0.0;
 
-    // Ranks, per thread over its own wpt consecutive words (wpt a power of
-    // two, THREADS * wpt >= nwords): one sweep gives the thread the mask of
-    // its non-empty words and their bit count, a block scan the rank of its
-    // first column; then only the non-empty words are ranked.  Lanes start
-    // their sweeps at different words so that a warp's loads hit 32 banks.
-    // C's columns are then written balanced by output position.
-    int wpt = 1;
+    // This thread's words [w0, w0 + wpt), wpt a power of two of at least 4
+    // with THREADS * wpt >= nwords.
+    int wpt = 4;
     while (wpt * THREADS < nwords) wpt <<= 1;
     const int w0 = tid * wpt;
-    const int rot = (lane * wpt) >> 5;
+    const uint32_t *src = kept ? a.wideBits + (size_t)a.wideSlot[row] * kRankWordsMax : bits;
+    uint32_t x[kWpt];
     uint32_t mask = 0u;
     int32_t cnt = 0;
-    for (int k = 0; k < wpt; ++k) {
-        const int q = (k + rot) & (wpt - 1);
-        if (w0 + q < nwords) {
-            const uint32_t x = bits[w0 + q];
-            if (x) mask |= 1u << q;
-            cnt += __popc(x);
+#pragma unroll
+    for (int k = 0; k < kWpt; k += 4) {
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (k < wpt && w0 + k < nwords) {
+            v = kept ? __ldcs(reinterpret_cast<const uint4 *>(src + w0 + k))
+                     : *reinterpret_cast<const uint4 *>(src + w0 + k);
+            // Words past the window hold another row's bits.
+            if (w0 + k + 1 >= nwords) v.y = 0u;
+            if (w0 + k + 2 >= nwords) v.z = 0u;
+            if (w0 + k + 3 >= nwords) v.w = 0u;
         }
+        x[k] = v.x;
+        x[k + 1] = v.y;
+        x[k + 2] = v.z;
+        x[k + 3] = v.w;
+    }
+#pragma unroll
+    for (int k = 0; k < kWpt; ++k) {
+        if (x[k]) mask |= 1u << k;
+        cnt += __popc(x[k]);
     }
     int32_t tot;
     const int32_t base = block_excl_scan<THREADS>(cnt, &tot, sh);
     if (tid == 0 && tot != expect) raise(a.err, DEV_COUNT_MISMATCH);
     {
         int32_t p = base;
-        for (uint32_t m = mask; m; m &= m - 1u) {
-            const int w = w0 + __ffs(m) - 1;
-            wpre[w] = p;
-            p += __popc(bits[w]);
+#pragma unroll
+        for (int k = 0; k < kWpt; k += 4) {
+            if (k < wpt && w0 + k < nwords) {
+                if (kept) *reinterpret_cast<uint4 *>(bits + w0 + k) = make_uint4(x[k], x[k + 1], x[k + 2], x[k + 3]);
+                pairRank[(w0 + k) >> 1] = (P)p;
+                p += __popc(x[k]) + __popc(x[k + 1]);
+                pairRank[((w0 + k) >> 1) + 1] = (P)p;
+                p += __popc(x[k + 2]) + __popc(x[k + 3]);
+            }
         }
         tbase[tid] = base;
         tmask[tid] = mask;
@@ -1502,71 +1523,41 @@ __device__ __forceinline__ void num_rank_rows(const NumArgs &a, int32_t lo, int 
     write_columns_balanced<THREADS>(bits, tbase, tmask, wpt, tot, a.Ci + obase, expect, obc);
     __syncthreads();
 
-    if constexpr (GLOBAL_ACC) {
-        double *cv = a.Cv + obase;
-        for (int64_t i = tid; i < expect; i += THREADS) cv[i] = 0.0;
+    for (int32_t eb = e0; eb < e1; eb += THREADS) {
+        int nb;
+        const int32_t total =
+            stage_entries<THREADS, true>(a.A, a.B, eb, min(THREADS, e1 - eb), pre, bst, av, &nb, sh);
+        int32_t tb, te;
+        warp_share<THREADS>(total, &tb, &te);
+        warp_range_ld<4>(
+            pre, bst, nb, tb, te,
+            [&](int32_t pos) { return ColVal{__ldg(&a.B.idx[pos]), __ldg(&a.B.val[pos])}; },
+            [&](bool v, const ColVal &x, int e) {
+                const uint32_t c = (uint32_t)(x.c - cbase);
+                if (v && c < (uint32_t)nwords * 32u) {
+                    const uint2 word = *reinterpret_cast<const uint2 *>(bits + (c >> 6) * 2u);
+                    const uint32_t below = (1u << (c & 31u)) - 1u;
+                    const uint32_t r = (uint32_t)pairRank[c >> 6] + ((c & 32u) ? __popc(word.x) + __popc(word.y & below)
+                                                                              : __popc(word.x & below));
+                    if (r < (uint32_t)expect) atomicAdd(&cv[r], __dmul_rn(av[e], x.v));
+                }
+            });
         __syncthreads();
-        for (int32_t eb = e0; eb < e1; eb += THREADS) {
-            int nb;
-            const int32_t total =
-                stage_entries<THREADS, true>(a.A, a.B, eb, min(THREADS, e1 - eb), pre, bst, av, &nb, sh);
-            int32_t tb, te;
-            warp_share<THREADS>(total, &tb, &te);
-            warp_range_ld<4>(
-                pre, bst, nb, tb, te,
-                [&](int32_t pos) { return ColVal{__ldg(&a.B.idx[pos]), __ldg(&a.B.val[pos])}; },
-                [&](bool v, const ColVal &x, int e) {
-                    const int32_t c = x.c - cbase;
-                    if (v && (uint32_t)c < (uint32_t)nwords * 32u) {
-                        const int w = c >> 5;
-                        const int64_t r = (int64_t)wpre[w] + __popc(bits[w] & ((1u << (c & 31)) - 1u));
-                        if (r < expect) atomicAdd(&cv[r], __dmul_rn(av[e], x.v));
-                    }
-                });
-            __syncthreads();
-        }
-    } else {
-        // Values, vcap ranks per pass.
-        for (int64_t s0 = 0; s0 < expect; s0 += vcap) {
-            const int ns = (int)min((int64_t)vcap, expect - s0);
-            for (int i = tid; i < ns; i += THREADS) vals[i] = 0.0;
-            for (int32_t eb = e0; eb < e1; eb += THREADS) {
-                int nb;
-                const int32_t total =
-                    stage_entries<THREADS, true>(a.A, a.B, eb, min(THREADS, e1 - eb), pre, bst, av, &nb, sh);
-                int32_t tb, te;
-                warp_share<THREADS>(total, &tb, &te);
-                warp_range_ld<4>(
-                    pre, bst, nb, tb, te,
-                    [&](int32_t pos) { return ColVal{__ldg(&a.B.idx[pos]), __ldg(&a.B.val[pos])}; },
-                    [&](bool v, const ColVal &x, int e) {
-                        const int32_t c = x.c - cbase;
-                        if (v && (uint32_t)c < (uint32_t)nwords * 32u) {
-                            const int w = c >> 5;
-                            const int64_t r = (int64_t)wpre[w] + __popc(bits[w] & ((1u << (c & 31)) - 1u)) - s0;
-                            if (r >= 0 && r < ns) atomic_fma(&vals[r], av[e], x.v);
-                        }
-                    });
-                __syncthreads();
-            }
-            for (int i = tid; i < ns; i += THREADS) a.Cv[obase + s0 + i] = vals[i];
-            __syncthreads();
-        }
     }
 }
 
-template <int THREADS, bool GLOBAL_ACC>
-__global__ void __launch_bounds__(THREADS, GLOBAL_ACC ? 3 : 1) k_num_rank(NumArgs a, int32_t lo, int maxWords, int vcap) {
-    num_rank_rows<THREADS, GLOBAL_ACC>(a, lo, maxWords, vcap, blockIdx.x);
+template <int THREADS, class P>
+__global__ void __launch_bounds__(THREADS, rank_ctas(THREADS)) k_num_rank(NumArgs a, int32_t lo, int maxWords) {
+    num_rank_rows<THREADS, P>(a, lo, maxWords, blockIdx.x);
 }
 
 // The same rows launched device-driven: the bin's rows from the bin table
 // on the device, covered by a grid-stride loop.
-template <int THREADS, bool GLOBAL_ACC>
-__global__ void __launch_bounds__(THREADS, GLOBAL_ACC ? 3 : 1) k_num_rank_dd(NumArgs a, int bin, int maxWords, int vcap) {
+template <int THREADS, class P>
+__global__ void __launch_bounds__(THREADS, rank_ctas(THREADS)) k_num_rank_dd(NumArgs a, int bin, int maxWords) {
     const int32_t lo = a.binStart[bin], count = a.binStart[bin + 1] - lo;
     for (int64_t vb = blockIdx.x; vb < count; vb += gridDim.x) {
-        num_rank_rows<THREADS, GLOBAL_ACC>(a, lo, maxWords, vcap, vb);
+        num_rank_rows<THREADS, P>(a, lo, maxWords, vb);
         __syncthreads();
     }
 }
@@ -2558,10 +2549,8 @@ constexpr size_t kSmemNumCtaS = StageLayout<kNumCtaSThreads>::bytes + (size_t)kN
 constexpr size_t kSmemNumCtaL = StageLayout<kNumCtaLThreads>::bytes + (size_t)kNumCtaLTable * 12;
 constexpr size_t kSmemDense = (size_t)kDenseWindow * 8 + kDenseWindow / 8 + (size_t)kDenseStage * 8;
 constexpr size_t kSmemWideBase = StageLayout<kWideThreads>::bytes;
-constexpr int kRankSThreads = 256, kRankSVcap = kNumCtaLMax;
-constexpr int kRankLThreads = 512;  // global accumulation: staging + bitmap + ranks only
-constexpr size_t kSmemRankSMax = StageLayout<kRankSThreads>::bytes + 8 * (size_t)kRankWordsMax + 8 * (size_t)kRankSVcap;
-constexpr size_t kSmemRankLMax = StageLayout<kRankLThreads>::bytes + 8 * (size_t)kRankWordsMax;
+constexpr int kRankSThreads = 256;  // rows of at most tune.rankSharedMax entries
+constexpr int kRankLThreads = 512;
 constexpr int kBitwRows = 8;
 constexpr int kRankwRows = 8;
 constexpr int kDensewRows = 4;  // 8 rows a CTA: 8.2 ms where 4 take 7.9
@@ -2577,6 +2566,18 @@ constexpr size_t kSmemRankm =
     (size_t)kRankmRows * (6 * (size_t)kMidSpanWords + 4 * (size_t)(kMidSpanWords / 32) + 8 * (size_t)kNumWarpMax);
 
 }  // namespace
+
+// Dynamic shared memory of the rank kernel: staging, bitmap and pair ranks of
+// maxWords words.
+static size_t smem_rank(int threads, int maxWords) {
+    return rank_bits_at(threads) + 4 * (size_t)maxWords + (threads == kRankSThreads ? 2 : 4) * (size_t)(maxWords / 2);
+}
+
+// Words of the rank kernels' bitmap: the threshold's, or all of C's columns
+// where they take fewer (a multiple of 4, as threads own aligned quads).
+static int rank_words(const Tuning &t, int64_t ncols) {
+    return (int)((std::min<int64_t>(t.rankWordsMax, ncols / 32 + 1) + 3) / 4 * 4);
+}
 
 void init_kernel_attributes() {
     cudaFuncSetAttribute(k_sym_hash_warp<kSymWarpRows, kSymWarpTable>,
@@ -2595,10 +2596,10 @@ void init_kernel_attributes() {
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemDense);
     cudaFuncSetAttribute(k_num_dense<kDenseThreads, kDenseWindow, kDenseStage, false>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemDense);
-    cudaFuncSetAttribute(k_num_rank<kRankSThreads, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kSmemRankSMax);
-    cudaFuncSetAttribute(k_num_rank<kRankLThreads, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kSmemRankLMax);
+    cudaFuncSetAttribute(k_num_rank<kRankSThreads, uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem_rank(kRankSThreads, kRankWordsMax));
+    cudaFuncSetAttribute(k_num_rank<kRankLThreads, int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem_rank(kRankLThreads, kRankWordsMax));
     cudaFuncSetAttribute(k_num_rankm<kRankmRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemRankm);
     cudaFuncSetAttribute(k_num_rankwin<kRankWinThreads, kRankWinWords>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kSmemRankWin);
@@ -2617,10 +2618,10 @@ void init_kernel_attributes() {
                          (int)kSmemNumCtaS);
     cudaFuncSetAttribute(k_num_hash_cta_dd<kNumCtaLThreads, kNumCtaLTable>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kSmemNumCtaL);
-    cudaFuncSetAttribute(k_num_rank_dd<kRankSThreads, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kSmemRankSMax);
-    cudaFuncSetAttribute(k_num_rank_dd<kRankLThreads, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kSmemRankLMax);
+    cudaFuncSetAttribute(k_num_rank_dd<kRankSThreads, uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem_rank(kRankSThreads, kRankWordsMax));
+    cudaFuncSetAttribute(k_num_rank_dd<kRankLThreads, int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem_rank(kRankLThreads, kRankWordsMax));
 }
 
 // Loads every symbolic and numeric kernel of this file now.  CUDA loads
@@ -2639,8 +2640,8 @@ cudaError_t preload_spgemm_kernels() {
         (const void *)k_num_densew<kDensewRows>,
         (const void *)k_num_rankm<kRankmRows>,
         (const void *)k_num_rankw<kRankwRows>,
-        (const void *)k_num_rank<kRankSThreads, false>,
-        (const void *)k_num_rank<kRankLThreads, true>,
+        (const void *)k_num_rank<kRankSThreads, uint16_t>,
+        (const void *)k_num_rank<kRankLThreads, int32_t>,
         (const void *)k_num_hash_cta<kNumCtaSThreads, kNumCtaSTable>,
         (const void *)k_num_hash_cta<kNumCtaLThreads, kNumCtaLTable>,
         (const void *)k_num_rankwin<kRankWinThreads, kRankWinWords>,
@@ -2656,13 +2657,6 @@ cudaError_t preload_spgemm_kernels() {
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
-}
-
-// Dynamic shared memory of the rank kernel: staging, bitmap and word ranks of
-// maxWords words, vcap shared values.
-static size_t smem_rank(int threads, int maxWords, int vcap) {
-    const size_t stage = threads == kRankSThreads ? StageLayout<kRankSThreads>::bytes : StageLayout<kRankLThreads>::bytes;
-    return stage + 8 * (size_t)maxWords + 8 * (size_t)vcap;
 }
 
 static int wide_window_bits(int64_t ncols) {
@@ -2801,17 +2795,19 @@ void launch_numeric_bin_dd(const NumArgs &a, int bin, cudaStream_t s, int *launc
             break;
         }
         case NB_RANKS: {
-            const size_t smem = smem_rank(kRankSThreads, a.tune.rankWordsMax, a.tune.rankSharedMax);
-            const void *fn = (const void *)k_num_rank_dd<kRankSThreads, false>;
-            k_num_rank_dd<kRankSThreads, false><<<resident_grid(fn, kRankSThreads, smem, a.numSms), kRankSThreads, smem,
-                                                  s>>>(a, bin, a.tune.rankWordsMax, a.tune.rankSharedMax);
+            const int words = rank_words(a.tune, a.B.n);
+            const size_t smem = smem_rank(kRankSThreads, words);
+            const void *fn = (const void *)k_num_rank_dd<kRankSThreads, uint16_t>;
+            k_num_rank_dd<kRankSThreads, uint16_t>
+                <<<resident_grid(fn, kRankSThreads, smem, a.numSms), kRankSThreads, smem, s>>>(a, bin, words);
             break;
         }
         case NB_RANKL: {
-            const size_t smem = smem_rank(kRankLThreads, a.tune.rankWordsMax, 0);
-            const void *fn = (const void *)k_num_rank_dd<kRankLThreads, true>;
-            k_num_rank_dd<kRankLThreads, true><<<resident_grid(fn, kRankLThreads, smem, a.numSms), kRankLThreads, smem,
-                                                 s>>>(a, bin, a.tune.rankWordsMax, 0);
+            const int words = rank_words(a.tune, a.B.n);
+            const size_t smem = smem_rank(kRankLThreads, words);
+            const void *fn = (const void *)k_num_rank_dd<kRankLThreads, int32_t>;
+            k_num_rank_dd<kRankLThreads, int32_t>
+                <<<resident_grid(fn, kRankLThreads, smem, a.numSms), kRankLThreads, smem, s>>>(a, bin, words);
             break;
         }
         case NB_HCTA_S: {
@@ -2856,10 +2852,10 @@ void prepare_dd_grids(const Tuning &t, int64_t bcols, int sms) {
     resident_grid((const void *)k_num_hash_warp_dd<kNumWarpRows, kNumWarpTable>, 32 * kNumWarpRows, kSmemNumWarp, sms);
     resident_grid((const void *)k_num_densew_dd<kDensewRows>, 32 * kDensewRows, 0, sms);
     resident_grid((const void *)k_num_rankw_dd<kRankwRows>, 32 * kRankwRows, 0, sms);
-    resident_grid((const void *)k_num_rank_dd<kRankSThreads, false>, kRankSThreads,
-                  smem_rank(kRankSThreads, t.rankWordsMax, t.rankSharedMax), sms);
-    resident_grid((const void *)k_num_rank_dd<kRankLThreads, true>, kRankLThreads,
-                  smem_rank(kRankLThreads, t.rankWordsMax, 0), sms);
+    resident_grid((const void *)k_num_rank_dd<kRankSThreads, uint16_t>, kRankSThreads,
+                  smem_rank(kRankSThreads, rank_words(t, bcols)), sms);
+    resident_grid((const void *)k_num_rank_dd<kRankLThreads, int32_t>, kRankLThreads,
+                  smem_rank(kRankLThreads, rank_words(t, bcols)), sms);
     resident_grid((const void *)k_num_hash_cta_dd<kNumCtaSThreads, kNumCtaSTable>, kNumCtaSThreads, kSmemNumCtaS, sms);
     resident_grid((const void *)k_num_hash_cta_dd<kNumCtaLThreads, kNumCtaLTable>, kNumCtaLThreads, kSmemNumCtaL, sms);
     resident_grid((const void *)k_num_rankwin<kRankWinThreads, kRankWinWords>, kRankWinThreads, kSmemRankWin, sms);
@@ -2890,15 +2886,18 @@ void launch_numeric_bin(const NumArgs &a, int bin, int32_t lo, int32_t hi, cudaS
         case NB_RANKW:
             k_num_rankw<kRankwRows><<<(unsigned)ceil_div(n, kRankwRows), 32 * kRankwRows, 0, s>>>(a, lo, n);
             break;
-        case NB_RANKS:
-            k_num_rank<kRankSThreads, false>
-                <<<(unsigned)n, kRankSThreads, smem_rank(kRankSThreads, a.tune.rankWordsMax, a.tune.rankSharedMax), s>>>(
-                    a, lo, a.tune.rankWordsMax, a.tune.rankSharedMax);
+        case NB_RANKS: {
+            const int words = rank_words(a.tune, a.B.n);
+            k_num_rank<kRankSThreads, uint16_t>
+                <<<(unsigned)n, kRankSThreads, smem_rank(kRankSThreads, words), s>>>(a, lo, words);
             break;
-        case NB_RANKL:
-            k_num_rank<kRankLThreads, true><<<(unsigned)n, kRankLThreads, smem_rank(kRankLThreads, a.tune.rankWordsMax, 0),
-                                             s>>>(a, lo, a.tune.rankWordsMax, 0);
+        }
+        case NB_RANKL: {
+            const int words = rank_words(a.tune, a.B.n);
+            k_num_rank<kRankLThreads, int32_t>
+                <<<(unsigned)n, kRankLThreads, smem_rank(kRankLThreads, words), s>>>(a, lo, words);
             break;
+        }
         case NB_HCTA_S:
             k_num_hash_cta<kNumCtaSThreads, kNumCtaSTable><<<(unsigned)n, kNumCtaSThreads, kSmemNumCtaS, s>>>(a, lo);
             break;

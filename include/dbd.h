@@ -133,8 +133,8 @@ typedef struct {
     int32_t criteria;         /* categoriser threshold (distributeWorkload.cpp:249-264) */
     int32_t n_chunks;         /* device output chunks streamed */
     int64_t blocks_per_category[3]; /* 0 dense, 1 light, 2 either (distributeWorkload.cpp:266-270) */
-    int64_t rows_per_bin[DBD_NUM_BINS];   /* numeric bins: empty, tiny, warp rank, warp hash, CTA rank (shared),
-                                             CTA rank (in place), CTA hash S, CTA hash L, dense windows,
+    int64_t rows_per_bin[DBD_NUM_BINS];   /* numeric bins: empty, tiny, warp rank, warp hash, CTA rank (small),
+                                             CTA rank (large), CTA hash S, CTA hash L, dense windows,
                                              warp dense window, warp rank window */
     int64_t sym_rows_per_bin[DBD_NUM_BINS]; /* symbolic bins: empty, tiny, warp flags, warp hash, CTA hash, CTA bitmap */
     int64_t bytes_d2h;
@@ -361,8 +361,8 @@ int dbd_batch_result(dbd_ctx *ctx, int64_t *c_row_off, int64_t *c_nnz_off, dbd_c
  *                          one-warp hash table (32..512)
  *   rank_words_max         CTA rank kernels take windows up to this many words;
  *                          wider rows use CTA hash tables or dense windows (1..8192)
- *   rank_shared_max_nnz    rank rows up to this size accumulate in shared
- *                          memory, larger ones in place in C (1..4096)
+ *   rank_shared_max_nnz    rank rows up to this size take CTAs of 256 threads
+ *                          and 16-bit ranks, larger ones 512 (1..4096)
  *   sym_hash_span_words    symbolic rows with at most 4096 products hash
  *                          (instead of a bitmap) above this span (>= 0)
  *   dense_warp_span_words  numeric rows whose window spans at most this many
