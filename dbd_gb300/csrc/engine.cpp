@@ -1879,8 +1879,16 @@ int dbd_spgemm_batched(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const d
     da.val = c->A.val.as<double>();
     c->A.pending = c->B.pending = false;
     c->b_is_a = square;
-    rc = check_operand(c, c->A, da);
-    if (rc) return rc;
+    if (square) {
+        rc = check_operand(c, c->A, da);
+        if (rc) return rc;
+    } else {
+        // The gather has checked A's pairs; its order and row ranges matter
+        // for a right operand only.
+        c->A.dev = da;
+        c->A.loaded = c->A.pending = true;
+        c->divided = false;
+    }
     if (!square) {
         CsrDev db;
         db.m = rowB[count];
