@@ -60,6 +60,14 @@ constexpr int kMaxSlabs = 64;                // rows spanning up to 2^22 columns
 constexpr int64_t kHeavyP = 65536;
 constexpr int kPieceNnz = 65536;
 constexpr int kPieceSlabs = 16;
+// The symbolic pass takes wide rows of at least sym_first_products() products
+// in a launch of their own beside the others, those of twice as many cut into
+// one item per slab: a CTA walks about 2 products a nanosecond, so a row of
+// 3.75M of the 381M products in 10,240 rows of R-MAT 2^21 set the pass's time
+// alone.  The line is half a CTA's share of all products (a shorter row can
+// hardly be the last one running), and no less than kSymFirstP, under which an
+// item is not worth its staging.
+constexpr int64_t kSymFirstP = 1 << 18;
 
 __host__ __device__ __forceinline__ int span_words(int32_t lo, int32_t hi) {
     return hi >= lo ? (hi >> 5) - (lo >> 5) + 1 : 0;
@@ -135,7 +143,8 @@ enum DevErr : int { DEV_OK = 0, DEV_TABLE_FULL = 1, DEV_COUNT_MISMATCH = 2, DEV_
 // Counter slots for dynamically scheduled kernels (zeroed per multiply).
 enum CounterSlot : int {
     CTR_SYM_TINY = 0, CTR_SYM_HWARP, CTR_SYM_HCTA, CTR_SYM_WIDE, CTR_NUM_GDENSE, CTR_NUM_RANKWIN, CTR_NUM_DSCR,
-    CTR_HEAVY, CTR_ITEMS, CTR_ADJOINT, CTR_COUNT = 16
+    CTR_HEAVY, CTR_ITEMS, CTR_ADJOINT, CTR_SYM_ITEMS, CTR_SYM_NEXT,
+    CTR_MAX_P, CTR_COUNT = 16
 };
 
 struct Binning {
@@ -159,6 +168,7 @@ enum CtlWord : int {
 struct Mailbox {
     int32_t flags[8];
     int32_t err, heavy;
+    int32_t maxP, pad;   // products of the largest row
     int64_t nnz;
     int32_t binStart[kMaxBins + 1];
     int64_t blockP[1];  // as many as the multiply has row blocks
@@ -188,10 +198,11 @@ void launch_row_minmax(const CsrDev &B, int2 *range, const int *unsorted, cudaSt
 void launch_row_products(const CsrDev &A, const int32_t *Bp, const int2 *range, const RowInfo &ri, uint8_t *symBin,
                          int *err, const int32_t *ctl, const Tuning &t, cudaStream_t s, int num_sms);
 // Row lists of the symbolic bins and (blockP not null) the products of every
-// rows_per_block rows; empty rows' entry counts are cleared.  tileSum:
-// tile_count(m) + 1 int64 of scratch.
+// rows_per_block rows and of the largest row (*maxP, zeroed by the caller);
+// empty rows' entry counts are cleared.  tileSum: tile_count(m) + 1 int64 of
+// scratch.
 void launch_sym_lists(int64_t m, const Binning &b, const RowInfo &ri, int32_t *rowNnz, int64_t *tileSum,
-                      int64_t rows_per_block, int64_t *blockP, const Mail &mail, cudaStream_t s);
+                      int64_t rows_per_block, int64_t *blockP, uint32_t *maxP, const Mail &mail, cudaStream_t s);
 // Numeric bins, their row lists and C's row pointers (m + 1) from the rows'
 // entry counts.
 void launch_num_lists(int64_t m, const Binning &b, const RowInfo &ri, const int32_t *Ap, const int32_t *rowNnz,
@@ -200,6 +211,21 @@ void launch_num_lists(int64_t m, const Binning &b, const RowInfo &ri, const int3
 void launch_row_scan(int64_t m, const int32_t *cnt, int64_t *part, int64_t *Cp, cudaStream_t s);
 
 // ---- launchers (k_spgemm.cu) ----
+// One work item of the largest symbolic wide rows: the idx-th row of the
+// bin, or its column slabs [s0, s1) (s0 < 0: the whole row).
+struct SymItem {
+    int32_t idx;
+    int16_t s0, s1;
+};
+inline int64_t sym_first_products(int64_t products, int num_sms) {
+    const int64_t share = products / (4 * (int64_t)(num_sms > 0 ? num_sms : 1));  // two CTAs an SM
+    return share > kSymFirstP ? share : kSymFirstP;
+}
+// Most items that rows of `products` products in all can make.
+inline int64_t sym_item_cap(int64_t products, int64_t firstP) {
+    return products / firstP + kMaxSlabs * (products / (2 * firstP));
+}
+
 struct SymArgs {
     CsrDev A, B;
     const int32_t *list;
@@ -226,7 +252,14 @@ struct SymArgs {
     int32_t *heavySlot = nullptr;
     int32_t *slabCnt = nullptr;
     int heavyCap = 0;
+    // Items of the wide rows launched on their own (null: none);
+    // their count is ctr[CTR_SYM_ITEMS], room for sym_item_cap().
+    SymItem *items = nullptr;
+    int64_t firstP = 0;  // products from which a row is an item
 };
+// Launches the items of the wide rows list[begin, begin + n) (a.items; the
+// bin's own launch then leaves their rows out).
+void launch_symbolic_items(const SymArgs &a, int32_t begin, int32_t n, cudaStream_t s, int *launches);
 // Launches the symbolic kernel of bin `bin` over list[begin, begin + n).
 void launch_symbolic_bin(const SymArgs &a, int bin, int32_t begin, int32_t n, cudaStream_t s, int *launches);
 // Device-driven launch of a symbolic bin: its rows from a.binStart on the

@@ -143,6 +143,7 @@ struct dbd_ctx {
     int gSlots = 0;
     int64_t gStride = 0;
     DevBuf heavySlot, slabCnt;  // slab counts of heavy rows (symbolic -> dense-bin pieces)
+    DevBuf symItems;            // items of the largest symbolic wide rows
     DevBuf items;               // dense-bin work items
     int heavyCap = 0, itemCap = 0;
     bool pieces = false;        // the dense bin cuts heavy rows into pieces in this multiply
@@ -178,7 +179,7 @@ struct dbd_ctx {
     bool capturing = false;
     bool replayOk = false;  // the last multiply left its plan and C on the device (kernel scope)
     Tuning tune;            // bin thresholds (dbd_set_tuning / dbd_autotune)
-    int64_t m = 0, ncols = 0, nnzC = 0, products = 0;
+    int64_t m = 0, ncols = 0, nnzC = 0, products = 0, maxRowP = 0;
     int64_t nblocks = 0, ntiles = 0;
     bool divided = false;
     std::vector<int64_t> blockP_h;
@@ -536,8 +537,8 @@ int divide_blocks(dbd_ctx *c) {
     mail.to = c->mail();
     mail.ctl = c->flags();
     mail.binStart = c->symStart.as<int32_t>();
-    launch_sym_lists(m, sb, row_info(c), c->rowNnz.as<int32_t>(), c->part.as<int64_t>(), rpb, c->mail()->blockP, mail,
-                     c->stream);
+    launch_sym_lists(m, sb, row_info(c), c->rowNnz.as<int32_t>(), c->part.as<int64_t>(), rpb, c->mail()->blockP,
+                     c->ctrs() + CTR_MAX_P, mail, c->stream);
     c->launches += 4;
     CK(c, cudaGetLastError());
     CK(c, cudaEventRecord(c->evPre, c->stream));
@@ -547,6 +548,7 @@ int divide_blocks(dbd_ctx *c) {
     rc = device_err(c, c->mail()->err, "work estimate");
     if (rc) return rc;
     memcpy(c->symStart_h, c->mail()->binStart, sizeof(c->symStart_h));
+    c->maxRowP = c->mail()->maxP;
     c->blockP_h.assign(c->mail()->blockP, c->mail()->blockP + c->nblocks);
 
     // Segmenter + categoriser on the per-block products (host, O(blocks)).
@@ -633,9 +635,23 @@ int symbolic(dbd_ctx *c) {
             c->wideKept = true;
         }
     }
+    // The largest wide rows go beside the others, cut by column.
+    const int32_t nwideRows = c->symStart_h[SB_WIDE + 1] - c->symStart_h[SB_WIDE];
+    const int64_t firstP = sym_first_products(c->products, c->num_sms);
+    if (nwideRows > 0 && c->maxRowP >= firstP) {
+        CK(c, c->symItems.ensure(sizeof(SymItem) * (size_t)sym_item_cap(c->products, firstP)));
+        sa.items = c->symItems.as<SymItem>();
+        sa.firstP = firstP;
+    }
     // Bins run concurrently, one stream each (heaviest first).
     static const int sorder[] = {SB_WIDE, SB_HCTA, SB_HWARP, SB_BITW, SB_TINY};
     Fork fk(c);
+    if (sa.items) {
+        cudaStream_t s = fk.stream(SB_EMPTY);  // its own, and first
+        cudaEvent_t e0 = c->time_ev(s);
+        launch_symbolic_items(sa, c->symStart_h[SB_WIDE], nwideRows, s, &c->launches);
+        if (e0) c->timed.push_back({0, SB_WIDE, e0, c->time_ev(s)});
+    }
     for (int b : sorder) {
         const int32_t n = c->symStart_h[b + 1] - c->symStart_h[b];
         if (n <= 0) continue;
@@ -1405,7 +1421,7 @@ void dbd_destroy(dbd_ctx *c) {
                       &c->adjA, &c->adjB, &c->adjT, &c->adjProd, &c->adjOff, &c->rowLo, &c->rowHi, &c->A.range, &c->B.range,
                       &c->gdense, &c->dgCount, &c->dgCol, &c->dgVal, &c->dgSum, &c->dgWsum,
                       &c->dgBad, &c->hashOut, &c->dscr, &c->heavySlot, &c->slabCnt,
-                      &c->items})
+                      &c->symItems, &c->items})
         b->release();
     c->mailBuf.release();
     c->hCp.release();
@@ -2088,7 +2104,7 @@ int dbd_batch_enqueue(dbd_ctx *c, void *stream) {
                         c->tune, s, c->num_sms);
     Binning sb{c->symBin.as<uint8_t>(), c->symList.as<int32_t>(), c->hist.as<int32_t>(), c->symTileOff.as<int32_t>(),
                c->symStart.as<int32_t>()};
-    launch_sym_lists(m, sb, row_info(c), c->rowNnz.as<int32_t>(), nullptr, 0, nullptr, Mail{}, s);
+    launch_sym_lists(m, sb, row_info(c), c->rowNnz.as<int32_t>(), nullptr, 0, nullptr, nullptr, Mail{}, s);
     SymArgs sa{};
     sa.A = A;
     sa.B = B;

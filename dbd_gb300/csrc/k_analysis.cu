@@ -301,7 +301,8 @@ enum TileMode : int { TILES_PLAIN = 0, TILES_BLOCKS, TILES_NUMERIC };
 __global__ void __launch_bounds__(kTileRows) k_tiles(int64_t m, int64_t ntiles, TileMode mode,
                                                      uint8_t *__restrict__ bin, int nbins, const int32_t *__restrict__ Ap,
                                                      RowInfo ri, int32_t *__restrict__ rowNnz, Tuning tune,
-                                                     int32_t *__restrict__ hist, int64_t *__restrict__ tileSum) {
+                                                     int32_t *__restrict__ hist, int64_t *__restrict__ tileSum,
+                                                     uint32_t *__restrict__ maxP) {
     __shared__ int32_t wc[kTileRows / 32][kMaxBins];
     __shared__ int64_t ws[kTileRows / 32];
     const int64_t r = (int64_t)blockIdx.x * kTileRows + threadIdx.x;
@@ -323,6 +324,11 @@ __global__ void __launch_bounds__(kTileRows) k_tiles(int64_t m, int64_t ntiles, 
     for (int q = 0; q < nbins; ++q) {
         const unsigned mk = __ballot_sync(FULL, b == q);
         if (lane == 0) wc[w][q] = __popc(mk);
+    }
+    if (maxP) {
+        // The largest row's products; below 2^31, as the work estimate checks.
+        const uint32_t most = __reduce_max_sync(FULL, (uint32_t)min(x, (int64_t)INT32_MAX));
+        if (lane == 0 && most > *(volatile uint32_t *)maxP) atomicMax(maxP, most);
     }
 #pragma unroll
     for (int d = 16; d; d >>= 1) x += __shfl_xor_sync(FULL, x, d);
@@ -465,6 +471,7 @@ __global__ void __launch_bounds__(kTileRows) k_tile_scatter(int64_t m, const uin
         else if (t < 8 + kMaxBins + 1) mail.to->binStart[t - 8] = mail.binStart[t - 8];
         else if (t == 32) mail.to->err = mail.ctl[CTL_ERR];
         else if (t == 33) mail.to->heavy = mail.ctl[CTL_CTR + CTR_HEAVY];
+        else if (t == 35) mail.to->maxP = mail.ctl[CTL_CTR + CTR_MAX_P];
         else if (t == 34 && mail.nnz) mail.to->nnz = *mail.nnz;
     }
     const int b = r < m ? (int)bin[r] : -1;
@@ -603,12 +610,12 @@ void launch_row_products(const CsrDev &A, const int32_t *Bp, const int2 *range, 
 }
 
 void launch_sym_lists(int64_t m, const Binning &b, const RowInfo &ri, int32_t *rowNnz, int64_t *tileSum,
-                      int64_t rows_per_block, int64_t *blockP, const Mail &mail, cudaStream_t s) {
+                      int64_t rows_per_block, int64_t *blockP, uint32_t *maxP, const Mail &mail, cudaStream_t s) {
     const int64_t nt = tile_count(m);
     const TileMode mode = blockP ? TILES_BLOCKS : TILES_PLAIN;
     if (nt > 0)
         k_tiles<<<(unsigned)nt, kTileRows, 0, s>>>(m, nt, mode, b.bin, SB_COUNT, nullptr, ri, rowNnz, Tuning{}, b.hist,
-                                                   blockP ? tileSum : nullptr);
+                                                   blockP ? tileSum : nullptr, blockP ? maxP : nullptr);
     k_tile_scan<<<kMaxBins + 1, kScanThreads, 0, s>>>(nt, mode, SB_COUNT, b.hist, b.tileOff, b.binStart, tileSum,
                                                       std::max<int64_t>(rows_per_block / kTileRows, 1), blockP);
     if (nt > 0 || mail.to)
@@ -621,7 +628,7 @@ void launch_num_lists(int64_t m, const Binning &b, const RowInfo &ri, const int3
     const int64_t nt = tile_count(m);
     if (nt > 0)
         k_tiles<<<(unsigned)nt, kTileRows, 0, s>>>(m, nt, TILES_NUMERIC, b.bin, NB_COUNT, Ap, ri,
-                                                   const_cast<int32_t *>(rowNnz), t, b.hist, tileSum);
+                                                   const_cast<int32_t *>(rowNnz), t, b.hist, tileSum, nullptr);
     k_tile_scan<<<kMaxBins + 1, kScanThreads, 0, s>>>(nt, TILES_NUMERIC, NB_COUNT, b.hist, b.tileOff, b.binStart,
                                                       tileSum, 1, Cp + m);
     if (nt > 0 || mail.to)

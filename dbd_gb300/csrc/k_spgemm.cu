@@ -585,15 +585,45 @@ __host__ __device__ __forceinline__ int wide_touch_cap(int winBits) {
     return min(kWideTouchMax, (winBits >> 5) / 4);
 }
 
+// Items of the wide rows list[begin, begin + n): rows of at least a.firstP
+// products, cut into one item per slab of columns from twice as many on (B's
+// rows ascending).  A cut row's count starts at zero
+// here, and its slab counts get their slot.
+__global__ void __launch_bounds__(256) k_sym_items(SymArgs a, int32_t begin, int32_t n) {
+    const int32_t i = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= n) return;
+    const int32_t row = a.list[begin + i];
+    const int64_t P = a.rowP[row];
+    if (P < a.firstP) return;
+    const int64_t base = (int64_t)(a.rowLo[row] >> 5) << 5;
+    const int ns = (int)((((int64_t)a.rowHi[row] + 1 - base) + (1 << kSlabShift) - 1) >> kSlabShift);
+    const bool cut = P >= 2 * a.firstP && b_sorted(a) && ns > 1 && ns <= kMaxSlabs;
+    const int k = cut ? ns : 1;
+    const uint32_t at = atomicAdd(&a.ctr[CTR_SYM_ITEMS], (uint32_t)k);
+    for (int s = 0; s < k; ++s) a.items[at + s] = cut ? SymItem{i, (int16_t)s, (int16_t)(s + 1)} : SymItem{i, -1, -1};
+    if (!cut) return;
+    a.rowNnz[row] = 0;
+    if (a.slabCnt) {
+        int32_t sl = (int32_t)atomicAdd(&a.ctr[CTR_HEAVY], 1u);
+        if (sl >= a.heavyCap) sl = -1;
+        a.heavySlot[row] = sl;
+    }
+}
+
 // Wide rows: persistent CTAs take rows from a counter (heavy rows spread
 // over the whole grid).  A shared bitmap over windows of winBits columns
 // stays zero between rows: every window records the words it touched and
 // clears only those (the whole window when more than kWideTouchMax were
 // touched).  The row's size is the sum of newly set bits, so no popcount
 // pass over the window either: a row costs its products, not its span.
-template <int THREADS>
+// Rows of at least a.firstP products are items of a launch of their own
+// (ITEMS, built by k_sym_items), the largest cut by column: a piece sets,
+// counts and keeps its slabs' columns and adds its count to the row's.  10,240 rows of R-MAT 2^21,
+// two of which hold 3.7M products each: 2.00 -> 1.14 ms (1.84 with 32-bit
+// window arithmetic alone).
+template <int THREADS, bool ITEMS>
 __global__ void __launch_bounds__(THREADS) k_sym_wide(SymArgs a, int32_t begin, int32_t count, int winBits) {
-    if (begin < 0) {  // device-driven: the bin's rows from the bin table
+    if (!ITEMS && begin < 0) {  // device-driven: the bin's rows from the bin table
         begin = a.binStart[SB_WIDE];
         count = a.binStart[SB_WIDE + 1] - begin;
     }
@@ -612,18 +642,30 @@ __global__ void __launch_bounds__(THREADS) k_sym_wide(SymArgs a, int32_t begin, 
     int32_t *cur = touched + cap;  // per staged entry: its B cursor across windows
     const int tid = threadIdx.x;
     for (int i = tid; i < (winBits >> 5); i += THREADS) bm[i] = 0u;
+    if constexpr (ITEMS) count = *(volatile int32_t *)&a.ctr[CTR_SYM_ITEMS];
     for (;;) {
-        if (tid == 0) next = (int32_t)atomicAdd(&a.ctr[CTR_SYM_WIDE], 1u);
+        if (tid == 0) next = (int32_t)atomicAdd(&a.ctr[ITEMS ? CTR_SYM_NEXT : CTR_SYM_WIDE], 1u);
         __syncthreads();
-        const int32_t item = next;
+        int32_t item = next;
         if (item >= count) break;
+        SymItem it{item, -1, -1};
+        if constexpr (ITEMS) {
+            it = a.items[item];
+            item = it.idx;
+        }
         const int32_t row = a.list[begin + item];
+        if (!ITEMS && a.items && a.rowP[row] >= a.firstP) {  // an item's
+            __syncthreads();  // every thread has read `next` before it changes
+            continue;
+        }
+        const bool piece = ITEMS && it.s0 >= 0;
         const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
         // The row's window [lo, hi], in windows of winBits columns from lo's word.
         const int32_t rlo = a.rowLo[row], rhi = a.rowHi[row];
         const int sw = span_words(rlo, rhi);
         const int64_t base = (int64_t)(rlo >> 5) << 5;
-        const int64_t end = (int64_t)rhi + 1;
+        const int64_t start = piece ? base + ((int64_t)it.s0 << kSlabShift) : base;
+        const int64_t end = piece ? min((int64_t)rhi + 1, base + ((int64_t)it.s1 << kSlabShift)) : (int64_t)rhi + 1;
         // Rows with more products than the list holds touch more words than
         // it holds as a rule: they set their bits with plain ORs (no old
         // values, no bookkeeping) and count, keep and clear the window in one
@@ -632,7 +674,8 @@ __global__ void __launch_bounds__(THREADS) k_sym_wide(SymArgs a, int32_t begin, 
         const bool keep = a.wideBits && sw <= kRankWordsMax;
         // Heavy rows record their entries per slab of 2^kSlabShift columns
         // (from `base`), for the numeric pass to cut them into pieces.
-        if (tid == 0) {
+        if (tid == 0 && piece) slot = a.heavySlot ? a.heavySlot[row] : -1;
+        if (tid == 0 && !piece) {
             int32_t sl = -1;
             const int64_t nslabs = ((end - base) + (1 << kSlabShift) - 1) >> kSlabShift;
             if (a.slabCnt && !rowCap && a.rowP[row] >= kHeavyP && winBits >= (1 << kSlabShift) &&
@@ -646,10 +689,12 @@ __global__ void __launch_bounds__(THREADS) k_sym_wide(SymArgs a, int32_t begin, 
         int cnt = 0;
         // Rows over several windows enumerate, per window, only the part of
         // each B row inside it (B's rows ascending).
-        const bool clip = b_sorted(a) && end - base > (int64_t)winBits;
+        const bool clip = b_sorted(a) && (piece || end - base > (int64_t)winBits);
         const bool once = e1 - e0 <= THREADS;  // one batch: its cursors carry over the windows
-        for (int64_t c_lo = base; c_lo < end; c_lo += winBits) {
+        for (int64_t c_lo = start; c_lo < end; c_lo += winBits) {
             const int words = (int)min((int64_t)winBits, end - c_lo + 31) >> 5;
+            // Columns of this window (a whole row has none past its end).
+            const uint32_t lim = ITEMS ? (uint32_t)min((int64_t)winBits, end - c_lo) : (uint32_t)winBits;
             if (tid == 0) nt = rowCap ? 0 : cap + 1;
             if (tid < (kWideWindowBitsMax >> kSlabShift)) slabSh[tid] = 0;
             __syncthreads();
@@ -657,29 +702,28 @@ __global__ void __launch_bounds__(THREADS) k_sym_wide(SymArgs a, int32_t begin, 
                 int nb;
                 const int32_t total =
                     stage_entries<THREADS, false>(a.A, a.B, eb, min(THREADS, e1 - eb), pre, bst, nullptr, &nb, sh, clip,
-                                                  c_lo, c_lo + winBits, once ? cur : nullptr, once && c_lo != base);
+                                                  c_lo, c_lo + lim, once ? cur : nullptr, once && c_lo != start);
                 int32_t tb, te;
                 warp_share<THREADS>(total, &tb, &te);
                 if (rowCap) {
                     warp_range_ld<kWideLoads>(
                         pre, bst, nb, tb, te, [&](int32_t pos) { return __ldg(&a.B.idx[pos]); },
                         [&](bool v, int32_t col, int) {
-                            const int64_t rel = v ? (int64_t)col - c_lo : -1;
-                            const bool in = rel >= 0 && rel < winBits;
-                            cnt += or_bits_count(bm, in, in ? (uint32_t)rel : 0u, touched, &nt, rowCap);
+                            const uint32_t rel = (uint32_t)col - (uint32_t)c_lo;  // columns below c_lo wrap past the window
+                            cnt += or_bits_count(bm, v && rel < lim, rel, touched, &nt, rowCap);
                         });
                 } else {
                     warp_range_ld<kWideLoads>(
                         pre, bst, nb, tb, te, [&](int32_t pos) { return __ldg(&a.B.idx[pos]); },
                         [&](bool v, int32_t col, int) {
-                            const int64_t rel = v ? (int64_t)col - c_lo : -1;
-                            if (rel >= 0 && rel < winBits) atomicOr(&bm[rel >> 5], 1u << (rel & 31));
+                            const uint32_t rel = (uint32_t)col - (uint32_t)c_lo;
+                            if (v && rel < lim) atomicOr(&bm[rel >> 5], 1u << (rel & 31));
                         });
                 }
                 __syncthreads();
             }
             if (!rowCap) {
-                uint32_t *dst = keep ? a.wideBits + (size_t)item * kRankWordsMax : nullptr;
+                uint32_t *dst = keep ? a.wideBits + (size_t)item * kRankWordsMax + ((c_lo - base) >> 5) : nullptr;
                 const int32_t sl = slot;
                 if (sl < 0) {
                     for (int i = tid; i < words; i += THREADS) {
@@ -732,7 +776,10 @@ __global__ void __launch_bounds__(THREADS) k_sym_wide(SymArgs a, int32_t begin, 
             __syncthreads();
         }
         cnt = block_sum_i<THREADS>(cnt, sh);
-        if (tid == 0) a.rowNnz[row] = cnt;
+        if (tid == 0) {
+            if (piece) atomicAdd(&a.rowNnz[row], cnt);
+            else a.rowNnz[row] = cnt;
+        }
     }
 }
 
@@ -2102,7 +2149,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_num_rankwin(NumArgs
                 warp_range_ld<4>(
                     pre, bst, nb, tb, te, [&](int32_t pos) { return __ldg(&a.B.idx[pos]); },
                     [&](bool v, int32_t col, int) {
-                        const uint32_t rel = v ? (uint32_t)((int64_t)col - c_lo) : 0u;
+                        const uint32_t rel = (uint32_t)col - (uint32_t)c_lo;
                         or_bit(bits, v && rel < nbits, rel);
                     });
                 __syncthreads();
@@ -2141,7 +2188,10 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_num_rankwin(NumArgs
                                             c_lo - shift);
             for (int64_t i = tid; i < tot && run + i < expect; i += THREADS) a.Cv[obase + run + i] = 0.0;
             __syncthreads();
-            // Pass 2: the window's products into C's row in place.
+            // Pass 2: the window's products into C's row in place (ranks
+            // within a window and its columns fit 32 bits).
+            double *cv = a.Cv + obase + run;
+            const uint32_t lim = (uint32_t)max((int64_t)0, min(expect - run, (int64_t)INT_MAX));
             for (int32_t eb = e0; eb < e1; eb += THREADS) {
                 int nb = nb1;
                 const int32_t total =
@@ -2154,12 +2204,12 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_num_rankwin(NumArgs
                     pre, bst, nb, tb, te,
                     [&](int32_t pos) { return ColVal{__ldg(&a.B.idx[pos]), __ldg(&a.B.val[pos])}; },
                     [&](bool v, const ColVal &x, int e) {
-                        const uint32_t c = v ? (uint32_t)((int64_t)x.c - c_lo) : 0u;
+                        const uint32_t c = (uint32_t)x.c - (uint32_t)c_lo;
                         if (v && c < nbits) {
-                            const int w = (int)(c >> 5);
-                            const int64_t r = run + (int64_t)gbase[w >> 8] + wpre[w] +
-                                              __popc(bits[w] & ((1u << (c & 31)) - 1u));
-                            if (r < expect) atomicAdd(&a.Cv[obase + r], __dmul_rn(av[e], x.v));
+                            const uint32_t w = c >> 5;
+                            const uint32_t r = (uint32_t)gbase[w >> 8] + wpre[w] +
+                                               __popc(bits[w] & ((1u << (c & 31)) - 1u));
+                            if (r < lim) atomicAdd(&cv[r], __dmul_rn(av[e], x.v));
                         }
                     });
                 __syncthreads();
@@ -2584,8 +2634,10 @@ void init_kernel_attributes() {
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemSymWarp);
     cudaFuncSetAttribute(k_sym_hash_cta<kSymCtaThreads, kSymCtaTable>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemSymCta);
-    cudaFuncSetAttribute(k_sym_wide<kWideThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(kSmemWideBase + kWideWindowBitsMax / 8 + 4 * (size_t)kWideTouchMax + 4 * kWideThreads));
+    for (const void *fn : {(const void *)k_sym_wide<kWideThreads, false>, (const void *)k_sym_wide<kWideThreads, true>})
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(kSmemWideBase + kWideWindowBitsMax / 8 + 4 * (size_t)kWideTouchMax +
+                                   4 * kWideThreads));
     cudaFuncSetAttribute(k_num_hash_warp<kNumWarpRows, kNumWarpTable>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemNumWarp);
     cudaFuncSetAttribute(k_num_hash_cta<kNumCtaSThreads, kNumCtaSTable>,
@@ -2634,7 +2686,9 @@ cudaError_t preload_spgemm_kernels() {
         (const void *)k_sym_flagw<kBitwRows>,
         (const void *)k_sym_hash_warp<kSymWarpRows, kSymWarpTable>,
         (const void *)k_sym_hash_cta<kSymCtaThreads, kSymCtaTable>,
-        (const void *)k_sym_wide<kWideThreads>,
+        (const void *)k_sym_items,
+        (const void *)k_sym_wide<kWideThreads, false>,
+        (const void *)k_sym_wide<kWideThreads, true>,
         (const void *)k_num_tiny,
         (const void *)k_num_hash_warp<kNumWarpRows, kNumWarpTable>,
         (const void *)k_num_densew<kDensewRows>,
@@ -2665,6 +2719,23 @@ static int wide_window_bits(int64_t ncols) {
     return (int)w;
 }
 
+static size_t smem_wide(int winBits) {
+    return kSmemWideBase + (size_t)winBits / 8 + 4 * (size_t)wide_touch_cap(winBits) + 4 * kWideThreads;
+}
+
+static int64_t wide_grid(int winBits, int sms) {
+    const int per_sm = std::max(1, std::min(2048 / kWideThreads, (int)((227 * 1024) / (smem_wide(winBits) + 1024))));
+    return (int64_t)std::max(sms, 1) * per_sm;
+}
+
+void launch_symbolic_items(const SymArgs &a, int32_t begin, int32_t n, cudaStream_t s, int *launches) {
+    const int wb = wide_window_bits(a.B.n);
+    k_sym_items<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(a, begin, n);
+    k_sym_wide<kWideThreads, true>
+        <<<(unsigned)wide_grid(wb, a.numSms), kWideThreads, smem_wide(wb), s>>>(a, begin, 0, wb);
+    *launches += 2;
+}
+
 // Symbolic kernel of bin b over list[begin, begin + n).
 void launch_symbolic_bin(const SymArgs &a, int bin, int32_t begin, int32_t n, cudaStream_t s,
                          int *launches) {
@@ -2687,10 +2758,8 @@ void launch_symbolic_bin(const SymArgs &a, int bin, int32_t begin, int32_t n, cu
             // Persistent: as many CTAs as fit on the GPU at once (two per SM
             // with the widest window), rows taken from a counter.
             const int wb = wide_window_bits(a.B.n);
-            const size_t smem = kSmemWideBase + (size_t)wb / 8 + 4 * (size_t)wide_touch_cap(wb) + 4 * kWideThreads;
-            const int per_sm = std::max(1, std::min(2048 / kWideThreads, (int)((227 * 1024) / (smem + 1024))));
-            const int grid = (int)std::min<int64_t>(n, (int64_t)std::max(a.numSms, 1) * per_sm);
-            k_sym_wide<kWideThreads><<<(unsigned)grid, kWideThreads, smem, s>>>(a, begin, n, wb);
+            const int grid = (int)std::min<int64_t>(n, wide_grid(wb, a.numSms));
+            k_sym_wide<kWideThreads, false><<<(unsigned)grid, kWideThreads, smem_wide(wb), s>>>(a, begin, n, wb);
             break;
         }
         default:
@@ -2750,9 +2819,10 @@ void launch_symbolic_bin_dd(const SymArgs &a, int bin, cudaStream_t s, int *laun
         }
         case SB_WIDE: {
             const int wb = wide_window_bits(a.B.n);
-            const size_t smem = kSmemWideBase + (size_t)wb / 8 + 4 * (size_t)wide_touch_cap(wb) + 4 * kWideThreads;
-            const int grid = resident_grid((const void *)k_sym_wide<kWideThreads>, kWideThreads, smem, a.numSms);
-            k_sym_wide<kWideThreads><<<(unsigned)grid, kWideThreads, smem, s>>>(a, -1, 0, wb);
+            const size_t smem = smem_wide(wb);
+            const void *fn = (const void *)k_sym_wide<kWideThreads, false>;
+            k_sym_wide<kWideThreads, false>
+                <<<(unsigned)resident_grid(fn, kWideThreads, smem, a.numSms), kWideThreads, smem, s>>>(a, -1, 0, wb);
             break;
         }
         default:
@@ -2846,8 +2916,7 @@ void prepare_dd_grids(const Tuning &t, int64_t bcols, int sms) {
     resident_grid((const void *)k_sym_flagw_dd<kBitwRows>, 32 * kBitwRows, 0, sms);
     resident_grid((const void *)k_sym_hash_warp_dd<kSymWarpRows, kSymWarpTable>, 32 * kSymWarpRows, kSmemSymWarp, sms);
     resident_grid((const void *)k_sym_hash_cta_dd<kSymCtaThreads, kSymCtaTable>, kSymCtaThreads, kSmemSymCta, sms);
-    resident_grid((const void *)k_sym_wide<kWideThreads>, kWideThreads,
-                  kSmemWideBase + (size_t)wb / 8 + 4 * (size_t)wide_touch_cap(wb) + 4 * kWideThreads, sms);
+    resident_grid((const void *)k_sym_wide<kWideThreads, false>, kWideThreads, smem_wide(wb), sms);
     resident_grid((const void *)k_num_tiny_dd, 32 * kNumTinyWarps, 0, sms);
     resident_grid((const void *)k_num_hash_warp_dd<kNumWarpRows, kNumWarpTable>, 32 * kNumWarpRows, kSmemNumWarp, sms);
     resident_grid((const void *)k_num_densew_dd<kDensewRows>, 32 * kDensewRows, 0, sms);

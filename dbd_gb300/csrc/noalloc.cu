@@ -229,7 +229,7 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     mail.to = box;
     mail.ctl = ctl;
     mail.binStart = symStart;
-    launch_sym_lists(m, sb, ri, rowNnz, nullptr, 0, nullptr, mail, s);
+    launch_sym_lists(m, sb, ri, rowNnz, nullptr, 0, nullptr, nullptr, mail, s);
     NA_CK(cudaStreamSynchronize(s));
     NA_CK(cudaGetLastError());
     for (const int32_t *f : {box->flags + CTL_A, box->flags + CTL_B}) {
