@@ -452,6 +452,8 @@ void launch_row_digest(int64_t r0, int64_t r1, const int64_t *Cp, int64_t outBas
                        const float *Cv, int64_t ncols, const RowDigest &d, cudaStream_t s, int num_sms);
 // dst[i] = src[i] rounded to float32, i < n.
 void launch_val_to_f32(const double *src, float *dst, int64_t n, cudaStream_t s, int num_sms);
+// The same into pinned host memory, at the host link's rate.
+void launch_val_to_host_f32(const double *src, float *dst, int64_t n, cudaStream_t s);
 
 // *acc += sum over i < n of mix64(((uint64)i << 32 | w[i]) ^ (salt * G)) (an
 // order-dependent hash of a device array of 32-bit words).

@@ -1009,10 +1009,12 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
     // out: one slot takes the whole remaining budget.  The copying scopes
     // keep two device slots (a chunk computes while the previous one is
     // copied) and two host ring slots, each a sixth of C's host bytes
-    // clamped to [1, 6] GiB (and within both budgets): at least six chunks
-    // overlap their copies with compute when C is small, and a large C
-    // keeps its chunks large (slots of 11.5 GiB copied slower than 6 GiB
-    // ones).
+    // clamped to 6 GiB (and within both budgets): at least six chunks
+    // overlap their copies with compute, and a large C keeps its chunks
+    // large (slots of 11.5 GiB copied slower than 6 GiB ones).  A slot is no
+    // less than 1 GiB where files are written, 128 MiB (0.7 ms of the host
+    // link) where C only crosses the link: 539 MB of C take 4.75 ms as one
+    // chunk, 4.20 ms as five.
     const int nslots_dev = copies ? 2 : 1;
     if (resident) {
         Chunk ch{0, m, 0, nnz};
@@ -1020,7 +1022,8 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
     } else {
         double slot_entries_f = std::max(0.0, dev_avail) / nslots_dev / dev_bpe;
         if (copies) {
-            double host_slot = std::min(6.0 * kGiB, std::max(1.0 * kGiB, host_bpe * (double)nnz / 6.0));
+            const double least = (scope == DBD_SCOPE_D2H ? 0.125 : 1.0) * kGiB;
+            double host_slot = std::min(6.0 * kGiB, std::max(least, host_bpe * (double)nnz / 6.0));
             if (!(scope == DBD_SCOPE_D2H && host_fits)) host_slot = std::min(host_slot, host_budget / 2.0);
             slot_entries_f = std::min(slot_entries_f, host_slot / host_bpe);
         }
@@ -1057,7 +1060,10 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
     const size_t slot_entries = resident ? (size_t)std::max<int64_t>(nnz, 1) : (size_t)cap_entries;
     CK(c, c->Ci.ensure(sizeof(int32_t) * slot_entries * nslots));
     CK(c, c->Cv.ensure(sizeof(double) * slot_entries * nslots));
-    if (f32out) CK(c, c->Cf.ensure(sizeof(float) * slot_entries * nslots));
+    // A device digest reads the float values on the device; otherwise they are
+    // rounded on their way to the host.
+    const bool devF32 = f32out && (c->digest & DBD_DIGEST_DEVICE) != 0;
+    if (devF32) CK(c, c->Cf.ensure(sizeof(float) * slot_entries * nslots));
     c->dev_resident = resident;
     c->host_f32 = f32out;
 
@@ -1189,8 +1195,8 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
             cudaStreamWaitEvent(c->stream, evCopy[i - nslots], 0);
         cudaEventRecord(evNum0[i], c->stream);
         numeric_rows(c, ch.r0, ch.r1, ch.c0, dCi, dCv);
-        float *dCf = f32out ? c->Cf.as<float>() + (size_t)ds * slot_entries : nullptr;
-        if (f32out && ch.c1 > ch.c0) {
+        float *dCf = devF32 ? c->Cf.as<float>() + (size_t)ds * slot_entries : nullptr;
+        if (devF32 && ch.c1 > ch.c0) {
             launch_val_to_f32(dCv, dCf, ch.c1 - ch.c0, c->stream, c->num_sms);
             c->launches++;
         }
@@ -1234,10 +1240,16 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
         if (n > 0) {
             cudaError_t e1 = cudaMemcpyAsync(hCi, dCi, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost,
                                              c->copy_stream);
-            cudaError_t e2 = f32out ? cudaMemcpyAsync(hCv, dCf, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost,
-                                                      c->copy_stream)
-                                    : cudaMemcpyAsync(hCv, dCv, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost,
-                                                      c->copy_stream);
+            cudaError_t e2 = cudaSuccess;
+            if (devF32) {
+                e2 = cudaMemcpyAsync(hCv, dCf, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, c->copy_stream);
+            } else if (f32out) {
+                launch_val_to_host_f32(dCv, reinterpret_cast<float *>(hCv), n, c->copy_stream);
+                e2 = cudaGetLastError();
+                c->launches++;
+            } else {
+                e2 = cudaMemcpyAsync(hCv, dCv, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, c->copy_stream);
+            }
             if (e1 != cudaSuccess || e2 != cudaSuccess) loop_rc = cuda_fail(c, e1 != cudaSuccess ? e1 : e2, "D2H");
         }
         cudaEventRecord(evCopy[i], c->copy_stream);
@@ -1361,6 +1373,13 @@ const char *dbd_error_string(int code) {
 
 const char *dbd_last_error(const dbd_ctx *ctx) { return ctx ? ctx->last_error.c_str() : ""; }
 
+// The copies' stream: its rounding kernels' CTAs go ahead of the next chunk's.
+static cudaError_t create_copy_stream(cudaStream_t *s) {
+    int least = 0, greatest = 0;
+    cudaError_t e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    return e != cudaSuccess ? e : cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, greatest);
+}
+
 int dbd_create(const dbd_config *cfg_in, dbd_ctx **out) {
     if (!out) return DBD_ERR_INVALID;
     *out = nullptr;
@@ -1377,7 +1396,7 @@ int dbd_create(const dbd_config *cfg_in, dbd_ctx **out) {
     c->cfg = cfg;
     cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, cfg.device);
     if (cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking) != cudaSuccess) {
+        create_copy_stream(&c->copy_stream) != cudaSuccess) {
         delete c;
         return DBD_ERR_CUDA;
     }
