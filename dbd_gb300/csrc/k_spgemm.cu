@@ -96,6 +96,9 @@ constexpr int kWideLoads = 4;
 constexpr int kHashWarpLoads = 2;
 // Warp-hash rows of at most this many products are sorted instead of hashed.
 constexpr int kEscMax = 512;
+constexpr int kEscShift = 9;  // bits of a product's number in their keys
+// Mean B row length from which their products are listed by groups of lanes.
+constexpr int kEscGroupLen = 6;
 
 // Position in B of product t (all lanes call; result valid when t < total).
 __device__ __forceinline__ int32_t chunk_pos(const Chunk &c, int32_t t, double *a_out) {
@@ -1118,7 +1121,8 @@ constexpr size_t warp_hash_bytes(int table) { return 12 * (size_t)table; }
 // runs of neighbouring lanes are merged: the first step of a merge compares
 // mirrored positions, the others positions one stride apart (Batcher's
 // bitonic merge, all comparators the same way round), strides of R and more
-// by shuffles, shorter ones inside the lane.
+// by shuffles, shorter ones inside the lane.  R need not be a power of two: the
+// runs' lengths halve down to a lane's R, which it sorts again.
 template <int R, class K>
 __device__ __forceinline__ void warp_sort(K (&key)[R]) {
     const int lane = threadIdx.x & 31;
@@ -1128,28 +1132,34 @@ __device__ __forceinline__ void warp_sort(K (&key)[R]) {
         K other[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) other[r] = __shfl_xor_sync(FULL, key[R - 1 - r], m - 1);
+        // The lower lane keeps the smaller key: one compare against the lane's
+        // side and one select (a minimum, a maximum and a select otherwise).
         const bool low = (lane & (m >> 1)) == 0;
 #pragma unroll
-        for (int r = 0; r < R; ++r) key[r] = low ? min(key[r], other[r]) : max(key[r], other[r]);
+        for (int r = 0; r < R; ++r) key[r] = (other[r] < key[r]) == low ? other[r] : key[r];
 #pragma unroll
         for (int d = m >> 2; d >= 1; d >>= 1) {
             const bool lo = (lane & d) == 0;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const K x = __shfl_xor_sync(FULL, key[r], d);
-                key[r] = lo ? min(key[r], x) : max(key[r], x);
+                key[r] = (x < key[r]) == lo ? x : key[r];
             }
         }
+        if constexpr ((R & (R - 1)) == 0) {
 #pragma unroll
-        for (int d = R >> 1; d >= 1; d >>= 1) {
+            for (int d = R >> 1; d >= 1; d >>= 1) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                if ((r & d) == 0) {
-                    const K lo = min(key[r], key[r + d]), hi = max(key[r], key[r + d]);
-                    key[r] = lo;
-                    key[r + d] = hi;
+                for (int r = 0; r < R; ++r) {
+                    if ((r & d) == 0) {
+                        const K lo = min(key[r], key[r + d]), hi = max(key[r], key[r + d]);
+                        key[r] = lo;
+                        key[r + d] = hi;
+                    }
                 }
             }
+        } else {
+            merge_exchange<R, 1, 1>(key);
         }
     }
 }
@@ -1159,64 +1169,115 @@ __device__ __forceinline__ void warp_sort(K (&key)[R]) {
 // so that neither hits a bank more than twice.
 __device__ __forceinline__ int rotated(int p) { return (p & ~31) | ((p + (p >> 5)) & 31); }
 
-// A row of at most 32 R products by one warp without a hash table (expand,
-// sort, compress): every product's value goes to shared memory and its
-// (column, product) key is sorted in registers (warp_sort), which puts equal
-// columns next to each other in Gustavson order.  A lane sums the runs inside
-// its R keys; a run over several lanes is finished by the lane that holds its
-// first key, from the others' leading sums.  The row's entries are gathered in
-// shared memory and written 32 consecutive ones a step.
+// Rows of at most kEscMax products by one warp without a hash table (expand,
+// sort, compress): every product's value goes to shared memory (esc_list) and
+// its (column, product) key is sorted in registers, 32 R of them (esc_sort,
+// warp_sort), which puts equal columns next to each other in Gustavson order.
+// A lane sums the runs inside its R keys; a run over several lanes is finished
+// by the lane that holds its first key, from the others' leading sums.  The
+// row's entries are gathered in shared memory and written 32 consecutive ones
+// a step.
 //
 // A bucket counting sort in shared memory with each lane writing R
 // consecutive entries, the form before, was bound by the L1: 60M bank
 // conflicts and 20M store requests for 100k rows of 256 products (91% of L1
-// throughput busy): 455 -> 227 us, 550k rows of about 144 products 1611 ->
-// 1106 us.  What bounds it now is latency, at 32 warps an SM (64 registers, 6 KB
-// a warp; at 92 registers and 20 warps 272 us).  kbuf and pv
-// hold 32 R entries each; columns lie in [rlo, rlo + 2^(bits of K - log2(32 R))).
-template <int R, class K>
-__device__ __forceinline__ void esc_row(const NumArgs &a, int32_t row, int32_t e0, int32_t e1, int n, int32_t rlo,
-                                        K *kbuf, double *pv) {
-    constexpr int N = 32 * R;
-    constexpr int SHIFT = ilog2(N);
-    constexpr K NONE = ~K(0);
-    constexpr int U = R < 4 ? R : 4;  // steps of B loads in flight
+// throughput busy): 455 -> 195 us, 550k rows of about 144 products 1611 ->
+// 973 us.  What bounds it now is instruction issue (65% busy, the ALU 68%) and
+// latency, at 32 warps an SM (64 registers, 6 KB a warp; at 92 registers and
+// 20 warps 272 us).  kbuf and pv hold a product each; columns lie in
+// [rlo, rlo + 2^(bits of K - kEscShift)).
+template <class K>
+__device__ __forceinline__ void esc_list(const NumArgs &a, int32_t e0, int32_t e1, int n, int32_t rlo, K *kbuf,
+                                         double *pv) {
     const int lane = threadIdx.x & 31;
     int32_t tb = 0;  // products of the earlier chunks
-    for (int32_t e = e0; e < e1; e += 32) {
-        const Chunk c = load_chunk(a.A, a.B, e, e1, lane);
-        for (int32_t t0 = 0; t0 < c.total; t0 += 32 * U) {
-            int32_t j[U];
-            double av[U];
+    if (n >= kEscGroupLen * (e1 - e0)) {
+        // Eight lanes an entry, two entries a group and two products of each
+        // a lane in flight: no search for a product's entry.
+        const int sub = lane & 7, grp = lane >> 3;
+        for (int32_t e = e0; e < e1; e += 32) {
+            const Chunk c = load_chunk(a.A, a.B, e, e1, lane);
+            const int32_t ex = tb + c.incl - c.len;
+            const int ne = min(32, e1 - e);
+            for (int q = 0; q < ne; q += 8) {
+                int32_t at[2], t[2], len[2];
+                double av[2];
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                j[u] = -1;
-                av[u] = 0.0;
-                const int32_t t = t0 + 32 * u + lane;
-                if (t0 + 32 * u < c.total) {
-                    const int32_t jj = chunk_pos(c, t, &av[u]);
-                    if (t < c.total && tb + t < n) j[u] = jj;
+                for (int h = 0; h < 2; ++h) {
+                    const int o = q + 4 * h + grp;  // lanes past the chunk's entries hold none
+                    at[h] = __shfl_sync(FULL, c.bs, o);
+                    len[h] = __shfl_sync(FULL, c.len, o);
+                    t[h] = __shfl_sync(FULL, ex, o);
+                    av[h] = __shfl_sync(FULL, c.a, o);
+                    len[h] = min(len[h], n - t[h]);
+                }
+                const int32_t most = max(len[0], len[1]);
+                for (int32_t i0 = sub; i0 < most; i0 += 16) {
+                    int32_t col[4];
+                    double bv[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int h = u >> 1, i = i0 + 8 * (u & 1);
+                        col[u] = i < len[h] ? __ldg(&a.B.idx[at[h] + i]) : 0;
+                        bv[u] = i < len[h] ? __ldg(&a.B.val[at[h] + i]) : 0.0;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int h = u >> 1, i = i0 + 8 * (u & 1);
+                        if (i < len[h]) {
+                            const int x = t[h] + i;
+                            kbuf[x] = (K)(uint32_t)(col[u] - rlo) << kEscShift | (K)x;
+                            pv[x] = __dmul_rn(av[h], bv[u]);
+                        }
+                    }
                 }
             }
-            int32_t col[U];
-            double bv[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                col[u] = j[u] >= 0 ? __ldg(&a.B.idx[j[u]]) : 0;
-                bv[u] = j[u] >= 0 ? __ldg(&a.B.val[j[u]]) : 0.0;
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (j[u] >= 0) {
-                    const int t = tb + t0 + 32 * u + lane;
-                    kbuf[t] = (K)(uint32_t)(col[u] - rlo) << SHIFT | (K)t;
-                    pv[t] = __dmul_rn(av[u], bv[u]);
-                }
-            }
+            tb += c.total;
         }
-        tb += c.total;
+    } else {
+        constexpr int U = 4;  // steps of B loads in flight
+        for (int32_t e = e0; e < e1; e += 32) {
+            const Chunk c = load_chunk(a.A, a.B, e, e1, lane);
+            for (int32_t t0 = 0; t0 < c.total; t0 += 32 * U) {
+                int32_t j[U];
+                double av[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    j[u] = -1;
+                    av[u] = 0.0;
+                    const int32_t t = t0 + 32 * u + lane;
+                    if (t0 + 32 * u < c.total) {
+                        const int32_t jj = chunk_pos(c, t, &av[u]);
+                        if (t < c.total && tb + t < n) j[u] = jj;
+                    }
+                }
+                int32_t col[U];
+                double bv[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    col[u] = j[u] >= 0 ? __ldg(&a.B.idx[j[u]]) : 0;
+                    bv[u] = j[u] >= 0 ? __ldg(&a.B.val[j[u]]) : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (j[u] >= 0) {
+                        const int t = tb + t0 + 32 * u + lane;
+                        kbuf[t] = (K)(uint32_t)(col[u] - rlo) << kEscShift | (K)t;
+                        pv[t] = __dmul_rn(av[u], bv[u]);
+                    }
+                }
+            }
+            tb += c.total;
+        }
     }
     __syncwarp();
+}
+
+template <int R, class K>
+__device__ __forceinline__ void esc_sort(const NumArgs &a, int32_t row, int n, int32_t rlo, K *kbuf, double *pv) {
+    constexpr int SHIFT = kEscShift;
+    constexpr K NONE = ~K(0);
+    const int lane = threadIdx.x & 31;
     K key[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) key[r] = 32 * r + lane < n ? kbuf[32 * r + lane] : NONE;
@@ -1228,7 +1289,7 @@ __device__ __forceinline__ void esc_row(const NumArgs &a, int32_t row, int32_t e
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const bool valid = R * lane + r < n;
-        v[r] = valid ? pv[(int)(key[r] & (K)(N - 1))] : 0.0;
+        v[r] = valid ? pv[min((int)(key[r] & (K)((1 << SHIFT) - 1)), 32 * R - 1)] : 0.0;
         const K prev = r > 0 ? key[r > 0 ? r - 1 : 0] : before;
         if (valid && ((r == 0 && lane == 0) || (key[r] >> SHIFT) != (prev >> SHIFT))) heads |= 1u << r;
     }
@@ -1238,7 +1299,9 @@ __device__ __forceinline__ void esc_row(const NumArgs &a, int32_t row, int32_t e
     double lead = 0.0;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        if (R * lane + r < n && !((heads >> r) & 1u)) {
+        const bool more = R * lane + r < n && !((heads >> r) & 1u);
+        if (!__any_sync(FULL, more)) continue;  // an addition takes the FP64 pipe 16 clocks, needed or not
+        if (more) {
             if ((heads & ((1u << r) - 1u)) == 0u) lead += v[r];
             else v[r] += v[r > 0 ? r - 1 : 0];
         }
@@ -1304,27 +1367,27 @@ __device__ __forceinline__ void num_hash_warp_rows(const NumArgs &a, int32_t lo,
     const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
     // Expand-sort-compress where the products fit the registers and the
     // columns the keys; the table takes the others.
-    static_assert(TABLE >= kEscMax, "the table's arrays hold the products");
+    static_assert(TABLE >= kEscMax && (1 << kEscShift) >= kEscMax, "the arrays and keys hold the products");
     const int64_t P = a.rowP[row];
     if (P <= kEscMax) {
         const int32_t rlo = a.rowLo[row];
         const int64_t span = (int64_t)a.rowHi[row] - rlo + 1;
         uint32_t *kb = reinterpret_cast<uint32_t *>(keys);
-        if (P <= 128 && span < (1 << 25)) {
-            esc_row<4, uint32_t>(a, row, e0, e1, (int)P, rlo, kb, vals);
-            return;
-        }
-        if (P <= 256 && span < (1 << 24)) {
-            esc_row<8, uint32_t>(a, row, e0, e1, (int)P, rlo, kb, vals);
+        // Three sizes and one listing: warps of an SM that run different code
+        // miss the instruction cache.  550k rows of 60 to 280 products: 0.97 ms;
+        // with 2, 4, 5, 6, 8 and 16 keys a lane, each with its own listing,
+        // 2.05 ms; with 8 and 16 only 1.02 ms.
+        if (span < ((int64_t)1 << (32 - kEscShift))) {
+            esc_list<uint32_t>(a, e0, e1, (int)P, rlo, kb, vals);
+            if (P <= 192) esc_sort<6, uint32_t>(a, row, (int)P, rlo, kb, vals);
+            else if (P <= 256) esc_sort<8, uint32_t>(a, row, (int)P, rlo, kb, vals);
+            else esc_sort<16, uint32_t>(a, row, (int)P, rlo, kb, vals);
             return;
         }
         if (P <= 256) {
-            esc_row<8, unsigned long long>(a, row, e0, e1, (int)P, rlo, reinterpret_cast<unsigned long long *>(keys),
-                                           vals);
-            return;
-        }
-        if (span < (1 << 23)) {
-            esc_row<16, uint32_t>(a, row, e0, e1, (int)P, rlo, kb, vals);
+            unsigned long long *kb64 = reinterpret_cast<unsigned long long *>(keys);
+            esc_list<unsigned long long>(a, e0, e1, (int)P, rlo, kb64, vals);
+            esc_sort<8, unsigned long long>(a, row, (int)P, rlo, kb64, vals);
             return;
         }
     }
