@@ -236,6 +236,7 @@ struct SymArgs {
     const int32_t *rowLo = nullptr;  // per-row column window (RowInfo)
     const int32_t *rowHi = nullptr;
     const int64_t *rowP = nullptr;   // per-row products (RowInfo)
+    const int2 *bRange = nullptr;    // first and last column of every row of B
     // Optional store of the wide rows' column bitmaps for the numeric rank
     // kernel (null: not kept): kRankWordsMax words per wide row (the row's
     // window from word lo/32 on), at the row's position in the wide bin;

@@ -605,6 +605,7 @@ int symbolic(dbd_ctx *c) {
     sa.err = c->err();
     sa.rowLo = c->rowLo.as<int32_t>();
     sa.rowP = c->rowP.as<int64_t>();
+    sa.bRange = (c->b_is_a ? c->A : c->B).range.as<int2>();
     sa.rowHi = c->rowHi.as<int32_t>();
     sa.tune = c->tune;
     // Slab counts of heavy rows for the dense bin's pieces (rank windows,
@@ -2135,6 +2136,7 @@ int dbd_batch_enqueue(dbd_ctx *c, void *stream) {
     sa.rowLo = c->rowLo.as<int32_t>();
     sa.rowHi = c->rowHi.as<int32_t>();
     sa.rowP = c->rowP.as<int64_t>();
+    sa.bRange = (c->b_is_a ? c->A : c->B).range.as<int2>();
     sa.tune = c->tune;
     sa.numSms = c->num_sms;
     sa.bSorted = 0;

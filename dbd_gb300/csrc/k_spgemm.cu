@@ -793,23 +793,32 @@ __global__ void __launch_bounds__(THREADS) k_sym_wide(SymArgs a, int32_t begin, 
 // [first_i, last_i] beyond every earlier run's end).  One warp, 32 entries a
 // step, no per-column work.  Returns false (count unset) when some B row is
 // not one run or the first columns decrease; B's rows must ascend strictly.
-__device__ __forceinline__ bool interval_union_count(const CsrDev &A, const CsrDev &B, int32_t e0, int32_t e1,
-                                                     int lane, int *count) {
+// The runs' ends come from the row ranges, loaded beside the row pointers
+// (B's columns would have to wait for them), and a step whose runs' ends
+// do not decrease either (a band's) needs no prefix maxima.  970k rows of 65
+// entries: 577 -> 344 us.
+__device__ __forceinline__ bool interval_union_count(const CsrDev &A, const CsrDev &B, const int2 *range, int32_t e0,
+                                                     int32_t e1, int lane, int *count) {
     int32_t endMax = INT32_MIN, firstMax = INT32_MIN;  // over the entries of earlier steps
-    int cnt = 0;
+    int add = 0;  // this lane's part of the union
     for (int32_t eb = e0; eb < e1; eb += 32) {
-        bool has = false;
-        int32_t f = INT32_MIN, l = INT32_MIN;
-        bool run = true;
-        if (eb + lane < e1) {
-            const int32_t k = A.idx[eb + lane];
-            const int32_t bs = B.ptr[k], len = B.ptr[k + 1] - bs;
-            if (len > 0) {
-                has = true;
-                f = __ldg(&B.idx[bs]);
-                l = __ldg(&B.idx[bs + len - 1]);
-                run = l - f == len - 1;
-            }
+        const int32_t k = eb + lane < e1 ? __ldg(&A.idx[eb + lane]) : -1;
+        const int32_t len = k >= 0 ? __ldg(&B.ptr[k + 1]) - __ldg(&B.ptr[k]) : 0;
+        const int2 r = k >= 0 ? __ldg(&range[k]) : make_int2(0, 0);
+        const bool has = len > 0;
+        const int32_t f = has ? r.x : INT32_MIN, l = has ? r.y : INT32_MIN;
+        const bool run = !has || l - f == len - 1;
+        int32_t fPrev = __shfl_up_sync(FULL, f, 1), lPrev = __shfl_up_sync(FULL, l, 1);
+        if (lane == 0) {
+            fPrev = firstMax;
+            lPrev = endMax;
+        }
+        const int last = min(31, e1 - eb - 1);
+        if (__all_sync(FULL, lane > last || (has && run && f >= fPrev && l >= lPrev))) {
+            if (has) add += (int)((long long)l - max((long long)f - 1, (long long)lPrev));
+            firstMax = __shfl_sync(FULL, f, last);
+            endMax = __shfl_sync(FULL, l, last);
+            continue;
         }
         // Inclusive prefix maxima of the first and last columns over lanes.
         int32_t fm = f, lm = l;
@@ -821,7 +830,8 @@ __device__ __forceinline__ bool interval_union_count(const CsrDev &A, const CsrD
                 lm = max(lm, yl);
             }
         }
-        int32_t fPrev = __shfl_up_sync(FULL, fm, 1), lPrev = __shfl_up_sync(FULL, lm, 1);
+        fPrev = __shfl_up_sync(FULL, fm, 1);
+        lPrev = __shfl_up_sync(FULL, lm, 1);
         if (lane == 0) {
             fPrev = INT32_MIN;
             lPrev = INT32_MIN;
@@ -829,13 +839,11 @@ __device__ __forceinline__ bool interval_union_count(const CsrDev &A, const CsrD
         fPrev = max(fPrev, firstMax);
         lPrev = max(lPrev, endMax);
         if (!__all_sync(FULL, run && (!has || f >= fPrev))) return false;
-        int add = 0;
-        if (has) add = (int)max(0LL, (long long)l - max((long long)f - 1, (long long)lPrev));
-        cnt += warp_sum_i(add);
+        if (has) add += (int)max(0LL, (long long)l - max((long long)f - 1, (long long)lPrev));
         firstMax = max(firstMax, __shfl_sync(FULL, fm, 31));
         endMax = max(endMax, __shfl_sync(FULL, lm, 31));
     }
-    *count = cnt;
+    *count = warp_sum_i(add);
     return true;
 }
 
@@ -877,19 +885,19 @@ __device__ __forceinline__ void sym_flagw_rows(const SymArgs &a, int32_t begin, 
     const int32_t base = (rlo >> 5) << 5;
     const int sw = min(span_words(rlo, a.rowHi[row]), kWarpSpanWords);
     const uint32_t nb = (uint32_t)sw * 32u;
-    for (int i = lane; i < sw * 8; i += 32) fw[i] = 0u;
-    __syncwarp();
     const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
     const bool rowwise = a.rowP[row] >= (int64_t)kRowwiseMinLen * (e1 - e0);
     int *err = a.err;
     const int32_t *bidx = a.B.idx;
     if (rowwise && b_sorted(a)) {
         int cnt;
-        if (interval_union_count(a.A, a.B, e0, e1, lane, &cnt)) {
+        if (interval_union_count(a.A, a.B, a.bRange, e0, e1, lane, &cnt)) {
             if (lane == 0) a.rowNnz[row] = cnt;
             return;
         }
     }
+    for (int i = lane; i < sw * 8; i += 32) fw[i] = 0u;
+    __syncwarp();
     if (rowwise) {
         // One A entry at a time.  A B row whose columns form one contiguous
         // run (banded and stencil matrices) flags its run a word (4 columns)

@@ -253,6 +253,7 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     sa.err = err;
     sa.rowLo = ri.lo;
     sa.rowP = ri.rowP;
+    sa.bRange = range;
     sa.rowHi = ri.hi;
     int launches = 0;
     for (int bin = SB_TINY; bin < SB_COUNT; ++bin)
