@@ -1514,24 +1514,27 @@ __global__ void __launch_bounds__(THREADS) k_num_hash_cta_dd(NumArgs a, int bin)
 
 // Rank rows (windows of at most 2^18 columns): one CTA per row.  The row's
 // columns are bits of a shared bitmap over its window (kept by the symbolic
-// pass, or set here by a pass over the products); each thread takes its own
-// consecutive words into registers, and a scan of their counts ranks every
-// pair of words, which gives a column's position in C's row by one 64-bit
-// load and a bit count.  Columns are written balanced by position, and a pass
-// over the products adds each one into C's row in place by an FP64 reduction
-// at L2.  No hashing, no sorting, no values in shared memory.
+// pass, or set here by a pass over the products); a scan of the words' counts
+// ranks every pair of words, which gives a column's position in C's row by
+// one 64-bit load and a bit count.  Columns are written balanced by position,
+// and a pass over the products adds each one into C's row in place by an FP64
+// reduction at L2.  No hashing, no sorting, no values in shared memory.
 //
 // P is the type of the pairs' ranks: 16 bits for the rows of the small CTAs
-// (at most kNumCtaLMax entries), which with 44 KB a CTA puts five of them on
-// an SM; a row is a chain of short phases with barriers between them, so what
-// bounds it is how many rows an SM has in flight.  Rows of up to 4096 entries used to
-// accumulate in shared memory (compare-and-swap loops around a multiply-add,
-// 102 KB and 256 threads a CTA, two CTAs per SM): R-MAT 2^18, 57k such rows
-// 3.13 -> 1.70 ms; 33k larger ones (512 threads, two CTAs an SM: three
-// spill and take 5.4) 5.01 -> 4.76 ms, where the reductions' 25 sectors a step
-// keep L1 at 62% and L2 at 54% of their throughput.
-// CTAs an SM is to hold: 64 registers a thread for the small ones.
-__host__ __device__ constexpr int rank_ctas(int threads) { return threads == 256 ? 4 : 2; }
+// (at most kNumCtaLMax entries), which with 44 KB a CTA at the widest window
+// puts five of them on an SM, six at narrower ones; a row is a chain of short
+// phases with barriers between them, so what bounds it is how many rows an SM
+// has in flight, as long as the ranking is free of bank conflicts.  Such rows
+// used to accumulate in shared memory (compare-and-swap loops around a
+// multiply-add, 102 KB and 256 threads a CTA, two CTAs per SM): 57k of R-MAT
+// 2^18 3.13 -> 1.37 ms, 18k of 2^16 0.55 -> 0.28.  The larger rows (512
+// threads, two CTAs an SM) are bound by the reductions' 25 sectors a step and
+// by what of C and B stays in L2 meanwhile: C's values are zeroed right before
+// the products, not earlier (33k rows of 2^18 4.76 -> 4.60 ms; 5.01 with the
+// ranks a group of words a thread), and a third CTA an SM, which 2^16 gains
+// 3% from, costs 2^18 6%.
+// CTAs an SM is to hold: 40 registers a thread for the small ones.
+__host__ __device__ constexpr int rank_ctas(int threads) { return threads == 256 ? 6 : 2; }
 
 // Where the rank kernel's bitmap starts behind the staging area.
 __host__ __device__ constexpr size_t rank_bits_at(int threads) {
@@ -1543,15 +1546,14 @@ __device__ __forceinline__ void num_rank_rows(const NumArgs &a, int32_t lo, int 
     extern __shared__ __align__(16) unsigned char smem[];
     using L = StageLayout<THREADS>;
     constexpr int NW = THREADS / 32;
-    constexpr int kWpt = kRankWordsMax / THREADS;  // words a thread owns at most
     __shared__ int32_t sh[NW];
     int32_t *pre = reinterpret_cast<int32_t *>(smem + L::pre);
     int32_t *bst = reinterpret_cast<int32_t *>(smem + L::bst);
     double *av = reinterpret_cast<double *>(smem + L::av);
     uint32_t *bits = reinterpret_cast<uint32_t *>(smem + rank_bits_at(THREADS));
     P *pairRank = reinterpret_cast<P *>(bits + maxWords);
-    // Per thread, the rank of its first column and its non-empty words, kept
-    // in the staging area (idle between the passes).
+    // Per group of words, the rank of its first column and its non-empty
+    // words, kept in the staging area (idle between the passes).
     static_assert(8 * THREADS <= L::bytes && kRankWordsMax <= 32 * THREADS, "rank groups");
     int32_t *tbase = pre;
     uint32_t *tmask = reinterpret_cast<uint32_t *>(pre + THREADS);
@@ -1570,7 +1572,7 @@ __device__ __forceinline__ void num_rank_rows(const NumArgs &a, int32_t lo, int 
 
     const bool kept = a.wideBits && sym_bin_of(a.rowP[row], e1 - e0, nwords, a.tune) == SB_WIDE;
     if (!kept) {
-        for (int i = tid; i < nwords; i += THREADS) bits[i] = 0u;
+        for (int i = tid; 4 * i < nwords; i += THREADS) reinterpret_cast<uint4 *>(bits)[i] = make_uint4(0u, 0u, 0u, 0u);
         for (int32_t eb = e0; eb < e1; eb += THREADS) {
             int nb;
             const int32_t total =
@@ -1586,59 +1588,68 @@ __device__ __forceinline__ void num_rank_rows(const NumArgs &a, int32_t lo, int 
             __syncthreads();
         }
     }
-    // C's values start at zero; the stores run while the row is ranked.
-    for (int i = tid; i < expect; i += THREADS) cv[i] = 0.0;
 
-    // This thread's words [w0, w0 + wpt), wpt a power of two of at least 4
-    // with THREADS * wpt >= nwords.
-    int wpt = 4;
-    while (wpt * THREADS < nwords) wpt <<= 1;
-    const int w0 = tid * wpt;
-    const uint32_t *src = kept ? a.wideBits + (size_t)a.wideSlot[row] * kRankWordsMax : bits;
-    uint32_t x[kWpt];
-    uint32_t mask = 0u;
+    // A warp ranks 32 groups of wpt words (a power of two of at least 4 with
+    // THREADS * wpt >= nwords), 128 consecutive words a step, four a lane.
+    // (With a group a thread, wide windows pay 8- and 16-way bank conflicts
+    // at each load and store: 57k rows of 2^18 1.74 ms instead of 1.39.)
+    int wpt = 4, lg = 2;
+    while (wpt * THREADS < nwords) wpt <<= 1, ++lg;
+    const int lane = tid & 31, n4 = wpt >> 2;
+    const int w0 = (tid >> 5) * 32 * wpt + 4 * lane;
     int32_t cnt = 0;
-#pragma unroll
-    for (int k = 0; k < kWpt; k += 4) {
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (k < wpt && w0 + k < nwords) {
-            v = kept ? __ldcs(reinterpret_cast<const uint4 *>(src + w0 + k))
-                     : *reinterpret_cast<const uint4 *>(src + w0 + k);
-            // Words past the window hold another row's bits.
-            if (w0 + k + 1 >= nwords) v.y = 0u;
-            if (w0 + k + 2 >= nwords) v.z = 0u;
-            if (w0 + k + 3 >= nwords) v.w = 0u;
+    const uint32_t *src = kept ? a.wideBits + (size_t)a.wideSlot[row] * kRankWordsMax : nullptr;
+#pragma unroll 4
+    for (int j = 0; j < n4; ++j) {
+        const int i = w0 + 128 * j;
+        if (i < nwords) {
+            uint4 v;
+            if (kept) {
+                v = __ldcs(reinterpret_cast<const uint4 *>(src + i));
+                // Words past the window hold another row's bits.
+                if (i + 1 >= nwords) v.y = 0u;
+                if (i + 2 >= nwords) v.z = 0u;
+                if (i + 3 >= nwords) v.w = 0u;
+                *reinterpret_cast<uint4 *>(bits + i) = v;
+            } else {
+                v = *reinterpret_cast<const uint4 *>(bits + i);
+            }
+            cnt += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
         }
-        x[k] = v.x;
-        x[k + 1] = v.y;
-        x[k + 2] = v.z;
-        x[k + 3] = v.w;
-    }
-#pragma unroll
-    for (int k = 0; k < kWpt; ++k) {
-        if (x[k]) mask |= 1u << k;
-        cnt += __popc(x[k]);
     }
     int32_t tot;
-    const int32_t base = block_excl_scan<THREADS>(cnt, &tot, sh);
+    int32_t run = __shfl_sync(FULL, block_excl_scan<THREADS>(cnt, &tot, sh), 0);
     if (tid == 0 && tot != expect) raise(a.err, DEV_COUNT_MISMATCH);
-    {
-        int32_t p = base;
+#pragma unroll 2
+    for (int j = 0; j < n4; ++j) {
+        const int i = w0 + 128 * j;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (i < nwords) v = *reinterpret_cast<const uint4 *>(bits + i);
+        const int32_t c2 = __popc(v.x) + __popc(v.y), c4 = c2 + __popc(v.z) + __popc(v.w);
+        int32_t x = c4;
 #pragma unroll
-        for (int k = 0; k < kWpt; k += 4) {
-            if (k < wpt && w0 + k < nwords) {
-                if (kept) *reinterpret_cast<uint4 *>(bits + w0 + k) = make_uint4(x[k], x[k + 1], x[k + 2], x[k + 3]);
-                pairRank[(w0 + k) >> 1] = (P)p;
-                p += __popc(x[k]) + __popc(x[k + 1]);
-                pairRank[((w0 + k) >> 1) + 1] = (P)p;
-                p += __popc(x[k + 2]) + __popc(x[k + 3]);
-            }
+        for (int d = 1; d < 32; d <<= 1) {
+            const int32_t y = __shfl_up_sync(FULL, x, d);
+            if (lane >= d) x += y;
         }
-        tbase[tid] = base;
-        tmask[tid] = mask;
+        const int32_t p = run + x - c4;
+        run += __shfl_sync(FULL, x, 31);
+        if (i < nwords) {
+            pairRank[i >> 1] = (P)p;
+            pairRank[(i >> 1) + 1] = (P)(p + c2);
+        }
+        uint32_t mask = ((v.x ? 1u : 0u) | (v.y ? 2u : 0u) | (v.z ? 4u : 0u) | (v.w ? 8u : 0u))
+                        << (4 * (lane & (n4 - 1)));
+        for (int d = 1; d < n4; d <<= 1) mask |= __shfl_xor_sync(FULL, mask, d);
+        if ((lane & (n4 - 1)) == 0) {
+            tbase[i >> lg] = p;
+            tmask[i >> lg] = mask;
+        }
     }
     __syncthreads();
     write_columns_balanced<THREADS>(bits, tbase, tmask, wpt, tot, a.Ci + obase, expect, obc);
+    // C's values start at zero.
+    for (int i = tid; i < expect; i += THREADS) cv[i] = 0.0;
     __syncthreads();
 
     for (int32_t eb = e0; eb < e1; eb += THREADS) {
