@@ -2145,18 +2145,20 @@ __global__ void __launch_bounds__(256) k_dense_items(NumArgs a, int32_t lo, int3
 // two per SM, take rows from a counter and apply the rank method over
 // windows of WIN words of the row's span (2^19 columns in shared memory).
 // Per window: a pass over the row's products sets the bits inside the
-// window; a sweep gives each thread the non-empty-word mask and bit count
-// of its 32 words (one summary word), and a scan of the counts gives every
-// thread the rank of its first column.  From there everything visits only
-// the non-empty words: their ranks (a 16-bit offset from a 32-bit base per
-// 256 words), C's columns (each thread writes a contiguous run of them), and
-// the clean-up that leaves the bitmap zero for the next window.  A second
-// pass adds every product inside the window into C's row in place at its
-// rank (FP64 L2 reductions).  Power-law rows spread thinly over millions of
-// columns pay for their entries, not for their span, past the one sweep.
+// window; its words are counted and ranked 128 a warp and step (a 16-bit
+// offset each from a 32-bit base per 256 words), and 32-word groups get the
+// rank of their first column and the mask of their non-empty words, from
+// which C's columns are written (each thread a contiguous run of them).  A
+// second pass adds every product inside the window into C's row in place at
+// its rank (FP64 L2 reductions).  Bound by instruction issue and the
+// reductions' 24 sectors a step (10,240 rows of R-MAT 2^21: 7 GB of DRAM
+// traffic and 59% of L1's throughput in 3.7 ms).  With a 32-word group a
+// thread, whose non-empty words it then visited one by one, the warp waited for the
+// fullest group: 3.92 -> 3.77 ms.  Half as many CTAs of 1024 threads and twice the
+// window: 4.07.
 template <int THREADS, int WIN>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_num_rankwin(NumArgs a, int32_t lo, int32_t count) {
-    static_assert(WIN == 32 * THREADS, "one summary word of 32 bitmap words per thread");
+    static_assert(WIN == 32 * THREADS, "whole groups of 256 words per warp");
     extern __shared__ __align__(16) unsigned char smem[];
     using L = StageLayout<THREADS>;
     constexpr int NW = THREADS / 32;
@@ -2165,7 +2167,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_num_rankwin(NumArgs
     int32_t *pre = reinterpret_cast<int32_t *>(smem + L::pre);
     int32_t *bst = reinterpret_cast<int32_t *>(smem + L::bst);
     double *av = reinterpret_cast<double *>(smem + L::av);
-    uint32_t *bits = reinterpret_cast<uint32_t *>(smem + L::bytes);
+    uint32_t *bits = reinterpret_cast<uint32_t *>(smem + rank_bits_at(THREADS));
     uint16_t *wpre = reinterpret_cast<uint16_t *>(bits + WIN);
     int32_t *gbase = reinterpret_cast<int32_t *>(wpre + WIN);
     int32_t *tbase = gbase + WIN / 256;                          // per thread: rank of its first column
@@ -2236,33 +2238,46 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_num_rankwin(NumArgs
                     });
                 __syncthreads();
             }
-            // This thread's 32 words [32 tid, 32 tid + 32): which are
-            // non-empty and how many bits they hold.  Lanes start at
-            // different words so that a warp's loads hit 32 banks.
-            uint32_t mask = 0;
+            // The words' ranks, 128 words a warp and step, four a lane, and
+            // per 32 words the rank of the first column and the non-empty
+            // words.
+            const int w0 = (tid >> 5) * (WIN / NW) + 4 * lane;
             int32_t cnt = 0;
-#pragma unroll 8
-            for (int k = 0; k < 32; ++k) {
-                const int q = (k + lane) & 31;
-                const uint32_t x = bits[32 * tid + q];
-                if (x) mask |= 1u << q;
-                cnt += __popc(x);
+#pragma unroll
+            for (int j = 0; j < WIN / NW / 128; ++j) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(bits + w0 + 128 * j);
+                cnt += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
             }
             int32_t tot;
-            const int32_t base = block_excl_scan<THREADS>(cnt, &tot, sh);
-            // 256-word groups are 8 threads: the group's base is its first
-            // thread's.
-            const int32_t gb = __shfl_sync(FULL, base, lane & ~7);
-            if ((lane & 7) == 0) gbase[tid >> 3] = base;
-            {
-                int32_t p = base;
-                for (uint32_t m = mask; m; m &= m - 1u) {
-                    const int w = 32 * tid + __ffs(m) - 1;
-                    wpre[w] = (uint16_t)(p - gb);
-                    p += __popc(bits[w]);
+            int32_t p0 = __shfl_sync(FULL, block_excl_scan<THREADS>(cnt, &tot, sh), 0), gb = p0;
+#pragma unroll 2
+            for (int j = 0; j < WIN / NW / 128; ++j) {
+                const int i = w0 + 128 * j;
+                const uint4 v = *reinterpret_cast<const uint4 *>(bits + i);
+                const int32_t c1 = __popc(v.x), c2 = c1 + __popc(v.y), c3 = c2 + __popc(v.z), c4 = c3 + __popc(v.w);
+                int32_t x = c4;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int32_t y = __shfl_up_sync(FULL, x, d);
+                    if (lane >= d) x += y;
                 }
-                tbase[tid] = base;
-                tmask[tid] = mask;
+                const int32_t p = p0 + x - c4;
+                if ((j & 1) == 0) {  // a group of 256 words starts
+                    gb = p0;
+                    if (lane == 0) gbase[i >> 8] = p0;
+                }
+                p0 += __shfl_sync(FULL, x, 31);
+                const int32_t q = p - gb;
+                *reinterpret_cast<ushort4 *>(wpre + i) = make_ushort4(
+                    (uint16_t)q, (uint16_t)(q + c1), (uint16_t)(q + c2), (uint16_t)(q + c3));
+                uint32_t mask = ((v.x ? 1u : 0u) | (v.y ? 2u : 0u) | (v.z ? 4u : 0u) | (v.w ? 8u : 0u))
+                                << (4 * (lane & 7));
+#pragma unroll
+                for (int d = 1; d < 8; d <<= 1) mask |= __shfl_xor_sync(FULL, mask, d);
+                if ((lane & 7) == 0) {
+                    tbase[i >> 5] = p;
+                    tmask[i >> 5] = mask;
+                }
             }
             __syncthreads();
             // C's columns, balanced over the threads by output position.
@@ -2296,8 +2311,9 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_num_rankwin(NumArgs
                     });
                 __syncthreads();
             }
-            // Leave the bitmap zero: only this thread's non-empty words.
-            for (uint32_t m = mask; m; m &= m - 1u) bits[32 * tid + __ffs(m) - 1] = 0u;
+            // Leave the bitmap zero.
+            for (int i = tid; 4 * i < nwords; i += THREADS)
+                reinterpret_cast<uint4 *>(bits)[i] = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();
             run += tot;
         }
@@ -2689,7 +2705,7 @@ constexpr int kDensewRows = 4;  // 8 rows a CTA: 8.2 ms where 4 take 7.9
 constexpr int kGdenseThreads = 512;
 constexpr int kRankWinThreads = 512;  // two CTAs per SM: one works while the other waits at a barrier
 constexpr int kRankWinWords = 16384;  // 2^19 columns per window
-constexpr size_t kSmemRankWin = StageLayout<kRankWinThreads>::bytes + 6 * (size_t)kRankWinWords +
+constexpr size_t kSmemRankWin = rank_bits_at(kRankWinThreads) + 6 * (size_t)kRankWinWords +
                                 4 * (size_t)(kRankWinWords / 256) + 12 * (size_t)kRankWinThreads;
 constexpr size_t kSmemGdenseBase = StageLayout<kGdenseThreads>::bytes;
 constexpr size_t kSmemDscr = StageLayout<kRankWinThreads>::bytes + 4 * (size_t)kRankWinWords;
