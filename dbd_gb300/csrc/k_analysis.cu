@@ -153,7 +153,17 @@ __global__ void k_row_minmax(CsrDev B, int2 *__restrict__ range, const int *__re
 // row; rows of more than kLongRow entries (power-law hubs, whose serial walk
 // by eight lanes would set the kernel's duration) are left to a second
 // stage in which a whole CTA takes each of them.
-constexpr int kLongRow = 256;
+//
+// Where the rows are short (at most kShortMean entries on average) a lane
+// takes a row: up to kShortRow entries with all their loads in flight, the
+// warp's longer rows four at a time by eight lanes each, and the second stage
+// starts at kLongRowShort.  2.1M five-entry rows 105 -> 36 us.  Its longest
+// warps are those of a power-law graph's hubs, so it takes kShortRows rows
+// and more: means of 2 to 5 entries over 2^20 rows 78 -> 56 us, 2^19 52 ->
+// 39, but 2^18 32 -> 37, 2^16 14 -> 21, 2^12 10 -> 14.
+constexpr int kLongRow = 256, kLongRowShort = 64;
+constexpr int kShortRow = 8;
+constexpr int64_t kShortMean = 6, kShortRows = 1 << 19;
 
 __device__ __forceinline__ void row_products_out(const CsrDev &A, int64_t row, int64_t sum, int32_t lo, int32_t hi,
                                                  RowInfo &ri, uint8_t *symBin, int *err, const Tuning &tune) {
@@ -165,7 +175,7 @@ __device__ __forceinline__ void row_products_out(const CsrDev &A, int64_t row, i
     if (sum > 0x7fffffffLL) atomicCAS(err, 0, (int)DEV_ROW_TOO_LONG);
 }
 
-template <int THREADS>
+template <int THREADS, bool SHORT>
 __global__ void __launch_bounds__(THREADS) k_row_products(CsrDev A, const int32_t *__restrict__ Bp,
                                                           const int2 *__restrict__ range, RowInfo ri,
                                                           uint8_t *__restrict__ symBin, int *err,
@@ -181,56 +191,116 @@ __global__ void __launch_bounds__(THREADS) k_row_products(CsrDev A, const int32_
     }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int sub = lane & 7;
+    constexpr int kLong = SHORT ? kLongRowShort : kLongRow;
     const unsigned gmask = 0xffu << (lane & 24);
-    const int64_t stride = ((int64_t)gridDim.x * THREADS) >> 3;
-    // kRowsAhead rows a group in flight: a row is a chain of three dependent
-    // loads, which one row at a time leaves the GPU waiting for (2.1M
-    // five-entry rows: 155 -> 105 us, with the ranges read as pairs).
-    constexpr int kRowsAhead = 4;
-    for (int64_t b = (blockIdx.x * (int64_t)THREADS + tid) >> 3; b < A.m; b += kRowsAhead * stride) {
-        int32_t s[kRowsAhead], e[kRowsAhead], k[kRowsAhead];
+    if constexpr (SHORT) {
+        for (int64_t b = blockIdx.x * (int64_t)THREADS + (tid & ~31); b < A.m; b += (int64_t)gridDim.x * THREADS) {
+            const int64_t row = b + lane;
+            const int32_t s = row < A.m ? __ldg(&A.ptr[row]) : 0;
+            const int32_t e = row < A.m ? __ldg(&A.ptr[row + 1]) : 0;
+            int32_t k[kShortRow], len[kShortRow];
+            int2 r[kShortRow];
+            const bool brief = e - s <= kShortRow;
 #pragma unroll
-        for (int u = 0; u < kRowsAhead; ++u) {
-            const int64_t row = b + u * stride;
-            s[u] = row < A.m ? __ldg(&A.ptr[row]) : 0;
-            e[u] = row < A.m ? __ldg(&A.ptr[row + 1]) : 0;
+            for (int i = 0; i < kShortRow; ++i) k[i] = brief && s + i < e ? __ldg(&A.idx[s + i]) : -1;
+#pragma unroll
+            for (int i = 0; i < kShortRow; ++i) {
+                r[i] = k[i] >= 0 ? __ldg(&range[k[i]]) : make_int2(INT32_MAX, -1);
+                len[i] = k[i] >= 0 ? __ldg(&Bp[k[i] + 1]) - __ldg(&Bp[k[i]]) : 0;
+            }
+            int64_t sum = 0;
+            int32_t lo = INT32_MAX, hi = -1;
+#pragma unroll
+            for (int i = 0; i < kShortRow; ++i) {
+                sum += len[i];
+                lo = min(lo, r[i].x);
+                hi = max(hi, r[i].y);
+            }
+            if (row < A.m && brief) row_products_out(A, row, sum, lo, hi, ri, symBin, err, tune);
+            // The others up to kLong: four at a time, eight lanes each.
+            unsigned more = __ballot_sync(FULL, !brief && e - s <= kLong);
+            while (more) {
+                int mine = -1;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    if (more && g == lane >> 3) mine = __ffs(more) - 1;
+                    more &= more - 1u;
+                }
+                const int32_t s8 = __shfl_sync(FULL, s, max(mine, 0)), e8 = __shfl_sync(FULL, e, max(mine, 0));
+                sum = 0;
+                lo = INT32_MAX;
+                hi = -1;
+                if (mine >= 0) {
+#pragma unroll 4
+                    for (int32_t i = s8 + sub; i < e8; i += 8) {
+                        const int32_t q = __ldg(&A.idx[i]);
+                        const int2 w = __ldg(&range[q]);
+                        sum += (int64_t)(__ldg(&Bp[q + 1]) - __ldg(&Bp[q]));
+                        lo = min(lo, w.x);
+                        hi = max(hi, w.y);
+                    }
+                }
+#pragma unroll
+                for (int d = 4; d; d >>= 1) {
+                    sum += __shfl_xor_sync(FULL, sum, d);
+                    lo = min(lo, __shfl_xor_sync(FULL, lo, d));
+                    hi = max(hi, __shfl_xor_sync(FULL, hi, d));
+                }
+                if (sub == 0 && mine >= 0) row_products_out(A, b + mine, sum, lo, hi, ri, symBin, err, tune);
+            }
         }
+    } else {
+        const int64_t stride = ((int64_t)gridDim.x * THREADS) >> 3;
+        // kRowsAhead rows a group in flight: a row is a chain of three dependent
+        // loads, which one row at a time leaves the GPU waiting for (2.1M
+        // five-entry rows: 155 -> 105 us, with the ranges read as pairs).
+        constexpr int kRowsAhead = 4;
+        for (int64_t b = (blockIdx.x * (int64_t)THREADS + tid) >> 3; b < A.m; b += kRowsAhead * stride) {
+            int32_t s[kRowsAhead], e[kRowsAhead], k[kRowsAhead];
 #pragma unroll
-        for (int u = 0; u < kRowsAhead; ++u) k[u] = s[u] + sub < e[u] ? __ldg(&A.idx[s[u] + sub]) : -1;
-        int64_t sum[kRowsAhead];
-        int32_t lo[kRowsAhead], hi[kRowsAhead];
-#pragma unroll
-        for (int u = 0; u < kRowsAhead; ++u) {
-            const int2 r = k[u] >= 0 ? __ldg(&range[k[u]]) : make_int2(INT32_MAX, -1);
-            sum[u] = k[u] >= 0 ? __ldg(&Bp[k[u] + 1]) - __ldg(&Bp[k[u]]) : 0;
-            lo[u] = r.x;
-            hi[u] = r.y;
-        }
-#pragma unroll
-        for (int u = 0; u < kRowsAhead; ++u) {
-            const int64_t row = b + u * stride;
-            if (row >= A.m || e[u] - s[u] > kLongRow) continue;  // the whole group skips together
-            for (int32_t i = s[u] + 8 + sub; i < e[u]; i += 8) {
-                const int32_t q = A.idx[i];
-                const int2 r = __ldg(&range[q]);
-                sum[u] += (int64_t)(Bp[q + 1] - Bp[q]);
-                lo[u] = min(lo[u], r.x);
-                hi[u] = max(hi[u], r.y);
+            for (int u = 0; u < kRowsAhead; ++u) {
+                const int64_t row = b + u * stride;
+                s[u] = row < A.m ? __ldg(&A.ptr[row]) : 0;
+                e[u] = row < A.m ? __ldg(&A.ptr[row + 1]) : 0;
             }
 #pragma unroll
-            for (int d = 4; d; d >>= 1) {
-                sum[u] += __shfl_xor_sync(gmask, sum[u], d, 8);
-                lo[u] = min(lo[u], __shfl_xor_sync(gmask, lo[u], d, 8));
-                hi[u] = max(hi[u], __shfl_xor_sync(gmask, hi[u], d, 8));
+            for (int u = 0; u < kRowsAhead; ++u) k[u] = s[u] + sub < e[u] ? __ldg(&A.idx[s[u] + sub]) : -1;
+            int64_t sum[kRowsAhead];
+            int32_t lo[kRowsAhead], hi[kRowsAhead];
+#pragma unroll
+            for (int u = 0; u < kRowsAhead; ++u) {
+                const int2 r = k[u] >= 0 ? __ldg(&range[k[u]]) : make_int2(INT32_MAX, -1);
+                sum[u] = k[u] >= 0 ? __ldg(&Bp[k[u] + 1]) - __ldg(&Bp[k[u]]) : 0;
+                lo[u] = r.x;
+                hi[u] = r.y;
             }
-            if (sub == 0) row_products_out(A, row, sum[u], lo[u], hi[u], ri, symBin, err, tune);
+#pragma unroll
+            for (int u = 0; u < kRowsAhead; ++u) {
+                const int64_t row = b + u * stride;
+                if (row >= A.m || e[u] - s[u] > kLong) continue;  // the whole group skips together
+                for (int32_t i = s[u] + 8 + sub; i < e[u]; i += 8) {
+                    const int32_t q = A.idx[i];
+                    const int2 r = __ldg(&range[q]);
+                    sum[u] += (int64_t)(Bp[q + 1] - Bp[q]);
+                    lo[u] = min(lo[u], r.x);
+                    hi[u] = max(hi[u], r.y);
+                }
+#pragma unroll
+                for (int d = 4; d; d >>= 1) {
+                    sum[u] += __shfl_xor_sync(gmask, sum[u], d, 8);
+                    lo[u] = min(lo[u], __shfl_xor_sync(gmask, lo[u], d, 8));
+                    hi[u] = max(hi[u], __shfl_xor_sync(gmask, hi[u], d, 8));
+                }
+                if (sub == 0) row_products_out(A, row, sum[u], lo[u], hi[u], ri, symBin, err, tune);
+            }
         }
     }
 
     // Long rows: CTA b takes the long rows r with r = b (mod gridDim.x), one
     // by one with all its threads.  Hubs sit close together in row order
-    // (power-law generators put them at small indices), so the modular
-    // assignment spreads them over the CTAs.
+    // (power-law generators put them at small indices, and at multiples of
+    // powers of two), so the modular assignment, by an odd number of CTAs,
+    // spreads them over the CTAs.
     __shared__ int32_t longRows[THREADS];
     __shared__ int nLong;
     __shared__ int64_t rs[THREADS / 32];
@@ -239,7 +309,7 @@ __global__ void __launch_bounds__(THREADS) k_row_products(CsrDev A, const int32_
         if (tid == 0) nLong = 0;
         __syncthreads();
         const int64_t row = t0 + blockIdx.x + (int64_t)gridDim.x * tid;
-        if (row < A.m && A.ptr[row + 1] - A.ptr[row] > kLongRow) longRows[atomicAdd(&nLong, 1)] = (int32_t)row;
+        if (row < A.m && A.ptr[row + 1] - A.ptr[row] > kLong) longRows[atomicAdd(&nLong, 1)] = (int32_t)row;
         __syncthreads();
         const int nl = nLong;
         for (int j = 0; j < nl; ++j) {
@@ -604,9 +674,18 @@ void launch_row_products(const CsrDev &A, const int32_t *Bp, const int2 *range, 
                          int *err, const int32_t *ctl, const Tuning &t, cudaStream_t s, int num_sms) {
     if (A.m == 0) return;
     constexpr int threads = 256;
-    const int64_t need = ceil_div(A.m * 8, threads);
-    const int grid = (int)std::min<int64_t>(need, (int64_t)num_sms * 8);
-    k_row_products<threads><<<grid, threads, 0, s>>>(A, Bp, range, ri, symBin, err, ctl, t);
+    const int64_t fit = (int64_t)num_sms * 8;
+    // Odd, for the long rows (262k rows of R-MAT 2^18, 5 entries on average: 58 -> 32 us).
+    const auto grid = [&](int64_t need) {
+        return (int)(need < fit ? need | 1 : (fit - 1) | 1);
+    };
+    if (A.m >= kShortRows && A.nnz <= kShortMean * A.m) {
+        k_row_products<threads, true><<<grid(ceil_div(A.m, threads)), threads, 0, s>>>(
+            A, Bp, range, ri, symBin, err, ctl, t);
+    } else {
+        k_row_products<threads, false><<<grid(ceil_div(A.m * 8, threads)), threads, 0, s>>>(
+            A, Bp, range, ri, symBin, err, ctl, t);
+    }
 }
 
 void launch_sym_lists(int64_t m, const Binning &b, const RowInfo &ri, int32_t *rowNnz, int64_t *tileSum,
@@ -656,7 +735,7 @@ void launch_f32_to_f64(const float *src, double *dst, int64_t n, cudaStream_t s)
 // launch, by default).  Returns the first error.
 cudaError_t preload_analysis_kernels() {
     const void *fns[] = {
-        (const void *)k_check_operand, (const void *)k_row_minmax, (const void *)k_row_products<256>,
+        (const void *)k_check_operand, (const void *)k_row_minmax, (const void *)k_row_products<256, true>, (const void *)k_row_products<256, false>,
         (const void *)k_tiles, (const void *)k_tile_scan, (const void *)k_tile_scatter,
         (const void *)k_scan_reduce, (const void *)k_scan_parts, (const void *)k_scan_final,
         (const void *)k_f32_to_f64,
