@@ -114,11 +114,14 @@ __global__ void __launch_bounds__(256) k_val_to_f32(const double *__restrict__ s
 
 // The same straight into pinned host memory: the rounding and the copy in one
 // pass over the FP64 values.  The host link bounds it (193 GB/s on the GB300,
-// what the copy engine reaches too), which 16 CTAs fill; kHostCtas leaves the
-// other SMs to the next chunk.  Warps write whole 128-byte lines of the
-// destination, whatever its alignment.  (A float array on the device and a
-// copy of it: 165 us more for 67M values.)
-constexpr int kHostCtas = 32, kHostThreads = 512;
+// what the copy engine reaches too): 16 CTAs fill it on an idle GPU, but
+// beside the next chunk's kernels 67M values take 1.57 ms with 16 CTAs of
+// 512 threads, 1.46 with 32 or 64, 1.41 with 128, and the same with
+// two small CTAs an SM, which leave those kernels more room (1.40 at the
+// link's rate).  Warps write whole 128-byte lines of the destination,
+// whatever its alignment.  (A float array on the device and a copy of it:
+// 165 us more.)
+constexpr int kHostCtas = 304, kHostThreads = 256;
 
 __global__ void __launch_bounds__(kHostThreads) k_val_to_host_f32(const double *__restrict__ src,
                                                                   float *__restrict__ dst, int64_t n) {
