@@ -143,7 +143,7 @@ enum DevErr : int { DEV_OK = 0, DEV_TABLE_FULL = 1, DEV_COUNT_MISMATCH = 2, DEV_
 // Counter slots for dynamically scheduled kernels (zeroed per multiply).
 enum CounterSlot : int {
     CTR_SYM_TINY = 0, CTR_SYM_HWARP, CTR_SYM_HCTA, CTR_SYM_WIDE, CTR_NUM_GDENSE, CTR_NUM_RANKWIN, CTR_NUM_DSCR,
-    CTR_HEAVY, CTR_ITEMS, CTR_ADJOINT, CTR_SYM_ITEMS, CTR_SYM_NEXT,
+    CTR_HEAVY, CTR_ITEMS, CTR_ADJOINT, CTR_ADJ_ITEMS, CTR_SYM_ITEMS, CTR_SYM_NEXT,
     CTR_MAX_P, CTR_COUNT = 16
 };
 
@@ -342,6 +342,24 @@ void launch_numeric_bin(const NumArgs &a, int bin, int32_t lo, int32_t hi, cudaS
 // (Cp, Ci), dA[e] = sum_k G(i,k) B(j,k) for e = (i,j) in A and
 // dB[f] += A(i,j) G(i,k) for f = (j,k) in B (dB null: dA only).  dA and dB
 // start at zero: entries without products are not written.
+// Part p of k of a heavy row's products in the CTA kernel.
+struct AdjItem {
+    int32_t row;
+    int16_t p, k;
+};
+constexpr int kAdjMaxParts = 128;
+// Rows of at least two parts' products are cut into parts of about a third of
+// a CTA's share of all products (five CTAs an SM), so that no row is the last
+// one running, and no less than 4096, under which a part is not worth its
+// staging (R-MAT 2^12 with 6 entries a row: 8192 78 us, 4096 65, 2048 40, but
+// 2^14 203, 205 and 269).
+inline int64_t adjoint_part_products(int64_t products, int num_sms) {
+    const int64_t share = products / (16 * (int64_t)(num_sms > 0 ? num_sms : 1));
+    return share > 4096 ? share : 4096;
+}
+// Most parts that rows of `products` products in all can make.
+inline int64_t adjoint_part_cap(int64_t products, int64_t partP) { return products / partP + products / (2 * partP); }
+
 struct AdjArgs {
     CsrDev A, B;
     const int64_t *Cp;
@@ -350,21 +368,26 @@ struct AdjArgs {
     double *dA;
     double *dB;
     const int32_t *order;  // rows of A in the forward's numeric bin order
-    uint32_t *ctr;         // row counter of the CTA kernel
+    uint32_t *ctr;         // row counter of the CTA kernel, then its items
     // With dB null: where to keep every product A(i,j) * G(i,k) for the
     // deterministic dB pass (null: nowhere), entry e's from off[e] on in B's
     // row order.
     double *prod = nullptr;
     const int64_t *off = nullptr;
     int64_t prodCap = 0;
+    // Rows of at least 2 * partP products (rowP) in parts (no items: none is
+    // cut); room for adjoint_part_cap() items, their count in ctr[1].
+    const int64_t *rowP = nullptr;
+    AdjItem *items = nullptr;
+    int64_t partP = 0, itemCap = 0;
     int *err;
 };
 // Rows order[lo, hi) whose rows of C hold at most 512 entries (one warp each).
 void launch_adjoint_warp(const AdjArgs &a, int32_t lo, int32_t hi, cudaStream_t s, int *launches);
 // Rows order[lo, hi) of any size, the last ones first.
 void launch_adjoint_cta(const AdjArgs &a, int32_t lo, int32_t hi, int num_sms, cudaStream_t s, int *launches);
-// dB = mask_B(A^T G) on its own: one warp per row k of B, each lane one
-// entry (k, j), summing A(i,k) * G(i,j) over column k of A in row order
+// dB = mask_B(A^T G) on its own: a thread per entry (k, j) of B, summing
+// A(i,k) * G(i,j) over column k of A in row order, long columns in segments
 // (colPtr / perm / rowOf: A's entries grouped by column, stably).
 struct AdjDbArgs {
     CsrDev B;

@@ -158,6 +158,7 @@ struct dbd_ctx {
     int64_t patA = -1, patB = -1;
     DevBuf adjG, adjA, adjB;    // device copies for host-side adjoint arguments
     DevBuf adjT;                // A grouped by column for the deterministic dB pass
+    DevBuf adjItems;            // parts of its heaviest rows
     DevBuf adjProd, adjOff;     // its products as the dA pass computed them, and where each A entry's start
     // Batched products: the pairs' placement (device copy of the pair
     // descriptors and offsets, staged through pinned memory), the per-row
@@ -1438,8 +1439,8 @@ void dbd_destroy(dbd_ctx *c) {
                       &c->rowP, &c->symBin, &c->numBin, &c->rowNnz, &c->symList, &c->numList, &c->hist,
                       &c->symTileOff, &c->numTileOff, &c->symStart, &c->numStart, &c->part, &c->Cp, &c->cursor,
                       &c->ctl, &c->Ci, &c->Cv, &c->wideBits, &c->wideSlot, &c->adjG,
-                      &c->adjA, &c->adjB, &c->adjT, &c->adjProd, &c->adjOff, &c->rowLo, &c->rowHi, &c->A.range, &c->B.range,
-                      &c->gdense, &c->dgCount, &c->dgCol, &c->dgVal, &c->dgSum, &c->dgWsum,
+                      &c->adjA, &c->adjB, &c->adjT, &c->adjProd, &c->adjOff, &c->adjItems, &c->rowLo, &c->rowHi,
+                      &c->A.range, &c->B.range, &c->gdense, &c->dgCount, &c->dgCol, &c->dgVal, &c->dgSum, &c->dgWsum,
                       &c->dgBad, &c->hashOut, &c->dscr, &c->heavySlot, &c->slabCnt,
                       &c->symItems, &c->items})
         b->release();
@@ -1713,6 +1714,14 @@ int dbd_spgemm_adjoint(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b,
     aa.order = c->numList.as<int32_t>();
     aa.ctr = c->ctrs() + CTR_ADJOINT;
     aa.err = c->err();
+    aa.rowP = c->rowP.as<int64_t>();
+    aa.partP = adjoint_part_products(c->products, c->num_sms);
+    if (c->maxRowP >= 2 * aa.partP) {
+        // Without the room no row is cut.
+        aa.itemCap = adjoint_part_cap(c->products, aa.partP);
+        if (c->adjItems.ensure(sizeof(AdjItem) * (size_t)aa.itemCap) == cudaSuccess) aa.items = c->adjItems.as<AdjItem>();
+        else cudaGetLastError();
+    }
     int launches = 0;
     if (det && B.nnz > 0 && A.nnz > 0 && 8.0 * (double)c->products <= c->cfg.gpu_gib * kGiB / 8) {
         // The products of the dA pass are kept for the dB pass within an

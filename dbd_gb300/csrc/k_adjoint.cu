@@ -39,6 +39,7 @@ __device__ __forceinline__ int64_t find_col(const int32_t *__restrict__ ci, int6
 // does.  100k rows of 256 products: 380 -> 242 us.
 constexpr int kAdjWarpNnz = 512;
 constexpr int kAdjWarpRows = 4;  // 24 KB a CTA
+constexpr int kAdjCtaThreads = 256, kAdjCtaPerSm = 5;
 
 __global__ void __launch_bounds__(32 * kAdjWarpRows) k_adjoint_warp(AdjArgs a, int32_t lo, int32_t n) {
     __shared__ double gs[kAdjWarpRows][kAdjWarpNnz];
@@ -123,21 +124,38 @@ __global__ void __launch_bounds__(32 * kAdjWarpRows) k_adjoint_warp(AdjArgs a, i
     }
 }
 
+// First product of the first staged entry that starts at product t or later
+// (the batch's products if none does; pre as stage_entries leaves it).
+__device__ __forceinline__ int32_t first_entry_at(const int32_t *pre, int nb, int32_t t) {
+    if (nb == 0) return 0;
+    const int e = find_entry(pre, nb, t);
+    return pre[e] < t ? pre[e + 1] : pre[e];
+}
+
 // Rows of more entries: persistent CTAs take rows from a counter, from the
 // heaviest bin on.  The row's entries are staged with their B rows' lengths
 // and the warps take equal contiguous shares of its products (a warp a row,
 // the form before, walked a power-law hub's half a million products alone:
-// 3.65 ms on R-MAT 2^14, 0.26 ms now, 0.30 keeping the products).  A row of C within kRankWordsMax
-// 32-column words is ranked through a bitmap and the words' first positions
-// in shared memory, two shared loads and a bit count a lookup; a wider one by
-// binary search.  Four steps of B loads, then their four loads of G, are in
-// flight together.
+// 3.65 ms on R-MAT 2^14).  Loads, shuffles and barriers set the pace, not the
+// FP64 pipe (42%) or L1 (27%): small CTAs, five an SM, and no row alone at
+// the end.  With the products kept, 2^14 takes 0.21 ms and 2^16 1.13; 0.30
+// and 1.68 with 512 threads, two CTAs an SM and whole rows, 0.26 and 1.37
+// with three, 0.33 with 256 threads and whole rows.
+// A row of C within kRankWordsMax 32-column words is ranked through a bitmap
+// and the words' first positions in shared memory, two shared loads and a bit
+// count a lookup; a wider one by binary search.  Four steps of B loads, then
+// their four loads of G, are in flight together.
 // dA of an entry is summed by the lanes it falls on, in registers while the
 // warp stays on it, and stored by the warp it starts in; the parts of an
 // entry that warps further on hold are added by one thread, in warp order
 // (a fixed order either way).
+//
+// Rows of at least 2 a.partP products are cut into items (built by
+// k_adjoint_items, and taken first): item p of k takes the entries of every
+// staged batch whose first products lie in the p-th of k equal shares of it,
+// so an entry's sum stays within a CTA.
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS) k_adjoint_cta(AdjArgs a, int32_t lo, int32_t n, int maxWords) {
+__global__ void __launch_bounds__(THREADS, kAdjCtaPerSm) k_adjoint_cta(AdjArgs a, int32_t lo, int32_t n, int maxWords) {
     extern __shared__ __align__(16) unsigned char smem[];
     using L = StageLayout<THREADS>;
     constexpr int NW = THREADS / 32;
@@ -152,12 +170,18 @@ __global__ void __launch_bounds__(THREADS) k_adjoint_cta(AdjArgs a, int32_t lo, 
     uint32_t *bits = reinterpret_cast<uint32_t *>(src + THREADS);
     int32_t *wpre = reinterpret_cast<int32_t *>(bits + maxWords);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int32_t parts = a.items ? (int32_t)min((int64_t)*(volatile uint32_t *)&a.ctr[1], a.itemCap) : 0;
     for (;;) {
         if (tid == 0) next = (int32_t)atomicAdd(a.ctr, 1u);
         __syncthreads();
         const int32_t item = next;
-        if (item >= n) break;
-        const int32_t row = a.order[lo + n - 1 - item];
+        if (item >= parts + n) break;
+        const AdjItem it = item < parts ? a.items[item] : AdjItem{a.order[lo + n - 1 - (item - parts)], 0, 1};
+        const int32_t row = it.row;
+        if (item >= parts && a.items && a.rowP[row] >= 2 * a.partP) {  // in parts
+            __syncthreads();  // every thread has read `next` before it changes
+            continue;
+        }
         const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
         const int64_t c0 = a.Cp[row], c1 = a.Cp[row + 1];
         const int32_t w0 = c1 > c0 ? a.Ci[c0] >> 5 : 0;
@@ -190,7 +214,15 @@ __global__ void __launch_bounds__(THREADS) k_adjoint_cta(AdjArgs a, int32_t lo, 
             const int32_t total = stage_entries<THREADS, true>(a.A, a.B, eb, min(THREADS, e1 - eb), pre, bst, av, &nb,
                                                                sh, false, 0, 0, nullptr, false, src);
             int32_t tb, te;
-            warp_share<THREADS>(total, &tb, &te);
+            if (it.k == 1) {
+                warp_share<THREADS>(total, &tb, &te);
+            } else {
+                const int32_t from = first_entry_at(pre, nb, (int32_t)((int64_t)total * it.p / it.k));
+                const int32_t to = first_entry_at(pre, nb, (int32_t)((int64_t)total * (it.p + 1) / it.k));
+                warp_share<THREADS>(to - from, &tb, &te);
+                tb += from;
+                te += from;
+            }
             if (lane == 0) partEnt[warp] = -1;
             // The batch's products follow each other in the kept array.
             double *keep = nullptr;
@@ -280,6 +312,19 @@ __global__ void __launch_bounds__(THREADS) k_adjoint_cta(AdjArgs a, int32_t lo, 
         }
         __syncthreads();  // every thread has read `next` before it changes
     }
+}
+
+// The parts of the rows order[lo, lo + n) that are cut.
+__global__ void __launch_bounds__(256) k_adjoint_items(AdjArgs a, int32_t lo, int32_t n) {
+    const int32_t i = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= n) return;
+    const int32_t row = a.order[lo + i];
+    const int64_t P = a.rowP[row];
+    if (P < 2 * a.partP) return;
+    const int k = (int)min((int64_t)kAdjMaxParts, P / a.partP);
+    const uint32_t at = atomicAdd(&a.ctr[1], (uint32_t)k);
+    if ((int64_t)at + k > a.itemCap) return raise(a.err, DEV_COUNT_MISMATCH);  // the products are not the forward's
+    for (int p = 0; p < k; ++p) a.items[at + p] = AdjItem{row, (int16_t)p, (int16_t)k};
 }
 
 // Products of every A entry (the length of its B row).
@@ -419,7 +464,6 @@ __global__ void __launch_bounds__(256) k_adjoint_db_sum(AdjDbArgs a) {
     a.dB[f] = acc;
 }
 
-constexpr int kAdjCtaThreads = 512;
 
 }  // namespace
 
@@ -469,9 +513,14 @@ void launch_adjoint_cta(const AdjArgs &a, int32_t lo, int32_t hi, int num_sms, c
     // A matrix of few columns needs no more bitmap than they take.
     const int words = (int)std::min<int64_t>(kRankWordsMax, a.B.n / 32 + 2);
     const size_t smem = smem_adjoint_cta(words);
-    const int per_sm = std::max(1, std::min(2048 / kAdjCtaThreads, (int)((227 * 1024) / (smem + 1024))));
-    const int grid = (int)std::min<int64_t>(hi - lo, (int64_t)std::max(num_sms, 1) * per_sm);
-    cudaMemsetAsync(a.ctr, 0, sizeof(uint32_t), s);
+    const int per_sm = std::max(1, std::min(kAdjCtaPerSm, (int)((227 * 1024) / (smem + 1024))));
+    const int64_t most = (int64_t)(hi - lo) * (a.items ? kAdjMaxParts : 1);
+    const int grid = (int)std::min<int64_t>(most, (int64_t)std::max(num_sms, 1) * per_sm);
+    cudaMemsetAsync(a.ctr, 0, 2 * sizeof(uint32_t), s);
+    if (a.items) {
+        k_adjoint_items<<<(unsigned)ceil_div(hi - lo, 256), 256, 0, s>>>(a, lo, hi - lo);
+        ++*launches;
+    }
     k_adjoint_cta<kAdjCtaThreads><<<(unsigned)grid, kAdjCtaThreads, smem, s>>>(a, lo, hi - lo, words);
     ++*launches;
 }
