@@ -29,9 +29,8 @@
 //                               of up to 2^19 columns that stays zero between
 //                               rows, kept for the numeric rank kernels
 //   dense rows  (numeric)       persistent CTAs, bitmap ranks over 2^19-column
-//                               windows in shared memory, work per window
-//                               over its non-empty words only, products
-//                               reduced into C in place
+//                               windows in shared memory, products reduced
+//                               into C in place
 //
 // Structure is decided by index only (a column belongs to a row as soon as a
 // product lands on it).  GB300's FP64 pipe is narrow (about two FP64
@@ -294,7 +293,7 @@ __device__ __forceinline__ int warp_sum_i(int v) {
 // instead of 32, and (numeric) issues 32 FP64 additions per row, 16 clocks of
 // the SM's FP64 pipe each, where a row needs one per product: 512 clocks a
 // row set its time.  2.1M five-point rows (25 products each): symbolic
-// 574 -> 88 us, numeric 4401 -> 407 us; 4096 rows: symbolic 8 -> 6 us, numeric
+// 574 -> 88 us, numeric 4401 -> 393 us; 4096 rows: symbolic 8 -> 6 us, numeric
 // 17 -> 17 us.  (Merging the products into a sorted list in shared
 // memory instead of sorting registers: 95, 422 and 19 us.)
 constexpr int kTinyPitch = 33;
@@ -370,10 +369,11 @@ __device__ __forceinline__ int tiny_count(const CsrDev &B, int n, const int32_t 
 __device__ __forceinline__ double first_term(double p) { return __double_as_longlong(p) == LLONG_MIN ? 0.0 : p; }
 
 // A lane's n <= N listed products (positions in col, A values in val) merged:
-// afterwards col and val hold its distinct columns, ascending and relative to
-// `base`, and their sums.  Returns how many.  Columns are below base + 2^27.
+// afterwards col and val hold its distinct columns less `shift`, ascending,
+// and their sums.  Returns how many.  Columns are in [base, base + 2^27).
 template <int N>
-__device__ __forceinline__ int tiny_sum(const CsrDev &B, int n, int32_t base, int32_t *col, double *val) {
+__device__ __forceinline__ int tiny_sum(const CsrDev &B, int n, int32_t base, int32_t shift, int32_t *col,
+                                        double *val) {
     uint32_t key[N];
 #pragma unroll
     for (int i0 = 0; i0 < N; i0 += 8) {
@@ -400,7 +400,7 @@ __device__ __forceinline__ int tiny_sum(const CsrDev &B, int n, int32_t base, in
             const bool head = i == 0 || (key[i] >> 5) != (key[i > 0 ? i - 1 : 0] >> 5);
             if (head) {
                 acc = first_term(p[i]);
-                col[kTinyPitch * m] = (int32_t)(key[i] >> 5);
+                col[kTinyPitch * m] = (int32_t)(key[i] >> 5) + (base - shift);
                 ++m;
             } else {
                 acc = __dadd_rn(acc, p[i]);
@@ -414,11 +414,11 @@ __device__ __forceinline__ int tiny_sum(const CsrDev &B, int n, int32_t base, in
 // The same for rows over 2^27 columns or more, whose keys would not fit 32
 // bits: products are merged one by one into the sorted list [0, m), which
 // never passes the product being taken.
-__device__ __noinline__ int tiny_sum_wide(const CsrDev &B, int n, int32_t base, int32_t *col, double *val) {
+__device__ __noinline__ int tiny_sum_wide(const CsrDev &B, int n, int32_t shift, int32_t *col, double *val) {
     int m = 0;
     for (int i = 0; i < n; ++i) {
         const int32_t q = col[kTinyPitch * i];
-        const int32_t c = __ldg(&B.idx[q]) - base;
+        const int32_t c = __ldg(&B.idx[q]) - shift;
         const double p = __dmul_rn(val[kTinyPitch * i], __ldg(&B.val[q]));
         int j = m;
         while (j > 0 && col[kTinyPitch * (j - 1)] > c) --j;
@@ -991,17 +991,17 @@ __device__ __forceinline__ void num_tiny_rows(const NumArgs &a, int32_t lo, int3
     const int listed = tiny_list<true>(a.A, a.B, row, live, col, val);
     const int most = __reduce_max_sync(FULL, listed);
     const int32_t cbase = live ? a.rowLo[row] : 0;
+    const int32_t shift = live ? col_shift(a, row) : 0;
     int m;
     if (__any_sync(FULL, live && listed > 0 && (int64_t)a.rowHi[row] - cbase >= (1 << 27)))
-        m = tiny_sum_wide(a.B, listed, cbase, col, val);
+        m = tiny_sum_wide(a.B, listed, shift, col, val);
     else if (most <= 8)
-        m = tiny_sum<8>(a.B, listed, cbase, col, val);
+        m = tiny_sum<8>(a.B, listed, cbase, shift, col, val);
     else if (most <= 16)
-        m = tiny_sum<16>(a.B, listed, cbase, col, val);
+        m = tiny_sum<16>(a.B, listed, cbase, shift, col, val);
     else
-        m = tiny_sum<kTinyMax>(a.B, listed, cbase, col, val);
+        m = tiny_sum<kTinyMax>(a.B, listed, cbase, shift, col, val);
     int64_t base = 0;
-    int32_t shift = 0;
     int n = 0;
     if (live) {
         const int64_t c0 = a.Cp[row];
@@ -1009,7 +1009,6 @@ __device__ __forceinline__ void num_tiny_rows(const NumArgs &a, int32_t lo, int3
         if (m != expect) raise(a.err, DEV_COUNT_MISMATCH);
         n = (int)min((int64_t)m, expect);
         base = c0 - a.outBase;
-        shift = col_shift(a, row) - cbase;
     }
     int incl = n;
 #pragma unroll
@@ -1017,23 +1016,42 @@ __device__ __forceinline__ void num_tiny_rows(const NumArgs &a, int32_t lo, int3
         const int y = __shfl_up_sync(FULL, incl, d);
         if (lane >= d) incl += y;
     }
-    base -= incl - n;  // entry t of the run goes to its row's base + t
+    const int start = incl - n;
+    base -= start;  // entry t of the run goes to its row's base + t
     const int total = __shfl_sync(FULL, incl, 31);
+    // Consecutive rows share their base, and lanes with entries lead the warp
+    // as a rule: entry t is then of the lane that the starts up to t count to
+    // (2.1M rows 408 -> 393 us against the search and its shuffles).
+    const unsigned have = __ballot_sync(FULL, n > 0);
+    const int64_t base0 = __shfl_sync(FULL, base, 0);
+    const bool plain = (have & (have + 1u)) == 0u && __all_sync(FULL, n == 0 || base == base0);
     __syncwarp();
+    int seen = 0, before = 0;  // rows that start before the step, and where the last of them does
     for (int t0 = 0; t0 < total; t0 += 32) {
         const int t = t0 + lane;
-        int o = 0;  // the lane whose row holds entry t
+        int o, first;
+        int64_t to = base0 + t;
+        if (plain) {
+            const uint32_t at = n > 0 ? (uint32_t)(start - t0) : 32u;
+            const uint32_t starts = __reduce_or_sync(FULL, at < 32u ? 1u << at : 0u);
+            const uint32_t upto = starts & (FULL >> (31 - lane));
+            o = seen + __popc(upto) - 1;
+            first = upto ? t0 + 31 - __clz(upto) : before;
+            seen += __popc(starts);
+            if (starts) before = t0 + 31 - __clz(starts);
+        } else {
+            o = 0;  // the lane whose row holds entry t
 #pragma unroll
-        for (int step = 16; step >= 1; step >>= 1) {
-            const int v = __shfl_sync(FULL, incl, o + step - 1);
-            if (v <= t) o += step;
+            for (int step = 16; step >= 1; step >>= 1) {
+                const int v = __shfl_sync(FULL, incl, o + step - 1);
+                if (v <= t) o += step;
+            }
+            first = __shfl_sync(FULL, start, o);
+            to = __shfl_sync(FULL, base, o) + t;
         }
-        const int64_t to = __shfl_sync(FULL, base, o) + t;
-        const int first = __shfl_sync(FULL, incl - n, o);
-        const int32_t sh = __shfl_sync(FULL, shift, o);
         if (t < total) {
             const int at = kTinyPitch * (t - first) + o;
-            a.Ci[to] = cols[g][at] - sh;
+            a.Ci[to] = cols[g][at];
             a.Cv[to] = vals[g][at];
         }
     }
