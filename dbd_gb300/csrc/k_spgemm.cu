@@ -102,11 +102,8 @@ constexpr int kEscGroupLen = 6;
 // Position in B of product t (all lanes call; result valid when t < total).
 __device__ __forceinline__ int32_t chunk_pos(const Chunk &c, int32_t t, double *a_out) {
     const int o = chunk_owner(c, t);
-    const int32_t incl_o = __shfl_sync(FULL, c.incl, o);
-    const int32_t len_o = __shfl_sync(FULL, c.len, o);
-    const int32_t bs_o = __shfl_sync(FULL, c.bs, o);
     if (a_out) *a_out = __shfl_sync(FULL, c.a, o);
-    return bs_o + (t - (incl_o - len_o));
+    return t + __shfl_sync(FULL, c.bs - (c.incl - c.len), o);
 }
 
 // ---------------------------------------------------------------------------

@@ -20,6 +20,7 @@ struct Chunk {
     int32_t incl;  // inclusive prefix of len over lanes
     double a;      // A value of this lane's entry
     int32_t total; // products of the chunk
+    bool lead;     // the lanes with products come first
 };
 
 __device__ __forceinline__ Chunk load_chunk(const CsrDev &A, const CsrDev &B, int32_t e, int32_t eEnd,
@@ -42,11 +43,25 @@ __device__ __forceinline__ Chunk load_chunk(const CsrDev &A, const CsrDev &B, in
     }
     c.incl = x;
     c.total = __shfl_sync(FULL, x, 31);
+    const unsigned have = __ballot_sync(FULL, c.len > 0);
+    c.lead = (have & (have + 1u)) == 0u;
     return c;
 }
 
-// Owner lane of product t (all 32 lanes must call; t may be out of range).
+// Owner lane of this lane's product t = t0 + lane (all 32 lanes must call, t0
+// the same on all; t may be out of range).  Where the lanes with products
+// come first it is the number of their first products up to t, less one: those
+// before the step by a vote, those inside it from a mask of them; otherwise a
+// search over the lanes (555k symbolic warp rows of a batch 502 -> 468
+// us against the search alone and three shuffles to the position).
 __device__ __forceinline__ int chunk_owner(const Chunk &c, int32_t t) {
+    if (c.lead) {
+        const int lane = threadIdx.x & 31;
+        const int32_t at = c.incl - c.len - (t - lane);
+        const unsigned before = __ballot_sync(FULL, c.len > 0 && at < 0);
+        const uint32_t in = __reduce_or_sync(FULL, c.len > 0 && at >= 0 && at < 32 ? 1u << at : 0u);
+        return max(__popc(before) + __popc(in & (FULL >> (31 - lane))) - 1, 0);
+    }
     int lo = 0;
 #pragma unroll
     for (int step = 16; step >= 1; step >>= 1) {
