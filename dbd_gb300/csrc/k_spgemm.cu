@@ -618,9 +618,9 @@ __global__ void __launch_bounds__(256) k_sym_items(SymArgs a, int32_t begin, int
 // pass over the window either: a row costs its products, not its span.
 // Rows of at least a.firstP products are items of a launch of their own
 // (ITEMS, built by k_sym_items), the largest cut by column: a piece sets,
-// counts and keeps its slabs' columns and adds its count to the row's.  10,240 rows of R-MAT 2^21,
-// two of which hold 3.7M products each: 2.00 -> 1.14 ms (1.84 with 32-bit
-// window arithmetic alone).
+// counts and keeps its slabs' columns and adds its count to the row's.
+// 10,240 rows of R-MAT 2^21, two of which hold 3.7M products each: 2.00 ->
+// 1.14 ms (1.84 with 32-bit window arithmetic alone).
 template <int THREADS, bool ITEMS>
 __global__ void __launch_bounds__(THREADS) k_sym_wide(SymArgs a, int32_t begin, int32_t count, int winBits) {
     if (!ITEMS && begin < 0) {  // device-driven: the bin's rows from the bin table
@@ -1542,7 +1542,7 @@ __global__ void __launch_bounds__(THREADS) k_num_hash_cta_dd(NumArgs a, int bin)
 // has in flight, as long as the ranking is free of bank conflicts.  Such rows
 // used to accumulate in shared memory (compare-and-swap loops around a
 // multiply-add, 102 KB and 256 threads a CTA, two CTAs per SM): 57k of R-MAT
-// 2^18 3.13 -> 1.37 ms, 18k of 2^16 0.55 -> 0.28.  The larger rows (512
+// 2^18 3.13 -> 1.36 ms, 18k of 2^16 0.75 -> 0.28.  The larger rows (512
 // threads, two CTAs an SM) are bound by the reductions' 25 sectors a step and
 // by what of C and B stays in L2 meanwhile: C's values are zeroed right before
 // the products, not earlier (33k rows of 2^18 4.76 -> 4.60 ms; 5.01 with the
@@ -2167,7 +2167,7 @@ __global__ void __launch_bounds__(256) k_dense_items(NumArgs a, int32_t lo, int3
 // second pass adds every product inside the window into C's row in place at
 // its rank (FP64 L2 reductions).  Bound by instruction issue and the
 // reductions' 24 sectors a step (10,240 rows of R-MAT 2^21: 7 GB of DRAM
-// traffic and 59% of L1's throughput in 3.7 ms).  With a 32-word group a
+// traffic and 59% of L1's throughput in 3.6 ms).  With a 32-word group a
 // thread, whose non-empty words it then visited one by one, the warp waited for the
 // fullest group: 3.92 -> 3.77 ms.  Half as many CTAs of 1024 threads and twice the
 // window: 4.07.
