@@ -191,8 +191,10 @@ inline int64_t tile_count(int64_t m) { return ceil_div(m, kTileRows); }
 // not ascend.
 void launch_check_operand(const CsrDev &M, int2 *range, int *badPtr, int *badIdx, int *unsorted, cudaStream_t s,
                           int num_sms);
-// Replaces them by the smallest and largest column when *unsorted is not 0.
-void launch_row_minmax(const CsrDev &B, int2 *range, const int *unsorted, cudaStream_t s, int num_sms);
+// Replaces them by the smallest and largest column when *unsorted is not 0
+// and *badPtr (may be null) is.
+void launch_row_minmax(const CsrDev &B, int2 *range, const int *badPtr, const int *unsorted, cudaStream_t s,
+                       int num_sms);
 // ctl (may be null): control words; with an operand's check failed every row is
 // left empty and neither operand is read.
 void launch_row_products(const CsrDev &A, const int32_t *Bp, const int2 *range, const RowInfo &ri, uint8_t *symBin,

@@ -415,7 +415,7 @@ int check_operand(dbd_ctx *c, Operand &op, const CsrDev &d) {
     CK(c, op.range.ensure(sizeof(int2) * (size_t)std::max<int64_t>(d.m, 1)));
     launch_check_operand(d, op.range.as<int2>(), flags, flags + 1, flags + 2, c->stream, c->num_sms);
     if (&op == &c->B || c->b_is_a)  // the right operand
-        launch_row_minmax(d, op.range.as<int2>(), flags + 2, c->stream, c->num_sms);
+        launch_row_minmax(d, op.range.as<int2>(), flags, flags + 2, c->stream, c->num_sms);
     CK(c, cudaGetLastError());
     op.loaded = op.pending = true;
     c->divided = false;
@@ -2128,7 +2128,7 @@ int dbd_batch_enqueue(dbd_ctx *c, void *stream) {
     const Operand &opb = c->bpSquare ? c->A : c->B;
     int launches = 0;
     launch_check_operand(B, opb.range.as<int2>(), nullptr, nullptr, flags + 2, s, c->num_sms);
-    launch_row_minmax(B, opb.range.as<int2>(), flags + 2, s, c->num_sms);
+    launch_row_minmax(B, opb.range.as<int2>(), nullptr, flags + 2, s, c->num_sms);
     launch_row_products(A, B.ptr, opb.range.as<int2>(), row_info(c), c->symBin.as<uint8_t>(), c->err(), nullptr,
                         c->tune, s, c->num_sms);
     Binning sb{c->symBin.as<uint8_t>(), c->symList.as<int32_t>(), c->hist.as<int32_t>(), c->symTileOff.as<int32_t>(),

@@ -125,16 +125,21 @@ __global__ void __launch_bounds__(256) k_check_operand(CsrDev M, int2 *__restric
 }
 
 // Smallest and largest column of every row of an operand that
-// k_check_operand found unsorted (one warp per row); nothing otherwise.
-__global__ void k_row_minmax(CsrDev B, int2 *__restrict__ range, const int *__restrict__ unsorted) {
-    if (*unsorted == 0) return;
+// k_check_operand found unsorted (one warp per row); nothing otherwise.  It is
+// enqueued before the host has read the checks' results, so an operand whose
+// row_ptr failed (*badPtr, where given) is left alone, and no row is read
+// outside [0, nnz) whatever its pointers say.
+__global__ void k_row_minmax(CsrDev B, int2 *__restrict__ range, const int *__restrict__ badPtr,
+                             const int *__restrict__ unsorted) {
+    if (*unsorted == 0 || (badPtr && *badPtr != 0)) return;
     const int lane = threadIdx.x & 31;
     int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (; row < B.m; row += stride) {
         int32_t lo = INT32_MAX, hi = -1;
         const int32_t s = B.ptr[row], e = B.ptr[row + 1];
-        for (int32_t i = s + lane; i < e; i += 32) {
+        if (s < 0 || e > B.nnz) continue;  // the whole warp
+        for (int64_t i = (int64_t)s + lane; i < e; i += 32) {
             const int32_t c = B.idx[i];
             lo = min(lo, c);
             hi = max(hi, c);
@@ -664,10 +669,11 @@ void launch_check_operand(const CsrDev &M, int2 *range, int *badPtr, int *badIdx
     k_check_operand<<<grid, 256, 0, s>>>(M, range, badPtr, badIdx, unsorted);
 }
 
-void launch_row_minmax(const CsrDev &B, int2 *range, const int *unsorted, cudaStream_t s, int num_sms) {
+void launch_row_minmax(const CsrDev &B, int2 *range, const int *badPtr, const int *unsorted, cudaStream_t s,
+                       int num_sms) {
     if (B.m == 0) return;
     const int grid = (int)std::min<int64_t>(ceil_div(B.m * 32, 256), (int64_t)num_sms * 8);
-    k_row_minmax<<<grid, 256, 0, s>>>(B, range, unsorted);
+    k_row_minmax<<<grid, 256, 0, s>>>(B, range, badPtr, unsorted);
 }
 
 void launch_row_products(const CsrDev &A, const int32_t *Bp, const int2 *range, const RowInfo &ri, uint8_t *symBin,

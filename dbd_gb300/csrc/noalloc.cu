@@ -221,7 +221,7 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     if (b != a)
         launch_check_operand(A, reinterpret_cast<int2 *>(rowP), ctl + CTL_A, ctl + CTL_A + 1, ctl + CTL_A + 2, s, sms);
     launch_check_operand(B, range, ctl + CTL_B, ctl + CTL_B + 1, ctl + CTL_B + 2, s, sms);
-    launch_row_minmax(B, range, ctl + CTL_B + 2, s, sms);
+    launch_row_minmax(B, range, ctl + CTL_B, ctl + CTL_B + 2, s, sms);
     // Analysis: products per row, symbolic bins, row lists.
     launch_row_products(A, B.ptr, range, ri, symBin, err, ctl, Tuning{}, s, sms);
     Binning sb{symBin, symList, hist, symTileOff, symStart};

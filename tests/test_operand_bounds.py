@@ -1,0 +1,151 @@
+"""No check of a device operand reads outside its columns, whatever its
+row_ptr holds.  The check kernels' own text is built for the host, where the
+columns end at pages that cannot be read; on the GPU every entry point refuses
+the same operands."""
+import ctypes
+import os
+import re
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+import dbd_gb300 as dbd
+from dbd_gb300 import generators as gen
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+HARNESS = r"""
+#include "kernel_on_host.h"
+#include <cstdio>
+#include <cstring>
+#include <sys/mman.h>
+#include <vector>
+%s
+// `n` columns with an unreadable page right behind them, or (front) before them.
+static int32_t *fenced(long n, bool front) {
+    const long page = 65536, bytes = (4 * n + page - 1) / page * page;
+    char *p = (char *)mmap(nullptr, bytes + 2 * page, PROT_NONE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    mprotect(p + page, bytes, PROT_READ | PROT_WRITE);
+    return (int32_t *)(front ? p + page : p + page + bytes - 4 * n);
+}
+// argv: rows, columns that there are, front; then row_ptr.
+int main(int argc, char **argv) {
+    const int m = atoi(argv[1]), have = atoi(argv[2]);
+    std::vector<int32_t> ptr;
+    for (int i = 4; i < argc; ++i) ptr.push_back(atoi(argv[i]));
+    CsrDev M;
+    M.m = m;
+    M.n = 1000;
+    M.nnz = atoi(getenv("NNZ"));
+    int32_t *idx = fenced(have, atoi(argv[3]));
+    for (int i = 0; i < have; ++i) idx[i] = (have - i) %% 7;
+    M.ptr = ptr.data();
+    M.idx = idx;
+    std::vector<int2> range(m);
+    int badPtr = 0, badIdx = 0, unsorted = 0;
+    each_thread(2, 256, [&] { k_check_operand(M, range.data(), &badPtr, &badIdx, &unsorted); });
+    unsorted = 1;
+    each_thread(2, 256, [&] { k_row_minmax(M, range.data(), &badPtr, &unsorted); });
+    each_thread(2, 256, [&] { k_row_minmax(M, range.data(), nullptr, &unsorted); });
+    printf("%%d %%d", badPtr, badIdx);
+}
+"""
+
+
+def _kernel(text, name):
+    """A kernel's definition out of the source."""
+    at = text.index("__global__", text.rindex("\n\n", 0, re.search(rf"\b{name}\(", text).start()))
+    depth, i = 0, text.index("{", at)
+    while True:
+        depth += (text[i] == "{") - (text[i] == "}")
+        i += 1
+        if depth == 0:
+            return text[at:i]
+
+
+@pytest.fixture(scope="module")
+def checks(tmp_path_factory):
+    with open(os.path.join(ROOT, "dbd_gb300", "csrc", "k_analysis.cu")) as f:
+        text = f.read()
+    d = tmp_path_factory.mktemp("checks")
+    src, exe = str(d / "checks.cpp"), str(d / "checks")
+    with open(src, "w") as f:
+        f.write(HARNESS % "\n".join(_kernel(text, k) for k in ("k_check_operand", "k_row_minmax")))
+    subprocess.run(["g++", "-O1", "-std=c++17", "-w", "-I", os.path.join(ROOT, "tests", "helpers"), src, "-o", exe],
+                   check=True)
+    return exe
+
+
+# Five rows over 20 entries; what a fault leaves of them.
+GOOD = [0, 4, 8, 12, 16, 20]
+FAULTS = {
+    "well formed": GOOD,
+    "far past the end": [0, 4, 1 << 30, 12, 16, 20],
+    "far below": [0, 4, -(1 << 30), 12, 16, 20],
+    "least": [0, 4, -(1 << 31), 12, 16, 20],
+    "largest": [0, 4, (1 << 31) - 1, 12, 16, 20],
+    "all far": [0, 1 << 30, 1 << 30, 1 << 30, 1 << 30, 20],
+    "decreasing": [0, 20, 0, 20, 0, 20],
+    "first": [1 << 20, 4, 8, 12, 16, 20],
+    "last": [0, 4, 8, 12, 16, 1 << 30],
+    "last negative": [0, 4, 8, 12, 16, -5],
+}
+
+
+@pytest.mark.parametrize("front", [0, 1])
+@pytest.mark.parametrize("fault", sorted(FAULTS))
+def test_checks_stay_inside_the_columns(checks, fault, front):
+    ptr = FAULTS[fault]
+    run = subprocess.run([checks, "5", "20", str(front)] + [str(x) for x in ptr], capture_output=True, text=True,
+                         env=dict(os.environ, NNZ="20"))
+    assert run.returncode == 0, f"ended by signal {-run.returncode}"
+    assert run.stdout == ("0 0" if fault == "well formed" else "1 0")
+
+
+def _device(torch, m, row_ptr):
+    t = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (row_ptr.astype(np.int32), m.col_idx, m.val)]
+    torch.cuda.synchronize()
+    return dbd.CSR.from_device(m.n_rows, m.n_cols, m.nnz, *(x.data_ptr() for x in t)), t
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fault", sorted(set(FAULTS) - {"well formed"}))
+def test_entry_points_refuse_far_row_pointers(fault):
+    """B's rows do not ascend, so that the unsorted operand's path is taken."""
+    torch = pytest.importorskip("torch")
+    from dbd_gb300 import _ffi
+    rng = np.random.default_rng(1)
+    ptr = np.array(GOOD, np.int32)
+    idx = np.concatenate([rng.permutation(5)[:4] for _ in range(5)]).astype(np.int32)
+    M = dbd.CSR(5, 5, ptr, idx, rng.standard_normal(20))
+    good, keep = _device(torch, M, ptr)
+    bad, keep2 = _device(torch, M, np.array(FAULTS[fault], np.int64))
+    out = [torch.empty(n, dtype=t, device="cuda") for n, t in
+           ((6, torch.int64), (25, torch.int32), (25, torch.float64))]
+    grads = torch.zeros(2, 25, dtype=torch.float64, device="cuda")
+    nnz = ctypes.c_int64()
+    with dbd.Context(cpu_gib=1, gpu_gib=1) as ctx:
+        want = ctx.spgemm(good).C
+        for a, b in ((bad, None), (good, bad), (bad, good)):
+            for call in (lambda: ctx.spgemm(a, b),
+                         lambda: ctx.spgemm_batched([good, a], [good, b] if b is not None else None)):
+                with pytest.raises(dbd.DBDError, match="row_ptr"):
+                    call()
+            va, vb = a.view()[0], None if b is None else b.view()[0]
+            assert _ffi.load().dbd_spgemm_noalloc(
+                ctypes.byref(va), None if vb is None else ctypes.byref(vb), out[0].data_ptr(), out[1].data_ptr(),
+                out[2].data_ptr(), 25, ctypes.byref(nnz), None) == -1
+        for load in (ctx.initialize_A, ctx.initialize_B):
+            with pytest.raises(dbd.DBDError, match="row_ptr"):
+                load(bad)
+        ctx.spgemm(good, good)  # an adjoint on the kept pattern
+        va, vb = bad.view()[0], good.view()[0]
+        for x, y in ((va, vb), (vb, va)):
+            assert ctx._lib.dbd_spgemm_adjoint(ctx.handle, ctypes.byref(x), ctypes.byref(y), out[2].data_ptr(),
+                                               grads[0].data_ptr(), grads[1].data_ptr(), 1, 0) == -1
+        again = ctx.spgemm(good).C
+    np.testing.assert_array_equal(again.col_idx, want.col_idx)
+    np.testing.assert_array_equal(again.val, want.val)
+    del keep, keep2
