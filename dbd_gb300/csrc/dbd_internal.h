@@ -269,7 +269,8 @@ void launch_symbolic_bin(const SymArgs &a, int bin, int32_t begin, int32_t n, cu
 // device, a grid of resident CTAs striding over them (no host read of the
 // bin sizes, so a stream capture holds it).
 void launch_symbolic_bin_dd(const SymArgs &a, int bin, cudaStream_t s, int *launches);
-void launch_f32_to_f64(const float *src, double *dst, int64_t n, cudaStream_t s);
+// Float32 values widened, unless *badPtr (the operand's row_ptr failed) is set.
+void launch_f32_to_f64(const float *src, double *dst, int64_t n, const int *badPtr, cudaStream_t s);
 
 // One work item of the dense bin: row, or the piece of it over the column
 // slabs [s0, s1) whose entries start `off` entries into C's row (s0 < 0:

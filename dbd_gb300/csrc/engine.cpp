@@ -359,6 +359,9 @@ int validate_host(dbd_ctx *c, const dbd_csr_view *v, const char *name) {
 
 int check_operand(dbd_ctx *c, Operand &op, const CsrDev &d);
 
+// The operand's three flags on the device.
+int *operand_flags(dbd_ctx *c, const Operand &op) { return c->flags() + (&op == &c->B ? CTL_B : CTL_A); }
+
 int load_operand(dbd_ctx *c, Operand &op, const dbd_csr_view *v, const char *name) {
     int rc = validate_host(c, v, name);
     if (rc) return rc;
@@ -371,12 +374,13 @@ int load_operand(dbd_ctx *c, Operand &op, const dbd_csr_view *v, const char *nam
     d.n = v->n_cols;
     d.nnz = v->nnz;
     const size_t ne = (size_t)v->nnz;
+    const float *narrow = nullptr;  // float32 values on the device, widened behind the check
     if (v->on_device) {
         d.ptr = v->row_ptr;
         d.idx = v->col_idx;
         if (v->val_fp32) {
             CK(c, op.val.ensure(sizeof(double) * ne));
-            launch_f32_to_f64((const float *)v->val, op.val.as<double>(), v->nnz, c->stream);
+            narrow = (const float *)v->val;
             d.val = op.val.as<double>();
         } else {
             d.val = (const double *)v->val;
@@ -391,7 +395,7 @@ int load_operand(dbd_ctx *c, Operand &op, const dbd_csr_view *v, const char *nam
         if (v->val_fp32) {
             CK(c, op.tmp.ensure(sizeof(float) * ne));
             CK(c, cudaMemcpyAsync(op.tmp.p, v->val, sizeof(float) * ne, cudaMemcpyHostToDevice, c->stream));
-            launch_f32_to_f64(op.tmp.as<float>(), op.val.as<double>(), v->nnz, c->stream);
+            narrow = op.tmp.as<float>();
         } else {
             CK(c, cudaMemcpyAsync(op.val.p, v->val, sizeof(double) * ne, cudaMemcpyHostToDevice, c->stream));
         }
@@ -399,7 +403,12 @@ int load_operand(dbd_ctx *c, Operand &op, const dbd_csr_view *v, const char *nam
         d.idx = op.idx.as<int32_t>();
         d.val = op.val.as<double>();
     }
-    return check_operand(c, op, d);
+    rc = check_operand(c, op, d);
+    if (!rc && narrow) {
+        launch_f32_to_f64(narrow, op.val.as<double>(), v->nnz, operand_flags(c, op), c->stream);
+        CK(c, cudaGetLastError());
+    }
+    return rc;
 }
 
 // Enqueues the checks of an operand now on the device (row_ptr spanning
@@ -411,7 +420,7 @@ int load_operand(dbd_ctx *c, Operand &op, const dbd_csr_view *v, const char *nam
 // checks and its work estimate once.
 int check_operand(dbd_ctx *c, Operand &op, const CsrDev &d) {
     op.dev = d;
-    int *flags = c->flags() + (&op == &c->B ? CTL_B : CTL_A);
+    int *flags = operand_flags(c, op);
     CK(c, op.range.ensure(sizeof(int2) * (size_t)std::max<int64_t>(d.m, 1)));
     launch_check_operand(d, op.range.as<int2>(), flags, flags + 1, flags + 2, c->stream, c->num_sms);
     if (&op == &c->B || c->b_is_a)  // the right operand

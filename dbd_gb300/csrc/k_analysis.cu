@@ -35,13 +35,15 @@ constexpr unsigned FULL = 0xffffffffu;
 // with a host round trip after each.  33M entries in 2^21 power-law rows:
 // 1082 us in three launches before, 41 us now (20 us at copy rate); a multiply
 // of 2.1M five-point rows takes 251 us less.
-// (A row_ptr that fails its check is never read through: a row's entries are
-// touched only when both its bounds lie in [0, nnz].)
+// (A row_ptr that fails its check is never read through: no entry is touched
+// unless ptr[m] is nnz, which is what says that there are so many, and a row's
+// only when both its bounds lie in [0, nnz].)
 __global__ void __launch_bounds__(256) k_check_operand(CsrDev M, int2 *__restrict__ range, int *__restrict__ badPtr,
                                                        int *__restrict__ badIdx, int *__restrict__ unsorted) {
     __shared__ int red[8];
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t nnz = M.ptr[M.m] == M.nnz ? M.nnz : 0;
     int down = 0;
     bool badI = false, badP = false;
     auto entry = [&](int32_t c, int32_t before, bool first) {
@@ -52,8 +54,8 @@ __global__ void __launch_bounds__(256) k_check_operand(CsrDev M, int2 *__restric
     // flight; an entry's predecessor comes from the same load or the lane
     // below, only a warp's first lane loads one.
     const int lane = threadIdx.x & 31;
-    const int64_t head = min(M.nnz, (int64_t)((16 - (reinterpret_cast<uintptr_t>(M.idx) & 15)) & 15) >> 2);
-    const int64_t quads = (M.nnz - head) >> 2;
+    const int64_t head = min(nnz, (int64_t)((16 - (reinterpret_cast<uintptr_t>(M.idx) & 15)) & 15) >> 2);
+    const int64_t quads = (nnz - head) >> 2;
     const int4 *q4 = reinterpret_cast<const int4 *>(M.idx + head);
     for (int64_t b = t0 - lane; b < quads; b += 2 * stride) {
         int4 c[2];
@@ -79,7 +81,7 @@ __global__ void __launch_bounds__(256) k_check_operand(CsrDev M, int2 *__restric
     // The unaligned entries before and the remainder behind.
     if (t0 < 8) {
         const int64_t i = t0 < 4 ? t0 : head + 4 * quads + (t0 - 4);
-        if (t0 < 4 ? i < head : i < M.nnz) entry(M.idx[i], i > 0 ? M.idx[i - 1] : -1, i == 0);
+        if (t0 < 4 ? i < head : i < nnz) entry(M.idx[i], i > 0 ? M.idx[i - 1] : -1, i == 0);
     }
     // Four rows a thread in flight.
     for (int64_t b = t0; b <= M.m; b += 4 * stride) {
@@ -93,7 +95,7 @@ __global__ void __launch_bounds__(256) k_check_operand(CsrDev M, int2 *__restric
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int64_t r = b + u * stride;
-            const bool has = r < M.m && v[u] >= 0 && v[u] < w[u] && w[u] <= M.nnz;
+            const bool has = r < M.m && v[u] >= 0 && v[u] < w[u] && w[u] <= nnz;
             lo[u] = has ? __ldg(&M.idx[v[u]]) : INT32_MAX;
             hi[u] = has ? __ldg(&M.idx[w[u] - 1]) : -1;
             before[u] = has && v[u] > 0 ? __ldg(&M.idx[v[u] - 1]) : -1;
@@ -654,8 +656,11 @@ __global__ void k_scan_final(int64_t m, const int32_t *__restrict__ cnt,
     if (blockIdx.x == 0 && threadIdx.x == 0) Cp[m] = part[nparts];
 }
 
-// Widens float32 values (a view with val_fp32) into the FP64 operand copy.
-__global__ void k_f32_to_f64(const float *__restrict__ src, double *__restrict__ dst, int64_t n) {
+// Widens float32 values (a view with val_fp32) into the FP64 operand copy;
+// nothing is read where the operand's row_ptr failed its check.
+__global__ void k_f32_to_f64(const float *__restrict__ src, double *__restrict__ dst, int64_t n,
+                             const int *__restrict__ badPtr) {
+    if (*badPtr != 0) return;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         dst[i] = (double)src[i];
 }
@@ -732,9 +737,9 @@ void launch_row_scan(int64_t m, const int32_t *rowNnz, int64_t *part, int64_t *C
     }
 }
 
-void launch_f32_to_f64(const float *src, double *dst, int64_t n, cudaStream_t s) {
+void launch_f32_to_f64(const float *src, double *dst, int64_t n, const int *badPtr, cudaStream_t s) {
     if (n <= 0) return;
-    k_f32_to_f64<<<(unsigned)std::min<int64_t>(ceil_div(n, 256), 4096), 256, 0, s>>>(src, dst, n);
+    k_f32_to_f64<<<(unsigned)std::min<int64_t>(ceil_div(n, 256), 4096), 256, 0, s>>>(src, dst, n, badPtr);
 }
 
 // Loads every kernel of this file now (CUDA loads kernels lazily, on first

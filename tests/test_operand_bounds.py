@@ -49,6 +49,8 @@ int main(int argc, char **argv) {
     unsorted = 1;
     each_thread(2, 256, [&] { k_row_minmax(M, range.data(), &badPtr, &unsorted); });
     each_thread(2, 256, [&] { k_row_minmax(M, range.data(), nullptr, &unsorted); });
+    std::vector<double> wide(M.nnz);
+    each_thread(2, 256, [&] { k_f32_to_f64((const float *)idx, wide.data(), M.nnz, &badPtr); });
     printf("%%d %%d", badPtr, badIdx);
 }
 """
@@ -72,7 +74,7 @@ def checks(tmp_path_factory):
     d = tmp_path_factory.mktemp("checks")
     src, exe = str(d / "checks.cpp"), str(d / "checks")
     with open(src, "w") as f:
-        f.write(HARNESS % "\n".join(_kernel(text, k) for k in ("k_check_operand", "k_row_minmax")))
+        f.write(HARNESS % "\n".join(_kernel(text, k) for k in ("k_check_operand", "k_row_minmax", "k_f32_to_f64")))
     subprocess.run(["g++", "-O1", "-std=c++17", "-w", "-I", os.path.join(ROOT, "tests", "helpers"), src, "-o", exe],
                    check=True)
     return exe
@@ -104,10 +106,21 @@ def test_checks_stay_inside_the_columns(checks, fault, front):
     assert run.stdout == ("0 0" if fault == "well formed" else "1 0")
 
 
-def _device(torch, m, row_ptr):
-    t = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (row_ptr.astype(np.int32), m.col_idx, m.val)]
+@pytest.mark.parametrize("front", [0, 1])
+@pytest.mark.parametrize("nnz", [19, 21, 24, 5000, 1 << 21])
+def test_checks_read_no_more_entries_than_row_ptr_ends_at(checks, nnz, front):
+    """Columns (and float32 values) are read only where row_ptr's end is the number of entries that was given."""
+    run = subprocess.run([checks, "5", "20", str(front)] + [str(x) for x in GOOD], capture_output=True, text=True,
+                         env=dict(os.environ, NNZ=str(nnz)))
+    assert run.returncode == 0, f"ended by signal {-run.returncode}"
+    assert run.stdout == "1 0"
+
+
+def _device(torch, m, row_ptr, nnz=None, fp32=False):
+    val = m.val.astype(np.float32) if fp32 else m.val
+    t = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (row_ptr.astype(np.int32), m.col_idx, val)]
     torch.cuda.synchronize()
-    return dbd.CSR.from_device(m.n_rows, m.n_cols, m.nnz, *(x.data_ptr() for x in t)), t
+    return dbd.CSR.from_device(m.n_rows, m.n_cols, nnz or m.nnz, *(x.data_ptr() for x in t), val_fp32=fp32), t
 
 
 @pytest.mark.gpu
@@ -148,4 +161,33 @@ def test_entry_points_refuse_far_row_pointers(fault):
         again = ctx.spgemm(good).C
     np.testing.assert_array_equal(again.col_idx, want.col_idx)
     np.testing.assert_array_equal(again.val, want.val)
+    del keep, keep2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nnz", [19, 21, 1 << 21])
+@pytest.mark.parametrize("fp32", [False, True])
+def test_entry_points_refuse_another_number_of_entries(nnz, fp32):
+    torch = pytest.importorskip("torch")
+    from dbd_gb300 import _ffi
+    M = gen.banded(7, 1, 0)
+    M = dbd.CSR(7, 7, M.row_ptr, M.col_idx, np.ones(M.nnz))
+    good, keep = _device(torch, M, M.row_ptr, fp32=fp32)
+    bad, keep2 = _device(torch, M, M.row_ptr, nnz=nnz if nnz != M.nnz else nnz + 1, fp32=fp32)
+    out = [torch.empty(n, dtype=t, device="cuda") for n, t in
+           ((8, torch.int64), (49, torch.int32), (49, torch.float64))]
+    count = ctypes.c_int64()
+    with dbd.Context(cpu_gib=1, gpu_gib=1) as ctx:
+        for a, b in ((bad, None), (good, bad), (bad, good)):
+            with pytest.raises(dbd.DBDError, match="malformed row_ptr"):
+                ctx.spgemm(a, b)
+            if not fp32:
+                va, vb = a.view()[0], None if b is None else b.view()[0]
+                assert _ffi.load().dbd_spgemm_noalloc(
+                    ctypes.byref(va), None if vb is None else ctypes.byref(vb), out[0].data_ptr(), out[1].data_ptr(),
+                    out[2].data_ptr(), 49, ctypes.byref(count), None) == -1
+        for load in (ctx.initialize_A, ctx.initialize_B):
+            with pytest.raises(dbd.DBDError, match="malformed row_ptr"):
+                load(bad)
+        assert ctx.spgemm(good).C.val.sum() == 5 * 9 + 2 * 4
     del keep, keep2
