@@ -72,10 +72,13 @@ k_batch_rows(const BatchPair *pairs, const int64_t *rowOff, int64_t count, int64
     }
 }
 
-// Column indices (shifted to the pair's column offset) and values.
+// Column indices (shifted to the pair's column offset) and values.  Runs behind
+// k_batch_rows: where a pair's row_ptr does not end at its nnz (*bad & 1), that
+// many entries may not be there, and nothing is read.
 __global__ void __launch_bounds__(kGatherThreads)
 k_batch_entries(const BatchPair *pairs, const int64_t *nnzOff, int64_t count, int64_t totalNnz, int32_t *outIdx,
                 double *outVal, int *bad) {
+    if (*(volatile int *)bad & 1) return;
     const int64_t t0 = (int64_t)blockIdx.x * kGatherTile;
     int64_t q = first_pair(nnzOff, count, t0);
     if (nnzOff[q + 1] >= t0 + kGatherTile) {

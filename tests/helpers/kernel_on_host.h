@@ -32,6 +32,7 @@ template <class T> T __ldg(const T *p) { return *p; }
 template <class T> T __shfl_up_sync(unsigned, T v, int) { return v; }
 template <class T> T __shfl_xor_sync(unsigned, T v, int) { return v; }
 inline int atomicAdd(int *p, int v) { return *p += v; }
+inline int atomicOr(int *p, int v) { return *p |= v; }
 inline int atomicExch(int *p, int v) {
     const int old = *p;
     *p = v;

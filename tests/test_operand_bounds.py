@@ -6,7 +6,6 @@ import ctypes
 import os
 import re
 import subprocess
-import sys
 
 import numpy as np
 import pytest
@@ -16,13 +15,12 @@ from dbd_gb300 import generators as gen
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
-HARNESS = r"""
+FENCED = r"""
 #include "kernel_on_host.h"
 #include <cstdio>
-#include <cstring>
+#include <cstdlib>
 #include <sys/mman.h>
 #include <vector>
-%s
 // `n` columns with an unreadable page right behind them, or (front) before them.
 static int32_t *fenced(long n, bool front) {
     const long page = 65536, bytes = (4 * n + page - 1) / page * page;
@@ -30,6 +28,10 @@ static int32_t *fenced(long n, bool front) {
     mprotect(p + page, bytes, PROT_READ | PROT_WRITE);
     return (int32_t *)(front ? p + page : p + page + bytes - 4 * n);
 }
+"""
+
+HARNESS = FENCED + r"""
+%s
 // argv: rows, columns that there are, front; then row_ptr.
 int main(int argc, char **argv) {
     const int m = atoi(argv[1]), have = atoi(argv[2]);
@@ -55,6 +57,43 @@ int main(int argc, char **argv) {
 }
 """
 
+# Two pairs of `have` entries; the second one's row_ptr does not end at its nnz.
+GATHER = FENCED + r"""
+struct BatchPair {
+    int64_t m, nnz, ncols, nnzOff, colOff;
+    int32_t shift;
+    const int32_t *ptr, *idx;
+    const double *val;
+};
+constexpr int kGatherThreads = 256, kGatherPerThread = 8, kGatherTile = 2048;
+static int64_t first_pair(const int64_t *off, int64_t count, int64_t x) {
+    int64_t q = count - 1;
+    while (off[q] > x) --q;
+    return q;
+}
+%s
+int main(int argc, char **argv) {
+    const int have = atoi(argv[1]), given = atoi(argv[2]);
+    BatchPair p[2] = {};
+    for (int q = 0; q < 2; ++q) {
+        p[q].ncols = 7;
+        p[q].nnz = q ? given : have;
+        p[q].nnzOff = q ? have : 0;
+        int32_t *idx = fenced(have, false);
+        for (int i = 0; i < have; ++i) idx[i] = i %% 7;
+        p[q].idx = idx;
+        p[q].val = (const double *)fenced(2 * have, false);
+    }
+    const int64_t off[3] = {0, have, have + given};
+    std::vector<int32_t> outIdx(off[2]);
+    std::vector<double> outVal(off[2]);
+    int bad = have != given;
+    each_thread((int)((off[2] + kGatherTile - 1) / kGatherTile), kGatherThreads,
+                [&] { k_batch_entries(p, off, 2, off[2], outIdx.data(), outVal.data(), &bad); });
+    printf("%%d", bad);
+}
+"""
+
 
 def _kernel(text, name):
     """A kernel's definition out of the source."""
@@ -67,17 +106,26 @@ def _kernel(text, name):
             return text[at:i]
 
 
-@pytest.fixture(scope="module")
-def checks(tmp_path_factory):
-    with open(os.path.join(ROOT, "dbd_gb300", "csrc", "k_analysis.cu")) as f:
+def _program(tmp, harness, source, kernels):
+    with open(os.path.join(ROOT, "dbd_gb300", "csrc", source)) as f:
         text = f.read()
-    d = tmp_path_factory.mktemp("checks")
-    src, exe = str(d / "checks.cpp"), str(d / "checks")
+    src, exe = str(tmp / "kernels.cpp"), str(tmp / "kernels")
     with open(src, "w") as f:
-        f.write(HARNESS % "\n".join(_kernel(text, k) for k in ("k_check_operand", "k_row_minmax", "k_f32_to_f64")))
+        f.write(harness % "\n".join(_kernel(text, k) for k in kernels))
     subprocess.run(["g++", "-O1", "-std=c++17", "-w", "-I", os.path.join(ROOT, "tests", "helpers"), src, "-o", exe],
                    check=True)
     return exe
+
+
+@pytest.fixture(scope="module")
+def checks(tmp_path_factory):
+    return _program(tmp_path_factory.mktemp("checks"), HARNESS, "k_analysis.cu",
+                    ("k_check_operand", "k_row_minmax", "k_f32_to_f64"))
+
+
+@pytest.fixture(scope="module")
+def gather(tmp_path_factory):
+    return _program(tmp_path_factory.mktemp("gather"), GATHER, "k_batch.cu", ("k_batch_entries",))
 
 
 # Five rows over 20 entries; what a fault leaves of them.
@@ -114,6 +162,13 @@ def test_checks_read_no_more_entries_than_row_ptr_ends_at(checks, nnz, front):
                          env=dict(os.environ, NNZ=str(nnz)))
     assert run.returncode == 0, f"ended by signal {-run.returncode}"
     assert run.stdout == "1 0"
+
+
+@pytest.mark.parametrize("have, given", [(20, 20), (3000, 3000), (20, 21), (20, 4096), (3000, 9000), (3000, 2999)])
+def test_gather_reads_no_more_entries_than_row_ptr_ends_at(gather, have, given):
+    run = subprocess.run([gather, str(have), str(given)], capture_output=True, text=True)
+    assert run.returncode == 0, f"ended by signal {-run.returncode}"
+    assert run.stdout == str(int(have != given))
 
 
 def _device(torch, m, row_ptr, nnz=None, fp32=False):
@@ -189,5 +244,14 @@ def test_entry_points_refuse_another_number_of_entries(nnz, fp32):
         for load in (ctx.initialize_A, ctx.initialize_B):
             with pytest.raises(dbd.DBDError, match="malformed row_ptr"):
                 load(bad)
+        if not fp32:
+            for b in (None, [good, good], [good, bad]):
+                with pytest.raises(dbd.DBDError, match="a pair's row_ptr"):
+                    ctx.spgemm_batched([good, bad], b)
+            ctx.batch_plan([good, bad], [good, good], capacity=98)
+            ctx.batch_enqueue()
+            torch.cuda.synchronize()
+            with pytest.raises(dbd.DBDError, match="a pair's row_ptr"):
+                ctx.batch_result(fetch=False)
         assert ctx.spgemm(good).C.val.sum() == 5 * 9 + 2 * 4
     del keep, keep2
