@@ -1986,6 +1986,7 @@ int dbd_batch_plan(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const dbd_c
     c->bpOk = false;
     c->batchCount = 0;
     c->replayOk = false;
+    c->patternOk = false;  // C's arrays are the plan's from here on
     drop_graph(c);
     c->A.loaded = c->B.loaded = false;
     c->divided = false;

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(THREADS, kAdjCtaPerSm) k_adjoint_cta(AdjArgs a
         const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
         const int64_t c0 = a.Cp[row], c1 = a.Cp[row + 1];
         const int32_t w0 = c1 > c0 ? a.Ci[c0] >> 5 : 0;
-        const int words = c1 > c0 ? (a.Ci[c1 - 1] >> 5) - w0 + 1 : 0;
+        const int words = c1 > c0 ? max(0, (a.Ci[c1 - 1] >> 5) - w0 + 1) : 0;
         const bool ranked = words <= maxWords;
         if (ranked) {
             for (int i = tid; i < words; i += THREADS) bits[i] = 0u;
@@ -194,6 +194,10 @@ __global__ void __launch_bounds__(THREADS, kAdjCtaPerSm) k_adjoint_cta(AdjArgs a
                 const int32_t c = __ldg(&a.Ci[i]);
                 const int32_t before = i > c0 ? __ldg(&a.Ci[i - 1]) : -1;
                 const int w = (c >> 5) - w0;
+                if ((uint32_t)w >= (uint32_t)words) {  // C's columns do not ascend
+                    raise(a.err, DEV_COUNT_MISMATCH);
+                    continue;
+                }
                 atomicOr(&bits[w], 1u << (c & 31));
                 if (before < 0 || (before >> 5) != (c >> 5)) wpre[w] = (int32_t)(i - c0);
             }
