@@ -17,7 +17,7 @@
 //                               each is one run); warp bitmap ranks
 //   short rows  (<= 256 nnz)    one warp per row: symbolic by a shared hash
 //                               table; numeric by expand-sort-compress in
-//                               registers for rows of at most 512 products, else by the
+//                               registers for rows of at most 256 products, else by the
 //                               table, compaction and a bitonic sort
 //   CTA rows                    the row's A entries staged in shared memory,
 //                               warps over consecutive products with several
@@ -94,8 +94,12 @@ constexpr int kWideLoads = 4;
 // Steps of B loads a warp-hash row keeps in flight.
 constexpr int kHashWarpLoads = 2;
 // Warp-hash rows of at most this many products are sorted instead of hashed.
-constexpr int kEscMax = 512;
-constexpr int kEscShift = 9;  // bits of a product's number in their keys
+// A sorted row rounds every product before it adds, the table's fused
+// multiply-adds do not: rows of 257 to 512 products have columns of several
+// products by necessity (they hold at most 256 entries), and sorted their
+// error was 0.62 units of the last place against 0.54 (rms, against exact sums).
+constexpr int kEscMax = 256;
+constexpr int kEscShift = 8;  // bits of a product's number in their keys
 // Mean B row length from which their products are listed by groups of lanes.
 constexpr int kEscGroupLen = 6;
 
@@ -1187,7 +1191,7 @@ __device__ __forceinline__ void warp_sort(K (&key)[R]) {
     }
 }
 
-// Where a warp keeps entry p of up to 1024 it writes R consecutive ones a lane
+// Where a warp keeps entry p of up to 256 it writes R consecutive ones a lane
 // and reads 32 consecutive ones a step: rotated by p / 32 in its group of 32,
 // so that neither hits a bank more than twice.
 __device__ __forceinline__ int rotated(int p) { return (p & ~31) | ((p + (p >> 5)) & 31); }
@@ -1204,8 +1208,8 @@ __device__ __forceinline__ int rotated(int p) { return (p & ~31) | ((p + (p >> 5
 // A bucket counting sort in shared memory with each lane writing R
 // consecutive entries, the form before, was bound by the L1: 60M bank
 // conflicts and 20M store requests for 100k rows of 256 products (91% of L1
-// throughput busy): 455 -> 195 us, 550k rows of about 144 products 1611 ->
-// 973 us.  What bounds it now is instruction issue (65% busy, the ALU 68%) and
+// throughput busy): 455 -> 190 us, 550k rows of about 144 products 1611 ->
+// 1007 us (the table's rows of 257 and more among them).  What bounds it now is instruction issue (65% busy, the ALU 68%) and
 // latency, at 32 warps an SM (64 registers, 6 KB a warp; at 92 registers and
 // 20 warps 272 us).  kbuf and pv hold a product each; columns lie in
 // [rlo, rlo + 2^(bits of K - kEscShift)).
@@ -1390,29 +1394,26 @@ __device__ __forceinline__ void num_hash_warp_rows(const NumArgs &a, int32_t lo,
     const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
     // Expand-sort-compress where the products fit the registers and the
     // columns the keys; the table takes the others.
-    static_assert(TABLE >= kEscMax && (1 << kEscShift) >= kEscMax, "the arrays and keys hold the products");
+    static_assert(TABLE >= 2 * kEscMax && (1 << kEscShift) >= kEscMax, "the arrays and keys hold the products");
     const int64_t P = a.rowP[row];
     if (P <= kEscMax) {
         const int32_t rlo = a.rowLo[row];
         const int64_t span = (int64_t)a.rowHi[row] - rlo + 1;
         uint32_t *kb = reinterpret_cast<uint32_t *>(keys);
-        // Three sizes and one listing: warps of an SM that run different code
-        // miss the instruction cache.  550k rows of 60 to 280 products: 0.97 ms;
-        // with 2, 4, 5, 6, 8 and 16 keys a lane, each with its own listing,
-        // 2.05 ms; with 8 and 16 only 1.02 ms.
+        // Two sizes and one listing: warps of an SM that run different code
+        // miss the instruction cache.  550k rows of 60 to 280 products: 1.0 ms;
+        // with six sizes of 2 to 16 keys a lane, each with its own listing,
+        // 2.05 ms.
         if (span < ((int64_t)1 << (32 - kEscShift))) {
             esc_list<uint32_t>(a, e0, e1, (int)P, rlo, kb, vals);
             if (P <= 192) esc_sort<6, uint32_t>(a, row, (int)P, rlo, kb, vals);
-            else if (P <= 256) esc_sort<8, uint32_t>(a, row, (int)P, rlo, kb, vals);
-            else esc_sort<16, uint32_t>(a, row, (int)P, rlo, kb, vals);
-            return;
-        }
-        if (P <= 256) {
+            else esc_sort<8, uint32_t>(a, row, (int)P, rlo, kb, vals);
+        } else {
             unsigned long long *kb64 = reinterpret_cast<unsigned long long *>(keys);
             esc_list<unsigned long long>(a, e0, e1, (int)P, rlo, kb64, vals);
             esc_sort<8, unsigned long long>(a, row, (int)P, rlo, kb64, vals);
-            return;
         }
+        return;
     }
     for (int i = lane; i < TABLE; i += 32) {
         keys[i] = EMPTY;

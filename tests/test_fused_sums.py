@@ -1,0 +1,42 @@
+"""Rows whose sums are fused multiply-adds, by their error against exact sums.
+
+Every column of C has two products, both in [1, 2).  A fused sum rounds the
+first product (by at most 2^-53) and then the sum, which lies in [2, 4) (by at
+most 2^-52): 3 * 2^-53 in all.  Products rounded one by one before they are
+added may be off by 4 * 2^-53, and one column in sixteen is by more than 3."""
+import numpy as np
+import pytest
+
+import dbd_gb300 as dbd
+
+pytestmark = pytest.mark.gpu
+HWARP, RANKS = 3, 4
+
+
+def _exact(x):
+    """The number as an integer multiple of 2^-52 (for x in [1, 2))."""
+    return [int(v) for v in np.ldexp(x, 52).astype(np.int64)]
+
+
+# Columns of a row, the columns they are drawn from, and the bin that takes them.
+@pytest.mark.parametrize("columns, n, bin_of", [(129, 70000, HWARP), (200, 70000, HWARP), (256, 70000, HWARP),
+                                                (256, 1 << 26, HWARP)])
+def test_two_products_a_column(columns, n, bin_of):
+    rng = np.random.default_rng(columns)
+    rows = max(8, 3000 // columns)
+    # Rows 2r and 2r + 1 of B have the same columns, and row r of A takes both.
+    cols = [np.unique(np.r_[0, rng.choice(n - 2, columns - 2, replace=False) + 1, n - 1]) for _ in range(rows)]
+    idx = np.concatenate([c for c in cols for _ in "ab"]).astype(np.int32)
+    B = dbd.CSR(2 * rows, n, (np.arange(2 * rows + 1) * columns).astype(np.int32), idx, rng.uniform(1.0, 1.4, idx.size))
+    A = dbd.CSR(rows, 2 * rows, (2 * np.arange(rows + 1)).astype(np.int32), np.arange(2 * rows, dtype=np.int32),
+                rng.uniform(1.0, 1.4, 2 * rows))
+    with dbd.Context(cpu_gib=1, gpu_gib=4) as ctx:
+        res = ctx.spgemm(A, B)
+    assert res.stats["rows_per_bin"][bin_of] == rows
+    np.testing.assert_array_equal(res.C.col_idx, np.concatenate(cols))
+    a, b = _exact(A.val), _exact(B.val)
+    got = [int(v) for v in np.ldexp(res.C.val, 51).astype(np.int64)]  # in [2, 4): multiples of 2^-51
+    for r in range(rows):
+        for j in range(columns):
+            want = sum(a[2 * r + h] * b[(2 * r + h) * columns + j] for h in (0, 1))  # multiples of 2^-104
+            assert abs((got[r * columns + j] << 53) - want) <= 3 << 51
