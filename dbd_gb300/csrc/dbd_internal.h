@@ -83,7 +83,7 @@ struct Tuning {
     int32_t numWarpMax = kNumWarpMax;         // numeric rows on one warp (rank or hash)
     int32_t symWarpMax = kSymWarpMax;         // symbolic rows on a warp hash table
     int32_t rankWordsMax = kRankWordsMax;     // CTA rank kernels for windows up to this many words
-    int32_t rankSharedMax = kNumCtaLMax;      // rank rows on the small CTAs (256 threads)
+    int32_t rankSharedMax = kNumCtaLMax;      // rank rows accumulating in shared memory (256 threads)
     int32_t symHashSpanWords = kWideHashSpanWords;  // symbolic CTA rows hash above this span
     int32_t denseWarpWords = kDenseWarpWords; // numeric rows on one warp's dense window
     int32_t midSpanWords = 0;                 // numeric rows on one warp's rank window (off: the

@@ -23,8 +23,9 @@
 //                               warps over consecutive products with several
 //                               B loads in flight (warp_range_ld): hash
 //                               tables for narrow-span rows, bitmap ranks
-//                               for rows within 2^18 columns (products
-//                               reduced into C in place)
+//                               for rows within 2^18 columns (sums in shared
+//                               memory up to 4096 entries, products reduced
+//                               into C in place above)
 //   wide rows   (symbolic)      persistent CTAs, a shared bitmap over windows
 //                               of up to 2^19 columns that stays zero between
 //                               rows, kept for the numeric rank kernels
@@ -1533,28 +1534,37 @@ __global__ void __launch_bounds__(THREADS) k_num_hash_cta_dd(NumArgs a, int bin)
 // pass, or set here by a pass over the products); a scan of the words' counts
 // ranks every pair of words, which gives a column's position in C's row by
 // one 64-bit load and a bit count.  Columns are written balanced by position,
-// and a pass over the products adds each one into C's row in place by an FP64
-// reduction at L2.  No hashing, no sorting, no values in shared memory.
+// and a pass over the products adds each one at its rank.  No hashing, no
+// sorting.
 //
 // P is the type of the pairs' ranks: 16 bits for the rows of the small CTAs
-// (at most kNumCtaLMax entries), which with 44 KB a CTA at the widest window
-// puts five of them on an SM, six at narrower ones; a row is a chain of short
-// phases with barriers between them, so what bounds it is how many rows an SM
-// has in flight, as long as the ranking is free of bank conflicts.  Such rows
-// used to accumulate in shared memory (compare-and-swap loops around a
-// multiply-add, 102 KB and 256 threads a CTA, two CTAs per SM): 57k of R-MAT
-// 2^18 3.13 -> 1.36 ms, 18k of 2^16 0.75 -> 0.28.  The larger rows (512
-// threads, two CTAs an SM) are bound by the reductions' 25 sectors a step and
+// (at most kNumCtaLMax entries).  Their sums are fused multiply-adds in shared
+// memory (compare-and-swap loops), kRankVals entries a pass over the products,
+// written out in whole sectors; with 75 KB a CTA at the widest window three of
+// them share an SM, five at 2^16 columns.  The compare-and-swap loops bound
+// them: four of a lane's in flight together, or more CTAs of a smaller
+// kRankVals, are no faster (57k rows of R-MAT 2^18 1.99 ms; 2.02 and 2.19), and
+// 384 or 512 threads a CTA are slower (2.19, 2.49).  The same rows reduced into
+// C in place, as the large ones are, take 1.36 ms but round every product
+// before it is added: 0.64 units of the last place instead of 0.56 (rms, R-MAT
+// 2^14, against exact sums).  57k rows of 2^18 3.13 ms before the ranks were 16
+// bits and taken by warp steps, 18k of 2^16 0.75 -> 0.39.
+//
+// The larger rows (512 threads, two CTAs an SM) add into C in place by FP64
+// reductions at L2 and are bound by the reductions' 25 sectors a step and
 // by what of C and B stays in L2 meanwhile: C's values are zeroed right before
 // the products, not earlier (33k rows of 2^18 4.76 -> 4.60 ms; 5.01 with the
 // ranks a group of words a thread), and a third CTA an SM, which 2^16 gains
 // 3% from, costs 2^18 6%.
-// CTAs an SM is to hold: 40 registers a thread for the small ones.
-__host__ __device__ constexpr int rank_ctas(int threads) { return threads == 256 ? 6 : 2; }
+constexpr int kRankSThreads = 256;  // rows of at most tune.rankSharedMax entries
+constexpr int kRankLThreads = 512;
+constexpr int kRankVals = 3960;  // with 2^18 columns, a third of an SM's shared memory
+// CTAs an SM is to hold: 48 registers a thread for the small ones.
+__host__ __device__ constexpr int rank_ctas(int threads) { return threads == kRankSThreads ? 5 : 2; }
 
 // Where the rank kernel's bitmap starts behind the staging area.
 __host__ __device__ constexpr size_t rank_bits_at(int threads) {
-    return (threads == 256 ? StageLayout<256>::bytes : StageLayout<512>::bytes) / 16 * 16 + 16;
+    return (threads == kRankSThreads ? StageLayout<kRankSThreads>::bytes : StageLayout<kRankLThreads>::bytes) / 16 * 16 + 16;
 }
 
 template <int THREADS, class P>
@@ -1567,7 +1577,9 @@ __device__ __forceinline__ void num_rank_rows(const NumArgs &a, int32_t lo, int 
     int32_t *bst = reinterpret_cast<int32_t *>(smem + L::bst);
     double *av = reinterpret_cast<double *>(smem + L::av);
     uint32_t *bits = reinterpret_cast<uint32_t *>(smem + rank_bits_at(THREADS));
-    P *pairRank = reinterpret_cast<P *>(bits + maxWords);
+    constexpr bool kShared = sizeof(P) == 2;  // the row's values in shared memory
+    double *vals = reinterpret_cast<double *>(bits + maxWords);
+    P *pairRank = reinterpret_cast<P *>(bits + maxWords + (kShared ? 2 * kRankVals : 0));
     // Per group of words, the rank of its first column and its non-empty
     // words, kept in the staging area (idle between the passes).
     static_assert(8 * THREADS <= L::bytes && kRankWordsMax <= 32 * THREADS, "rank groups");
@@ -1664,30 +1676,49 @@ __device__ __forceinline__ void num_rank_rows(const NumArgs &a, int32_t lo, int 
     }
     __syncthreads();
     write_columns_balanced<THREADS>(bits, tbase, tmask, wpt, tot, a.Ci + obase, expect, obc);
-    // C's values start at zero.
-    for (int i = tid; i < expect; i += THREADS) cv[i] = 0.0;
-    __syncthreads();
-
-    for (int32_t eb = e0; eb < e1; eb += THREADS) {
-        int nb;
-        const int32_t total =
-            stage_entries<THREADS, true>(a.A, a.B, eb, min(THREADS, e1 - eb), pre, bst, av, &nb, sh);
-        int32_t tb, te;
-        warp_share<THREADS>(total, &tb, &te);
-        warp_range_ld<4>(
-            pre, bst, nb, tb, te,
-            [&](int32_t pos) { return ColVal{__ldg(&a.B.idx[pos]), __ldg(&a.B.val[pos])}; },
-            [&](bool v, const ColVal &x, int e) {
-                const uint32_t c = (uint32_t)(x.c - cbase);
-                if (v && c < (uint32_t)nwords * 32u) {
-                    const uint2 word = *reinterpret_cast<const uint2 *>(bits + (c >> 6) * 2u);
-                    const uint32_t below = (1u << (c & 31u)) - 1u;
-                    const uint32_t r = (uint32_t)pairRank[c >> 6] + ((c & 32u) ? __popc(word.x) + __popc(word.y & below)
-                                                                              : __popc(word.x & below));
-                    if (r < (uint32_t)expect) atomicAdd(&cv[r], __dmul_rn(av[e], x.v));
-                }
+    // Every product, as add(its rank, A value, B value).
+    auto products = [&](auto &&add) {
+        for (int32_t eb = e0; eb < e1; eb += THREADS) {
+            int nb;
+            const int32_t total =
+                stage_entries<THREADS, true>(a.A, a.B, eb, min(THREADS, e1 - eb), pre, bst, av, &nb, sh);
+            int32_t tb, te;
+            warp_share<THREADS>(total, &tb, &te);
+            warp_range_ld<4>(
+                pre, bst, nb, tb, te,
+                [&](int32_t pos) { return ColVal{__ldg(&a.B.idx[pos]), __ldg(&a.B.val[pos])}; },
+                [&](bool v, const ColVal &x, int e) {
+                    const uint32_t c = (uint32_t)(x.c - cbase);
+                    if (v && c < (uint32_t)nwords * 32u) {
+                        const uint2 word = *reinterpret_cast<const uint2 *>(bits + (c >> 6) * 2u);
+                        const uint32_t below = (1u << (c & 31u)) - 1u;
+                        add((uint32_t)pairRank[c >> 6] + ((c & 32u) ? __popc(word.x) + __popc(word.y & below)
+                                                                    : __popc(word.x & below)),
+                            av[e], x.v);
+                    }
+                });
+            __syncthreads();
+        }
+    };
+    if constexpr (kShared) {
+        for (int32_t r0 = 0; r0 < expect; r0 += kRankVals) {  // once, but for the largest rows
+            const int n = min(expect - r0, kRankVals);
+            for (int i = tid; i < n; i += THREADS) vals[i] = 0.0;
+            __syncthreads();
+            products([&](uint32_t r, double x, double y) {
+                r -= (uint32_t)r0;
+                if (r < (uint32_t)n) atomic_fma(&vals[r], x, y);
             });
+            for (int i = tid; i < n; i += THREADS) cv[r0 + i] = vals[i];
+            __syncthreads();
+        }
+    } else {
+        // C's values start at zero.
+        for (int i = tid; i < expect; i += THREADS) cv[i] = 0.0;
         __syncthreads();
+        products([&](uint32_t r, double x, double y) {
+            if (r < (uint32_t)expect) atomicAdd(&cv[r], __dmul_rn(x, y));
+        });
     }
 }
 
@@ -2713,8 +2744,6 @@ constexpr size_t kSmemNumCtaS = StageLayout<kNumCtaSThreads>::bytes + (size_t)kN
 constexpr size_t kSmemNumCtaL = StageLayout<kNumCtaLThreads>::bytes + (size_t)kNumCtaLTable * 12;
 constexpr size_t kSmemDense = (size_t)kDenseWindow * 8 + kDenseWindow / 8 + (size_t)kDenseStage * 8;
 constexpr size_t kSmemWideBase = StageLayout<kWideThreads>::bytes;
-constexpr int kRankSThreads = 256;  // rows of at most tune.rankSharedMax entries
-constexpr int kRankLThreads = 512;
 constexpr int kBitwRows = 8;
 constexpr int kRankwRows = 8;
 constexpr int kDensewRows = 4;  // 8 rows a CTA: 8.2 ms where 4 take 7.9
@@ -2732,9 +2761,11 @@ constexpr size_t kSmemRankm =
 }  // namespace
 
 // Dynamic shared memory of the rank kernel: staging, bitmap and pair ranks of
-// maxWords words.
+// maxWords words, and the small CTAs' values.
 static size_t smem_rank(int threads, int maxWords) {
-    return rank_bits_at(threads) + 4 * (size_t)maxWords + (threads == kRankSThreads ? 2 : 4) * (size_t)(maxWords / 2);
+    const bool small = threads == kRankSThreads;
+    return rank_bits_at(threads) + 4 * (size_t)maxWords + (small ? 2 : 4) * (size_t)(maxWords / 2) +
+           (small ? 8 * (size_t)kRankVals : 0);
 }
 
 // Words of the rank kernels' bitmap: the threshold's, or all of C's columns

@@ -361,8 +361,9 @@ int dbd_batch_result(dbd_ctx *ctx, int64_t *c_row_off, int64_t *c_nnz_off, dbd_c
  *                          one-warp hash table (32..512)
  *   rank_words_max         CTA rank kernels take windows up to this many words;
  *                          wider rows use CTA hash tables or dense windows (1..8192)
- *   rank_shared_max_nnz    rank rows up to this size take CTAs of 256 threads
- *                          and 16-bit ranks, larger ones 512 (1..4096)
+ *   rank_shared_max_nnz    rank rows up to this size accumulate in shared
+ *                          memory (fused multiply-adds), larger ones in place
+ *                          in C (rounded products, added at L2) (1..4096)
  *   sym_hash_span_words    symbolic rows with at most 4096 products hash
  *                          (instead of a bitmap) above this span (>= 0)
  *   dense_warp_span_words  numeric rows whose window spans at most this many

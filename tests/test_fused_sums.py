@@ -20,7 +20,8 @@ def _exact(x):
 
 # Columns of a row, the columns they are drawn from, and the bin that takes them.
 @pytest.mark.parametrize("columns, n, bin_of", [(129, 70000, HWARP), (200, 70000, HWARP), (256, 70000, HWARP),
-                                                (256, 1 << 26, HWARP)])
+                                                (256, 1 << 26, HWARP), (257, 70000, RANKS), (1000, 4000, RANKS),
+                                                (3960, 250000, RANKS), (3961, 250000, RANKS), (4096, 250000, RANKS)])
 def test_two_products_a_column(columns, n, bin_of):
     rng = np.random.default_rng(columns)
     rows = max(8, 3000 // columns)
