@@ -899,6 +899,21 @@ int product_fingerprint(dbd_ctx *c, uint64_t *out) {
 
 // ---- stage 3: the distributor --------------------------------------------
 
+// Device memory held by operands and work arrays.
+double work_bytes(const dbd_ctx *c) {
+    return (double)(c->A.ptr.cap + c->A.idx.cap + c->A.val.cap + c->B.ptr.cap + c->B.idx.cap + c->B.val.cap +
+                    c->rowP.cap + c->symBin.cap + c->numBin.cap + c->rowNnz.cap + c->symList.cap + c->numList.cap +
+                    c->hist.cap + c->symTileOff.cap + c->numTileOff.cap + c->part.cap + c->Cp.cap + c->cursor.cap +
+                    (c->gSlots ? c->gdense.cap : 0) + (c->scrSlots ? c->dscr.cap : 0) + c->wideBits.cap +
+                    c->heavySlot.cap + c->slabCnt.cap + c->items.cap);
+}
+
+// And by what only the last adjoint or symbolic pass used: a multiply whose C
+// does not fit beside it gives it back.
+double lent_bytes(const dbd_ctx *c) {
+    return (double)(c->adjProd.cap + c->adjOff.cap + c->adjItems.cap + c->symItems.cap);
+}
+
 int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
     if (!c->divided) {
         int rc = divide_blocks(c);
@@ -943,14 +958,7 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
     const int64_t m = c->m, nnz = c->nnzC;
     const double gpu_budget = c->cfg.gpu_gib * kGiB;
     const double host_budget = c->cfg.host_gib * kGiB;
-    // Device memory already held by operands and work arrays.
-    const double used = (double)(c->A.ptr.cap + c->A.idx.cap + c->A.val.cap + c->B.ptr.cap + c->B.idx.cap +
-                                 c->B.val.cap + c->rowP.cap + c->symBin.cap + c->numBin.cap + c->rowNnz.cap +
-                                 c->symList.cap + c->numList.cap + c->hist.cap + c->symTileOff.cap +
-                                 c->numTileOff.cap + c->part.cap + c->Cp.cap + c->cursor.cap +
-                                 (c->gSlots ? c->gdense.cap : 0) + (c->scrSlots ? c->dscr.cap : 0) +
-                                 c->wideBits.cap + c->heavySlot.cap + c->slabCnt.cap + c->items.cap);
-    double dev_avail = gpu_budget - used;
+    double dev_avail = gpu_budget - work_bytes(c) - lent_bytes(c);
     // What the device has free matters where C's arrays have yet to be
     // allocated (asking takes 25 us).
     const size_t held = (size_t)std::max<int64_t>(nnz, 1);
@@ -959,6 +967,12 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
         size_t free_b = 0, total_b = 0;
         CK(c, cudaMemGetInfo(&free_b, &total_b));
         dev_avail = std::min(dev_avail, (double)free_b - 512.0 * 1024 * 1024);
+        // C goes before what an adjoint may need again.
+        if (lent_bytes(c) > 0 && 16.0 * (double)nnz > std::max(0.0, dev_avail)) {
+            for (DevBuf *b : {&c->adjProd, &c->adjOff, &c->adjItems, &c->symItems}) b->release();
+            CK(c, cudaMemGetInfo(&free_b, &total_b));
+            dev_avail = std::min(gpu_budget - work_bytes(c), (double)free_b - 512.0 * 1024 * 1024);
+        }
     }
     const bool copies = scope != DBD_SCOPE_KERNEL;
     // The reference's output layout (float32 values): the copying scopes
@@ -1732,10 +1746,14 @@ int dbd_spgemm_adjoint(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b,
         else cudaGetLastError();
     }
     int launches = 0;
-    if (det && B.nnz > 0 && A.nnz > 0 && 8.0 * (double)c->products <= c->cfg.gpu_gib * kGiB / 8) {
+    const double gpu_budget = c->cfg.gpu_gib * kGiB;
+    const double beside = work_bytes(c) + (double)(c->Ci.cap + c->Cv.cap + c->adjItems.cap + c->symItems.cap);
+    if (det && B.nnz > 0 && A.nnz > 0 && 8.0 * (double)c->products <= gpu_budget / 8 &&
+        beside + 8.0 * (double)c->products + 12.0 * (double)A.nnz <= gpu_budget) {
         // The products of the dA pass are kept for the dB pass within an
-        // eighth of the GPU budget (as the wide rows' bitmaps are) and where
-        // the device has the room; otherwise the dB pass looks G up again.
+        // eighth of the GPU budget (as the wide rows' bitmaps are), what the
+        // context holds leaves of it, and where the device has the room;
+        // otherwise the dB pass looks G up again.
         const size_t oLen = (8 * (size_t)(A.nnz + 1) + 15) / 16 * 16;
         const size_t oScan = oLen + (4 * (size_t)A.nnz + 15) / 16 * 16;
         if (c->adjProd.ensure(8 * (size_t)std::max<int64_t>(c->products, 1)) == cudaSuccess &&
