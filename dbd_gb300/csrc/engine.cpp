@@ -976,11 +976,13 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
     }
     const bool copies = scope != DBD_SCOPE_KERNEL;
     // The reference's output layout (float32 values): the copying scopes
-    // round each chunk's FP64 values once on the device, so 8 bytes per
-    // entry cross the link instead of 12.  Device slots then hold 16 bytes
-    // per entry (FP64 accumulators + their float32 copy).
+    // round each value once on its way to the host, so 8 bytes per entry
+    // cross the link instead of 12.  A device digest reads the float values
+    // on the device: its slots hold them beside the FP64 ones.
     const bool f32out = copies && c->cfg.out_val_fp32 != 0;
-    const double dev_bpe = f32out ? 16.0 : 12.0;
+    const bool devF32 = f32out && (c->digest & DBD_DIGEST_DEVICE) != 0;
+    if (f32out && !devF32) c->Cf.release();
+    const double dev_bpe = devF32 ? 16.0 : 12.0;
     const double host_bpe = f32out ? 8.0 : 12.0;
     const size_t hve = f32out ? sizeof(float) : sizeof(double);  // host bytes per value
     const double out_bytes = 12.0 * (double)nnz;
@@ -1085,9 +1087,6 @@ int distribute(dbd_ctx *c, dbd_scope scope, const char *out_dir) {
     const size_t slot_entries = resident ? (size_t)std::max<int64_t>(nnz, 1) : (size_t)cap_entries;
     CK(c, c->Ci.ensure(sizeof(int32_t) * slot_entries * nslots));
     CK(c, c->Cv.ensure(sizeof(double) * slot_entries * nslots));
-    // A device digest reads the float values on the device; otherwise they are
-    // rounded on their way to the host.
-    const bool devF32 = f32out && (c->digest & DBD_DIGEST_DEVICE) != 0;
     if (devF32) CK(c, c->Cf.ensure(sizeof(float) * slot_entries * nslots));
     c->dev_resident = resident;
     c->host_f32 = f32out;
