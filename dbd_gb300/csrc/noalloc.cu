@@ -69,8 +69,12 @@ int device_scratch(int dev, unsigned char **out, Mailbox **mail) {
             snprintf(g_msg, sizeof(g_msg), "cudaGetSymbolAddress: %s", cudaGetErrorString(e));
             return report(DBD_ERR_CUDA);
         }
+        // Allowed beside another thread's capture, which it has no part in.
         void *h = nullptr;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
         e = cudaMallocHost(&h, sizeof(Mailbox));
+        cudaThreadExchangeStreamCaptureMode(&mode);
         if (e != cudaSuccess) {
             snprintf(g_msg, sizeof(g_msg), "cudaMallocHost: %s", cudaGetErrorString(e));
             return report(DBD_ERR_OOM_HOST);
@@ -163,15 +167,10 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
                  need, (long long)m, (long long)a->nnz, kDbdNoallocScratchBytes);
         return report(DBD_ERR_BUDGET);
     }
-    int dev = 0;
-    NA_CK(cudaGetDevice(&dev));
-    unsigned char *base = nullptr;
-    Mailbox *box = nullptr;
-    int rc = device_scratch(dev, &base, &box);
-    if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream_handle;
-    // The call synchronises with the host twice (bin sizes, nnz(C)), which a
-    // stream capture cannot hold: refuse it before anything is enqueued.
+    // The call synchronises with the host (bin sizes, nnz(C), the error word),
+    // which a stream capture cannot hold: refuse it before anything is enqueued,
+    // and before the set-up, whose pinned allocation would break the capture.
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
         cudaGetLastError();
@@ -179,6 +178,12 @@ extern "C" int dbd_spgemm_noalloc(const dbd_csr_view *a, const dbd_csr_view *b, 
     }
     if (cap != cudaStreamCaptureStatusNone)
         return fail(DBD_ERR_INVALID, "the stream is capturing: this call synchronises and cannot be captured");
+    int dev = 0;
+    NA_CK(cudaGetDevice(&dev));
+    unsigned char *base = nullptr;
+    Mailbox *box = nullptr;
+    int rc = device_scratch(dev, &base, &box);
+    if (rc) return rc;
     Carver c{base};  // the layout of scratch_bytes()
     const size_t nt = (size_t)ceil_div(m, kTileRows) + 1;
     int2 *range = c.take<int2>((size_t)b->n_rows);
