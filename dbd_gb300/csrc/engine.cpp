@@ -442,16 +442,17 @@ int clear_ctl(dbd_ctx *c) {
 // The pending checks' results, from flags the host has read.
 int judge_operands(dbd_ctx *c, const int32_t *flags) {
     int rc = DBD_OK;
-    if (const int32_t bad = flags[CTL_PAIR])
+    if (const int32_t bad = flags[CTL_PAIR]) {
+        c->A.loaded = c->B.loaded = false;
         rc = set_err(c, DBD_ERR_INVALID, (bad & 1) ? "a pair's row_ptr does not span [0, nnz] monotonically"
                                                    : "a pair's column index is out of range");
+    }
     for (Operand *op : {&c->A, &c->B}) {
         if (!op->pending) continue;
         op->pending = false;
         const bool isB = op == &c->B;
         const int32_t *f = flags + (isB ? CTL_B : CTL_A);
         op->sorted = f[2] ? 0 : 1;
-        if (flags[CTL_PAIR]) op->loaded = false;
         if (f[0] || f[1]) {
             op->loaded = false;
             if (!rc)
@@ -470,10 +471,19 @@ int settle_operands(dbd_ctx *c) {
     return judge_operands(c, c->mail()->flags);
 }
 
+// Operands whose checks a failed call left unread are not loaded: their flags
+// are about to be cleared.
+void drop_pending(dbd_ctx *c) {
+    for (Operand *op : {&c->A, &c->B}) {
+        if (op->pending) op->loaded = false;
+        op->pending = false;
+    }
+}
+
 // Loads A and B (null: A again), their checks pending.  A fault of A's is
 // reported ahead of one of B's.
 int load_pair(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b) {
-    c->A.pending = c->B.pending = false;
+    drop_pending(c);
     c->b_is_a = b == nullptr;
     int rc = clear_ctl(c);
     if (!rc) rc = load_operand(c, c->A, a, "A");
@@ -1524,6 +1534,7 @@ int dbd_load_a(dbd_ctx *c, const dbd_csr_view *a) {
     if (!c || !a) return DBD_ERR_INVALID;
     cudaSetDevice(c->cfg.device);
     c->b_is_a = false;
+    drop_pending(c);
     CK(c, cudaMemsetAsync(c->flags(), 0, sizeof(int32_t) * CTL_ERR, c->stream));
     int rc = load_operand(c, c->A, a, "A");
     return rc ? rc : settle_operands(c);
@@ -1533,6 +1544,7 @@ int dbd_load_b(dbd_ctx *c, const dbd_csr_view *b) {
     if (!c || !b) return DBD_ERR_INVALID;
     cudaSetDevice(c->cfg.device);
     c->b_is_a = false;
+    drop_pending(c);
     CK(c, cudaMemsetAsync(c->flags(), 0, sizeof(int32_t) * CTL_ERR, c->stream));
     int rc = load_operand(c, c->B, b, "B");
     return rc ? rc : settle_operands(c);
@@ -1841,6 +1853,7 @@ int dbd_spgemm_batched(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const d
     c->batchCount = 0;
     c->replayOk = false;
     drop_graph(c);
+    drop_pending(c);
     c->A.loaded = c->B.loaded = false;
     c->divided = false;
     const bool square = b == nullptr;
@@ -1948,16 +1961,16 @@ int dbd_spgemm_batched(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const d
     da.ptr = c->A.ptr.as<int32_t>();
     da.idx = c->A.idx.as<int32_t>();
     da.val = c->A.val.as<double>();
-    c->A.pending = c->B.pending = false;
     c->b_is_a = square;
     if (square) {
         rc = check_operand(c, c->A, da);
         if (rc) return rc;
     } else {
         // The gather has checked A's pairs; its order and row ranges matter
-        // for a right operand only.
+        // for a right operand only, and are not known.
         c->A.dev = da;
-        c->A.loaded = c->A.pending = true;
+        c->A.loaded = true;
+        c->A.sorted = 0;
         c->divided = false;
     }
     if (!square) {
@@ -2005,6 +2018,7 @@ int dbd_batch_plan(dbd_ctx *c, int64_t count, const dbd_csr_view *a, const dbd_c
     c->replayOk = false;
     c->patternOk = false;  // C's arrays are the plan's from here on
     drop_graph(c);
+    drop_pending(c);
     c->A.loaded = c->B.loaded = false;
     c->divided = false;
     const bool square = b == nullptr;
