@@ -142,9 +142,9 @@ enum DevErr : int { DEV_OK = 0, DEV_TABLE_FULL = 1, DEV_COUNT_MISMATCH = 2, DEV_
 
 // Counter slots for dynamically scheduled kernels (zeroed per multiply).
 enum CounterSlot : int {
-    CTR_SYM_TINY = 0, CTR_SYM_HWARP, CTR_SYM_HCTA, CTR_SYM_WIDE, CTR_NUM_GDENSE, CTR_NUM_RANKWIN, CTR_NUM_DSCR,
-    CTR_HEAVY, CTR_ITEMS, CTR_ADJOINT, CTR_ADJ_ITEMS, CTR_SYM_ITEMS, CTR_SYM_NEXT,
-    CTR_MAX_P, CTR_COUNT = 16
+    CTR_SYM_WIDE = 0, CTR_NUM_GDENSE, CTR_NUM_RANKWIN, CTR_NUM_DSCR, CTR_HEAVY, CTR_ITEMS,
+    CTR_ADJOINT,  // the adjoint's: next item, then AdjCounter
+    CTR_SYM_ITEMS = CTR_ADJOINT + 6, CTR_SYM_NEXT, CTR_MAX_P, CTR_COUNT = 16
 };
 
 struct Binning {
@@ -362,6 +362,14 @@ inline int64_t adjoint_part_products(int64_t products, int num_sms) {
 }
 // Most parts that rows of `products` products in all can make.
 inline int64_t adjoint_part_cap(int64_t products, int64_t partP) { return products / partP + products / (2 * partP); }
+// Counters behind the next item's: parts, and rows that a CTA, four warps (over
+// more entries of C or fewer) and a warp take.
+enum AdjCounter : int { ADJ_PARTS = 1, ADJ_CTA, ADJ_WIDE, ADJ_QUAD, ADJ_WARP, ADJ_COUNTERS };
+// Rows of the CTA bins from which on they are told apart by their shape: two
+// rounds of the CTAs that fit at once.  2000 rows of 289 to 1600 products are as
+// fast either way (90 to 126 us); with 300 rows the further launches show (96 to
+// 131 us).
+inline int64_t adjoint_apart_rows(int num_sms) { return 10 * (int64_t)num_sms; }
 
 struct AdjArgs {
     CsrDev A, B;
@@ -371,24 +379,32 @@ struct AdjArgs {
     double *dA;
     double *dB;
     const int32_t *order;  // rows of A in the forward's numeric bin order
-    uint32_t *ctr;         // row counter of the CTA kernel, then its items
+    uint32_t *ctr;         // next item of the CTA kernel, then AdjCounter
     // With dB null: where to keep every product A(i,j) * G(i,k) for the
     // deterministic dB pass (null: nowhere), entry e's from off[e] on in B's
     // row order.
     double *prod = nullptr;
     const int64_t *off = nullptr;
     int64_t prodCap = 0;
-    // Rows of at least 2 * partP products (rowP) in parts (no items: none is
-    // cut); room for adjoint_part_cap() items, their count in ctr[1].
+    // With items, the rows of the CTA bins are told apart (launch_adjoint_split):
+    // those of at least 2 * partP products (rowP) go in parts, room for
+    // adjoint_part_cap() of them; the others' lists are by AdjCounter (only
+    // ADJ_CTA's given: a CTA takes each of them).
     const int64_t *rowP = nullptr;
     AdjItem *items = nullptr;
+    int32_t *rows[ADJ_COUNTERS] = {};
     int64_t partP = 0, itemCap = 0;
     int *err;
 };
 // Rows order[lo, hi) whose rows of C hold at most 512 entries (one warp each).
 void launch_adjoint_warp(const AdjArgs &a, int32_t lo, int32_t hi, cudaStream_t s, int *launches);
-// Rows order[lo, hi) of any size, the last ones first.
+// Clears the counters and, with a.items, tells the rows order[lo, hi) apart.
+void launch_adjoint_split(const AdjArgs &a, int32_t lo, int32_t hi, cudaStream_t s, int *launches);
+// Behind it: the parts and the rows of order[lo, hi) that a CTA takes, the last
+// ones first; and the rows among n that four warps (kind ADJ_WIDE, ADJ_QUAD) or
+// one warp (ADJ_WARP) take.
 void launch_adjoint_cta(const AdjArgs &a, int32_t lo, int32_t hi, int num_sms, cudaStream_t s, int *launches);
+void launch_adjoint_rows(const AdjArgs &a, int kind, int32_t n, int num_sms, cudaStream_t s, int *launches);
 // dB = mask_B(A^T G) on its own: a thread per entry (k, j) of B, summing
 // A(i,k) * G(i,j) over column k of A in row order, long columns in segments
 // (colPtr / perm / rowOf: A's entries grouped by column, stably).

@@ -1750,11 +1750,20 @@ int dbd_spgemm_adjoint(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b,
     aa.err = c->err();
     aa.rowP = c->rowP.as<int64_t>();
     aa.partP = adjoint_part_products(c->products, c->num_sms);
-    if (c->maxRowP >= 2 * aa.partP) {
-        // Without the room no row is cut.
+    const int32_t ctaLo = c->numStart_h[NB_RANKS], ctaHi = c->numStart_h[NB_DENSEW], ctaRows = ctaHi - ctaLo;
+    const bool apart = ctaRows >= adjoint_apart_rows(c->num_sms);
+    if (ctaRows > 0 && (apart || c->maxRowP >= 2 * aa.partP)) {
+        // Without the room a CTA takes each of their rows.
         aa.itemCap = adjoint_part_cap(c->products, aa.partP);
-        if (c->adjItems.ensure(sizeof(AdjItem) * (size_t)aa.itemCap) == cudaSuccess) aa.items = c->adjItems.as<AdjItem>();
-        else cudaGetLastError();
+        const int lists = apart ? ADJ_COUNTERS - ADJ_CTA : 1;
+        if (c->adjItems.ensure(sizeof(AdjItem) * (size_t)aa.itemCap +
+                               sizeof(int32_t) * (size_t)lists * (size_t)ctaRows) == cudaSuccess) {
+            aa.items = c->adjItems.as<AdjItem>();
+            int32_t *at = reinterpret_cast<int32_t *>(aa.items + aa.itemCap);
+            for (int q = 0; q < lists; ++q) aa.rows[ADJ_CTA + q] = at + (size_t)q * (size_t)ctaRows;
+        } else {
+            cudaGetLastError();
+        }
     }
     int launches = 0;
     const double gpu_budget = c->cfg.gpu_gib * kGiB;
@@ -1780,14 +1789,25 @@ int dbd_spgemm_adjoint(dbd_ctx *c, const dbd_csr_view *a, const dbd_csr_view *b,
         }
     }
     // The numeric bins between the CTA rank rows and the dense ones hold the
-    // rows of C that need a CTA (numWarpMax entries or more); a warp takes the
-    // others, at most kDenseWarpWords * 32 entries long.
+    // rows of C of more than numWarpMax entries, which are told apart on the
+    // device; a warp takes the others, at most kDenseWarpWords * 32 entries long.
     c->sused = 0;
     {
         Fork fk(c);
-        launch_adjoint_cta(aa, c->numStart_h[NB_RANKS], c->numStart_h[NB_DENSEW], c->num_sms, fk.stream(0), &launches);
-        launch_adjoint_warp(aa, c->numStart_h[NB_TINY], c->numStart_h[NB_RANKS], fk.stream(1), &launches);
-        launch_adjoint_warp(aa, c->numStart_h[NB_DENSEW], c->numStart_h[NB_COUNT], fk.stream(2), &launches);
+        if (ctaRows > 0) {
+            cudaStream_t s = fk.stream(0);
+            launch_adjoint_split(aa, ctaLo, ctaHi, s, &launches);
+            cudaEvent_t told = c->sync_ev();
+            cudaEventRecord(told, s);
+            launch_adjoint_cta(aa, ctaLo, ctaHi, c->num_sms, s, &launches);
+            for (int kind = ADJ_WIDE; kind <= ADJ_WARP; ++kind) {
+                if (!aa.rows[kind]) continue;
+                cudaStreamWaitEvent(fk.stream(kind), told, 0);
+                launch_adjoint_rows(aa, kind, ctaRows, c->num_sms, fk.stream(kind), &launches);
+            }
+        }
+        launch_adjoint_warp(aa, c->numStart_h[NB_TINY], ctaLo, fk.stream(1), &launches);
+        launch_adjoint_warp(aa, ctaHi, c->numStart_h[NB_COUNT], fk.stream(2), &launches);
         fk.join();
     }
     if (det && B.nnz > 0) {

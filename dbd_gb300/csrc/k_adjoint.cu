@@ -4,8 +4,9 @@
 // device (CSR, columns ascending in every row):
 //   dA = mask_A(G * B^T)   dA(i,k) = sum_j G(i,j) * B(k,j)
 //   dB = mask_B(A^T * G)   dB(k,j) = sum_i A(i,k) * G(i,j)
-// k_adjoint_warp and k_adjoint_cta take both from A's rows (dB by FP64 reductions); with the
-// deterministic option dB comes from its own pass over B's pattern
+// k_adjoint_rows and k_adjoint_cta take both from A's rows (dB by FP64
+// reductions); with the deterministic option dB comes from its own pass over B's
+// pattern
 // (k_entry_rows, the stable radix sort of k_mtx.cu, k_col_ptr, then the
 // k_adjoint_db kernels).
 #include "cta_stage.cuh"
@@ -29,43 +30,65 @@ __device__ __forceinline__ int64_t find_col(const int32_t *__restrict__ ci, int6
     return (lo < end && ci[lo] == k) ? lo : end;
 }
 
-// Rows of C of at most kAdjWarpNnz entries: one warp per row of A.  The row's
+// Rows of C of at most NNZ entries: WARPS warps per row of A.  The row's
 // columns and G sit in shared memory, so a product's G(i,j) is a binary
 // search there instead of one through L2 (each step of which the product
-// would wait for); eight lanes take one entry of A at a time, four entries a
-// step, so that short B rows fill the warp without an owner search and an
-// entry's dA is one sum over eight lanes.  Two FP64 instructions a product:
-// the fused multiply-add into dA and the multiply whose sum into dB the L2
-// does.  100k rows of 256 products: 380 -> 242 us.
-constexpr int kAdjWarpNnz = 512;
-constexpr int kAdjWarpRows = 4;  // 24 KB a CTA
+// would wait for); L lanes take one entry of A at a time, 32 / L entries a warp
+// and step and two products of each a lane, so that B rows fill the warp without
+// an owner search and an entry's dA is one sum over L lanes.  Two FP64
+// instructions a product: the fused multiply-add into dA and the multiply whose
+// sum into dB the L2 does.  100k rows of 256 products: 380 -> 242 us.
+//
+// L follows the mean number of products an entry (30k rows of 200 entries of 1,
+// 3 and 5 products: 575, 775 and 1025 us with eight lanes whatever the mean, 232,
+// 475 and 690 so); rows of a few entries, which fill no step however few lanes
+// they get, take more, whose reductions into dB are next to each other (300k
+// rows of 3 entries of 3 products 627 -> 484 us).  A single lane gains for
+// entries of one product only (932 -> 863 us) and loses for those of three.
+//
+// Rows of 513 entries and more take four warps a row: 24 KB a CTA for 2048 of
+// them, 12 KB for 1024, which leaves the L1 its room (100k rows of 576 products
+// 851 -> 736 us).
+constexpr int kAdjWarpNnz = 512, kAdjQuadNnz = 1024, kAdjWideNnz = 2048;
+constexpr int kAdjWarps = 4;  // a CTA
 constexpr int kAdjCtaThreads = 256, kAdjCtaPerSm = 5;
 
-__global__ void __launch_bounds__(32 * kAdjWarpRows) k_adjoint_warp(AdjArgs a, int32_t lo, int32_t n) {
-    __shared__ double gs[kAdjWarpRows][kAdjWarpNnz];
-    __shared__ int32_t cs[kAdjWarpRows][kAdjWarpNnz];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t item = (int64_t)blockIdx.x * kAdjWarpRows + w;
-    if (item >= n) return;
-    const int32_t row = a.order[lo + item];
-    const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
-    const int64_t c0 = a.Cp[row], nc64 = a.Cp[row + 1] - c0;
-    if (nc64 > kAdjWarpNnz) {  // not the bins' row
-        if (lane == 0) raise(a.err, DEV_COUNT_MISMATCH);
-        return;
+// Which rows of the CTA bins these kernels take (k_adjoint_split), by the steps
+// that one warp would walk.  A step is about 0.08 us of an SM's time, a CTA's
+// row 1.5 us a batch of its entries and 1.9 ns a product: rows of few steps for
+// their products, whose entries are of like lengths, are worth taking.  100k
+// rows of 289, 400, 576 and 1024 products in 17 to 32 entries: 1605, 1683, 1766
+// and 2031 us by CTAs, 455, 505, 780 and 1137 so.  Longer walks are left to the
+// CTAs, as one row would be the last one running: with 24 steps for a warp 20k
+// rows of one entry of 400 products take 291 us instead of 233; with 24 for four
+// warps and a product in 45 steps, 1209 us instead of 1137 on the last case
+// above.  Power-law graphs stay as they are (R-MAT 2^16 1.10 ms; 1.42 if rows
+// were taken by their products alone).
+constexpr int kAdjWarpSteps = 32, kAdjQuadSteps = 16, kAdjBase = 20, kAdjPer = 30;
+
+// Lanes an entry, for a row of n entries whose row of C holds nc.
+__device__ __forceinline__ int adjoint_lanes(int64_t nc, int32_t n) {
+    if (n <= 4 || nc > 8 * (int64_t)n) return 8;
+    return n <= 8 || nc > 4 * (int64_t)n ? 4 : 2;
+}
+
+template <int WARPS, int L>
+__device__ __forceinline__ void adjoint_row(const AdjArgs &a, int32_t e0, int32_t e1, int64_t c0, int nc, double *gs,
+                                            int32_t *cs) {
+    constexpr int T = 32 * WARPS, PER = 32 / L;
+    const int lane = threadIdx.x & 31, w = WARPS == 1 ? 0 : threadIdx.x >> 5, tid = 32 * w + lane;
+    const double *g = gs;
+    const int32_t *c = cs;
+    for (int i = tid; i < nc; i += T) {
+        cs[i] = __ldg(&a.Ci[c0 + i]);
+        gs[i] = __ldg(&a.G[c0 + i]);
     }
-    const int nc = (int)nc64;
-    const double *g = gs[w];
-    const int32_t *c = cs[w];
-    for (int i = lane; i < nc; i += 32) {
-        cs[w][i] = __ldg(&a.Ci[c0 + i]);
-        gs[w][i] = __ldg(&a.G[c0 + i]);
-    }
-    __syncwarp();
+    if constexpr (WARPS == 1) __syncwarp();
+    else __syncthreads();
     int top = 1;
     while (2 * top < nc) top <<= 1;
-    const int sub = lane & 7, grp = lane >> 3;
-    const unsigned gmask = 0xffu << (lane & 24);
+    const int sub = lane & (L - 1), grp = lane / L;
+    const unsigned gmask = ((1u << L) - 1u) << (lane & (32 - L));
     for (int32_t eb = e0; eb < e1; eb += 32) {
         int32_t bs = 0, len = 0;
         double av = 0.0;
@@ -78,7 +101,7 @@ __global__ void __launch_bounds__(32 * kAdjWarpRows) k_adjoint_warp(AdjArgs a, i
             av = __ldg(&a.A.val[eb + lane]);
         }
         const int ne = min(32, e1 - eb);
-        for (int q = 0; q < ne; q += 4) {
+        for (int q = PER * w; q < ne; q += PER * WARPS) {
             const int32_t s = __shfl_sync(FULL, bs, q + grp), l = __shfl_sync(FULL, len, q + grp);
             const double x = __shfl_sync(FULL, av, q + grp);
             double *keep = nullptr;
@@ -88,14 +111,14 @@ __global__ void __launch_bounds__(32 * kAdjWarpRows) k_adjoint_warp(AdjArgs a, i
                 else raise(a.err, DEV_COUNT_MISMATCH);  // the patterns are not the forward's
             }
             double acc = 0.0;
-            for (int32_t i0 = sub; i0 < l; i0 += 16) {
+            for (int32_t i0 = sub; i0 < l; i0 += 2 * L) {
                 // Two products a lane in flight.
                 int32_t k[2];
                 double b[2];
                 int at[2] = {0, 0};
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    const int32_t i = i0 + 8 * u;
+                    const int32_t i = i0 + L * u;
                     k[u] = i < l ? __ldg(&a.B.idx[s + i]) : -1;
                     b[u] = i < l ? __ldg(&a.B.val[s + i]) : 0.0;
                 }
@@ -113,14 +136,40 @@ __global__ void __launch_bounds__(32 * kAdjWarpRows) k_adjoint_warp(AdjArgs a, i
                     }
                     const double gv = g[at[u]];
                     acc = __fma_rn(gv, b[u], acc);
-                    if (a.dB) atomicAdd(&a.dB[s + i0 + 8 * u], __dmul_rn(x, gv));
-                    else if (keep) keep[i0 + 8 * u] = __dmul_rn(x, gv);
+                    if (a.dB) atomicAdd(&a.dB[s + i0 + L * u], __dmul_rn(x, gv));
+                    else if (keep) keep[i0 + L * u] = __dmul_rn(x, gv);
                 }
             }
 #pragma unroll
-            for (int d = 4; d; d >>= 1) acc += __shfl_xor_sync(gmask, acc, d, 8);
+            for (int d = L / 2; d; d >>= 1) acc += __shfl_xor_sync(gmask, acc, d, L);
             if (sub == 0 && q + grp < ne) a.dA[eb + q + grp] = acc;
         }
+    }
+}
+
+// Rows list[0, n), or as many as *count says.
+template <int WARPS, int NNZ>
+__global__ void __launch_bounds__(32 * kAdjWarps) k_adjoint_rows(AdjArgs a, const int32_t *__restrict__ list, int32_t n,
+                                                                 const uint32_t *__restrict__ count) {
+    constexpr int ROWS = kAdjWarps / WARPS;
+    __shared__ double gs[ROWS][NNZ];
+    __shared__ int32_t cs[ROWS][NNZ];
+    const int r = WARPS == 1 ? threadIdx.x >> 5 : 0;
+    if (count) n = (int32_t)min((int64_t)n, (int64_t)*count);
+    for (int64_t i = (int64_t)blockIdx.x * ROWS + r; i < n; i += (int64_t)gridDim.x * ROWS) {
+        const int32_t row = list[i];
+        const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
+        const int64_t c0 = a.Cp[row], nc = a.Cp[row + 1] - c0;
+        if (nc > NNZ) {  // not the list's row
+            if ((threadIdx.x & (32 * WARPS - 1)) == 0) raise(a.err, DEV_COUNT_MISMATCH);
+            continue;
+        }
+        const int lanes = adjoint_lanes(nc, e1 - e0);
+        if (lanes == 2) adjoint_row<WARPS, 2>(a, e0, e1, c0, (int)nc, gs[r], cs[r]);
+        else if (lanes == 4) adjoint_row<WARPS, 4>(a, e0, e1, c0, (int)nc, gs[r], cs[r]);
+        else adjoint_row<WARPS, 8>(a, e0, e1, c0, (int)nc, gs[r], cs[r]);
+        if constexpr (WARPS == 1) __syncwarp();
+        else __syncthreads();
     }
 }
 
@@ -151,7 +200,7 @@ __device__ __forceinline__ int32_t first_entry_at(const int32_t *pre, int nb, in
 // (a fixed order either way).
 //
 // Rows of at least 2 a.partP products are cut into items (built by
-// k_adjoint_items, and taken first): item p of k takes the entries of every
+// k_adjoint_split, and taken first): item p of k takes the entries of every
 // staged batch whose first products lie in the p-th of k equal shares of it,
 // so an entry's sum stays within a CTA.
 template <int THREADS>
@@ -170,18 +219,16 @@ __global__ void __launch_bounds__(THREADS, kAdjCtaPerSm) k_adjoint_cta(AdjArgs a
     uint32_t *bits = reinterpret_cast<uint32_t *>(src + THREADS);
     int32_t *wpre = reinterpret_cast<int32_t *>(bits + maxWords);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int32_t parts = a.items ? (int32_t)min((int64_t)*(volatile uint32_t *)&a.ctr[1], a.itemCap) : 0;
+    const int32_t parts = a.items ? (int32_t)min((int64_t)a.ctr[ADJ_PARTS], a.itemCap) : 0;
+    if (a.items) n = (int32_t)a.ctr[ADJ_CTA];
     for (;;) {
         if (tid == 0) next = (int32_t)atomicAdd(a.ctr, 1u);
         __syncthreads();
         const int32_t item = next;
         if (item >= parts + n) break;
-        const AdjItem it = item < parts ? a.items[item] : AdjItem{a.order[lo + n - 1 - (item - parts)], 0, 1};
+        const AdjItem it = item < parts ? a.items[item]
+                                        : AdjItem{a.items ? a.rows[ADJ_CTA][item - parts] : a.order[lo + n - 1 - item], 0, 1};
         const int32_t row = it.row;
-        if (item >= parts && a.items && a.rowP[row] >= 2 * a.partP) {  // in parts
-            __syncthreads();  // every thread has read `next` before it changes
-            continue;
-        }
         const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
         const int64_t c0 = a.Cp[row], c1 = a.Cp[row + 1];
         const int32_t w0 = c1 > c0 ? a.Ci[c0] >> 5 : 0;
@@ -318,15 +365,63 @@ __global__ void __launch_bounds__(THREADS, kAdjCtaPerSm) k_adjoint_cta(AdjArgs a
     }
 }
 
-// The parts of the rows order[lo, lo + n) that are cut.
-__global__ void __launch_bounds__(256) k_adjoint_items(AdjArgs a, int32_t lo, int32_t n) {
-    const int32_t i = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (i >= n) return;
-    const int32_t row = a.order[lo + i];
-    const int64_t P = a.rowP[row];
-    if (P < 2 * a.partP) return;
+// Tells the rows order[lo, lo + n) apart, the last ones first, a warp a row:
+// the parts of those that are cut, and which of the others a CTA, four warps or a
+// warp take.
+__global__ void __launch_bounds__(256) k_adjoint_split(AdjArgs a, int32_t lo, int32_t n) {
+    __shared__ int kinds[8];
+    __shared__ uint32_t first[ADJ_COUNTERS];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t i = (int64_t)blockIdx.x * 8 + w;
+    const int32_t row = i < n ? a.order[lo + n - 1 - i] : -1;
+    int kind = 0;
+    int64_t P = 0;
+    if (row >= 0) {
+        P = a.rowP[row];
+        const int64_t nc = a.Cp[row + 1] - a.Cp[row];
+        const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
+        kind = P >= 2 * a.partP ? ADJ_PARTS : ADJ_CTA;
+        if (a.rows[ADJ_WARP] && nc <= kAdjWideNnz && e1 - e0 <= 4096) {
+            // Steps of the row by one warp, and the longest of them.
+            const int L = adjoint_lanes(nc, e1 - e0), per = 32 / L;
+            int steps = 0, longest = 0;
+            for (int32_t e = e0; e < e1; e += 32) {
+                int32_t len = 0;
+                if (e + lane < e1) {
+                    const int32_t k = __ldg(&a.A.idx[e + lane]);
+                    len = __ldg(&a.B.ptr[k + 1]) - __ldg(&a.B.ptr[k]);
+                }
+                for (int d = 1; d < per; d <<= 1) len = max(len, __shfl_xor_sync(FULL, len, d));
+                const int x = (len + 2 * L - 1) / (2 * L);
+                if (lane % per == 0) steps += x;
+                longest = max(longest, x);
+            }
+            steps = __reduce_add_sync(FULL, steps);
+            longest = __reduce_max_sync(FULL, longest);
+            const int batches = (e1 - e0 + kAdjCtaThreads - 1) / kAdjCtaThreads;
+            if (steps <= kAdjBase * batches + P / kAdjPer) {
+                if (nc <= kAdjWarpNnz && steps <= kAdjWarpSteps) kind = ADJ_WARP;
+                else if (max(steps / kAdjWarps, longest) <= kAdjQuadSteps) kind = nc <= kAdjQuadNnz ? ADJ_QUAD : ADJ_WIDE;
+            }
+        }
+    }
+    if (lane == 0) kinds[w] = kind;
+    __syncthreads();
+    if (threadIdx.x < ADJ_COUNTERS) {
+        uint32_t k = 0;
+        for (int r = 0; r < 8; ++r) k += kinds[r] == (int)threadIdx.x;
+        if (threadIdx.x >= ADJ_CTA && k) first[threadIdx.x] = atomicAdd(&a.ctr[threadIdx.x], k);
+    }
+    __syncthreads();
+    if (lane != 0 || kind == 0) return;
+    if (kind != ADJ_PARTS) {
+        uint32_t at = first[kind];
+        for (int r = 0; r < w; ++r) at += kinds[r] == kind;
+        a.rows[kind][at] = row;
+        return;
+    }
     const int k = (int)min((int64_t)kAdjMaxParts, P / a.partP);
-    const uint32_t at = atomicAdd(&a.ctr[1], (uint32_t)k);
+    const uint32_t at = atomicAdd(&a.ctr[ADJ_PARTS], (uint32_t)k);
     if ((int64_t)at + k > a.itemCap) return raise(a.err, DEV_COUNT_MISMATCH);  // the products are not the forward's
     for (int p = 0; p < k; ++p) a.items[at + p] = AdjItem{row, (int16_t)p, (int16_t)k};
 }
@@ -508,8 +603,29 @@ static size_t smem_adjoint_cta(int words) {
 
 void launch_adjoint_warp(const AdjArgs &a, int32_t lo, int32_t hi, cudaStream_t s, int *launches) {
     if (hi <= lo) return;
-    k_adjoint_warp<<<(unsigned)ceil_div(hi - lo, kAdjWarpRows), 32 * kAdjWarpRows, 0, s>>>(a, lo, hi - lo);
+    k_adjoint_rows<1, kAdjWarpNnz><<<(unsigned)ceil_div(hi - lo, kAdjWarps), 32 * kAdjWarps, 0, s>>>(a, a.order + lo,
+                                                                                                   hi - lo, nullptr);
     ++*launches;
+}
+
+void launch_adjoint_rows(const AdjArgs &a, int kind, int32_t n, int num_sms, cudaStream_t s, int *launches) {
+    // At most 64 CTAs an SM: a short list of many candidates costs little.
+    const int rows = kind == ADJ_WARP ? kAdjWarps : 1;
+    const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(n, rows), (int64_t)std::max(num_sms, 1) * 64);
+    const auto fn = kind == ADJ_WARP   ? k_adjoint_rows<1, kAdjWarpNnz>
+                    : kind == ADJ_QUAD ? k_adjoint_rows<kAdjWarps, kAdjQuadNnz>
+                                       : k_adjoint_rows<kAdjWarps, kAdjWideNnz>;
+    fn<<<grid, 32 * kAdjWarps, 0, s>>>(a, a.rows[kind], n, a.ctr + kind);
+    ++*launches;
+}
+
+void launch_adjoint_split(const AdjArgs &a, int32_t lo, int32_t hi, cudaStream_t s, int *launches) {
+    if (hi <= lo) return;
+    cudaMemsetAsync(a.ctr, 0, ADJ_COUNTERS * sizeof(uint32_t), s);
+    if (a.items) {
+        k_adjoint_split<<<(unsigned)ceil_div(hi - lo, 8), 256, 0, s>>>(a, lo, hi - lo);
+        ++*launches;
+    }
 }
 
 void launch_adjoint_cta(const AdjArgs &a, int32_t lo, int32_t hi, int num_sms, cudaStream_t s, int *launches) {
@@ -520,11 +636,6 @@ void launch_adjoint_cta(const AdjArgs &a, int32_t lo, int32_t hi, int num_sms, c
     const int per_sm = std::max(1, std::min(kAdjCtaPerSm, (int)((227 * 1024) / (smem + 1024))));
     const int64_t most = (int64_t)(hi - lo) * (a.items ? kAdjMaxParts : 1);
     const int grid = (int)std::min<int64_t>(most, (int64_t)std::max(num_sms, 1) * per_sm);
-    cudaMemsetAsync(a.ctr, 0, 2 * sizeof(uint32_t), s);
-    if (a.items) {
-        k_adjoint_items<<<(unsigned)ceil_div(hi - lo, 256), 256, 0, s>>>(a, lo, hi - lo);
-        ++*launches;
-    }
     k_adjoint_cta<kAdjCtaThreads><<<(unsigned)grid, kAdjCtaThreads, smem, s>>>(a, lo, hi - lo, words);
     ++*launches;
 }
