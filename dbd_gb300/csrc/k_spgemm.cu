@@ -1762,7 +1762,16 @@ __device__ __forceinline__ uint32_t run_bits(int w, int r0, int r1) {
 // from the runs' ends, so B's indices are not read.  A band's rows take 2.05
 // steps an entry instead of 3: 970k rows of 4225 products 10.95 -> 7.86 ms
 // (6.5 ms at the pipe's rate).
-template <int ROWS>
+//
+// Few rows leave most of the pipe idle and are bound by a warp's chain of steps:
+// up to kDensewFew rows an SM take the products six steps at a time, which,
+// where they lie in one entry, share no column and need no order among them
+// (512 rows of 512 entries of 512 products 1560 -> 1105 us, 1245 entry by entry;
+// 2000 rows of 256 of 256 458 -> 398).  With 5000 such rows that is slower (898
+// us instead of 767), the pipe being busy and the registers fewer.
+constexpr int kDensewFew = 16;
+
+template <int ROWS, int U>
 __device__ __forceinline__ void num_densew_rows(const NumArgs &a, int32_t lo, int32_t count, int64_t vb) {
     constexpr int kCols = kDenseWarpWords * 32;
     __shared__ double vs[ROWS][kCols];
@@ -1836,10 +1845,10 @@ __device__ __forceinline__ void num_densew_rows(const NumArgs &a, int32_t lo, in
                 int32_t p0 = __shfl_sync(FULL, posAt, 0), p1 = __shfl_sync(FULL, posAt, 1);
                 int32_t c0 = __shfl_sync(FULL, relAt, 0), c1 = __shfl_sync(FULL, relAt, 1);
                 double a0 = __shfl_sync(FULL, avl, 0), a1 = __shfl_sync(FULL, avl, 1);
-                constexpr int U = 3;  // steps whose loads are in flight together
-                for (int32_t t0 = 0; t0 < total; t0 += 32 * U) {
+                for (int32_t t0 = 0; t0 < total; t0 += 32 * U) {  // U steps' loads in flight together
                     int32_t rel[U];
                     double av[U], bv[U];
+                    const int q0 = q;
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
                         const int32_t s = t0 + 32 * u, t = s + lane;
@@ -1857,6 +1866,16 @@ __device__ __forceinline__ void num_densew_rows(const NumArgs &a, int32_t lo, in
                         rel[u] = t < total ? (next ? c1 : c0) + t : -1;
                         av[u] = next ? a1 : a0;
                         bv[u] = t < total ? __ldg(&bval[(next ? p1 : p0) + t]) : 0.0;
+                    }
+                    if (U > 3 && q == q0 && t0 + 32 * U <= end) {
+                        // All in one entry: no column twice.
+                        double x[U];
+#pragma unroll
+                        for (int u = 0; u < U; ++u) x[u] = vals[rel[u]];
+#pragma unroll
+                        for (int u = 0; u < U; ++u) vals[rel[u]] = __fma_rn(av[u], bv[u], x[u]);
+                        __syncwarp();
+                        continue;
                     }
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
@@ -1909,9 +1928,9 @@ __device__ __forceinline__ void num_densew_rows(const NumArgs &a, int32_t lo, in
     if (lane == 0 && p != expect) raise(a.err, DEV_COUNT_MISMATCH);
 }
 
-template <int ROWS>
+template <int ROWS, int U>
 __global__ void __launch_bounds__(32 * ROWS) k_num_densew(NumArgs a, int32_t lo, int32_t count) {
-    num_densew_rows<ROWS>(a, lo, count, blockIdx.x);
+    num_densew_rows<ROWS, U>(a, lo, count, blockIdx.x);
 }
 
 // The same rows launched device-driven: the bin's rows from the bin table
@@ -1920,7 +1939,7 @@ template <int ROWS>
 __global__ void __launch_bounds__(32 * ROWS) k_num_densew_dd(NumArgs a, int bin) {
     const int32_t lo = a.binStart[bin], count = a.binStart[bin + 1] - lo;
     for (int64_t vb = blockIdx.x; vb * ROWS < count; vb += gridDim.x) {
-        num_densew_rows<ROWS>(a, lo, count, vb);
+        num_densew_rows<ROWS, 3>(a, lo, count, vb);
         __syncthreads();
     }
 }
@@ -2836,7 +2855,8 @@ cudaError_t preload_spgemm_kernels() {
         (const void *)k_sym_wide<kWideThreads, true>,
         (const void *)k_num_tiny,
         (const void *)k_num_hash_warp<kNumWarpRows, kNumWarpTable>,
-        (const void *)k_num_densew<kDensewRows>,
+        (const void *)k_num_densew<kDensewRows, 3>,
+        (const void *)k_num_densew<kDensewRows, 6>,
         (const void *)k_num_rankm<kRankmRows>,
         (const void *)k_num_rankw<kRankwRows>,
         (const void *)k_num_rank<kRankSThreads, uint16_t>,
@@ -3089,7 +3109,10 @@ void launch_numeric_bin(const NumArgs &a, int bin, int32_t lo, int32_t hi, cudaS
                 <<<(unsigned)ceil_div(n, kNumWarpRows), 32 * kNumWarpRows, kSmemNumWarp, s>>>(a, lo, n);
             break;
         case NB_DENSEW:
-            k_num_densew<kDensewRows><<<(unsigned)ceil_div(n, kDensewRows), 32 * kDensewRows, 0, s>>>(a, lo, n);
+            if (n <= kDensewFew * std::max(a.numSms, 1))
+                k_num_densew<kDensewRows, 6><<<(unsigned)ceil_div(n, kDensewRows), 32 * kDensewRows, 0, s>>>(a, lo, n);
+            else
+                k_num_densew<kDensewRows, 3><<<(unsigned)ceil_div(n, kDensewRows), 32 * kDensewRows, 0, s>>>(a, lo, n);
             break;
         case NB_RANKM: {
             // Persistent: three CTAs of kRankmRows warps per SM.
