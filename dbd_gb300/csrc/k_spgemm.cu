@@ -17,7 +17,7 @@
 //                               each is one run); warp bitmap ranks
 //   short rows  (<= 256 nnz)    one warp per row: symbolic by a shared hash
 //                               table; numeric by expand-sort-compress in
-//                               registers for rows of at most 256 products, else by the
+//                               registers for rows of at most 512 products, else by the
 //                               table, compaction and a bitonic sort
 //   CTA rows                    the row's A entries staged in shared memory,
 //                               warps over consecutive products with several
@@ -95,19 +95,22 @@ constexpr int kWideLoads = 4;
 // Steps of B loads a warp-hash row keeps in flight.
 constexpr int kHashWarpLoads = 2;
 // Warp-hash rows of at most this many products are sorted instead of hashed.
-// A sorted row rounds every product before it adds, the table's fused
-// multiply-adds do not: rows of 257 to 512 products have columns of several
-// products by necessity (they hold at most 256 entries), and sorted their
-// error was 0.62 units of the last place against 0.54 (rms, against exact sums).
-constexpr int kEscMax = 256;
-constexpr int kEscShift = 8;  // bits of a product's number in their keys
+// Up to kEscMax every product is rounded before it is added; past it, to
+// kFusedMax, the sums are fused multiply-adds, as the table's are: such rows
+// have columns of several products by necessity (they hold at most 256 entries),
+// whose rms error would be 0.62 units of the last place instead of 0.54
+// (against exact sums).
+constexpr int kEscMax = 256, kFusedMax = 512;
+constexpr int kEscShift = 8, kFusedShift = 9;  // bits of a product's number in their keys
 // Mean B row length from which their products are listed by groups of lanes.
 constexpr int kEscGroupLen = 6;
 
-// Position in B of product t (all lanes call; result valid when t < total).
-__device__ __forceinline__ int32_t chunk_pos(const Chunk &c, int32_t t, double *a_out) {
+// Position in B of product t and the lane its entry is on (all lanes call;
+// results valid when t < total).
+__device__ __forceinline__ int32_t chunk_pos(const Chunk &c, int32_t t, double *a_out, int32_t *owner = nullptr) {
     const int o = chunk_owner(c, t);
     if (a_out) *a_out = __shfl_sync(FULL, c.a, o);
+    if (owner) *owner = o;
     return t + __shfl_sync(FULL, c.bs - (c.incl - c.len), o);
 }
 
@@ -1141,8 +1144,9 @@ __device__ __forceinline__ void table_write_sorted(const NumArgs &a, int32_t row
 }
 
 // Shared bytes per warp of the warp hash kernel: keys and values (which rows
-// sorted in registers use for their products).  6 KB per warp.
-constexpr size_t warp_hash_bytes(int table) { return 12 * (size_t)table; }
+// sorted in registers use for their products) and those rows' entries.  6.5 KB
+// per warp.
+constexpr size_t warp_hash_bytes(int table) { return 13 * (size_t)table; }
 
 // Sorts 32 R keys ascending over a warp's registers: key[r] of lane l is the
 // (R l + r)-th afterwards.  Each lane sorts its own R (merge_exchange); then
@@ -1210,13 +1214,17 @@ __device__ __forceinline__ int rotated(int p) { return (p & ~31) | ((p + (p >> 5
 // consecutive entries, the form before, was bound by the L1: 60M bank
 // conflicts and 20M store requests for 100k rows of 256 products (91% of L1
 // throughput busy): 455 -> 190 us, 550k rows of about 144 products 1611 ->
-// 1007 us (the table's rows of 257 and more among them).  What bounds it now is instruction issue (65% busy, the ALU 68%) and
+// 954 us.  What bounds it now is instruction issue (65% busy, the ALU 68%) and
 // latency, at 32 warps an SM (64 registers, 6 KB a warp; at 92 registers and
 // 20 warps 272 us).  kbuf and pv hold a product each; columns lie in
 // [rlo, rlo + 2^(bits of K - kEscShift)).
-template <class K>
+//
+// SHIFT is the bits of a product's number in its key.  With ent (rows past
+// kEscMax products, of at most 256 entries) pv takes the B values and ent the
+// products' entries, for esc_fused.
+template <int SHIFT, class K>
 __device__ __forceinline__ void esc_list(const NumArgs &a, int32_t e0, int32_t e1, int n, int32_t rlo, K *kbuf,
-                                         double *pv) {
+                                         double *pv, uint8_t *ent) {
     const int lane = threadIdx.x & 31;
     int32_t tb = 0;  // products of the earlier chunks
     if (n >= kEscGroupLen * (e1 - e0)) {
@@ -1254,8 +1262,9 @@ __device__ __forceinline__ void esc_list(const NumArgs &a, int32_t e0, int32_t e
                         const int h = u >> 1, i = i0 + 8 * (u & 1);
                         if (i < len[h]) {
                             const int x = t[h] + i;
-                            kbuf[x] = (K)(uint32_t)(col[u] - rlo) << kEscShift | (K)x;
-                            pv[x] = __dmul_rn(av[h], bv[u]);
+                            kbuf[x] = (K)(uint32_t)(col[u] - rlo) << SHIFT | (K)x;
+                            pv[x] = ent ? bv[u] : __dmul_rn(av[h], bv[u]);
+                            if (ent) ent[x] = (uint8_t)(e - e0 + q + 4 * h + grp);
                         }
                     }
                 }
@@ -1267,15 +1276,16 @@ __device__ __forceinline__ void esc_list(const NumArgs &a, int32_t e0, int32_t e
         for (int32_t e = e0; e < e1; e += 32) {
             const Chunk c = load_chunk(a.A, a.B, e, e1, lane);
             for (int32_t t0 = 0; t0 < c.total; t0 += 32 * U) {
-                int32_t j[U];
+                int32_t j[U], own[U];
                 double av[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     j[u] = -1;
                     av[u] = 0.0;
+                    own[u] = 0;
                     const int32_t t = t0 + 32 * u + lane;
                     if (t0 + 32 * u < c.total) {
-                        const int32_t jj = chunk_pos(c, t, &av[u]);
+                        const int32_t jj = chunk_pos(c, t, &av[u], &own[u]);
                         if (t < c.total && tb + t < n) j[u] = jj;
                     }
                 }
@@ -1290,8 +1300,9 @@ __device__ __forceinline__ void esc_list(const NumArgs &a, int32_t e0, int32_t e
                 for (int u = 0; u < U; ++u) {
                     if (j[u] >= 0) {
                         const int t = tb + t0 + 32 * u + lane;
-                        kbuf[t] = (K)(uint32_t)(col[u] - rlo) << kEscShift | (K)t;
-                        pv[t] = __dmul_rn(av[u], bv[u]);
+                        kbuf[t] = (K)(uint32_t)(col[u] - rlo) << SHIFT | (K)t;
+                        pv[t] = ent ? bv[u] : __dmul_rn(av[u], bv[u]);
+                        if (ent) ent[t] = (uint8_t)(e - e0 + own[u]);
                     }
                 }
             }
@@ -1381,6 +1392,77 @@ __device__ __forceinline__ void esc_sort(const NumArgs &a, int32_t row, int n, i
     }
 }
 
+// The same for rows of kEscMax to kFusedMax products, whose columns have several
+// products by necessity (they hold at most kNumWarpMax entries): every sum is one
+// chain of fused multiply-adds, as in the table.  A lane sums the runs that
+// start in it; where its keys begin inside a run it goes on from the sum of the
+// lane before, once that one has it.  20k rows of about 400 products 323 us by
+// the table, 121 so (143 with rounded products).
+__device__ __forceinline__ void esc_fused(const NumArgs &a, int32_t row, int32_t e0, int n, int32_t rlo, uint32_t *kbuf,
+                                          double *pv, const uint8_t *ent) {
+    constexpr int R = kFusedMax / 32, SHIFT = kFusedShift;
+    const int lane = threadIdx.x & 31;
+    uint32_t key[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) key[r] = 32 * r + lane < n ? kbuf[32 * r + lane] : ~0u;
+    warp_sort<R>(key);
+    const int have = min(max(n - R * lane, 0), R);  // this lane's keys
+    uint32_t heads = 0;
+    const uint32_t before = __shfl_up_sync(FULL, key[R - 1], 1);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t prev = r > 0 ? key[r > 0 ? r - 1 : 0] : before;
+        if (r < have && ((r == 0 && lane == 0) || (key[r] >> SHIFT) != (prev >> SHIFT))) heads |= 1u << r;
+    }
+    const int first = heads ? __ffs(heads) - 1 : have;  // keys before it continue the run of the lane before
+    const int begins = __shfl_down_sync(FULL, first > 0 ? 1 : 0, 1);
+    const bool goesOn = lane < 31 && begins;  // the last run does, in the next lane
+    const int mine = __popc(heads);
+    int incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(FULL, incl, d);
+        if (lane >= d) incl += y;
+    }
+    const int64_t obase = a.Cp[row] - a.outBase;
+    const int32_t expect = (int32_t)(a.Cp[row + 1] - a.Cp[row]);
+    if (lane == 31 && incl != expect) raise(a.err, DEV_COUNT_MISMATCH);
+    const int32_t shift = col_shift(a, row) - rlo;
+    auto fused = [&](uint32_t k, double acc) {
+        const int x = (int)(k & ((1u << SHIFT) - 1u));
+        return __fma_rn(__ldg(&a.A.val[e0 + ent[x]]), pv[x], acc);
+    };
+    // Entries go out lane by lane: such rows are few (a batch's tail), and the
+    // registers and shared memory for their order would be every row's.
+    int p = incl - mine;
+    double acc = 0.0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (r < first || r >= have) continue;
+        const bool head = (heads >> r) & 1u;
+        acc = fused(key[r], head ? 0.0 : acc);
+        if (head && p < expect) a.Ci[obase + p] = (int32_t)(key[r] >> SHIFT) - shift;
+        p += head;
+        const bool ends = r + 1 == have ? !goesOn : ((heads >> (r + 1)) & 1u) != 0u;
+        if (ends && p <= expect) a.Cv[obase + p - 1] = acc;
+    }
+    bool wait = first > 0;
+    bool known = !wait || heads != 0u;  // the sum so far of this lane's last run
+    while (__any_sync(FULL, wait)) {
+        const double from = __shfl_up_sync(FULL, acc, 1);
+        const bool ready = __shfl_up_sync(FULL, known ? 1 : 0, 1);
+        if (!wait || !ready) continue;
+        double lead = from;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (r < first) lead = fused(key[r], lead);
+        if (heads == 0u) acc = lead;
+        if ((heads != 0u || !goesOn) && incl - mine <= expect) a.Cv[obase + incl - mine - 1] = lead;
+        known = true;
+        wait = false;
+    }
+}
+
 template <int ROWS, int TABLE>
 __device__ __forceinline__ void num_hash_warp_rows(const NumArgs &a, int32_t lo, int32_t count, int64_t vb) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1395,25 +1477,32 @@ __device__ __forceinline__ void num_hash_warp_rows(const NumArgs &a, int32_t lo,
     const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
     // Expand-sort-compress where the products fit the registers and the
     // columns the keys; the table takes the others.
-    static_assert(TABLE >= 2 * kEscMax && (1 << kEscShift) >= kEscMax, "the arrays and keys hold the products");
+    static_assert(TABLE >= 2 * kEscMax && TABLE >= kFusedMax && (1 << kEscShift) >= kEscMax &&
+                      (1 << kFusedShift) >= kFusedMax, "the arrays and keys hold the products");
     const int64_t P = a.rowP[row];
+    const int32_t rlo = a.rowLo[row];
+    const int64_t span = (int64_t)a.rowHi[row] - rlo + 1;
+    uint32_t *kb = reinterpret_cast<uint32_t *>(keys);
     if (P <= kEscMax) {
-        const int32_t rlo = a.rowLo[row];
-        const int64_t span = (int64_t)a.rowHi[row] - rlo + 1;
-        uint32_t *kb = reinterpret_cast<uint32_t *>(keys);
         // Two sizes and one listing: warps of an SM that run different code
-        // miss the instruction cache.  550k rows of 60 to 280 products: 1.0 ms;
+        // miss the instruction cache.  550k rows of 60 to 280 products: 0.95 ms;
         // with six sizes of 2 to 16 keys a lane, each with its own listing,
         // 2.05 ms.
         if (span < ((int64_t)1 << (32 - kEscShift))) {
-            esc_list<uint32_t>(a, e0, e1, (int)P, rlo, kb, vals);
+            esc_list<kEscShift, uint32_t>(a, e0, e1, (int)P, rlo, kb, vals, nullptr);
             if (P <= 192) esc_sort<6, uint32_t>(a, row, (int)P, rlo, kb, vals);
             else esc_sort<8, uint32_t>(a, row, (int)P, rlo, kb, vals);
         } else {
             unsigned long long *kb64 = reinterpret_cast<unsigned long long *>(keys);
-            esc_list<unsigned long long>(a, e0, e1, (int)P, rlo, kb64, vals);
+            esc_list<kEscShift, unsigned long long>(a, e0, e1, (int)P, rlo, kb64, vals, nullptr);
             esc_sort<8, unsigned long long>(a, row, (int)P, rlo, kb64, vals);
         }
+        return;
+    }
+    if (P <= kFusedMax && e1 - e0 <= 256 && span < ((int64_t)1 << (32 - kFusedShift))) {
+        uint8_t *ent = reinterpret_cast<uint8_t *>(vals + TABLE);
+        esc_list<kFusedShift, uint32_t>(a, e0, e1, (int)P, rlo, kb, vals, ent);
+        esc_fused(a, row, e0, (int)P, rlo, kb, vals, ent);
         return;
     }
     for (int i = lane; i < TABLE; i += 32) {

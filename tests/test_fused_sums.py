@@ -41,3 +41,47 @@ def test_two_products_a_column(columns, n, bin_of):
         for j in range(columns):
             want = sum(a[2 * r + h] * b[(2 * r + h) * columns + j] for h in (0, 1))  # multiples of 2^-104
             assert abs((got[r * columns + j] << 53) - want) <= 3 << 51
+
+
+@pytest.mark.parametrize("products", [257, 300, 480, 511, 512])
+@pytest.mark.parametrize("distinct", [2, 3, 9, 70, 240])
+@pytest.mark.parametrize("per", [1.2, 3, 12])
+def test_warp_rows_are_chains_in_order(products, distinct, per):
+    """Warp rows of 257 to 512 products of at most 256 entries: every sum is the fused multiply-adds of its
+    products in A's entry order, bit for bit; with more entries a row takes the table, which adds in any order."""
+    from fractions import Fraction
+    rng = np.random.default_rng(products + distinct)
+    n = 70000
+    pool = np.unique(np.r_[0, rng.choice(n - 2, distinct - 2, replace=False) + 1, n - 1])
+    lens = []
+    while sum(lens) < products:
+        top = min(pool.size, products - sum(lens))
+        lens.append(int(min(top, 1 + rng.poisson(per - 1))))
+    cols = [np.sort(rng.choice(pool, l, replace=False)) for l in lens]
+    cols[0][:1], cols[-1][-1:] = pool[0], pool[-1]  # the window's ends
+    cols = [np.unique(c) for c in cols]
+    idx = np.concatenate(cols).astype(np.int32)
+    if not 256 < idx.size <= 512:
+        pytest.skip("another class of rows")
+    B = dbd.CSR(len(cols), n, np.r_[0, np.cumsum([c.size for c in cols])].astype(np.int32), idx,
+                rng.standard_normal(idx.size))
+    A = dbd.CSR(2, len(cols), (np.arange(3) * len(cols)).astype(np.int32), np.tile(np.arange(len(cols)), 2).astype(np.int32),
+                rng.standard_normal(2 * len(cols)))
+    with dbd.Context(cpu_gib=1, gpu_gib=4) as ctx:
+        res = ctx.spgemm(A, B)
+    assert res.stats["rows_per_bin"][HWARP] == 2
+    for r in range(2):
+        want, size = {}, {}
+        for e in range(len(cols)):
+            x = A.val[r * len(cols) + e]
+            for f in range(B.row_ptr[e], B.row_ptr[e + 1]):
+                c = int(B.col_idx[f])
+                want[c] = float(Fraction(x) * Fraction(B.val[f]) + Fraction(want.get(c, 0.0)))
+                size[c] = size.get(c, 0.0) + abs(x * B.val[f])
+        s, t = res.C.row_ptr[r], res.C.row_ptr[r + 1]
+        assert res.C.col_idx[s:t].tolist() == sorted(want)
+        exact = np.array([want[c] for c in sorted(want)])
+        if len(cols) <= 256:
+            np.testing.assert_array_equal(res.C.val[s:t], exact)
+        else:
+            assert np.all(np.abs(res.C.val[s:t] - exact) <= 1e-12 * np.array([size[c] for c in sorted(want)]))
