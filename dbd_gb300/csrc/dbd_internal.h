@@ -60,14 +60,15 @@ constexpr int kMaxSlabs = 64;                // rows spanning up to 2^22 columns
 constexpr int64_t kHeavyP = 65536;
 constexpr int kPieceNnz = 65536;
 constexpr int kPieceSlabs = 16;
-// The symbolic pass takes wide rows of at least sym_first_products() products
-// in a launch of their own beside the others, those of twice as many cut into
-// one item per slab: a CTA walks about 2 products a nanosecond, so a row of
-// 3.75M of the 381M products in 10,240 rows of R-MAT 2^21 set the pass's time
-// alone.  The line is half a CTA's share of all products (a shorter row can
-// hardly be the last one running), and no less than kSymFirstP, under which an
-// item is not worth its staging.
-constexpr int64_t kSymFirstP = 1 << 18;
+// The symbolic pass cuts wide rows of at least sym_cut_products() products into
+// one item per slab, in a launch of their own beside the others: a CTA walks
+// about 2 products a nanosecond, so a row of 3.75M of the 381M products in
+// 10,240 rows of R-MAT 2^21 set the pass's time alone.  The line is a CTA's share
+// of all products (a shorter row can hardly be the last one running), and no
+// less than kSymCutP.  A row of 520k, 1.04M and 2.07M products alone: 130, 236
+// and 446 us whole, 49, 73 and 120 cut.  (In the other launch without being cut,
+// rows of half as many and more took 10 us longer, 40 of them 30.)
+constexpr int64_t kSymCutP = 1 << 19;
 
 __host__ __device__ __forceinline__ int span_words(int32_t lo, int32_t hi) {
     return hi >= lo ? (hi >> 5) - (lo >> 5) + 1 : 0;
@@ -213,20 +214,18 @@ void launch_num_lists(int64_t m, const Binning &b, const RowInfo &ri, const int3
 void launch_row_scan(int64_t m, const int32_t *cnt, int64_t *part, int64_t *Cp, cudaStream_t s);
 
 // ---- launchers (k_spgemm.cu) ----
-// One work item of the largest symbolic wide rows: the idx-th row of the
-// bin, or its column slabs [s0, s1) (s0 < 0: the whole row).
+// One work item of the largest symbolic wide rows: column slabs [s0, s1) of the
+// idx-th row of the bin.
 struct SymItem {
     int32_t idx;
     int16_t s0, s1;
 };
-inline int64_t sym_first_products(int64_t products, int num_sms) {
-    const int64_t share = products / (4 * (int64_t)(num_sms > 0 ? num_sms : 1));  // two CTAs an SM
-    return share > kSymFirstP ? share : kSymFirstP;
+inline int64_t sym_cut_products(int64_t products, int num_sms) {
+    const int64_t share = products / (2 * (int64_t)(num_sms > 0 ? num_sms : 1));  // two CTAs an SM
+    return share > kSymCutP ? share : kSymCutP;
 }
 // Most items that rows of `products` products in all can make.
-inline int64_t sym_item_cap(int64_t products, int64_t firstP) {
-    return products / firstP + kMaxSlabs * (products / (2 * firstP));
-}
+inline int64_t sym_item_cap(int64_t products, int64_t cutP) { return kMaxSlabs * (products / cutP); }
 
 struct SymArgs {
     CsrDev A, B;
@@ -258,7 +257,7 @@ struct SymArgs {
     // Items of the wide rows launched on their own (null: none);
     // their count is ctr[CTR_SYM_ITEMS], room for sym_item_cap().
     SymItem *items = nullptr;
-    int64_t firstP = 0;  // products from which a row is an item
+    int64_t cutP = 0;  // products from which a row is cut
 };
 // Launches the items of the wide rows list[begin, begin + n) (a.items; the
 // bin's own launch then leaves their rows out).

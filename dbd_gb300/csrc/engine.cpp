@@ -658,11 +658,11 @@ int symbolic(dbd_ctx *c) {
     }
     // The largest wide rows go beside the others, cut by column.
     const int32_t nwideRows = c->symStart_h[SB_WIDE + 1] - c->symStart_h[SB_WIDE];
-    const int64_t firstP = sym_first_products(c->products, c->num_sms);
-    if (nwideRows > 0 && c->maxRowP >= firstP) {
-        CK(c, c->symItems.ensure(sizeof(SymItem) * (size_t)sym_item_cap(c->products, firstP)));
+    const int64_t cutP = sym_cut_products(c->products, c->num_sms);
+    if (nwideRows > 0 && c->maxRowP >= cutP && opB_sorted(c)) {
+        CK(c, c->symItems.ensure(sizeof(SymItem) * (size_t)sym_item_cap(c->products, cutP)));
         sa.items = c->symItems.as<SymItem>();
-        sa.firstP = firstP;
+        sa.cutP = cutP;
     }
     // Bins run concurrently, one stream each (heaviest first).
     static const int sorder[] = {SB_WIDE, SB_HCTA, SB_HWARP, SB_BITW, SB_TINY};

@@ -167,7 +167,10 @@ __global__ void k_row_minmax(CsrDev B, int2 *__restrict__ range, const int *__re
 // starts at kLongRowShort.  2.1M five-entry rows 105 -> 36 us.  Its longest
 // warps are those of a power-law graph's hubs, so it takes kShortRows rows
 // and more: means of 2 to 5 entries over 2^20 rows 78 -> 56 us, 2^19 52 ->
-// 39, but 2^18 32 -> 37, 2^16 14 -> 21, 2^12 10 -> 14.
+// 39, but 2^18 32 -> 37, 2^16 14 -> 21, 2^12 10 -> 14.  The mean's line is on the
+// safe side: on rows of Poisson lengths lanes gain up to a mean of 10 (the whole
+// work estimate of 2^21 rows, mean 5 217 -> 177 us, 8 278 -> 239, 12 335 -> 331),
+// on R-MAT 2^20 up to 12 (6 165 -> 153, 8 176 -> 169, 12 210 -> 202).
 constexpr int kLongRow = 256, kLongRowShort = 64;
 constexpr int kShortRow = 8;
 constexpr int64_t kShortMean = 6, kShortRows = 1 << 19;

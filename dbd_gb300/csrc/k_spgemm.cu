@@ -102,7 +102,10 @@ constexpr int kHashWarpLoads = 2;
 // (against exact sums).
 constexpr int kEscMax = 256, kFusedMax = 512;
 constexpr int kEscShift = 8, kFusedShift = 9;  // bits of a product's number in their keys
-// Mean B row length from which their products are listed by groups of lanes.
+// Mean B row length from which their products are listed by groups of lanes, at
+// which both ways take the same time: 100k rows of about 200 products, groups
+// against one flat sequence, mean 3 289 and 262 us, 4 246 and 225, 5 221 and 227,
+// 6 218 and 221, 8 195 and 198, 12 158 and 172.
 constexpr int kEscGroupLen = 6;
 
 // Position in B of product t and the lane its entry is on (all lanes call;
@@ -593,23 +596,25 @@ __host__ __device__ __forceinline__ int wide_touch_cap(int winBits) {
     return min(kWideTouchMax, (winBits >> 5) / 4);
 }
 
-// Items of the wide rows list[begin, begin + n): rows of at least a.firstP
-// products, cut into one item per slab of columns from twice as many on (B's
-// rows ascending).  A cut row's count starts at zero
-// here, and its slab counts get their slot.
+// Column slabs that a wide row is cut into, an item each; 0 for a row that is
+// not (fewer than a.cutP products, one slab, or B's rows not ascending).
+__device__ __forceinline__ int sym_cut_slabs(const SymArgs &a, int32_t row) {
+    if (a.rowP[row] < a.cutP || !b_sorted(a)) return 0;
+    const int64_t base = (int64_t)(a.rowLo[row] >> 5) << 5;
+    const int64_t ns = (((int64_t)a.rowHi[row] + 1 - base) + (1 << kSlabShift) - 1) >> kSlabShift;
+    return ns > 1 && ns <= kMaxSlabs ? (int)ns : 0;
+}
+
+// Items of the wide rows list[begin, begin + n) that are cut.  A cut row's count
+// starts at zero here, and its slab counts get their slot.
 __global__ void __launch_bounds__(256) k_sym_items(SymArgs a, int32_t begin, int32_t n) {
     const int32_t i = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= n) return;
     const int32_t row = a.list[begin + i];
-    const int64_t P = a.rowP[row];
-    if (P < a.firstP) return;
-    const int64_t base = (int64_t)(a.rowLo[row] >> 5) << 5;
-    const int ns = (int)((((int64_t)a.rowHi[row] + 1 - base) + (1 << kSlabShift) - 1) >> kSlabShift);
-    const bool cut = P >= 2 * a.firstP && b_sorted(a) && ns > 1 && ns <= kMaxSlabs;
-    const int k = cut ? ns : 1;
+    const int k = sym_cut_slabs(a, row);
+    if (k == 0) return;
     const uint32_t at = atomicAdd(&a.ctr[CTR_SYM_ITEMS], (uint32_t)k);
-    for (int s = 0; s < k; ++s) a.items[at + s] = cut ? SymItem{i, (int16_t)s, (int16_t)(s + 1)} : SymItem{i, -1, -1};
-    if (!cut) return;
+    for (int s = 0; s < k; ++s) a.items[at + s] = SymItem{i, (int16_t)s, (int16_t)(s + 1)};
     a.rowNnz[row] = 0;
     if (a.slabCnt) {
         int32_t sl = (int32_t)atomicAdd(&a.ctr[CTR_HEAVY], 1u);
@@ -624,9 +629,9 @@ __global__ void __launch_bounds__(256) k_sym_items(SymArgs a, int32_t begin, int
 // clears only those (the whole window when more than kWideTouchMax were
 // touched).  The row's size is the sum of newly set bits, so no popcount
 // pass over the window either: a row costs its products, not its span.
-// Rows of at least a.firstP products are items of a launch of their own
-// (ITEMS, built by k_sym_items), the largest cut by column: a piece sets,
-// counts and keeps its slabs' columns and adds its count to the row's.
+// The largest rows, cut by column, are items of a launch of their own (ITEMS,
+// built by k_sym_items): a piece sets, counts and keeps its slabs' columns and
+// adds its count to the row's.
 // 10,240 rows of R-MAT 2^21, two of which hold 3.7M products each: 2.00 ->
 // 1.14 ms (1.84 with 32-bit window arithmetic alone).
 template <int THREADS, bool ITEMS>
@@ -662,11 +667,11 @@ __global__ void __launch_bounds__(THREADS) k_sym_wide(SymArgs a, int32_t begin, 
             item = it.idx;
         }
         const int32_t row = a.list[begin + item];
-        if (!ITEMS && a.items && a.rowP[row] >= a.firstP) {  // an item's
+        if (!ITEMS && a.items && sym_cut_slabs(a, row) > 0) {  // its pieces are items
             __syncthreads();  // every thread has read `next` before it changes
             continue;
         }
-        const bool piece = ITEMS && it.s0 >= 0;
+        constexpr bool piece = ITEMS;
         const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
         // The row's window [lo, hi], in windows of winBits columns from lo's word.
         const int32_t rlo = a.rowLo[row], rhi = a.rowHi[row];
