@@ -39,7 +39,7 @@ __device__ __forceinline__ int64_t find_col(const int32_t *__restrict__ ci, int6
 // instructions a product: the fused multiply-add into dA and the multiply whose
 // sum into dB the L2 does.  100k rows of 256 products: 380 -> 242 us.
 //
-// L follows the mean number of products an entry (30k rows of 200 entries of 1,
+// L follows the mean number of products of 32 entries (30k rows of 200 entries of 1,
 // 3 and 5 products: 575, 775 and 1025 us with eight lanes whatever the mean, 232,
 // 475 and 690 so); rows of a few entries, which fill no step however few lanes
 // they get, take more, whose reductions into dB are next to each other (300k
@@ -66,19 +66,72 @@ constexpr int kAdjCtaThreads = 256, kAdjCtaPerSm = 5;
 // were taken by their products alone).
 constexpr int kAdjWarpSteps = 32, kAdjQuadSteps = 16, kAdjBase = 20, kAdjPer = 30;
 
-// Lanes an entry, for a row of n entries whose row of C holds nc.
-__device__ __forceinline__ int adjoint_lanes(int64_t nc, int32_t n) {
-    if (n <= 4 || nc > 8 * (int64_t)n) return 8;
-    return n <= 8 || nc > 4 * (int64_t)n ? 4 : 2;
+// Lanes an entry, for n entries of P products in all (of each no more than 1024
+// counted).
+__device__ __forceinline__ int adjoint_lanes(int P, int n) {
+    if (n <= 4 || P > 8 * n) return 8;
+    return n <= 8 || P > 4 * n ? 4 : 2;
 }
 
+// Up to 32 entries of a row (from eb on; each lane holds one), L lanes an entry:
+// groups q0 / PER, q0 / PER + WARPS, ... of 32 / L entries.
 template <int WARPS, int L>
+__device__ __forceinline__ void adjoint_entries(const AdjArgs &a, int32_t eb, int ne, int q0, int32_t bs, int32_t len,
+                                                double av, int64_t off, const double *g, const int32_t *c, int nc,
+                                                int top) {
+    constexpr int PER = 32 / L;
+    const int lane = threadIdx.x & 31, sub = lane & (L - 1), grp = lane / L;
+    const unsigned gmask = ((1u << L) - 1u) << (lane & (32 - L));
+    for (int q = PER * q0; q < ne; q += PER * WARPS) {
+        const int32_t s = __shfl_sync(FULL, bs, q + grp), l = __shfl_sync(FULL, len, q + grp);
+        const double x = __shfl_sync(FULL, av, q + grp);
+        double *keep = nullptr;
+        if (a.prod) {
+            const int64_t o = __shfl_sync(FULL, off, q + grp);
+            if (o + l <= a.prodCap) keep = a.prod + o;
+            else raise(a.err, DEV_COUNT_MISMATCH);  // the patterns are not the forward's
+        }
+        double acc = 0.0;
+        for (int32_t i0 = sub; i0 < l; i0 += 2 * L) {
+            // Two products a lane in flight.
+            int32_t k[2];
+            double b[2];
+            int at[2] = {0, 0};
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int32_t i = i0 + L * u;
+                k[u] = i < l ? __ldg(&a.B.idx[s + i]) : -1;
+                b[u] = i < l ? __ldg(&a.B.val[s + i]) : 0.0;
+            }
+            for (int step = top; step >= 1; step >>= 1) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+                    if (at[u] + step < nc && c[at[u] + step] <= k[u]) at[u] += step;
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (k[u] < 0) continue;
+                if (nc == 0 || c[at[u]] != k[u]) {
+                    raise(a.err, DEV_COUNT_MISMATCH);
+                    continue;
+                }
+                const double gv = g[at[u]];
+                acc = __fma_rn(gv, b[u], acc);
+                if (a.dB) atomicAdd(&a.dB[s + i0 + L * u], __dmul_rn(x, gv));
+                else if (keep) keep[i0 + L * u] = __dmul_rn(x, gv);
+            }
+        }
+#pragma unroll
+        for (int d = L / 2; d; d >>= 1) acc += __shfl_xor_sync(gmask, acc, d, L);
+        if (sub == 0 && q + grp < ne) a.dA[eb + q + grp] = acc;
+    }
+}
+
+template <int WARPS>
 __device__ __forceinline__ void adjoint_row(const AdjArgs &a, int32_t e0, int32_t e1, int64_t c0, int nc, double *gs,
                                             int32_t *cs) {
-    constexpr int T = 32 * WARPS, PER = 32 / L;
+    constexpr int T = 32 * WARPS;
     const int lane = threadIdx.x & 31, w = WARPS == 1 ? 0 : threadIdx.x >> 5, tid = 32 * w + lane;
-    const double *g = gs;
-    const int32_t *c = cs;
     for (int i = tid; i < nc; i += T) {
         cs[i] = __ldg(&a.Ci[c0 + i]);
         gs[i] = __ldg(&a.G[c0 + i]);
@@ -87,9 +140,8 @@ __device__ __forceinline__ void adjoint_row(const AdjArgs &a, int32_t e0, int32_
     else __syncthreads();
     int top = 1;
     while (2 * top < nc) top <<= 1;
-    const int sub = lane & (L - 1), grp = lane / L;
-    const unsigned gmask = ((1u << L) - 1u) << (lane & (32 - L));
-    for (int32_t eb = e0; eb < e1; eb += 32) {
+    int q0 = w;  // 32 entries make two groups of two lanes: the next two warps take the next ones'
+    for (int32_t eb = e0; eb < e1; eb += 32, q0 = (q0 + WARPS / 2) % WARPS) {
         int32_t bs = 0, len = 0;
         double av = 0.0;
         int64_t off = 0;
@@ -101,49 +153,10 @@ __device__ __forceinline__ void adjoint_row(const AdjArgs &a, int32_t e0, int32_
             av = __ldg(&a.A.val[eb + lane]);
         }
         const int ne = min(32, e1 - eb);
-        for (int q = PER * w; q < ne; q += PER * WARPS) {
-            const int32_t s = __shfl_sync(FULL, bs, q + grp), l = __shfl_sync(FULL, len, q + grp);
-            const double x = __shfl_sync(FULL, av, q + grp);
-            double *keep = nullptr;
-            if (a.prod) {
-                const int64_t o = __shfl_sync(FULL, off, q + grp);
-                if (o + l <= a.prodCap) keep = a.prod + o;
-                else raise(a.err, DEV_COUNT_MISMATCH);  // the patterns are not the forward's
-            }
-            double acc = 0.0;
-            for (int32_t i0 = sub; i0 < l; i0 += 2 * L) {
-                // Two products a lane in flight.
-                int32_t k[2];
-                double b[2];
-                int at[2] = {0, 0};
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int32_t i = i0 + L * u;
-                    k[u] = i < l ? __ldg(&a.B.idx[s + i]) : -1;
-                    b[u] = i < l ? __ldg(&a.B.val[s + i]) : 0.0;
-                }
-                for (int step = top; step >= 1; step >>= 1) {
-#pragma unroll
-                    for (int u = 0; u < 2; ++u)
-                        if (at[u] + step < nc && c[at[u] + step] <= k[u]) at[u] += step;
-                }
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    if (k[u] < 0) continue;
-                    if (nc == 0 || c[at[u]] != k[u]) {
-                        raise(a.err, DEV_COUNT_MISMATCH);
-                        continue;
-                    }
-                    const double gv = g[at[u]];
-                    acc = __fma_rn(gv, b[u], acc);
-                    if (a.dB) atomicAdd(&a.dB[s + i0 + L * u], __dmul_rn(x, gv));
-                    else if (keep) keep[i0 + L * u] = __dmul_rn(x, gv);
-                }
-            }
-#pragma unroll
-            for (int d = L / 2; d; d >>= 1) acc += __shfl_xor_sync(gmask, acc, d, L);
-            if (sub == 0 && q + grp < ne) a.dA[eb + q + grp] = acc;
-        }
+        const int lanes = adjoint_lanes(__reduce_add_sync(FULL, min(len, 1024)), ne);
+        if (lanes == 2) adjoint_entries<WARPS, 2>(a, eb, ne, q0, bs, len, av, off, gs, cs, nc, top);
+        else if (lanes == 4) adjoint_entries<WARPS, 4>(a, eb, ne, q0, bs, len, av, off, gs, cs, nc, top);
+        else adjoint_entries<WARPS, 8>(a, eb, ne, q0, bs, len, av, off, gs, cs, nc, top);
     }
 }
 
@@ -164,10 +177,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps) k_adjoint_rows(AdjArgs a, cons
             if ((threadIdx.x & (32 * WARPS - 1)) == 0) raise(a.err, DEV_COUNT_MISMATCH);
             continue;
         }
-        const int lanes = adjoint_lanes(nc, e1 - e0);
-        if (lanes == 2) adjoint_row<WARPS, 2>(a, e0, e1, c0, (int)nc, gs[r], cs[r]);
-        else if (lanes == 4) adjoint_row<WARPS, 4>(a, e0, e1, c0, (int)nc, gs[r], cs[r]);
-        else adjoint_row<WARPS, 8>(a, e0, e1, c0, (int)nc, gs[r], cs[r]);
+        adjoint_row<WARPS>(a, e0, e1, c0, (int)nc, gs[r], cs[r]);
         if constexpr (WARPS == 1) __syncwarp();
         else __syncthreads();
     }
@@ -383,7 +393,6 @@ __global__ void __launch_bounds__(256) k_adjoint_split(AdjArgs a, int32_t lo, in
         kind = P >= 2 * a.partP ? ADJ_PARTS : ADJ_CTA;
         if (a.rows[ADJ_WARP] && nc <= kAdjWideNnz && e1 - e0 <= 4096) {
             // Steps of the row by one warp, and the longest of them.
-            const int L = adjoint_lanes(nc, e1 - e0), per = 32 / L;
             int steps = 0, longest = 0;
             for (int32_t e = e0; e < e1; e += 32) {
                 int32_t len = 0;
@@ -391,6 +400,7 @@ __global__ void __launch_bounds__(256) k_adjoint_split(AdjArgs a, int32_t lo, in
                     const int32_t k = __ldg(&a.A.idx[e + lane]);
                     len = __ldg(&a.B.ptr[k + 1]) - __ldg(&a.B.ptr[k]);
                 }
+                const int L = adjoint_lanes(__reduce_add_sync(FULL, min(len, 1024)), min(32, e1 - e)), per = 32 / L;
                 for (int d = 1; d < per; d <<= 1) len = max(len, __shfl_xor_sync(FULL, len, d));
                 const int x = (len + 2 * L - 1) / (2 * L);
                 if (lane % per == 0) steps += x;
