@@ -66,8 +66,9 @@ constexpr int kPieceSlabs = 16;
 // 10,240 rows of R-MAT 2^21 set the pass's time alone.  The line is a CTA's share
 // of all products (a shorter row can hardly be the last one running), and no
 // less than kSymCutP.  A row of 520k, 1.04M and 2.07M products alone: 130, 236
-// and 446 us whole, 49, 73 and 120 cut.  (In the other launch without being cut,
-// rows of half as many and more took 10 us longer, 40 of them 30.)
+// and 446 us whole, 49, 73 and 120 cut; 260k 78 and 37, so the least is on the
+// safe side.  (In the other launch without being cut, rows of half as many and
+// more took 10 us longer, 40 of them 30.)
 constexpr int64_t kSymCutP = 1 << 19;
 
 __host__ __device__ __forceinline__ int span_words(int32_t lo, int32_t hi) {

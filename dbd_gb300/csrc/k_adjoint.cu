@@ -236,8 +236,9 @@ __global__ void __launch_bounds__(THREADS, kAdjCtaPerSm) k_adjoint_cta(AdjArgs a
         __syncthreads();
         const int32_t item = next;
         if (item >= parts + n) break;
-        const AdjItem it = item < parts ? a.items[item]
-                                        : AdjItem{a.items ? a.rows[ADJ_CTA][item - parts] : a.order[lo + n - 1 - item], 0, 1};
+        AdjItem it{0, 0, 1};
+        if (item < parts) it = a.items[item];
+        else it.row = a.items ? a.rows[ADJ_CTA][item - parts] : a.order[lo + n - 1 - item];
         const int32_t row = it.row;
         const int32_t e0 = a.A.ptr[row], e1 = a.A.ptr[row + 1];
         const int64_t c0 = a.Cp[row], c1 = a.Cp[row + 1];
@@ -411,7 +412,8 @@ __global__ void __launch_bounds__(256) k_adjoint_split(AdjArgs a, int32_t lo, in
             const int batches = (e1 - e0 + kAdjCtaThreads - 1) / kAdjCtaThreads;
             if (steps <= kAdjBase * batches + P / kAdjPer) {
                 if (nc <= kAdjWarpNnz && steps <= kAdjWarpSteps) kind = ADJ_WARP;
-                else if (max(steps / kAdjWarps, longest) <= kAdjQuadSteps) kind = nc <= kAdjQuadNnz ? ADJ_QUAD : ADJ_WIDE;
+                else if (max(steps / kAdjWarps, longest) <= kAdjQuadSteps)
+                    kind = nc <= kAdjQuadNnz ? ADJ_QUAD : ADJ_WIDE;
             }
         }
     }

@@ -379,8 +379,9 @@ __global__ void __launch_bounds__(THREADS) k_row_products(CsrDev A, const int32_
 enum TileMode : int { TILES_PLAIN = 0, TILES_BLOCKS, TILES_NUMERIC };
 
 __global__ void __launch_bounds__(kTileRows) k_tiles(int64_t m, int64_t ntiles, TileMode mode,
-                                                     uint8_t *__restrict__ bin, int nbins, const int32_t *__restrict__ Ap,
-                                                     RowInfo ri, int32_t *__restrict__ rowNnz, Tuning tune,
+                                                     uint8_t *__restrict__ bin, int nbins,
+                                                     const int32_t *__restrict__ Ap, RowInfo ri,
+                                                     int32_t *__restrict__ rowNnz, Tuning tune,
                                                      int32_t *__restrict__ hist, int64_t *__restrict__ tileSum,
                                                      uint32_t *__restrict__ maxP) {
     __shared__ int32_t wc[kTileRows / 32][kMaxBins];
@@ -749,7 +750,8 @@ void launch_f32_to_f64(const float *src, double *dst, int64_t n, const int *badP
 // launch, by default).  Returns the first error.
 cudaError_t preload_analysis_kernels() {
     const void *fns[] = {
-        (const void *)k_check_operand, (const void *)k_row_minmax, (const void *)k_row_products<256, true>, (const void *)k_row_products<256, false>,
+        (const void *)k_check_operand, (const void *)k_row_minmax,
+        (const void *)k_row_products<256, true>, (const void *)k_row_products<256, false>,
         (const void *)k_tiles, (const void *)k_tile_scan, (const void *)k_tile_scatter,
         (const void *)k_scan_reduce, (const void *)k_scan_parts, (const void *)k_scan_final,
         (const void *)k_f32_to_f64,

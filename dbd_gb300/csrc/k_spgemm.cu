@@ -9,8 +9,8 @@
 // bin of rows (by products, size and column window) has its own kernels:
 //
 //   tiny rows   (P_r <= 32)     one lane per row, products listed in shared
-//                               memory and merged in place by column, summed
-//                               in Gustavson order (bit-exact FP64)
+//                               memory, sorted by column in registers and
+//                               summed in Gustavson order (bit-exact FP64)
 //   narrow rows (small window)  one warp per row over a window of flag bytes
 //                               and FP64 accumulators (symbolic: the length of
 //                               the union of the B rows' column runs when
@@ -38,10 +38,11 @@
 // instructions per SM per clock), so the numeric kernels spend one FP64
 // instruction per product: a fused multiply-add into the accumulator (plain,
 // or inside a compare-and-swap loop where lanes may collide), or a multiply
-// whose sum the L2 performs (global reductions).  The tiny path rounds each
-// product (__dmul_rn) and adds in the oracle's order, reproducing it bit for
-// bit; the other paths differ from it by summation order and by the fused
-// roundings, well inside the 1e-12 tolerance.
+// whose sum the L2 performs (global reductions: rank rows past 4096 entries and
+// dense rows), or, in warp rows of at most 256 products, sorts add up.  The tiny
+// path rounds each product (__dmul_rn) and adds in the oracle's order,
+// reproducing it bit for bit; the other paths differ from it by summation order
+// and by the fused roundings, well inside the 1e-12 tolerance.
 #include "cta_stage.cuh"
 #include "dbd_internal.h"
 #include "warp_chunk.cuh"
@@ -722,7 +723,7 @@ __global__ void __launch_bounds__(THREADS) k_sym_wide(SymArgs a, int32_t begin, 
                     warp_range_ld<kWideLoads>(
                         pre, bst, nb, tb, te, [&](int32_t pos) { return __ldg(&a.B.idx[pos]); },
                         [&](bool v, int32_t col, int) {
-                            const uint32_t rel = (uint32_t)col - (uint32_t)c_lo;  // columns below c_lo wrap past the window
+                            const uint32_t rel = (uint32_t)col - (uint32_t)c_lo;  // below c_lo it wraps past lim
                             cnt += or_bits_count(bm, v && rel < lim, rel, touched, &nt, rowCap);
                         });
                 } else {
@@ -987,8 +988,9 @@ __device__ __forceinline__ int32_t col_shift(const NumArgs &a, int32_t row) {
     return a.colShift ? a.colShift[row] : 0;
 }
 
-// Tiny rows, numeric: the warp then writes its rows' entries as one flat run, 32 consecutive ones a step, so that rows next to each other in C
-// go out in whole sectors.
+// Tiny rows, numeric: the warp then writes its rows' entries as one flat run, 32
+// consecutive ones a step, so that rows next to each other in C go out in whole
+// sectors.
 __device__ __forceinline__ void num_tiny_rows(const NumArgs &a, int32_t lo, int32_t count, int64_t vb) {
     __shared__ double vals[kNumTinyWarps][kTinyWords];
     __shared__ int32_t cols[kNumTinyWarps][kTinyWords];
@@ -1658,7 +1660,9 @@ __host__ __device__ constexpr int rank_ctas(int threads) { return threads == kRa
 
 // Where the rank kernel's bitmap starts behind the staging area.
 __host__ __device__ constexpr size_t rank_bits_at(int threads) {
-    return (threads == kRankSThreads ? StageLayout<kRankSThreads>::bytes : StageLayout<kRankLThreads>::bytes) / 16 * 16 + 16;
+    const size_t staged =
+        threads == kRankSThreads ? StageLayout<kRankSThreads>::bytes : StageLayout<kRankLThreads>::bytes;
+    return staged / 16 * 16 + 16;
 }
 
 template <int THREADS, class P>
@@ -1946,7 +1950,7 @@ __device__ __forceinline__ void num_densew_rows(const NumArgs &a, int32_t lo, in
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
                         const int32_t s = t0 + 32 * u, t = s + lane;
-                        if (s >= end && s < total) {  // the step starts in the next entry (no entry is shorter than a step)
+                        if (s >= end && s < total) {  // the step starts in the next entry (none is shorter than a step)
                             ++q;
                             end = __shfl_sync(FULL, incl, q);
                             p0 = p1;
