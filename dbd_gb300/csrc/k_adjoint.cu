@@ -434,8 +434,8 @@ __global__ void __launch_bounds__(256) k_adjoint_split(AdjArgs a, int32_t lo, in
     }
     const int k = (int)min((int64_t)kAdjMaxParts, P / a.partP);
     const uint32_t at = atomicAdd(&a.ctr[ADJ_PARTS], (uint32_t)k);
-    if ((int64_t)at + k > a.itemCap) return raise(a.err, DEV_COUNT_MISMATCH);  // the products are not the forward's
-    for (int p = 0; p < k; ++p) a.items[at + p] = AdjItem{row, (int16_t)p, (int16_t)k};
+    if ((int64_t)at + k > a.itemCap) raise(a.err, DEV_COUNT_MISMATCH);  // the products are not the forward's
+    for (int p = 0; p < k && (int64_t)at + p < a.itemCap; ++p) a.items[at + p] = AdjItem{row, (int16_t)p, (int16_t)k};
 }
 
 // Products of every A entry (the length of its B row).
